@@ -346,7 +346,15 @@ double residual_into(Ctx& c, cudaStream_t s, const double* x, const double* b, d
 // geometric multigrid (pg_mg.cu)
 int mg_pcg_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStream_t s);
 int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s);
-void mg_precondition(Ctx& c, bool f32, cudaStream_t s, const double* r, double* z);
+void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z);
+// CG preconditioned by the V-cycle on every RVE of the context; host copies
+// of the scalars (8 per RVE: ..., 4 tol^2, 5 b.b) and flags (4 per RVE: done,
+// breakdown, iterations, coarsest operator singular), valid until the next call
+struct MgCgResult {
+    const double* scalars = nullptr;
+    const int* flags = nullptr;
+};
+int mg_cg(Ctx& c, const pg_solver_cfg& cfg, MgCgResult& res, cudaStream_t s);
 void mg_free(Ctx& c);
 // ||v||^2 of a device vector (synchronises)
 double dev_norm2(Ctx& c, const double* v, int n, cudaStream_t s);

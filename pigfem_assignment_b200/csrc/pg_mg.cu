@@ -1,77 +1,119 @@
-// Geometric multigrid preconditioner for the IGFEM system (sm_100a).
+// Geometric multigrid preconditioner for the IGFEM system, and the CG around it (sm_100a).
 //
 // The reference factors K_ff directly (MUMPS through PETSc,
 // src/Solver.cpp:56-142); on the GPU the masked system is solved by CG whose
 // preconditioner is one V-cycle over the structured background grid:
 //   level 0     the IGFEM system itself (2x2-block CSR, regular + enrichment nodes)
 //   level l>0   grid of ceil(n_{l-1}/2) cells per side, 9-point block stencil
+// A context made of several RVEs (a batch) has one such hierarchy per RVE, of
+// its own depth; every kernel covers all of them, each RVE with its own CG
+// scalars, tolerance and end.
+//
 // Prolongation interpolates the coarse correction bilinearly (in grid index
 // space) onto the regular nodes of the finer grid and leaves enrichment
 // DOFs to the smoother (their shape functions vanish at the regular nodes,
 // so a smooth error lives in the regular DOFs).  Coarse operators are the
 // Galerkin products P^T A P of the masked finer operator; a coarse DOF is
-// fixed when the finer node at its position is fixed.  Smoothing is damped
-// block Jacobi (2x2 node blocks), the coarsest grid (at most 4 cells per
-// side) is solved by a dense LU with partial pivoting in one CTA.
+// fixed when the finer node at its position is fixed.
+//
+// Level 0 is smoothed once each way, in two factors: a damped block-Jacobi
+// sweep of the regular nodes, and a Chebyshev polynomial of the enrichment
+// block (k_mg_enr); before the coarse correction in this order, after it in
+// the reverse one, so that the cycle is symmetric.  Both factors reduce the
+// error in the energy norm (kOmegaReg and the polynomial's bound), so the
+// cycle is positive definite.  Coarse levels take two sweeps of damped block
+// Jacobi each way, the coarsest grid (at most 4 cells per side) its inverse.
+// Against two sweeps over all of level 0 each way: 74 -> 51 CG iterations at
+// 512^2 (rtol 1e-12), each with three products by K instead of five.
+//
+// A CG iteration is 7 launches and two per coarse level that has more than
+// kBottomNodes nodes; it was 43 at 512^2.  Below 512^2 all of them are bound
+// by launch and dependent-load latency, above by the reads of K.
 //
 // Precision: the outer CG always runs in FP64 (operator, vectors, dots and
-// the returned residual).  PG_PRECISION_MIXED runs the whole V-cycle in FP32
-// (FP32 copies of every level's operator and FP32 vectors); only the
-// preconditioner changes, so the FP64 result and its residual are unchanged
-// in kind.
+// the returned residual).  PG_PRECISION_MIXED runs the V-cycle in FP32 (FP32
+// copies of every level's operator and FP32 vectors; rows of level 0 are
+// summed in FP64); only the preconditioner changes, so the FP64 result and
+// its residual are unchanged in kind.
 //
-// Every kernel a CG iteration launches returns at once after the device
-// "done" flag is set, so captured graphs of several iterations may run past
-// convergence without changing the result.
+// Every kernel of a CG iteration returns at once for an RVE whose "done" flag
+// is set, so captured graphs of several iterations may run past convergence
+// without changing the result.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
-#include "pg_solve_kernels.cuh"
+#include "pg_mg_kernels.cuh"
 
 namespace pgb {
 
+using namespace mg;
+
 namespace {
 
-constexpr int kMgMaxLevels = 16;
-constexpr int kMgCoarseCells = 4;        // coarsen until both sides have at most this many cells
-constexpr int kMgCoarseMaxDof = 2 * (kMgCoarseCells + 1) * (kMgCoarseCells + 1);
-constexpr int kMgNu1 = 2, kMgNu2 = 2;    // pre- and post-smoothing sweeps
-constexpr double kMgOmega = 0.5;         // block-Jacobi damping: lambda_max(D^-1 K) reaches ~3.9 on IGFEM meshes
+constexpr int kMaxLevels = 16;
+constexpr int kSpanCtasPerSm = 5;        // CTAs of the level-0 kernels that an SM holds
+constexpr int kChunk = 2;                // CG iterations per graph (the parity of p and r.z is baked in)
 
-struct MgLevel {
-    int nx = 0, ny = 0, n = 0;           // cells per side, nodes
-    double* A = nullptr;                 // 36 per node: stencil block (dj+1)*3+(di+1), 2x2 row-major
-    float* Af = nullptr;
-    double* Dinv = nullptr;              // 4 per node
-    float* Dinvf = nullptr;
+// Level vectors in the V-cycle's precision
+template <typename T>
+struct LevelArrays {
+    T *A = nullptr, *Dinv = nullptr;     // 36 and 4 per node: stencil block (dj+1)*3+(di+1), 2x2 row-major
+    T *b = nullptr, *x = nullptr, *xo = nullptr;  // 2 per node
+};
+
+struct Tiles {
+    int4* tile = nullptr;                // RVE, first node column and row, 1 for the RVE's first tile
+    int n = 0;
+};
+
+struct Level {
+    int n = 0;                           // nodes of all RVEs
+    int* node_rve = nullptr;             // (several RVEs)
+    Pair* pair = nullptr;                // per RVE: the transfer from the finer level
     uint8_t* fixed = nullptr;            // 2 per node
-    double *x = nullptr, *x2 = nullptr, *b = nullptr, *r = nullptr;
-    float *xf = nullptr, *x2f = nullptr, *bf = nullptr, *rf = nullptr;
+    Tiles down, up;                      // of the transfer to this level, and of this level's post-smoothing
+    LevelArrays<double> d;
+    LevelArrays<float> f;
 };
 
 }  // namespace
 
 struct MgHierarchy {
-    int nlev = 0;                        // coarse levels 1..nlev (nlev is the coarsest)
-    MgLevel L[kMgMaxLevels + 1];
-    // level-0 V-cycle vectors
-    double *x0 = nullptr, *x0b = nullptr, *r0 = nullptr;
-    float *b0f = nullptr, *x0f = nullptr, *x0bf = nullptr, *r0f = nullptr;
-    float* Dinv0f = nullptr;
-    // coarsest dense LU (row-major, n_c x n_c) and pivots
-    int nc = 0;
-    double* LU = nullptr;
-    int* piv = nullptr;
-    // CG scalars: 0 pq, 1 rz, 2 rz_new, 3 rr, 4 tol2; flags: 0 done, 1 breakdown, 2 iterations, 3 coarse-singular
+    int R = 0;                           // RVEs
+    int nlev = 0;                        // coarse levels 1..nlev
+    Level L[kMaxLevels + 1];
+    Spans spans{};
+    int n_cta = 0;
+    int* node_end = nullptr;             // per RVE
+    // enrichment nodes
+    int n_enr = 0, n_pieces = 0, max_piece = 0;
+    int *enr_node = nullptr, *enr_rve = nullptr;
+    Enr enr{};
+    unsigned long long* bound = nullptr; // per RVE
+    double* coef = nullptr;
+    // the bottom of every RVE's cycle
+    Bottom* bottom = nullptr;
+    size_t bottom_smem[2] = {0, 0};      // FP64, FP32
+    Coarse* coarse = nullptr;
+    double* XT = nullptr;
+    // level-0 vectors of the cycle: x, and the enrichment nodes' after post-smoothing
+    double *x0 = nullptr, *x0e = nullptr;
+    float *x0f = nullptr, *x0ef = nullptr, *Dinv0f = nullptr;
+    bool f32_ready = false;
+    // CG: partials (p.q, r.r, r.z), scalars, flags, and their pinned host copies (two slots of flags)
+    double *part_pq = nullptr, *part_rr = nullptr, *part_rz = nullptr;
     double* sc = nullptr;
     int* fl = nullptr;
+    double* h_sc = nullptr;
+    int* h_fl = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[4] = {};       // of kChunk iterations: FP64 / FP32 cycle, without / with inclusion modes
     // inclusion rigid modes (cohesive meshes): 3 per inclusion, supports disjoint
     int n_inc = 0;                       // 0: no mode space
-    bool use_modes = false;
     int* z_inc = nullptr;                // per node: the inclusion whose modes touch it, -1 none
     double* zval = nullptr;              // per node: [d][k], 2 x 3
     double* E = nullptr;                 // per inclusion: Z_i^T K Z_i (3 x 3)
@@ -82,657 +124,7 @@ struct MgHierarchy {
 
 namespace {
 
-// ---------------------------------------------------------------------------
-// Grid transfer weights (grid index space).  Coarse index I sits at fine
-// index pos(I) = min(2I, nf); nf is the finer grid's cell count.
-// ---------------------------------------------------------------------------
-__host__ __device__ __forceinline__ int mg_pos(int I, int nf) { return 2 * I < nf ? 2 * I : nf; }
-
-__host__ __device__ __forceinline__ double mg_w(int g, int nf, int I) {
-    if ((g & 1) == 0) return (g >> 1) == I ? 1.0 : 0.0;
-    if (g == nf) return I == ((nf + 1) >> 1) ? 1.0 : 0.0;
-    return (I == ((g - 1) >> 1) || I == ((g + 1) >> 1)) ? 0.5 : 0.0;
-}
-
-// ---------------------------------------------------------------------------
-// Set-up kernels
-// ---------------------------------------------------------------------------
-struct GalArgs {
-    int nxf, nyf, nxc, nyc;
-    // finer operator: BSR (level 0) or stencil
-    const int* row_ptr;
-    const int* col;
-    const double* K;
-    int n_reg;
-    const double* A;
-    const uint8_t* fixed_f;
-    const uint8_t* fixed_c;
-    double* Ac;
-};
-
-// Ac(a, a + o) = sum_{i child of a} sum_{j in row i} P_ia M_i A_ij M_j P_jb, masked by the coarse mask.
-template <bool FINE_BSR>
-__global__ void k_mg_galerkin(GalArgs g) {
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ncn = (g.nxc + 1) * (g.nyc + 1);
-    if (tid >= 9 * ncn) return;
-    const int a = tid / 9, o = tid - 9 * a;
-    const int Ia = a % (g.nxc + 1), Ja = a / (g.nxc + 1);
-    const int Ib = Ia + (o % 3) - 1, Jb = Ja + (o / 3) - 1;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    if (Ib >= 0 && Ib <= g.nxc && Jb >= 0 && Jb <= g.nyc) {
-        const int px = mg_pos(Ia, g.nxf), py = mg_pos(Ja, g.nyf);
-        for (int cy = py - 1; cy <= py + 1; ++cy) {
-            if (cy < 0 || cy > g.nyf) continue;
-            const double wy = mg_w(cy, g.nyf, Ja);
-            if (wy == 0.0) continue;
-            for (int cx = px - 1; cx <= px + 1; ++cx) {
-                if (cx < 0 || cx > g.nxf) continue;
-                const double wx = mg_w(cx, g.nxf, Ia);
-                if (wx == 0.0) continue;
-                const int i = cx + cy * (g.nxf + 1);
-                const double wi = wx * wy;
-                const bool fi0 = !g.fixed_f[2 * i], fi1 = !g.fixed_f[2 * i + 1];
-                if (FINE_BSR) {
-                    for (int q = g.row_ptr[i]; q < g.row_ptr[i + 1]; ++q) {
-                        const int j = g.col[q];
-                        if (j >= g.n_reg) continue;
-                        const int gx = j % (g.nxf + 1), gy = j / (g.nxf + 1);
-                        const double wj = mg_w(gx, g.nxf, Ib) * mg_w(gy, g.nyf, Jb);
-                        if (wj == 0.0) continue;
-                        const bool fj0 = !g.fixed_f[2 * j], fj1 = !g.fixed_f[2 * j + 1];
-                        const double* blk = g.K + 4 * (size_t)q;
-                        const double w = wi * wj;
-                        if (fi0 && fj0) acc[0] += w * blk[0];
-                        if (fi0 && fj1) acc[1] += w * blk[1];
-                        if (fi1 && fj0) acc[2] += w * blk[2];
-                        if (fi1 && fj1) acc[3] += w * blk[3];
-                    }
-                } else {
-                    for (int s = 0; s < 9; ++s) {
-                        const int gx = cx + (s % 3) - 1, gy = cy + (s / 3) - 1;
-                        if (gx < 0 || gx > g.nxf || gy < 0 || gy > g.nyf) continue;
-                        const double wj = mg_w(gx, g.nxf, Ib) * mg_w(gy, g.nyf, Jb);
-                        if (wj == 0.0) continue;
-                        const int j = gx + gy * (g.nxf + 1);
-                        const bool fj0 = !g.fixed_f[2 * j], fj1 = !g.fixed_f[2 * j + 1];
-                        const double* blk = g.A + 36 * (size_t)i + 4 * s;
-                        const double w = wi * wj;
-                        if (fi0 && fj0) acc[0] += w * blk[0];
-                        if (fi0 && fj1) acc[1] += w * blk[1];
-                        if (fi1 && fj0) acc[2] += w * blk[2];
-                        if (fi1 && fj1) acc[3] += w * blk[3];
-                    }
-                }
-            }
-        }
-        const int b = Ib + Jb * (g.nxc + 1);
-        if (g.fixed_c[2 * a]) acc[0] = acc[1] = 0.0;
-        if (g.fixed_c[2 * a + 1]) acc[2] = acc[3] = 0.0;
-        if (g.fixed_c[2 * b]) acc[0] = acc[2] = 0.0;
-        if (g.fixed_c[2 * b + 1]) acc[1] = acc[3] = 0.0;
-    }
-    double* out = g.Ac + 36 * (size_t)a + 4 * o;
-    for (int k = 0; k < 4; ++k) out[k] = acc[k];
-}
-
-// Coarse mask by injection: the coarse node takes the mask of the finer node at its position.
-__global__ void k_mg_inject_mask(int nxf, int nxc, int nyc, int nyf, const uint8_t* fixed_f, uint8_t* fixed_c) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= (nxc + 1) * (nyc + 1)) return;
-    const int I = a % (nxc + 1), J = a / (nxc + 1);
-    const int i = mg_pos(I, nxf) + mg_pos(J, nyf) * (nxf + 1);
-    fixed_c[2 * a] = fixed_f[2 * i];
-    fixed_c[2 * a + 1] = fixed_f[2 * i + 1];
-}
-
-// Inverse of each node's masked diagonal block (stencil centre), as k_prec_setup does for level 0.
-__global__ void k_mg_dinv(int n, const double* A, const uint8_t* fixed, double* Dinv, float* Dinvf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* b = A + 36 * (size_t)i + 16;
-    const bool f0 = fixed[2 * i], f1 = fixed[2 * i + 1];
-    double m[4] = {0.0, 0.0, 0.0, 0.0};
-    if (!f0 && !f1) {
-        const double det = b[0] * b[3] - b[1] * b[2];
-        if (det != 0.0) {
-            m[0] = b[3] / det;
-            m[1] = -b[1] / det;
-            m[2] = -b[2] / det;
-            m[3] = b[0] / det;
-        }
-    } else {
-        m[0] = (f0 || b[0] == 0.0) ? 0.0 : 1.0 / b[0];
-        m[3] = (f1 || b[3] == 0.0) ? 0.0 : 1.0 / b[3];
-    }
-    for (int k = 0; k < 4; ++k) {
-        Dinv[4 * (size_t)i + k] = m[k];
-        if (Dinvf) Dinvf[4 * (size_t)i + k] = (float)m[k];
-    }
-}
-
-__global__ void k_mg_to_f32(size_t n, const double* a, float* b) {
-    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (float)a[i];
-}
-
-// Dense LU with partial pivoting of the coarsest operator, one CTA.
-// Fixed DOFs get identity rows and columns.  fl[3] = 1 on a zero pivot.
-__global__ void k_mg_coarse_factor(int nx, int ny, const double* A, const uint8_t* fixed, double* LU, int* piv,
-                                   int* fl) {
-    __shared__ double M[kMgCoarseMaxDof][kMgCoarseMaxDof + 1];
-    __shared__ int sp[kMgCoarseMaxDof];
-    __shared__ int s_pivot;
-    const int nn = (nx + 1) * (ny + 1), n = 2 * nn;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) M[e / n][e % n] = 0.0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < 9 * nn; t += blockDim.x) {
-        const int a = t / 9, o = t - 9 * a;
-        const int I = a % (nx + 1) + (o % 3) - 1, J = a / (nx + 1) + (o / 3) - 1;
-        if (I < 0 || I > nx || J < 0 || J > ny) continue;
-        const int b = I + J * (nx + 1);
-        const double* blk = A + 36 * (size_t)a + 4 * o;
-        for (int d = 0; d < 2; ++d)
-            for (int f = 0; f < 2; ++f)
-                if (!fixed[2 * a + d] && !fixed[2 * b + f]) M[2 * a + d][2 * b + f] = blk[2 * d + f];
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        if (fixed[r]) M[r][r] = 1.0;
-        sp[r] = r;
-    }
-    __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        if (threadIdx.x == 0) {
-            int best = k;
-            for (int r = k + 1; r < n; ++r)
-                if (fabs(M[r][k]) > fabs(M[best][k])) best = r;
-            s_pivot = best;
-            if (M[best][k] == 0.0) fl[3] = 1;
-        }
-        __syncthreads();
-        const int pr = s_pivot;
-        if (pr != k) {
-            for (int c2 = threadIdx.x; c2 < n; c2 += blockDim.x) {
-                const double t2 = M[k][c2];
-                M[k][c2] = M[pr][c2];
-                M[pr][c2] = t2;
-            }
-            if (threadIdx.x == 0) {
-                const int t3 = sp[k];
-                sp[k] = sp[pr];
-                sp[pr] = t3;
-            }
-        }
-        __syncthreads();
-        const double d = M[k][k];
-        for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x)
-            if (d != 0.0) M[r][k] /= d;
-        __syncthreads();
-        for (int e = threadIdx.x; e < (n - k - 1) * (n - k - 1); e += blockDim.x) {
-            const int r = k + 1 + e / (n - k - 1), c2 = k + 1 + e % (n - k - 1);
-            M[r][c2] -= M[r][k] * M[k][c2];
-        }
-        __syncthreads();
-    }
-    // The coarse solve runs once per V-cycle; two substitutions of n steps,
-    // each behind a barrier, cost tens of microseconds.  So the inverse is
-    // formed here (column j solves L U x = P e_j, one thread per column) and
-    // stored transposed in LU (LU[j n + r] = X[r][j]), with the rows and
-    // columns of fixed DOFs zeroed: the solve is then one matrix-vector product.
-    __shared__ double W[kMgCoarseMaxDof][kMgCoarseMaxDof + 1];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        double* y = W[j];
-        for (int r = 0; r < n; ++r) y[r] = (sp[r] == j && !fixed[j]) ? 1.0 : 0.0;
-        for (int k = 0; k < n; ++k) {
-            const double yk = y[k];
-            for (int r = k + 1; r < n; ++r) y[r] -= M[r][k] * yk;
-        }
-        for (int k = n - 1; k >= 0; --k) {
-            y[k] = M[k][k] != 0.0 ? y[k] / M[k][k] : 0.0;
-            const double yk = y[k];
-            for (int r = 0; r < k; ++r) y[r] -= M[r][k] * yk;
-        }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int j = e / n, r = e - j * n;
-        LU[e] = fixed[r] ? 0.0 : W[j][r];
-    }
-    for (int r = threadIdx.x; r < n; r += blockDim.x) piv[r] = sp[r];
-}
-
-// ---------------------------------------------------------------------------
-// V-cycle kernels (T = double or float; arithmetic in T)
-// ---------------------------------------------------------------------------
-// level 0: xout = xin + omega D^-1 mask(b - A xin) (xin null: zero)
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_mg_smooth_bsr(int n, const int* __restrict__ row_ptr,
-                                                            const int* __restrict__ col, const T* __restrict__ K,
-                                                            const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                                            const T* __restrict__ b, const T* __restrict__ xin,
-                                                            T* __restrict__ xout, T omega, const int* done, int resid_only) {
-    if (done && done[0]) return;
-    // kRowLanes lanes per block row (bsr_row_group); lane 0 of each group finishes the row
-    const int t = blockIdx.x * kThreads + threadIdx.x;
-    const int i = t / kRowLanes, g = t % kRowLanes;
-    double y0 = 0.0, y1 = 0.0;
-    if (xin) bsr_row_group<T, T>(i, i < n, g, row_ptr, col, K, xin, y0, y1);
-    if (i >= n || g != 0) return;
-    T r0 = b[2 * i], r1 = b[2 * i + 1];
-    if (xin) {
-        r0 -= (T)y0;
-        r1 -= (T)y1;
-    }
-    if (fixed[2 * i]) r0 = 0;
-    if (fixed[2 * i + 1]) r1 = 0;
-    if (resid_only) {
-        xout[2 * i] = r0;
-        xout[2 * i + 1] = r1;
-        return;
-    }
-    const T* m = Dinv + 4 * (size_t)i;
-    const T z0 = m[0] * r0 + m[1] * r1, z1 = m[2] * r0 + m[3] * r1;
-    xout[2 * i] = (xin ? xin[2 * i] : (T)0) + omega * z0;
-    xout[2 * i + 1] = (xin ? xin[2 * i + 1] : (T)0) + omega * z1;
-}
-
-// GLOBAL: A and Dinv are in global memory and read as whole 2x2 blocks
-// (load_block); otherwise (shared memory) element by element.
-template <typename T, bool GLOBAL>
-__device__ __forceinline__ void mg_smooth_node(int i, int nx, int ny, const T* __restrict__ A,
-                                               const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                               const T* __restrict__ b, const T* __restrict__ xin, T* __restrict__ xout,
-                                               T omega, int resid_only) {
-    T r0 = b[2 * i], r1 = b[2 * i + 1];
-    if (xin) {
-        const int I = i % (nx + 1), J = i / (nx + 1);
-        T y0 = 0, y1 = 0;
-        for (int s = 0; s < 9; ++s) {
-            const int gx = I + (s % 3) - 1, gy = J + (s / 3) - 1;
-            if (gx < 0 || gx > nx || gy < 0 || gy > ny) continue;
-            const int j = gx + gy * (nx + 1);
-            const T* k = A + 36 * (size_t)i + 4 * s;
-            T k0, k1, k2, k3;
-            if constexpr (GLOBAL) {
-                double d0, d1, d2, d3;
-                load_block(k, d0, d1, d2, d3);
-                k0 = (T)d0; k1 = (T)d1; k2 = (T)d2; k3 = (T)d3;
-            } else {
-                k0 = k[0]; k1 = k[1]; k2 = k[2]; k3 = k[3];
-            }
-            const T x0 = xin[2 * j], x1 = xin[2 * j + 1];
-            y0 += k0 * x0 + k1 * x1;
-            y1 += k2 * x0 + k3 * x1;
-        }
-        r0 -= y0;
-        r1 -= y1;
-    }
-    if (fixed[2 * i]) r0 = 0;
-    if (fixed[2 * i + 1]) r1 = 0;
-    if (resid_only) {
-        xout[2 * i] = r0;
-        xout[2 * i + 1] = r1;
-        return;
-    }
-    const T* m = Dinv + 4 * (size_t)i;
-    T m0, m1, m2, m3;
-    if constexpr (GLOBAL) {
-        double d0, d1, d2, d3;
-        load_block(m, d0, d1, d2, d3);
-        m0 = (T)d0; m1 = (T)d1; m2 = (T)d2; m3 = (T)d3;
-    } else {
-        m0 = m[0]; m1 = m[1]; m2 = m[2]; m3 = m[3];
-    }
-    const T z0 = m0 * r0 + m1 * r1, z1 = m2 * r0 + m3 * r1;
-    xout[2 * i] = (xin ? xin[2 * i] : (T)0) + omega * z0;
-    xout[2 * i + 1] = (xin ? xin[2 * i + 1] : (T)0) + omega * z1;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_mg_smooth_st(int nx, int ny, const T* __restrict__ A,
-                                                           const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                                           const T* __restrict__ b, const T* __restrict__ xin,
-                                                           T* __restrict__ xout, T omega, const int* done, int resid_only) {
-    if (done && done[0]) return;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= (nx + 1) * (ny + 1)) return;
-    mg_smooth_node<T, true>(i, nx, ny, A, Dinv, fixed, b, xin, xout, omega, resid_only);
-}
-
-// bc(a) = mask_c(sum_{i child of a} P_ia rf(i))
-template <typename T>
-__device__ __forceinline__ void mg_restrict_node(int a, int nxf, int nyf, int nxc, const T* __restrict__ rf,
-                                                 const uint8_t* fixed_c, T* __restrict__ bc) {
-    const int Ia = a % (nxc + 1), Ja = a / (nxc + 1);
-    const int px = mg_pos(Ia, nxf), py = mg_pos(Ja, nyf);
-    T s0 = 0, s1 = 0;
-    for (int cy = py - 1; cy <= py + 1; ++cy) {
-        if (cy < 0 || cy > nyf) continue;
-        const double wy = mg_w(cy, nyf, Ja);
-        if (wy == 0.0) continue;
-        for (int cx = px - 1; cx <= px + 1; ++cx) {
-            if (cx < 0 || cx > nxf) continue;
-            const double wx = mg_w(cx, nxf, Ia);
-            if (wx == 0.0) continue;
-            const int i = cx + cy * (nxf + 1);
-            const T w = (T)(wx * wy);
-            s0 += w * rf[2 * i];
-            s1 += w * rf[2 * i + 1];
-        }
-    }
-    bc[2 * a] = fixed_c[2 * a] ? (T)0 : s0;
-    bc[2 * a + 1] = fixed_c[2 * a + 1] ? (T)0 : s1;
-}
-
-template <typename T>
-__global__ void k_mg_restrict(int nxf, int nyf, int nxc, int nyc, const T* __restrict__ rf, const uint8_t* fixed_c,
-                              T* __restrict__ bc, const int* done) {
-    if (done && done[0]) return;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= (nxc + 1) * (nyc + 1)) return;
-    mg_restrict_node(a, nxf, nyf, nxc, rf, fixed_c, bc);
-}
-
-// xf(i) += mask_f(sum_a P_ia xc(a)) over the finer grid's nodes
-template <typename T>
-__device__ __forceinline__ void mg_prolong_node(int i, int nxf, int nyf, int nxc, const T* __restrict__ xc,
-                                                const uint8_t* fixed_f, T* __restrict__ xf) {
-    const int gx = i % (nxf + 1), gy = i / (nxf + 1);
-    int Ix[2], Iy[2];
-    T wxs[2], wys[2];
-    int nxp, nyp;
-    if ((gx & 1) == 0) { Ix[0] = gx >> 1; wxs[0] = 1; nxp = 1; }
-    else if (gx == nxf) { Ix[0] = (nxf + 1) >> 1; wxs[0] = 1; nxp = 1; }
-    else { Ix[0] = (gx - 1) >> 1; Ix[1] = (gx + 1) >> 1; wxs[0] = wxs[1] = (T)0.5; nxp = 2; }
-    if ((gy & 1) == 0) { Iy[0] = gy >> 1; wys[0] = 1; nyp = 1; }
-    else if (gy == nyf) { Iy[0] = (nyf + 1) >> 1; wys[0] = 1; nyp = 1; }
-    else { Iy[0] = (gy - 1) >> 1; Iy[1] = (gy + 1) >> 1; wys[0] = wys[1] = (T)0.5; nyp = 2; }
-    T s0 = 0, s1 = 0;
-    for (int py = 0; py < nyp; ++py)
-        for (int px = 0; px < nxp; ++px) {
-            const int a = Ix[px] + Iy[py] * (nxc + 1);
-            const T w = wxs[px] * wys[py];
-            s0 += w * xc[2 * a];
-            s1 += w * xc[2 * a + 1];
-        }
-    if (!fixed_f[2 * i]) xf[2 * i] += s0;
-    if (!fixed_f[2 * i + 1]) xf[2 * i + 1] += s1;
-}
-
-template <typename T>
-__global__ void k_mg_prolong(int nxf, int nyf, int nxc, const T* __restrict__ xc, const uint8_t* fixed_f,
-                             T* __restrict__ xf, const int* done) {
-    if (done && done[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (nxf + 1) * (nyf + 1)) return;
-    mg_prolong_node(i, nxf, nyf, nxc, xc, fixed_f, xf);
-}
-
-// The bottom of the V-cycle in one launch.  Below a few hundred nodes every
-// level's kernels are latency-bound (a launch of one block costs about as
-// much as one of a thousand), and the V-cycle has seven of them per level.
-// So the levels from `first` down to the coarsest run in one CTA, phase after
-// phase between block barriers, in the same order and with the same per-node
-// arithmetic as the per-level kernels: restrict the finer residual,
-// pre-smooth, residual, ..., coarse solve, then prolongate and post-smooth
-// back up.  Their operators, diagonal inverses and vectors are first copied
-// into shared memory (one coalesced pass), so no phase waits on L2; the
-// result of level `first` goes back to its x for the caller's prolongation.
-// (taking the 33x33 level as well, its operators read from L2, made the bottom
-// 151 us instead of 34 us per cycle: slower than that level's seven launches)
-constexpr int kMgBottomNodes = 300;        // levels at most this size may run in k_mg_bottom
-constexpr int kMgBottomSmem = 220 * 1024;  // and their shared-memory copy at most this many bytes
-constexpr int kMgBottomThreads = 512;
-constexpr int kMgBottomLevels = 8;
-
-template <typename T>
-struct MgBottomArgs {
-    int nlev;                               // levels here, the last the coarsest
-    int nxf, nyf;                           // grid of the finer level restricted first
-    const T* rf;                            // its residual
-    int nx[kMgBottomLevels], ny[kMgBottomLevels];
-    const T* A[kMgBottomLevels];
-    const T* Dinv[kMgBottomLevels];
-    const uint8_t* fixed[kMgBottomLevels];
-    int staged[kMgBottomLevels];            // 1: A and D^-1 copied into shared memory; 0: read from global (L2)
-    T* x0;                                  // level `first`'s x (global): the result
-    const double* XT;                       // coarsest: transposed masked inverse
-    int nc;
-    T omega;
-};
-
-// shared-memory bytes of k_mg_bottom for a level of n nodes: b, x, x2, r (2 n
-// each) and fixed (2 n bytes, rounded to 8), and with its operator staged A
-// (36 n) and D^-1 (4 n) too
-template <typename T>
-size_t mg_bottom_vec_bytes(int n) {
-    return (size_t)8 * n * sizeof(T) + (((size_t)2 * n + 7) & ~(size_t)7);
-}
-template <typename T>
-size_t mg_bottom_op_bytes(int n) {
-    return (size_t)(36 + 4) * n * sizeof(T);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kMgBottomThreads) k_mg_bottom(MgBottomArgs<T> a, const int* done) {
-    if (done && done[0]) return;
-    extern __shared__ __align__(16) unsigned char g_bottom_smem[];
-    __shared__ double bs[kMgCoarseMaxDof];
-    const int tid = threadIdx.x;
-    // carve and stage
-    T* sA[kMgBottomLevels];
-    T* sD[kMgBottomLevels];
-    T* sb[kMgBottomLevels];
-    T* sx[kMgBottomLevels];
-    T* sx2[kMgBottomLevels];
-    T* sr[kMgBottomLevels];
-    uint8_t* sf[kMgBottomLevels];
-    unsigned char* p = g_bottom_smem;
-    for (int k = 0; k < a.nlev; ++k) {
-        const int n = (a.nx[k] + 1) * (a.ny[k] + 1);
-        T* q0 = reinterpret_cast<T*>(p);
-        if (a.staged[k]) {
-            sA[k] = q0;
-            sD[k] = sA[k] + 36 * n;
-            q0 = sD[k] + 4 * n;
-        } else {
-            // a larger level: its operator stays in global memory (L2), only its vectors here
-            sA[k] = const_cast<T*>(a.A[k]);
-            sD[k] = const_cast<T*>(a.Dinv[k]);
-        }
-        sb[k] = q0;
-        sx[k] = sb[k] + 2 * n;
-        sx2[k] = sx[k] + 2 * n;
-        sr[k] = sx2[k] + 2 * n;
-        sf[k] = reinterpret_cast<uint8_t*>(sr[k] + 2 * n);
-        p = reinterpret_cast<unsigned char*>(sf[k]) + ((2 * n + 7) & ~7);
-        if (k < a.nlev - 1 && a.staged[k]) {
-            for (int q = tid; q < 36 * n; q += kMgBottomThreads) sA[k][q] = a.A[k][q];
-            for (int q = tid; q < 4 * n; q += kMgBottomThreads) sD[k][q] = a.Dinv[k][q];
-        }
-        for (int q = tid; q < 2 * n; q += kMgBottomThreads) sf[k][q] = a.fixed[k][q];
-    }
-    __syncthreads();
-    int nxf = a.nxf, nyf = a.nyf;
-    const T* rf = a.rf;
-    T* xs[kMgBottomLevels];
-    for (int k = 0; k < a.nlev; ++k) {
-        const int nx = a.nx[k], ny = a.ny[k], n = (nx + 1) * (ny + 1);
-        for (int i = tid; i < n; i += kMgBottomThreads) mg_restrict_node(i, nxf, nyf, nx, rf, sf[k], sb[k]);
-        __syncthreads();
-        if (k == a.nlev - 1) {
-            // coarsest: x = XT^T b (fixed DOFs 0)
-            for (int q = tid; q < a.nc; q += kMgBottomThreads) bs[q] = sf[k][q] ? 0.0 : (double)sb[k][q];
-            __syncthreads();
-            for (int q = tid; q < a.nc; q += kMgBottomThreads) {
-                double acc = 0.0;
-                for (int j = 0; j < a.nc; ++j) acc += a.XT[(size_t)j * a.nc + q] * bs[j];
-                sx[k][q] = sf[k][q] ? (T)0 : (T)acc;
-            }
-            __syncthreads();
-            xs[k] = sx[k];
-            break;
-        }
-        T* lc = sx[k];
-        T* la = sx2[k];
-        for (int i = tid; i < n; i += kMgBottomThreads)
-            mg_smooth_node<T, false>(i, nx, ny, (const T*)sA[k], (const T*)sD[k], sf[k], (const T*)sb[k], (const T*)nullptr, lc,
-                           a.omega, 0);
-        __syncthreads();
-        for (int it = 1; it < kMgNu1; ++it) {
-            for (int i = tid; i < n; i += kMgBottomThreads)
-                mg_smooth_node<T, false>(i, nx, ny, (const T*)sA[k], (const T*)sD[k], sf[k], (const T*)sb[k], (const T*)lc, la,
-                               a.omega, 0);
-            __syncthreads();
-            T* t = lc;
-            lc = la;
-            la = t;
-        }
-        for (int i = tid; i < n; i += kMgBottomThreads)
-            mg_smooth_node<T, false>(i, nx, ny, (const T*)sA[k], (const T*)sD[k], sf[k], (const T*)sb[k], (const T*)lc, sr[k],
-                           a.omega, 1);
-        __syncthreads();
-        xs[k] = lc;
-        rf = sr[k];
-        nxf = nx;
-        nyf = ny;
-    }
-    for (int k = a.nlev - 2; k >= 0; --k) {
-        const int nx = a.nx[k], ny = a.ny[k], n = (nx + 1) * (ny + 1);
-        T* lc = xs[k];
-        T* la = lc == sx[k] ? sx2[k] : sx[k];
-        for (int i = tid; i < n; i += kMgBottomThreads)
-            mg_prolong_node(i, nx, ny, a.nx[k + 1], (const T*)xs[k + 1], sf[k], lc);
-        __syncthreads();
-        for (int it = 0; it < kMgNu2; ++it) {
-            for (int i = tid; i < n; i += kMgBottomThreads)
-                mg_smooth_node<T, false>(i, nx, ny, (const T*)sA[k], (const T*)sD[k], sf[k], (const T*)sb[k], (const T*)lc, la,
-                               a.omega, 0);
-            __syncthreads();
-            T* t = lc;
-            lc = la;
-            la = t;
-        }
-        xs[k] = lc;
-    }
-    const int n0 = 2 * (a.nx[0] + 1) * (a.ny[0] + 1);
-    for (int q = tid; q < n0; q += kMgBottomThreads) a.x0[q] = xs[0][q];
-}
-
-__global__ void k_mg_f64_to_f32(int n, const double* __restrict__ a, float* __restrict__ b, const int* done) {
-    if (done && done[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (float)a[i];
-}
-
-__global__ void k_mg_f32_to_f64(int n, const float* __restrict__ a, double* __restrict__ b, const int* done) {
-    if (done && done[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (double)a[i];
-}
-
-// ---------------------------------------------------------------------------
-// CG kernels (FP64).  Scalars: sc[0] p.q, sc[1] r.z, sc[2] new r.z, sc[3] r.r, sc[4] tol^2.
-// ---------------------------------------------------------------------------
-__global__ void k_mgcg_s1(double* sc, const int* fl) {
-    if (fl[0]) return;
-    sc[1] = sc[2];
-    sc[0] = 0.0;
-    sc[3] = 0.0;
-}
-
-__global__ void __launch_bounds__(kThreads) k_mgcg_spmv(int n, const int* __restrict__ row_ptr,
-                                                        const int* __restrict__ col, const double* __restrict__ K,
-                                                        const double* __restrict__ p, const uint8_t* __restrict__ fixed,
-                                                        double* __restrict__ q, double* sc, const int* fl,
-                                                        double* ws) {
-    if (fl[0]) return;
-    // kRowLanes lanes per block row (bsr_row_group); lane 0 of each group finishes the row
-    const int t = blockIdx.x * kThreads + threadIdx.x;
-    const int i = t / kRowLanes, g = t % kRowLanes;
-    double part = 0.0;
-    double y0, y1;
-    bsr_row_group<double, double>(i, i < n, g, row_ptr, col, K, p, y0, y1);
-    if (i < n && g == 0) {
-        if (fixed[2 * i]) y0 = 0.0;
-        if (fixed[2 * i + 1]) y1 = 0.0;
-        q[2 * i] = y0;
-        q[2 * i + 1] = y1;
-        part = p[2 * i] * y0 + p[2 * i + 1] * y1;
-    }
-    const double s = block_sum(part);
-    grid_add(ws, 0, s, &sc[0]);
-}
-
-__global__ void __launch_bounds__(kThreads) k_mgcg_update(int nd, double* __restrict__ x, double* __restrict__ r,
-                                                          const double* __restrict__ p, const double* __restrict__ q,
-                                                          double* sc, int* fl, double* ws) {
-    if (fl[0]) return;
-    const double pq = sc[0];
-    if (!(pq > 0.0)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            fl[1] = 1;
-            fl[0] = 1;
-        }
-        return;
-    }
-    const double alpha = sc[1] / pq;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    double part = 0.0;
-    if (i < nd) {
-        x[i] += alpha * p[i];
-        const double ri = r[i] - alpha * q[i];
-        r[i] = ri;
-        part = ri * ri;
-    }
-    const double s = block_sum(part);
-    grid_add(ws, 1, s, &sc[3]);
-}
-
-__global__ void k_mgcg_s2(double* sc, int* fl) {
-    if (fl[0]) return;
-    fl[2] += 1;
-    if (sc[3] <= sc[4]) fl[0] = 1;
-    sc[2] = 0.0;
-}
-
-__global__ void __launch_bounds__(kThreads) k_mgcg_dot(int nd, const double* __restrict__ a, const double* __restrict__ b,
-                                                       double* out, const int* fl, double* ws) {
-    if (fl[0]) return;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    const double v = i < nd ? a[i] * b[i] : 0.0;
-    const double s = block_sum(v);
-    grid_add(ws, 2, s, out);
-}
-
-__global__ void __launch_bounds__(kThreads) k_mgcg_pupdate(int nd, const double* __restrict__ z, double* __restrict__ p,
-                                                           const double* sc, const int* fl) {
-    if (fl[0]) return;
-    const double beta = sc[2] / sc[1];
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < nd) p[i] = z[i] + beta * p[i];
-}
-
-__global__ void __launch_bounds__(kThreads) k_mgcg_start(int nd, const uint8_t* __restrict__ fixed,
-                                                         const double* __restrict__ b, double* __restrict__ r,
-                                                         double* __restrict__ x, double* sc, double* ws) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    double part = 0.0;
-    if (i < nd) {
-        const double v = fixed[i] ? 0.0 : b[i];
-        r[i] = v;
-        x[i] = 0.0;
-        part = v * v;
-    }
-    const double s = block_sum(part);
-    grid_add(ws, 1, s, &sc[3]);
-}
-
-__global__ void k_mgcg_tol(double* sc, double rtol2) { sc[4] = rtol2 * sc[3]; }
-
-inline int nb(int n, int t = kThreads) { return (n + t - 1) / t; }
-
+inline int nb(long long n, int t = kThreads) { return (int)((n + t - 1) / t); }
 
 // ---------------------------------------------------------------------------
 // Inclusion rigid modes.  With cohesive interfaces an inclusion whose
@@ -841,14 +233,60 @@ __global__ void k_modes_add(int n, const int* __restrict__ z_inc, const double* 
     }
 }
 
+
+// ---------------------------------------------------------------------------
+// Structure (once per mesh)
+// ---------------------------------------------------------------------------
 template <typename T>
 int mg_alloc(MgHierarchy& m, T** p, size_t n) {
     *p = nullptr;
     PG_CUDA(cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T)));
-    PG_CUDA(fill_sync(*p, 0, std::max<size_t>(n, 1) * sizeof(T)));
     m.owned.push_back((void*)*p);
     return PG_OK;
 }
+
+template <typename T>
+int mg_upload(MgHierarchy& m, T** p, const std::vector<T>& v) {
+    const int rc = mg_alloc(m, p, v.size());
+    if (rc) return rc;
+    if (!v.empty()) PG_CUDA(h2d_sync(*p, v.data(), v.size() * sizeof(T)));
+    return PG_OK;
+}
+
+// Device memory of many arrays in one allocation (each 256-byte aligned): a
+// hierarchy has some sixty, and an allocation each took longer than a solve.
+struct Arena {
+    struct Item {
+        void** p;
+        size_t bytes;
+        const void* src;
+    };
+    std::vector<Item> items;
+    template <typename T>
+    void add(T** p, size_t n) {
+        items.push_back({(void**)p, std::max<size_t>(n, 1) * sizeof(T), nullptr});
+    }
+    // with contents (kept by the caller until commit)
+    template <typename T>
+    void add(T** p, const std::vector<T>& v) {
+        items.push_back({(void**)p, std::max<size_t>(v.size(), 1) * sizeof(T), v.empty() ? nullptr : v.data()});
+    }
+    int commit(MgHierarchy& m) {
+        size_t total = 0;
+        for (const Item& it : items) total += (it.bytes + 255) & ~size_t(255);
+        char* base = nullptr;
+        int rc = mg_alloc(m, &base, total);
+        if (rc) return rc;
+        for (const Item& it : items) {
+            *it.p = base;
+            if (it.src) PG_CUDA(cudaMemcpy(base, it.src, it.bytes, cudaMemcpyHostToDevice));
+            base += (it.bytes + 255) & ~size_t(255);
+        }
+        PG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        items.clear();
+        return PG_OK;
+    }
+};
 
 // Inclusion rigid modes of a cohesive mesh (host, once per mesh).
 int modes_build(Ctx& c, MgHierarchy& m) {
@@ -902,354 +340,511 @@ int modes_build(Ctx& c, MgHierarchy& m) {
                 zval[6 * (size_t)n + 3 * d + q] = Rn[d][q] - ((1.0 - t) * Ra[d][q] + t * Rb[d][q]);
     }
     int rc;
-    if ((rc = mg_alloc(m, &m.z_inc, (size_t)nn)) || (rc = mg_alloc(m, &m.zval, 6 * (size_t)nn)) ||
-        (rc = mg_alloc(m, &m.E, 9 * (size_t)ni)) || (rc = mg_alloc(m, &m.Einv, 9 * (size_t)ni)) ||
-        (rc = mg_alloc(m, &m.w, 3 * (size_t)ni)))
+    if ((rc = mg_upload(m, &m.z_inc, zinc)) || (rc = mg_upload(m, &m.zval, zval)) || (rc = mg_alloc(m, &m.E, 9 * (size_t)ni)) ||
+        (rc = mg_alloc(m, &m.Einv, 9 * (size_t)ni)) || (rc = mg_alloc(m, &m.w, 3 * (size_t)ni)))
         return rc;
-    PG_CUDA(h2d_sync(m.z_inc, zinc.data(), zinc.size() * sizeof(int)));
-    PG_CUDA(h2d_sync(m.zval, zval.data(), zval.size() * sizeof(double)));
     m.n_inc = ni;
     return PG_OK;
 }
 
-// Structure of the hierarchy (once per mesh).
-int mg_build(Ctx& c) {
-    if (c.mg) return PG_OK;
-    {   // k_mg_bottom's shared-memory limit, once per device (before any graph capture)
-        static bool done_dev[64] = {};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev < 0 || dev >= 64 || !done_dev[dev]) {
-            PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMgBottomSmem));
-            PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMgBottomSmem));
-            if (dev >= 0 && dev < 64) done_dev[dev] = true;
+// The enrichment pieces of one RVE (see k_mg_enr): its enrichment nodes in
+// depth-first order of the K_ee graph (along the interfaces), cut into cores
+// of kPieceRows; around each core the nodes within kChebSteps - 1 steps.
+struct RvePieces {
+    std::vector<Piece> piece;
+    std::vector<int> node, eptr;
+    std::vector<int2> ent;
+};
+
+void build_pieces(const HostMesh& hm, int rve, int lo, int hi, RvePieces& out) {
+    const int n = hi - lo;
+    std::vector<int> order, stack, local(n, -1);
+    std::vector<char> seen(n, 0);
+    order.reserve(n);
+    for (int s = 0; s < n; ++s) {
+        if (seen[s]) continue;
+        stack.push_back(s);
+        while (!stack.empty()) {
+            const int v = stack.back();
+            stack.pop_back();
+            if (seen[v]) continue;
+            seen[v] = 1;
+            order.push_back(v);
+            for (int q = hm.row_ptr[lo + v + 1] - 1; q >= hm.row_ptr[lo + v]; --q) {
+                const int j = hm.col[q];
+                if (j >= lo && j < hi && !seen[j - lo]) stack.push_back(j - lo);
+            }
         }
     }
-    const int nx0 = c.hm.spec.nx, ny0 = c.hm.spec.ny;
-    if (nx0 < 1 || ny0 < 1) {
+    std::vector<int> loc;
+    for (int c0 = 0; c0 < n; c0 += kPieceRows) {
+        Piece p{};
+        p.rve = rve;
+        p.row0 = (int)out.node.size();
+        loc.assign(order.begin() + c0, order.begin() + std::min(n, c0 + kPieceRows));
+        for (size_t k = 0; k < loc.size(); ++k) local[loc[k]] = (int)k;
+        p.end[0] = (int)loc.size();
+        for (int d = 1; d < kChebSteps; ++d) {
+            const int b = d == 1 ? 0 : p.end[d - 2], e = p.end[d - 1];
+            for (int k = b; k < e; ++k)
+                for (int q = hm.row_ptr[lo + loc[k]]; q < hm.row_ptr[lo + loc[k] + 1]; ++q) {
+                    const int j = hm.col[q];
+                    if (j < lo || j >= hi || local[j - lo] >= 0) continue;
+                    local[j - lo] = (int)loc.size();
+                    loc.push_back(j - lo);
+                }
+            p.end[d] = (int)loc.size();
+        }
+        for (size_t k = 0; k < loc.size(); ++k) {
+            out.node.push_back(lo + loc[k]);
+            out.eptr.push_back((int)out.ent.size());
+            if ((int)k >= p.end[kChebSteps - 2]) continue;  // the outermost ring only starts the recurrence
+            for (int q = hm.row_ptr[lo + loc[k]]; q < hm.row_ptr[lo + loc[k] + 1]; ++q) {
+                const int j = hm.col[q];
+                if (j >= lo && j < hi) out.ent.push_back(make_int2(q, local[j - lo]));
+            }
+        }
+        for (int v : loc) local[v] = -1;
+        out.piece.push_back(p);
+    }
+}
+
+int build_hierarchy(Ctx& c) {
+    const HostMesh& hm = c.hm;
+    const int R = (int)hm.grids.size();
+    if (R < 1) {
         set_error("multigrid: mesh without a structured background grid");
         return PG_ERR_ARG;
     }
-    MgHierarchy* m = new MgHierarchy();
-    c.mg = m;
-    int rc;
-    const int nd0 = c.n_dof;
-    if ((rc = mg_alloc(*m, &m->x0, nd0)) || (rc = mg_alloc(*m, &m->x0b, nd0)) || (rc = mg_alloc(*m, &m->r0, nd0)))
-        return rc;
-    if ((rc = mg_alloc(*m, &m->b0f, nd0)) || (rc = mg_alloc(*m, &m->x0f, nd0)) || (rc = mg_alloc(*m, &m->x0bf, nd0)) ||
-        (rc = mg_alloc(*m, &m->r0f, nd0)) || (rc = mg_alloc(*m, &m->Dinv0f, 4 * (size_t)c.n_nodes)))
-        return rc;
-    int nx = nx0, ny = ny0, l = 0;
-    while ((nx > kMgCoarseCells || ny > kMgCoarseCells) && l < kMgMaxLevels) {
-        nx = (nx + 1) / 2;
-        ny = (ny + 1) / 2;
-        ++l;
-        MgLevel& L = m->L[l];
-        L.nx = nx;
-        L.ny = ny;
-        L.n = (nx + 1) * (ny + 1);
-        const size_t n = L.n;
-        if ((rc = mg_alloc(*m, &L.A, 36 * n)) || (rc = mg_alloc(*m, &L.Af, 36 * n)) || (rc = mg_alloc(*m, &L.Dinv, 4 * n)) ||
-            (rc = mg_alloc(*m, &L.Dinvf, 4 * n)) || (rc = mg_alloc(*m, &L.fixed, 2 * n)))
-            return rc;
-        if ((rc = mg_alloc(*m, &L.x, 2 * n)) || (rc = mg_alloc(*m, &L.x2, 2 * n)) || (rc = mg_alloc(*m, &L.b, 2 * n)) ||
-            (rc = mg_alloc(*m, &L.r, 2 * n)))
-            return rc;
-        if ((rc = mg_alloc(*m, &L.xf, 2 * n)) || (rc = mg_alloc(*m, &L.x2f, 2 * n)) || (rc = mg_alloc(*m, &L.bf, 2 * n)) ||
-            (rc = mg_alloc(*m, &L.rf, 2 * n)))
-            return rc;
+    // each RVE's grids, coarsened until both sides have at most kCoarseCells cells
+    std::vector<std::vector<std::pair<int, int>>> dims(R);
+    int nlev = 0;
+    for (int r = 0; r < R; ++r) {
+        int nx = hm.grids[r].nx, ny = hm.grids[r].ny;
+        dims[r].push_back({nx, ny});
+        while ((nx > kCoarseCells || ny > kCoarseCells) && (int)dims[r].size() <= kMaxLevels) {
+            nx = (nx + 1) / 2;
+            ny = (ny + 1) / 2;
+            dims[r].push_back({nx, ny});
+        }
+        if (dims[r].size() < 2 || nx > kCoarseCells || ny > kCoarseCells) {
+            set_error("multigrid: grid too small or too large to coarsen");
+            return PG_ERR_ARG;
+        }
+        nlev = std::max(nlev, (int)dims[r].size() - 1);
     }
-    if (l == 0 || (nx > kMgCoarseCells || ny > kMgCoarseCells)) {
-        set_error("multigrid: grid too small or too large to coarsen");
-        return PG_ERR_ARG;
+    auto nodes = [&](int r, int l) { return (dims[r][l].first + 1) * (dims[r][l].second + 1); };
+    MgHierarchy* mp = new MgHierarchy();
+    c.mg = mp;
+    MgHierarchy& m = *mp;
+    m.R = R;
+    m.nlev = nlev;
+    Arena ar;
+    // the bottom of each RVE's cycle: its levels of at most kBottomNodes nodes
+    std::vector<Bottom> bottom(R);
+    std::vector<int> kb(R);
+    size_t smem[2] = {0, 0};
+    for (int r = 0; r < R; ++r) {
+        const int depth = (int)dims[r].size() - 1;
+        int k = depth;
+        while (k > 1 && depth - k + 1 < kBottomLevels && nodes(r, k - 1) <= kBottomNodes) --k;
+        kb[r] = k;
+        for (int t = 0; t < 2; ++t) {
+            size_t bytes = 0;
+            for (int l = k; l <= depth; ++l) bytes += bottom_level_bytes(nodes(r, l), t ? sizeof(float) : sizeof(double), l == depth);
+            smem[t] = std::max(smem[t], bytes);
+        }
     }
-    m->nlev = l;
-    m->nc = 2 * m->L[l].n;
-    if ((rc = mg_alloc(*m, &m->LU, (size_t)m->nc * m->nc)) || (rc = mg_alloc(*m, &m->piv, m->nc)) ||
-        (rc = mg_alloc(*m, &m->sc, 8)) || (rc = mg_alloc(*m, &m->fl, 8)))
-        return rc;
+    m.bottom_smem[0] = smem[0];
+    m.bottom_smem[1] = smem[1];
+    // levels: offsets, transfers, tiles
+    std::vector<std::vector<int>> off(nlev + 1, std::vector<int>(R, 0));
+    std::vector<std::vector<Pair>> pairs(nlev + 1);
+    std::vector<std::vector<int4>> down(nlev + 1), up(nlev + 1);
+    std::vector<std::vector<int>> node_rve(nlev + 1);
+    for (int r = 0; r < R; ++r) off[0][r] = hm.grids[r].node_off;
+    for (int l = 1; l <= nlev; ++l) {
+        Level& L = m.L[l];
+        pairs[l].assign(R, Pair{0, 0, 0, 0, -1, -1});
+        for (int r = 0; r < R; ++r) {
+            if ((int)dims[r].size() <= l) continue;
+            off[l][r] = L.n;
+            const int nx = dims[r][l].first, ny = dims[r][l].second;
+            pairs[l][r] = Pair{off[l - 1][r], dims[r][l - 1].first, dims[r][l - 1].second, L.n, nx, ny};
+            if (R > 1) node_rve[l].insert(node_rve[l].end(), nodes(r, l), r);
+            L.n += nodes(r, l);
+            if (l <= kb[r])
+                for (int J = 0; J <= ny; J += kDownTile)
+                    for (int I = 0; I <= nx; I += kDownTile) down[l].push_back(make_int4(r, I, J, I == 0 && J == 0));
+            if (l < kb[r])
+                for (int J = 0; J <= ny; J += kUpTile)
+                    for (int I = 0; I <= nx; I += kUpTile) up[l].push_back(make_int4(r, I, J, 0));
+        }
+        L.down.n = (int)down[l].size();
+        L.up.n = (int)up[l].size();
+        ar.add(&L.pair, pairs[l]);
+        ar.add(&L.down.tile, down[l]);
+        ar.add(&L.up.tile, up[l]);
+        if (R > 1) ar.add(&L.node_rve, node_rve[l]);
+        ar.add(&L.fixed, 2 * (size_t)L.n);
+        ar.add(&L.d.A, 36 * (size_t)L.n);
+        ar.add(&L.d.Dinv, 4 * (size_t)L.n);
+        for (double** v : {&L.d.b, &L.d.x, &L.d.xo}) ar.add(v, 2 * (size_t)L.n);
+    }
+    for (int r = 0; r < R; ++r) {
+        const int depth = (int)dims[r].size() - 1;
+        Bottom& B = bottom[r];
+        B = Bottom{};
+        B.first = kb[r];
+        B.nlev = depth - kb[r] + 1;
+        for (int k = 0; k < B.nlev; ++k) {
+            B.nx[k] = dims[r][kb[r] + k].first;
+            B.ny[k] = dims[r][kb[r] + k].second;
+            B.off[k] = off[kb[r] + k][r];
+        }
+        B.foff = off[kb[r] - 1][r];
+        B.fnx = dims[r][kb[r] - 1].first;
+        B.fny = dims[r][kb[r] - 1].second;
+    }
+    // row spans of the level-0 kernels: as many CTAs as the GPU holds, each with about as many blocks of K, in
+    // steps of the rows a CTA takes at once
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    constexpr int kStep = kSpanThreads / kRowLanes;
+    const long long total = hm.n_blocks() + 2LL * c.n_nodes;
+    const double per_cta = std::max((double)total / (sms * kSpanCtasPerSm), 1.0);
+    std::vector<int4> span;
+    std::vector<int2> range(R);
+    std::vector<int> reg_end(R), node_end(R);
+    for (int r = 0; r < R; ++r) {
+        const auto& gb = hm.grids[r];
+        const int lo = gb.node_off, hi = r + 1 < R ? hm.grids[r + 1].node_off : c.n_nodes;
+        reg_end[r] = lo + gb.n_reg;
+        node_end[r] = hi;
+        range[r].x = (int)span.size();
+        int row = lo;
+        while (row < hi) {
+            int end = row;
+            double w = 0.0;
+            while (end < hi && (end == row || w + 0.5 * (hm.row_ptr[std::min(end + kStep, hi)] - hm.row_ptr[end]) < per_cta)) {
+                const int e = std::min(end + kStep, hi);
+                w += hm.row_ptr[e] - hm.row_ptr[end] + 2.0 * (e - end);
+                end = e;
+            }
+            span.push_back(make_int4(r, row, end, 0));
+            row = end;
+        }
+        range[r].y = (int)span.size();
+    }
+    m.n_cta = (int)span.size();
+    int4* d_span;
+    int2* d_range;
+    int* d_reg;
+    ar.add(&d_span, span);
+    ar.add(&d_range, range);
+    ar.add(&d_reg, reg_end);
+    ar.add(&m.node_end, node_end);
+    // enrichment pieces, RVE by RVE in parallel
+    std::vector<RvePieces> rp(R);
+    parallel_for(R, 1, [&](long long r) { build_pieces(hm, (int)r, reg_end[r], node_end[r], rp[r]); });
+    std::vector<Piece> piece;
+    std::vector<int> pnode, peptr, enr_node, enr_rve;
+    std::vector<int2> pent;
+    for (int r = 0; r < R; ++r) {
+        const int n0 = (int)pnode.size(), e0 = (int)pent.size();
+        for (Piece p : rp[r].piece) {
+            p.row0 += n0;
+            m.max_piece = std::max(m.max_piece, p.end[kChebSteps - 1]);
+            piece.push_back(p);
+        }
+        pnode.insert(pnode.end(), rp[r].node.begin(), rp[r].node.end());
+        for (int e : rp[r].eptr) peptr.push_back(e + e0);
+        pent.insert(pent.end(), rp[r].ent.begin(), rp[r].ent.end());
+        for (int i = reg_end[r]; i < node_end[r]; ++i) {
+            enr_node.push_back(i);
+            enr_rve.push_back(r);
+        }
+    }
+    peptr.push_back((int)pent.size());
+    m.n_pieces = (int)piece.size();
+    m.n_enr = (int)enr_node.size();
+    Piece* d_piece;
+    int *d_pnode, *d_peptr;
+    int2* d_pent;
+    ar.add(&d_piece, piece);
+    ar.add(&d_pnode, pnode);
+    ar.add(&d_peptr, peptr);
+    ar.add(&d_pent, pent);
+    ar.add(&m.enr_node, enr_node);
+    ar.add(&m.enr_rve, enr_rve);
+    ar.add(&m.bound, (size_t)R);
+    ar.add(&m.coef, (size_t)kChebCoef * R);
+    ar.add(&m.bottom, bottom);
+    std::vector<Coarse> coarse(R);  // (device pointers are known after the commit)
+    ar.add(&m.coarse, (size_t)R);
+    ar.add(&m.XT, (size_t)kCoarseStride * R);
+    ar.add(&m.x0, (size_t)c.n_dof);
+    ar.add(&m.x0e, (size_t)c.n_dof);
+    for (double** v : {&m.part_pq, &m.part_rr, &m.part_rz}) ar.add(v, (size_t)m.n_cta);
+    ar.add(&m.sc, (size_t)kScal * R);
+    ar.add(&m.fl, (size_t)kFlags * R);
+    int rc = ar.commit(m);
+    if (rc) return rc;
+    m.spans = Spans{d_span, d_range, d_reg};
+    m.enr = Enr{d_piece, d_pnode, d_peptr, d_pent, m.coef};
+    for (int r = 0; r < R; ++r) {
+        const int l = (int)dims[r].size() - 1;
+        coarse[r] = Coarse{m.L[l].d.A, m.L[l].fixed, off[l][r], dims[r][l].first, dims[r][l].second, 0};
+    }
+    PG_CUDA(h2d_sync(m.coarse, coarse.data(), coarse.size() * sizeof(Coarse)));
+    PG_CUDA(cudaMallocHost((void**)&m.h_sc, (size_t)kScal * R * sizeof(double)));
+    PG_CUDA(cudaMallocHost((void**)&m.h_fl, 2 * (size_t)kFlags * R * sizeof(int)));
+    for (cudaEvent_t& e : m.ev) PG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    // kernels whose shared memory exceeds the default (the attribute belongs to the device, so the largest any
+    // hierarchy on it may ask for)
+    constexpr int kSmemMax = 190 * 1024;
+    if (smem[0] > kSmemMax || (size_t)m.max_piece * 8 * sizeof(double) > 100 * 1024) {
+        set_error("multigrid: level too large for shared memory");
+        return PG_ERR_LIMIT;
+    }
+    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    for (auto k : {k_mg_enr<double, false>, k_mg_enr<double, true>})
+        PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    for (auto k : {k_mg_enr<float, false>, k_mg_enr<float, true>})
+        PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     // coarse masks by injection
     cudaStream_t s = c.stream;
     const uint8_t* ff = c.fixed;
-    int nxf = nx0, nyf = ny0;
-    for (int k = 1; k <= l; ++k) {
-        MgLevel& L = m->L[k];
-        k_mg_inject_mask<<<nb(L.n), kThreads, 0, s>>>(nxf, L.nx, L.ny, nyf, ff, L.fixed);
+    for (int l = 1; l <= nlev; ++l) {
+        Level& L = m.L[l];
+        k_mg_inject_mask<<<nb(L.n), kThreads, 0, s>>>(L.n, L.node_rve, L.pair, ff, L.fixed);
         ff = L.fixed;
-        nxf = L.nx;
-        nyf = L.ny;
     }
     PG_CUDA(cudaGetLastError());
     PG_CUDA(cudaStreamSynchronize(s));
-    return modes_build(c, *m);
+    return R == 1 ? modes_build(c, m) : PG_OK;
+}
+
+int mg_build(Ctx& c) {
+    if (c.mg) return PG_OK;
+    const int rc = build_hierarchy(c);
+    if (rc != PG_OK) mg_free(c);
+    return rc;
+}
+
+// the FP32 cycle's arrays, on its first use
+int ensure_f32(Ctx& c, MgHierarchy& m) {
+    if (m.f32_ready) return PG_OK;
+    Arena ar;
+    for (int l = 1; l <= m.nlev; ++l) {
+        Level& L = m.L[l];
+        ar.add(&L.f.A, 36 * (size_t)L.n);
+        ar.add(&L.f.Dinv, 4 * (size_t)L.n);
+        for (float** v : {&L.f.b, &L.f.x, &L.f.xo}) ar.add(v, 2 * (size_t)L.n);
+    }
+    ar.add(&m.x0f, (size_t)c.n_dof);
+    ar.add(&m.x0ef, (size_t)c.n_dof);
+    ar.add(&m.Dinv0f, 4 * (size_t)c.n_nodes);
+    const int rc = ar.commit(m);
+    if (rc == PG_OK) m.f32_ready = true;
+    return rc;
 }
 
 // Numeric set-up for the current K (every solve: K changes between Newton iterations).
-int mg_numeric(Ctx& c, bool f32, cudaStream_t s) {
+int mg_numeric(Ctx& c, bool f32, bool modes, cudaStream_t s) {
     MgHierarchy& m = *c.mg;
     const int n0 = c.n_nodes;
-    // level 0 smoother: block Jacobi of the masked K
+    int rc;
+    if (f32 && (rc = ensure_f32(c, m))) return rc;
+    cudaMemsetAsync(m.fl, 0, (size_t)kFlags * m.R * sizeof(int), s);
+    // level 0: block Jacobi of the masked K, and the enrichment block's polynomial
     k_prec_setup<double><<<nb(n0), kThreads, 0, s>>>(n0, c.diag, c.K, c.fixed, 1, 0, c.minv);
     if (f32) {
         launch_to_fp32(c, s);
-        k_mg_to_f32<<<nb(4 * n0), kThreads, 0, s>>>(4 * (size_t)n0, c.minv, m.Dinv0f);
+        k_mg_to_f32<<<nb(4LL * n0), kThreads, 0, s>>>(4 * (size_t)n0, c.minv, m.Dinv0f);
     }
-    int nxf = c.hm.spec.nx, nyf = c.hm.spec.ny;
-    for (int k = 1; k <= m.nlev; ++k) {
-        MgLevel& L = m.L[k];
-        GalArgs g;
-        g.nxf = nxf;
-        g.nyf = nyf;
-        g.nxc = L.nx;
-        g.nyc = L.ny;
-        g.row_ptr = c.row_ptr;
-        g.col = c.col;
-        g.K = c.K;
-        g.n_reg = c.n_reg;
-        g.A = k > 1 ? m.L[k - 1].A : nullptr;
-        g.fixed_f = k > 1 ? m.L[k - 1].fixed : c.fixed;
-        g.fixed_c = L.fixed;
-        g.Ac = L.A;
-        if (k == 1)
-            k_mg_galerkin<true><<<nb(9 * L.n), kThreads, 0, s>>>(g);
+    if (m.n_enr > 0) {
+        cudaMemsetAsync(m.bound, 0, (size_t)m.R * sizeof(unsigned long long), s);
+        k_enr_bound<<<nb(m.n_enr, 128), 128, 0, s>>>(m.n_enr, m.enr_node, m.enr_rve, m.spans.reg_end, m.node_end, c.row_ptr,
+                                                      c.col, c.diag, c.K, m.bound);
+        k_enr_coef<<<nb(m.R), kThreads, 0, s>>>(m.R, m.bound, m.coef);
+    }
+    for (int l = 1; l <= m.nlev; ++l) {
+        Level& L = m.L[l];
+        const uint8_t* ff = l > 1 ? m.L[l - 1].fixed : c.fixed;
+        float* Af = f32 ? L.f.A : nullptr;
+        float* Df = f32 ? L.f.Dinv : nullptr;
+        if (l == 1)
+            k_mg_galerkin<true><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, c.row_ptr, c.col, c.K,
+                                                                           nullptr, ff, L.fixed, L.d.A, Af, L.d.Dinv, Df);
         else
-            k_mg_galerkin<false><<<nb(9 * L.n), kThreads, 0, s>>>(g);
-        k_mg_dinv<<<nb(L.n), kThreads, 0, s>>>(L.n, L.A, L.fixed, L.Dinv, f32 ? L.Dinvf : nullptr);
-        if (f32) k_mg_to_f32<<<nb(36 * L.n), kThreads, 0, s>>>(36 * (size_t)L.n, L.A, L.Af);
-        nxf = L.nx;
-        nyf = L.ny;
+            k_mg_galerkin<false><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, nullptr, nullptr, nullptr,
+                                                                            m.L[l - 1].d.A, ff, L.fixed, L.d.A, Af, L.d.Dinv,
+                                                                            Df);
     }
-    if (m.n_inc > 0 && m.use_modes) {
+    if (m.n_inc > 0 && modes) {
         cudaMemsetAsync(m.E, 0, 9 * (size_t)m.n_inc * sizeof(double), s);
         k_modes_E<<<nb(n0), kThreads, 0, s>>>(n0, m.z_inc, m.zval, c.row_ptr, c.col, c.K, c.fixed, m.E);
         k_modes_inv<<<nb(m.n_inc), kThreads, 0, s>>>(m.n_inc, m.E, m.Einv);
     }
-    const MgLevel& C = m.L[m.nlev];
-    cudaMemsetAsync(m.fl, 0, 8 * sizeof(int), s);
-    k_mg_coarse_factor<<<1, 128, 0, s>>>(C.nx, C.ny, C.A, C.fixed, m.LU, m.piv, m.fl);
+    k_mg_coarse_inverse<<<m.R, kFactorThreads, 2 * kCoarseStride * sizeof(double), s>>>(m.coarse, m.XT, m.fl);
     PG_CUDA(cudaGetLastError());
     return PG_OK;
 }
 
-// One V-cycle: returns the level-0 buffer holding V(b0).  Records launches on s.
+// What the V-cycle's precision decides: the level-0 operator and vectors and the levels' arrays
 template <typename T>
-const T* vcycle(Ctx& c, MgHierarchy& m, cudaStream_t s, const T* b0, const int* done);
-
-// First level of the fused bottom (k_mg_bottom) and which of its levels have
-// their operator staged in shared memory: going up from the coarsest, the
-// levels of at most kMgBottomNodes nodes (at most kMgBottomLevels) whose
-// vectors fit in kMgBottomSmem bytes together; then, coarsest first, each
-// level's operator is staged while it still fits (the coarsest level, solved
-// by its explicit inverse, needs none); the others read theirs from L2.
-template <typename T>
-int mg_bottom_first(const MgHierarchy& m, size_t* smem, int* staged) {
-    int kb = m.nlev;
-    size_t bytes = mg_bottom_vec_bytes<T>(m.L[m.nlev].n);
-    for (int k = m.nlev - 1; k >= 1 && m.nlev - k + 1 <= kMgBottomLevels; --k) {
-        const size_t add = mg_bottom_vec_bytes<T>(m.L[k].n);
-        if (m.L[k].n > kMgBottomNodes || bytes + add > (size_t)kMgBottomSmem) break;
-        bytes += add;
-        kb = k;
-    }
-    for (int k = m.nlev; k >= kb; --k) {
-        int& st = staged[k - kb];
-        st = 0;
-        if (k == m.nlev) continue;
-        const size_t add = mg_bottom_op_bytes<T>(m.L[k].n);
-        if (bytes + add <= (size_t)kMgBottomSmem) {
-            bytes += add;
-            st = 1;
-        }
-    }
-    *smem = bytes;
-    return kb;
-}
-
-// Levels kb .. nlev in one launch; level kb's result ends in its x (xf).
-template <typename T>
-void launch_bottom(MgHierarchy& m, int kb, size_t smem, const int* staged, int nxf, int nyf, const T* rf,
-                   cudaStream_t s, const int* done) {
-    MgBottomArgs<T> a;
-    a.nlev = m.nlev - kb + 1;
-    a.nxf = nxf;
-    a.nyf = nyf;
-    a.rf = rf;
-    for (int k = kb; k <= m.nlev; ++k) {
-        MgLevel& L = m.L[k];
-        const int j = k - kb;
-        a.nx[j] = L.nx;
-        a.ny[j] = L.ny;
-        a.fixed[j] = L.fixed;
-        a.staged[j] = staged[j];
-        if constexpr (std::is_same<T, float>::value) {
-            a.A[j] = L.Af;
-            a.Dinv[j] = L.Dinvf;
-        } else {
-            a.A[j] = L.A;
-            a.Dinv[j] = L.Dinv;
-        }
-    }
-    if constexpr (std::is_same<T, float>::value) a.x0 = m.L[kb].xf;
-    else a.x0 = m.L[kb].x;
-    a.XT = m.LU;
-    a.nc = m.nc;
-    a.omega = (T)kMgOmega;
-    k_mg_bottom<T><<<1, kMgBottomThreads, smem, s>>>(a, done);
-}
-
+struct Cycle;
 template <>
-const double* vcycle<double>(Ctx& c, MgHierarchy& m, cudaStream_t s, const double* b0, const int* done) {
-    const int n0 = c.n_nodes;
-    const double om = kMgOmega;
-    // level 0 pre-smoothing
-    double* cur = m.x0;
-    double* alt = m.x0b;
-    k_mg_smooth_bsr<double><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.K, c.minv, c.fixed, b0, nullptr, cur, om,
-                                                          done, 0);
-    for (int it = 1; it < kMgNu1; ++it) {
-        k_mg_smooth_bsr<double><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.K, c.minv, c.fixed, b0, cur, alt, om,
-                                                              done, 0);
-        std::swap(cur, alt);
-    }
-    k_mg_smooth_bsr<double><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.K, c.minv, c.fixed, b0, cur, m.r0, om,
-                                                          done, 1);
-    int nxf = c.hm.spec.nx, nyf = c.hm.spec.ny;
-    const double* rf = m.r0;
-    double* xs[kMgMaxLevels + 1];
-    xs[0] = cur;
-    size_t bsm = 0;
-    int staged[kMgBottomLevels];
-    const int kb = mg_bottom_first<double>(m, &bsm, staged);
-    for (int k = 1; k <= m.nlev; ++k) {
-        MgLevel& L = m.L[k];
-        if (k == kb) {  // this level and all coarser ones: one launch
-            launch_bottom<double>(m, kb, bsm, staged, nxf, nyf, rf, s, done);
-            xs[k] = L.x;
-            break;
-        }
-        k_mg_restrict<double><<<nb(L.n), kThreads, 0, s>>>(nxf, nyf, L.nx, L.ny, rf, L.fixed, L.b, done);
-        double* lc = L.x;
-        double* la = L.x2;
-        k_mg_smooth_st<double><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.A, L.Dinv, L.fixed, L.b, nullptr, lc, om, done, 0);
-        for (int it = 1; it < kMgNu1; ++it) {
-            k_mg_smooth_st<double><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.A, L.Dinv, L.fixed, L.b, lc, la, om, done, 0);
-            std::swap(lc, la);
-        }
-        k_mg_smooth_st<double><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.A, L.Dinv, L.fixed, L.b, lc, L.r, om, done, 1);
-        xs[k] = lc;
-        rf = L.r;
-        nxf = L.nx;
-        nyf = L.ny;
-    }
-    for (int k = kb - 1; k >= 0; --k) {
-        const MgLevel& Lc = m.L[k + 1];
-        if (k == 0) {
-            k_mg_prolong<double><<<nb(c.n_reg), kThreads, 0, s>>>(c.hm.spec.nx, c.hm.spec.ny, Lc.nx, xs[1], c.fixed, cur,
-                                                                    done);
-            for (int it = 0; it < kMgNu2; ++it) {
-                k_mg_smooth_bsr<double><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.K, c.minv, c.fixed, b0, cur,
-                                                                      alt, om, done, 0);
-                std::swap(cur, alt);
-            }
-            return cur;
-        }
-        MgLevel& L = m.L[k];
-        double* lc = xs[k];
-        double* la = lc == L.x ? L.x2 : L.x;
-        k_mg_prolong<double><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, Lc.nx, xs[k + 1], L.fixed, lc, done);
-        for (int it = 0; it < kMgNu2; ++it) {
-            k_mg_smooth_st<double><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.A, L.Dinv, L.fixed, L.b, lc, la, om, done, 0);
-            std::swap(lc, la);
-        }
-        xs[k] = lc;
-    }
-    return cur;
-}
-
+struct Cycle<double> {
+    static const double* K(const Ctx& c) { return c.K; }
+    static const double* Dinv(const Ctx& c, const MgHierarchy&) { return c.minv; }
+    static double* x(const MgHierarchy& m) { return m.x0; }
+    static double* xe(const MgHierarchy& m) { return m.x0e; }
+    static LevelArrays<double>& lev(Level& L) { return L.d; }
+    static size_t bottom_smem(const MgHierarchy& m) { return m.bottom_smem[0]; }
+};
 template <>
-const float* vcycle<float>(Ctx& c, MgHierarchy& m, cudaStream_t s, const float* b0, const int* done) {
-    const int n0 = c.n_nodes;
-    const float om = (float)kMgOmega;
-    float* cur = m.x0f;
-    float* alt = m.x0bf;
-    k_mg_smooth_bsr<float><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.Kf, m.Dinv0f, c.fixed, b0, nullptr, cur, om,
-                                                         done, 0);
-    for (int it = 1; it < kMgNu1; ++it) {
-        k_mg_smooth_bsr<float><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.Kf, m.Dinv0f, c.fixed, b0, cur, alt, om,
-                                                             done, 0);
-        std::swap(cur, alt);
-    }
-    k_mg_smooth_bsr<float><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.Kf, m.Dinv0f, c.fixed, b0, cur, m.r0f, om,
-                                                         done, 1);
-    int nxf = c.hm.spec.nx, nyf = c.hm.spec.ny;
-    const float* rf = m.r0f;
-    float* xs[kMgMaxLevels + 1];
-    xs[0] = cur;
-    size_t bsm = 0;
-    int staged[kMgBottomLevels];
-    const int kb = mg_bottom_first<float>(m, &bsm, staged);
-    for (int k = 1; k <= m.nlev; ++k) {
-        MgLevel& L = m.L[k];
-        if (k == kb) {  // this level and all coarser ones: one launch
-            launch_bottom<float>(m, kb, bsm, staged, nxf, nyf, rf, s, done);
-            xs[k] = L.xf;
-            break;
-        }
-        k_mg_restrict<float><<<nb(L.n), kThreads, 0, s>>>(nxf, nyf, L.nx, L.ny, rf, L.fixed, L.bf, done);
-        float* lc = L.xf;
-        float* la = L.x2f;
-        k_mg_smooth_st<float><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.Af, L.Dinvf, L.fixed, L.bf, nullptr, lc, om, done, 0);
-        for (int it = 1; it < kMgNu1; ++it) {
-            k_mg_smooth_st<float><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.Af, L.Dinvf, L.fixed, L.bf, lc, la, om, done, 0);
-            std::swap(lc, la);
-        }
-        k_mg_smooth_st<float><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.Af, L.Dinvf, L.fixed, L.bf, lc, L.rf, om, done, 1);
-        xs[k] = lc;
-        rf = L.rf;
-        nxf = L.nx;
-        nyf = L.ny;
-    }
-    for (int k = kb - 1; k >= 0; --k) {
-        const MgLevel& Lc = m.L[k + 1];
-        if (k == 0) {
-            k_mg_prolong<float><<<nb(c.n_reg), kThreads, 0, s>>>(c.hm.spec.nx, c.hm.spec.ny, Lc.nx, xs[1], c.fixed, cur, done);
-            for (int it = 0; it < kMgNu2; ++it) {
-                k_mg_smooth_bsr<float><<<nb(kRowLanes * n0), kThreads, 0, s>>>(n0, c.row_ptr, c.col, c.Kf, m.Dinv0f, c.fixed, b0, cur,
-                                                                     alt, om, done, 0);
-                std::swap(cur, alt);
-            }
-            return cur;
-        }
-        MgLevel& L = m.L[k];
-        float* lc = xs[k];
-        float* la = lc == L.xf ? L.x2f : L.xf;
-        k_mg_prolong<float><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, Lc.nx, xs[k + 1], L.fixed, lc, done);
-        for (int it = 0; it < kMgNu2; ++it) {
-            k_mg_smooth_st<float><<<nb(L.n), kThreads, 0, s>>>(L.nx, L.ny, L.Af, L.Dinvf, L.fixed, L.bf, lc, la, om, done, 0);
-            std::swap(lc, la);
-        }
-        xs[k] = lc;
-    }
-    return cur;
-}
+struct Cycle<float> {
+    static const float* K(const Ctx& c) { return c.Kf; }
+    static const float* Dinv(const Ctx&, const MgHierarchy& m) { return m.Dinv0f; }
+    static float* x(const MgHierarchy& m) { return m.x0f; }
+    static float* xe(const MgHierarchy& m) { return m.x0ef; }
+    static LevelArrays<float>& lev(Level& L) { return L.f; }
+    static size_t bottom_smem(const MgHierarchy& m) { return m.bottom_smem[1]; }
+};
 
-// z = M^-1 r through one V-cycle (FP64 in, FP64 out).
-void mg_apply(Ctx& c, MgHierarchy& m, bool f32, cudaStream_t s, const double* r, double* z, const int* done) {
-    const int nd = c.n_dof;
-    if (f32) {
-        k_mg_f64_to_f32<<<nb(nd), kThreads, 0, s>>>(nd, r, m.b0f, done);
-        const float* x = vcycle<float>(c, m, s, m.b0f, done);
-        k_mg_f32_to_f64<<<nb(nd), kThreads, 0, s>>>(nd, x, z, done);
-    } else {
-        const double* x = vcycle<double>(c, m, s, r, done);
-        k_copy<double><<<nb(nd), kThreads, 0, s>>>(nd, x, z);
+// The V-cycle after its first sweep (which CG's update has formed): z = V(r)
+// and the partials of r.z.  fl null outside CG; check: this cycle follows a
+// CG update, whose r.r it tests.
+template <typename T>
+void mg_cycle(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s, const double* r, double* z, int* fl, bool check) {
+    using C = Cycle<T>;
+    const T *K = C::K(c), *D0 = C::Dinv(c, m);
+    T *x0 = C::x(m), *xe = C::xe(m);
+    const size_t esm = (size_t)m.max_piece * 4 * sizeof(Vec2<T>);
+    if (m.n_pieces > 0)
+        k_mg_enr<T, false><<<m.n_pieces, kPieceThreads, esm, s>>>(m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
+                                                                  x0, x0, fl);
+    k_mg_down0<T><<<m.L[1].down.n, kSpanThreads, 0, s>>>(m.L[1].down.tile, m.L[1].pair, c.row_ptr, c.col, K, c.fixed, r, x0,
+                                                         m.L[1].fixed, C::lev(m.L[1]).b, m.spans, m.part_rr, m.sc, fl,
+                                                         check ? 1 : 0);
+    for (int l = 2; l <= m.nlev && m.L[l].down.n > 0; ++l) {
+        Level &F = m.L[l - 1], &L = m.L[l];
+        LevelArrays<T>& f = C::lev(F);
+        k_mg_down<T><<<L.down.n, kTileThreads, 0, s>>>(L.down.tile, L.pair, f.A, f.Dinv, F.fixed, f.b, f.x, L.fixed,
+                                                       C::lev(L).b, fl);
     }
-    if (m.n_inc > 0 && m.use_modes) {
+    BottomArrays<T> ba{};
+    for (int l = 1; l <= m.nlev; ++l) {
+        LevelArrays<T>& v = C::lev(m.L[l]);
+        ba.A[l] = v.A;
+        ba.Dinv[l] = v.Dinv;
+        ba.fixed[l] = m.L[l].fixed;
+        ba.b[l] = v.b;
+        ba.xo[l] = v.xo;
+    }
+    k_mg_bottom<T><<<m.R, kBottomThreads, C::bottom_smem(m), s>>>(m.bottom, ba, m.XT, c.fixed, x0, fl);
+    for (int l = m.nlev - 1; l >= 1; --l) {
+        Level& L = m.L[l];
+        if (L.up.n == 0) continue;
+        LevelArrays<T>& v = C::lev(L);
+        const T* xc = C::lev(m.L[l + 1]).xo;
+        if (l == 1)
+            k_mg_up<T, true><<<L.up.n, kTileThreads, 0, s>>>(L.up.tile, L.pair, m.L[2].pair, v.A, v.Dinv, L.fixed, v.b, v.x, xc,
+                                                             nullptr, c.fixed, x0, fl);
+        else
+            k_mg_up<T, false><<<L.up.n, kTileThreads, 0, s>>>(L.up.tile, L.pair, m.L[l + 1].pair, v.A, v.Dinv, L.fixed, v.b,
+                                                              v.x, xc, v.xo, nullptr, nullptr, fl);
+    }
+    if (m.n_pieces > 0)
+        k_mg_enr<T, true><<<m.n_pieces, kPieceThreads, esm, s>>>(m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
+                                                                 x0, xe, fl);
+    k_mg_post<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.row_ptr, c.col, K, D0, c.fixed, r, x0, xe, z, fl, m.part_rz);
+    if (m.n_inc > 0 && modes) {
         const int n = c.n_nodes;
-        k_modes_zero<<<nb(3 * m.n_inc), kThreads, 0, s>>>(3 * m.n_inc, m.w, done);
-        k_modes_dot<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, r, m.w, done);
-        k_modes_add<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, m.Einv, m.w, z, done);
+        k_modes_zero<<<nb(3 * m.n_inc), kThreads, 0, s>>>(3 * m.n_inc, m.w, fl);
+        k_modes_dot<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, r, m.w, fl);
+        k_modes_add<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, m.Einv, m.w, z, fl);
+        k_cg_dot<<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, r, z, fl, m.part_rz);
     }
+}
+
+// kChunk CG iterations
+template <typename T>
+void cg_iterations(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s) {
+    double* pb[2] = {c.p, c.xi};
+    for (int it = 0; it < kChunk; ++it) {
+        const int P = it & 1;
+        k_cg_spmv<<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.row_ptr, c.col, c.K, c.fixed, c.z, pb[1 - P], pb[P], c.q,
+                                                   m.part_rz, m.sc, m.fl, m.part_pq, P);
+        k_cg_update<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.dx, c.r, pb[P], c.q, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
+                                                        m.part_pq, m.sc, m.fl, m.part_rr, P);
+        mg_cycle<T>(c, m, modes, s, c.r, c.z, m.fl, true);
+    }
+}
+
+// CG on mask(K) dx = mask(b) (b = c.b, dx = c.dx) for every RVE; the host
+// copies of the flags and scalars are current when it returns PG_OK.
+template <typename T>
+int cg_run(Ctx& c, MgHierarchy& m, bool modes, const pg_solver_cfg& cfg, cudaStream_t s) {
+    const bool f32 = std::is_same<T, float>::value;
+    const size_t fl_bytes = (size_t)kFlags * m.R * sizeof(int);
+    int rc = mg_numeric(c, f32, modes, s);
+    if (rc) return rc;
+    k_cg_start<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, c.b, c.r, c.dx, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
+                                                   m.part_rr);
+    k_cg_tol<<<m.R, kSpanThreads, 0, s>>>(m.spans, m.part_rr, cfg.rtol * cfg.rtol, m.sc, m.fl);
+    cudaMemsetAsync(c.xi, 0, (size_t)c.n_dof * sizeof(double), s);  // p before the first iteration
+    mg_cycle<T>(c, m, modes, s, c.r, c.z, nullptr, false);
+    cudaMemcpyAsync(m.h_sc, m.sc, (size_t)kScal * m.R * sizeof(double), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(m.h_fl, m.fl, fl_bytes, cudaMemcpyDeviceToHost, s);
+    cudaGraphExec_t& exec = m.graph[(f32 ? 1 : 0) + (modes ? 2 : 0)];
+    if (!exec && cfg.max_iter > 0) {
+        // every pointer in it belongs to the context, so one graph serves all its solves
+        cudaGraph_t graph;
+        PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        cg_iterations<T>(c, m, modes, s);
+        PG_CUDA(cudaStreamEndCapture(s, &graph));
+        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (ie != cudaSuccess) {
+            exec = nullptr;
+            return cuda_fail(ie, "multigrid CG graph");
+        }
+    }
+    PG_CUDA(cudaStreamSynchronize(s));
+    for (int r = 0; r < m.R; ++r)
+        if (m.h_fl[kFlags * r + 3]) {
+            set_error("multigrid: singular coarsest operator");
+            return PG_ERR_BREAKDOWN;
+        }
+    auto all_done = [&](const int* f) {
+        for (int r = 0; r < m.R; ++r)
+            if (!f[kFlags * r]) return false;
+        return true;
+    };
+    int* slot[2] = {m.h_fl, m.h_fl + kFlags * m.R};
+    int launched = 0, last = 0;
+    if (!all_done(slot[0])) {
+        // the next graph is in flight while the host looks at the last one's flags
+        while (launched < cfg.max_iter) {
+            const int k = (launched / kChunk) & 1;
+            PG_CUDA(cudaGraphLaunch(exec, s));
+            cudaMemcpyAsync(slot[k], m.fl, fl_bytes, cudaMemcpyDeviceToHost, s);
+            cudaEventRecord(m.ev[k], s);
+            launched += kChunk;
+            last = k;
+            if (launched > kChunk) {
+                PG_CUDA(cudaEventSynchronize(m.ev[1 - k]));
+                if (all_done(slot[1 - k])) break;
+            }
+        }
+        PG_CUDA(cudaEventSynchronize(m.ev[last]));
+        if (last != 0) std::copy(slot[1], slot[1] + kFlags * m.R, slot[0]);
+    }
+    return PG_OK;
 }
 
 }  // namespace
@@ -1257,98 +852,70 @@ void mg_apply(Ctx& c, MgHierarchy& m, bool f32, cudaStream_t s, const double* r,
 int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s) {
     int rc = mg_build(c);
     if (rc != PG_OK) return rc;
-    c.mg->use_modes = modes;
-    if ((rc = mg_numeric(c, f32, s))) return rc;
-    int fl[8] = {};
-    cudaMemcpyAsync(fl, c.mg->fl, sizeof fl, cudaMemcpyDeviceToHost, s);
+    MgHierarchy& m = *c.mg;
+    if ((rc = mg_numeric(c, f32, modes, s))) return rc;
+    cudaMemcpyAsync(m.h_fl, m.fl, (size_t)kFlags * m.R * sizeof(int), cudaMemcpyDeviceToHost, s);
     PG_CUDA(cudaStreamSynchronize(s));
-    if (fl[3]) {
+    if (m.h_fl[3]) {
         set_error("multigrid: singular coarsest operator");
         return PG_ERR_BREAKDOWN;
     }
     return PG_OK;
 }
 
-void mg_precondition(Ctx& c, bool f32, cudaStream_t s, const double* r, double* z) {
-    mg_apply(c, *c.mg, f32, s, r, z, nullptr);
+void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z) {
+    MgHierarchy& m = *c.mg;
+    if (f32) {
+        k_mg_pre<float><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, r, m.Dinv0f, m.x0f);
+        mg_cycle<float>(c, m, modes, s, r, z, nullptr, false);
+    } else {
+        k_mg_pre<double><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, r, c.minv, m.x0);
+        mg_cycle<double>(c, m, modes, s, r, z, nullptr, false);
+    }
 }
 
 void mg_free(Ctx& c) {
     if (!c.mg) return;
-    for (void* p : c.mg->owned) cudaFree(p);
+    MgHierarchy& m = *c.mg;
+    for (cudaGraphExec_t g : m.graph)
+        if (g) cudaGraphExecDestroy(g);
+    for (cudaEvent_t e : m.ev)
+        if (e) cudaEventDestroy(e);
+    if (m.h_sc) cudaFreeHost(m.h_sc);
+    if (m.h_fl) cudaFreeHost(m.h_fl);
+    for (void* p : m.owned) cudaFree(p);
     delete c.mg;
     c.mg = nullptr;
+}
+
+int mg_cg(Ctx& c, const pg_solver_cfg& cfg, MgCgResult& res, cudaStream_t s) {
+    int rc = mg_build(c);
+    if (rc != PG_OK) return rc;
+    MgHierarchy& m = *c.mg;
+    const bool modes = cfg.inclusion_modes != 0 && m.n_inc > 0;
+    rc = cfg.precision == PG_PRECISION_MIXED ? cg_run<float>(c, m, modes, cfg, s) : cg_run<double>(c, m, modes, cfg, s);
+    res.scalars = m.h_sc;
+    res.flags = m.h_fl;
+    return rc;
 }
 
 // CG on mask(K) dx = mask(b) (b = c.b, dx = c.dx) preconditioned by one
 // V-cycle per iteration.  Fills st.iterations, st.rel_residual (true FP64
 // residual) and st.status.
 int mg_pcg_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStream_t s) {
-    int rc = mg_build(c);
-    if (rc != PG_OK) return rc;
-    MgHierarchy& m = *c.mg;
-    const bool f32 = cfg.precision == PG_PRECISION_MIXED;
-    m.use_modes = cfg.inclusion_modes != 0;
-    if ((rc = mg_numeric(c, f32, s))) return rc;
-    const int n = c.n_nodes, nd = c.n_dof;
-    cudaMemsetAsync(m.sc, 0, 8 * sizeof(double), s);
-    k_mgcg_start<<<nb(nd), kThreads, 0, s>>>(nd, c.fixed, c.b, c.r, c.dx, m.sc, c.red_active);
-    k_mgcg_tol<<<1, 1, 0, s>>>(m.sc, cfg.rtol * cfg.rtol);
-    // z = V(r), p = z, sc[2] = r.z
-    mg_apply(c, m, f32, s, c.r, c.z, nullptr);
-    k_copy<double><<<nb(nd), kThreads, 0, s>>>(nd, c.z, c.p);
-    k_mgcg_dot<<<nb(nd), kThreads, 0, s>>>(nd, c.r, c.z, m.sc + 2, m.fl, c.red_active);
-    int hf[8] = {};
-    double hs[8] = {};
-    cudaMemcpyAsync(hs, m.sc, sizeof hs, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(hf, m.fl, sizeof hf, cudaMemcpyDeviceToHost, s);
-    PG_CUDA(cudaStreamSynchronize(s));
-    if (hf[3]) {
-        set_error("multigrid: singular coarsest operator");
-        st.status = PG_ERR_BREAKDOWN;
+    MgCgResult res;
+    const int rc = mg_cg(c, cfg, res, s);
+    if (rc == PG_ERR_BREAKDOWN) {
+        st.status = rc;
         return PG_OK;
     }
-    const double bb = hs[3];
-    int iters = 0;
-    bool breakdown = false;
-    if (bb > 0.0 && cfg.max_iter > 0) {
-        constexpr int kChunk = 2;
-        cudaGraph_t graph;
-        PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < kChunk; ++it) {
-            k_mgcg_s1<<<1, 1, 0, s>>>(m.sc, m.fl);
-            k_mgcg_spmv<<<nb(kRowLanes * n), kThreads, 0, s>>>(n, c.row_ptr, c.col, c.K, c.p, c.fixed, c.q, m.sc, m.fl,
-                                                                 c.red_active);
-            k_mgcg_update<<<nb(nd), kThreads, 0, s>>>(nd, c.dx, c.r, c.p, c.q, m.sc, m.fl, c.red_active);
-            k_mgcg_s2<<<1, 1, 0, s>>>(m.sc, m.fl);
-            mg_apply(c, m, f32, s, c.r, c.z, m.fl);
-            k_mgcg_dot<<<nb(nd), kThreads, 0, s>>>(nd, c.r, c.z, m.sc + 2, m.fl, c.red_active);
-            k_mgcg_pupdate<<<nb(nd), kThreads, 0, s>>>(nd, c.z, c.p, m.sc, m.fl);
-        }
-        PG_CUDA(cudaStreamEndCapture(s, &graph));
-        cudaGraphExec_t exec = nullptr;
-        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) return cuda_fail(ie, "multigrid CG graph");
-        while (true) {
-            cudaGraphLaunch(exec, s);
-            cudaMemcpyAsync(hf, m.fl, sizeof hf, cudaMemcpyDeviceToHost, s);
-            const cudaError_t e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) {
-                cudaGraphExecDestroy(exec);
-                return cuda_fail(e, "multigrid CG");
-            }
-            iters = hf[2];
-            if (hf[0] || iters >= cfg.max_iter) break;
-        }
-        cudaGraphExecDestroy(exec);
-        breakdown = hf[1] != 0;
-    }
+    if (rc != PG_OK) return rc;
+    const double bb = res.scalars[5];
     const double rr = residual_into(c, s, c.dx, c.b, c.r);
-    st.iterations = iters;
+    st.iterations = res.flags[2];
     st.refinements = 0;
     st.rel_residual = bb > 0.0 ? std::sqrt(rr / bb) : 0.0;
-    if (breakdown)
+    if (res.flags[1])
         st.status = PG_ERR_BREAKDOWN;
     else
         st.status = rr <= 4.0 * cfg.rtol * cfg.rtol * bb ? PG_OK : PG_ERR_NOT_CONVERGED;

@@ -1,0 +1,1286 @@
+// Kernels of the multigrid V-cycle and of the CG around it (see pg_mg.cu).
+//
+// Every kernel covers all the RVEs of a context (one, or a batch): the work
+// is cut into tiles or row spans that lie in one RVE each, listed in a table,
+// and a CTA whose RVE is done returns at once.
+#pragma once
+
+#include "pg_solve_kernels.cuh"
+
+namespace pgb {
+namespace mg {
+
+constexpr double kOmegaReg = 0.6;     // level 0, regular nodes: P1 triangles, three nodes each, so
+                                      // lambda_max(D^-1 K_rr) <= 3 and 0.6 * 3 < 2
+constexpr double kOmega = 0.5;        // coarse levels: four nodes per cell, lambda_max(D^-1 A) <= 4
+constexpr int kChebSteps = 4;         // level 0, enrichment nodes
+constexpr double kChebRatio = 16.0;   // of the largest to the smallest eigenvalue the polynomial is made for
+constexpr int kChebCoef = 8;          // doubles per RVE: 1 / theta, then per later step its two factors
+constexpr int kScal = 8;              // doubles per RVE: r.z of even and odd iterations, -, -, tol^2, b.b, true r.r
+constexpr int kFlags = 4;             // ints per RVE: done, breakdown, iterations, coarsest operator singular
+constexpr int kSpanThreads = 256;
+constexpr int kCoarseCells = 4;       // an RVE is coarsened until both sides have at most this many cells
+constexpr int kCoarseMaxDof = 2 * (kCoarseCells + 1) * (kCoarseCells + 1);
+constexpr int kCoarseStride = kCoarseMaxDof * kCoarseMaxDof;
+
+// One RVE's grids on the two sides of a transfer: first node and cells per
+// side (cnx < 0: the RVE has no such coarse grid).
+struct Pair {
+    int foff, fnx, fny, coff, cnx, cny;
+};
+
+// Row spans of the level-0 kernels: a CTA's RVE and rows, and per RVE its CTAs and where its regular nodes end.
+struct Spans {
+    const int4* span;       // RVE, first row, end row
+    const int2* range;      // per RVE: first CTA, end CTA
+    const int* reg_end;     // per RVE
+};
+
+// ---------------------------------------------------------------------------
+// Grid transfer weights (grid index space).  Coarse index I sits at fine
+// index pos(I) = min(2I, nf); nf is the finer grid's cell count.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ int grid_pos(int I, int nf) { return 2 * I < nf ? 2 * I : nf; }
+
+__host__ __device__ __forceinline__ double grid_w(int g, int nf, int I) {
+    if ((g & 1) == 0) return (g >> 1) == I ? 1.0 : 0.0;
+    if (g == nf) return I == ((nf + 1) >> 1) ? 1.0 : 0.0;
+    return (I == ((g - 1) >> 1) || I == ((g + 1) >> 1)) ? 0.5 : 0.0;
+}
+
+// the coarse indices a fine index interpolates from (I0 = I1 where it is only one) and the weight of each
+template <typename T>
+__device__ __forceinline__ void parents(int g, int nf, int& I0, int& I1, T& w) {
+    if ((g & 1) == 0) {
+        I0 = I1 = g >> 1;
+        w = (T)0.5;
+    } else if (g == nf) {
+        I0 = I1 = (nf + 1) >> 1;
+        w = (T)0.5;
+    } else {
+        I0 = (g - 1) >> 1;
+        I1 = (g + 1) >> 1;
+        w = (T)0.5;
+    }
+}
+
+template <typename T>
+struct alignas(2 * sizeof(T)) Vec2 {
+    T x, y;
+};
+
+template <typename T>
+__device__ __forceinline__ Vec2<T> ld2(const T* p, size_t i) {
+    return reinterpret_cast<const Vec2<T>*>(p)[i];
+}
+template <typename T>
+__device__ __forceinline__ void st2(T* p, size_t i, T x, T y) {
+    Vec2<T> v;
+    v.x = x;
+    v.y = y;
+    reinterpret_cast<Vec2<T>*>(p)[i] = v;
+}
+
+// one 2x2 block of a stencil or a diagonal inverse (volatile: the compiler keeps a row's loads together, ahead
+// of the first use, instead of spacing them out to save registers)
+__device__ __forceinline__ void load4(const double* p, double& a, double& b, double& c, double& d) {
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
+}
+__device__ __forceinline__ void load4(const float* p, float& a, float& b, float& c, float& d) {
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "l"(p));
+}
+
+// block_sum, valid in every thread
+__device__ __forceinline__ double block_sum_all(double v) {
+    __shared__ double s_all;
+    v = block_sum(v);
+    if (threadIdx.x == 0) s_all = v;
+    __syncthreads();
+    v = s_all;
+    __syncthreads();
+    return v;
+}
+
+// The sum of one RVE's partials, in CTA order.  A reduction's kernel leaves
+// one partial per CTA and the next kernel's CTAs each add them up: the kernel
+// boundary orders the two, so no CTA waits on a fence and a ticket (which held
+// every CTA of the earlier fused sums: 33 us against 21 us for the same matrix
+// product without a sum at 512^2), and the result is the same bits on every run.
+__device__ __forceinline__ double range_sum(const double* __restrict__ part, int2 rg) {
+    double v = 0.0;
+    for (int k = rg.x + threadIdx.x; k < rg.y; k += blockDim.x) v += part[k];
+    return block_sum_all(v);
+}
+
+// Block row i of K times a vector, kRowLanes lanes per row (bsr_row_group);
+// get(j) gives the vector's pair at column node j (a Vec2<double>), and
+// columns with skip(j) are left out.
+template <typename MT, typename Get>
+__device__ __forceinline__ void row_lanes(int r0, int r1, int g, const int* __restrict__ col, const MT* __restrict__ K,
+                                          Get get, double& y0, double& y1) {
+    double a0 = 0.0, a1 = 0.0;
+    for (int base = r0 + g; base < r1; base += kRowLanes * kRowUnroll) {
+        int j[kRowUnroll];
+        double b[kRowUnroll][4];
+#pragma unroll
+        for (int u = 0; u < kRowUnroll; ++u) {
+            const int k = base + u * kRowLanes;
+            j[u] = -1;
+            b[u][0] = b[u][1] = b[u][2] = b[u][3] = 0.0;
+            if (k < r1) {
+                j[u] = __ldg(&col[k]);
+                load_block(K + 4 * (size_t)k, b[u][0], b[u][1], b[u][2], b[u][3]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kRowUnroll; ++u) {
+            if (j[u] >= 0) {
+                const Vec2<double> v = get(j[u]);
+                a0 += b[u][0] * v.x + b[u][1] * v.y;
+                a1 += b[u][2] * v.x + b[u][3] * v.y;
+            }
+        }
+    }
+    a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+    a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+    y0 = a0;
+    y1 = a1;
+}
+
+// ---------------------------------------------------------------------------
+// CG.  Iteration parity P; part_* hold one partial per CTA of the spans.
+// ---------------------------------------------------------------------------
+
+// x = 0, r = mask(b); partials of r.r; the first regular smoothing sweep x1 = omega D^-1 r
+template <typename T>
+__global__ void __launch_bounds__(kSpanThreads) k_cg_start(Spans sp, const uint8_t* __restrict__ fixed,
+                                                           const double* __restrict__ b, double* __restrict__ r,
+                                                           double* __restrict__ x, const T* __restrict__ Dinv,
+                                                           T* __restrict__ x1, double* part_rr) {
+    const int4 S = sp.span[blockIdx.x];
+    const int reg = sp.reg_end[S.x];
+    double acc = 0.0;
+    for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
+        const Vec2<double> v = ld2(b, i);
+        const double r0 = fixed[2 * i] ? 0.0 : v.x, r1 = fixed[2 * i + 1] ? 0.0 : v.y;
+        st2(r, i, r0, r1);
+        st2(x, i, 0.0, 0.0);
+        acc += r0 * r0 + r1 * r1;
+        if (i < reg) {
+            T m0, m1, m2, m3;
+            load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+            st2(x1, i, (T)kOmegaReg * (m0 * (T)r0 + m1 * (T)r1), (T)kOmegaReg * (m2 * (T)r0 + m3 * (T)r1));
+        }
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
+}
+
+// the first regular smoothing sweep alone (a V-cycle applied outside CG)
+template <typename T>
+__global__ void __launch_bounds__(kSpanThreads) k_mg_pre(Spans sp, const uint8_t* __restrict__ fixed,
+                                                         const double* __restrict__ r, const T* __restrict__ Dinv,
+                                                         T* __restrict__ x1) {
+    const int4 S = sp.span[blockIdx.x];
+    const int end = min(S.z, sp.reg_end[S.x]);
+    for (int i = S.y + threadIdx.x; i < end; i += kSpanThreads) {
+        const Vec2<double> v = ld2(r, i);
+        const T r0 = fixed[2 * i] ? (T)0 : (T)v.x, r1 = fixed[2 * i + 1] ? (T)0 : (T)v.y;
+        T m0, m1, m2, m3;
+        load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+        st2(x1, i, (T)kOmegaReg * (m0 * r0 + m1 * r1), (T)kOmegaReg * (m2 * r0 + m3 * r1));
+    }
+}
+
+// per RVE: tol^2 = rtol^2 b.b, and the r.z that the first iteration divides by
+__global__ inline void k_cg_tol(Spans sp, const double* part_rr, double rtol2, double* sc, int* fl) {
+    const int r = blockIdx.x;
+    const double bb = range_sum(part_rr, sp.range[r]);
+    if (threadIdx.x == 0) {
+        double* s = sc + kScal * r;
+        s[0] = 0.0;
+        s[1] = 1.0;
+        s[4] = rtol2 * bb;
+        s[5] = bb;
+        if (bb == 0.0) fl[kFlags * r] = 1;
+    }
+}
+
+// p = z + beta p_old, q = mask(K p), partials of p.q.  p is formed where it is
+// read: a row gathers z and p_old of its columns instead of waiting for a
+// kernel that writes p.  Bound by the reads of K (32 bytes a block).
+__global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* __restrict__ row_ptr,
+                                                          const int* __restrict__ col, const double* __restrict__ K,
+                                                          const uint8_t* __restrict__ fixed,
+                                                          const double* __restrict__ z, const double* __restrict__ p_old,
+                                                          double* __restrict__ p, double* __restrict__ q,
+                                                          const double* __restrict__ part_rz, double* sc, const int* fl,
+                                                          double* part_pq, int P) {
+    const int4 S = sp.span[blockIdx.x];
+    if (fl[kFlags * S.x]) return;
+    const int2 rg = sp.range[S.x];
+    const double rz = range_sum(part_rz, rg);
+    double* s = sc + kScal * S.x;
+    const double beta = rz / s[1 - P];
+    if ((int)blockIdx.x == rg.x && threadIdx.x == 0) s[P] = rz;
+    const int g = threadIdx.x % kRowLanes;
+    double acc = 0.0;
+    for (int base = S.y; base < S.z; base += kSpanThreads / kRowLanes) {
+        const int i = base + threadIdx.x / kRowLanes;
+        const bool valid = i < S.z;
+        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        double y0, y1;
+        row_lanes(r0, r1, g, col, K, [&](int j) {
+            Vec2<double> a = ld2(z, j);
+            const Vec2<double> b = ld2(p_old, j);
+            a.x += beta * b.x;
+            a.y += beta * b.y;
+            return a;
+        }, y0, y1);
+        if (valid && g == 0) {
+            const Vec2<double> a = ld2(z, i), b = ld2(p_old, i);
+            const double p0 = a.x + beta * b.x, p1 = a.y + beta * b.y;
+            if (fixed[2 * i]) y0 = 0.0;
+            if (fixed[2 * i + 1]) y1 = 0.0;
+            st2(p, i, p0, p1);
+            st2(q, i, y0, y1);
+            acc += p0 * y0 + p1 * y1;
+        }
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part_pq[blockIdx.x] = acc;
+}
+
+// x += alpha p, r -= alpha q, partials of r.r, and the first regular smoothing sweep of the coming V-cycle
+template <typename T>
+__global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* __restrict__ x, double* __restrict__ r,
+                                                            const double* __restrict__ p, const double* __restrict__ q,
+                                                            const T* __restrict__ Dinv, T* __restrict__ x1,
+                                                            const double* __restrict__ part_pq, const double* sc, int* fl,
+                                                            double* part_rr, int P) {
+    const int4 S = sp.span[blockIdx.x];
+    int* f = fl + kFlags * S.x;
+    if (f[0]) return;
+    const int2 rg = sp.range[S.x];
+    const double pq = range_sum(part_pq, rg);
+    const bool first = (int)blockIdx.x == rg.x && threadIdx.x == 0;
+    if (!(pq > 0.0)) {
+        if (first) {
+            f[1] = 1;
+            f[0] = 1;
+        }
+        return;
+    }
+    if (first) f[2] += 1;
+    const double alpha = sc[kScal * S.x + P] / pq;
+    const int reg = sp.reg_end[S.x];
+    double acc = 0.0;
+    for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
+        const Vec2<double> xv = ld2((const double*)x, i), rv = ld2((const double*)r, i), pv = ld2(p, i), qv = ld2(q, i);
+        const double r0 = rv.x - alpha * qv.x, r1 = rv.y - alpha * qv.y;
+        st2(x, i, xv.x + alpha * pv.x, xv.y + alpha * pv.y);
+        st2(r, i, r0, r1);
+        acc += r0 * r0 + r1 * r1;
+        if (i < reg) {
+            T m0, m1, m2, m3;
+            load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+            st2(x1, i, (T)kOmegaReg * (m0 * (T)r0 + m1 * (T)r1), (T)kOmegaReg * (m2 * (T)r0 + m3 * (T)r1));
+        }
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
+}
+
+// partials of a.b
+__global__ inline void __launch_bounds__(kSpanThreads) k_cg_dot(Spans sp, const double* __restrict__ a,
+                                                                const double* __restrict__ b, const int* fl, double* part) {
+    const int4 S = sp.span[blockIdx.x];
+    if (fl && fl[kFlags * S.x]) return;
+    double acc = 0.0;
+    for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
+        const Vec2<double> u = ld2(a, i), v = ld2(b, i);
+        acc += u.x * v.x + u.y * v.y;
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part[blockIdx.x] = acc;
+}
+
+// ---------------------------------------------------------------------------
+// Level 0
+// ---------------------------------------------------------------------------
+
+// The enrichment nodes' part of the smoother: x_e (+)= q(D^-1 K_ee) D^-1 r_e
+// with the Chebyshev polynomial q of degree kChebSteps - 1 for the spectrum
+// (bound / kChebRatio, bound), r_e the residual at x.  The enrichment block
+// couples each interface's nodes along a chain; damped block Jacobi sweeps of
+// the whole system resolve it slowly (72 CG iterations at 128^2, 154 with
+// softened cohesive interfaces; 53 and 84 with one regular sweep and this).
+//
+// A piece is up to kPieceRows enrichment nodes and those around it that its
+// steps need: step k reads the previous iterate one node further out, so the
+// nodes within kChebSteps - 1 - k steps are recomputed and the piece needs no
+// exchange with others (the result is the polynomial of the whole K_ee).
+// Four lanes per row; one latency chain per step is what bounds it.
+struct Piece {
+    int row0;                  // its first local row; then rows at distance 0, <= 1, <= 2, <= 3
+    int end[kChebSteps];
+    int rve, pad0, pad1;
+};
+constexpr int kPieceRows = 48;
+constexpr int kPieceThreads = 256;
+
+struct Enr {
+    const Piece* piece;
+    const int* node;           // per local row: its node
+    const int* eptr;           // per local row: its entries in K_ee
+    const int2* ent;           // block slot in K, local column
+    const double* coef;        // kChebCoef per RVE
+};
+
+template <typename T, bool POST>
+__global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                                          const T* __restrict__ K, const T* __restrict__ Dinv,
+                                                          const uint8_t* __restrict__ fixed, const int* __restrict__ reg_end,
+                                                          const double* __restrict__ b, const T* __restrict__ xin,
+                                                          T* __restrict__ xout, const int* fl) {
+    extern __shared__ __align__(16) unsigned char enr_smem[];
+    const Piece pc = e.piece[blockIdx.x];
+    if (fl && fl[kFlags * pc.rve]) return;
+    const int n = pc.end[kChebSteps - 1];
+    Vec2<T>* sx = reinterpret_cast<Vec2<T>*>(enr_smem);  // two copies of x, then d and r
+    Vec2<T>* sx2 = sx + n;
+    Vec2<T>* sd = sx2 + n;
+    Vec2<T>* sr = sd + n;
+    const double* cf = e.coef + kChebCoef * pc.rve;
+    const int reg = reg_end[pc.rve];
+    const int g = threadIdx.x % kRowLanes;
+    constexpr int kRows = kPieceThreads / kRowLanes;
+    const T ith = (T)cf[0];
+    for (int base = 0; base < n; base += kRows) {
+        const int l = base + threadIdx.x / kRowLanes;
+        const bool valid = l < n;
+        const int i = valid ? e.node[pc.row0 + l] : 0;
+        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        double y0, y1;
+        row_lanes(r0, r1, g, col, K, [&](int j) {
+            Vec2<double> v;
+            v.x = v.y = 0.0;
+            if (POST || j < reg) {  // before the coarse correction x_e is zero
+                const Vec2<T> a = ld2(xin, j);
+                v.x = (double)a.x;
+                v.y = (double)a.y;
+            }
+            return v;
+        }, y0, y1);
+        if (valid && g == 0) {
+            const Vec2<double> bv = ld2(b, i);
+            Vec2<T> rv, dv;
+            rv.x = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0;
+            rv.y = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
+            T m0, m1, m2, m3;
+            load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+            dv.x = ith * (m0 * rv.x + m1 * rv.y);
+            dv.y = ith * (m2 * rv.x + m3 * rv.y);
+            sr[l] = rv;
+            sd[l] = dv;
+            sx[l] = dv;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 1; k < kChebSteps; ++k) {
+        const T c1 = (T)cf[2 * k - 1], c2 = (T)cf[2 * k];
+        const int rows = pc.end[kChebSteps - 1 - k];
+        const Vec2<T>* xa = (k & 1) ? sx : sx2;
+        Vec2<T>* xb = (k & 1) ? sx2 : sx;
+        for (int base = 0; base < rows; base += kRows) {
+            const int l = base + threadIdx.x / kRowLanes;
+            const bool valid = l < rows;
+            const int e0 = valid ? e.eptr[pc.row0 + l] : 0, e1 = valid ? e.eptr[pc.row0 + l + 1] : 0;
+            double a0 = 0.0, a1 = 0.0;
+            for (int q = e0 + g; q < e1; q += kRowLanes) {
+                const int2 en = __ldg(&e.ent[q]);
+                double k0, k1, k2, k3;
+                load_block(K + 4 * (size_t)en.x, k0, k1, k2, k3);
+                const Vec2<T> v = xa[en.y];
+                a0 += k0 * (double)v.x + k1 * (double)v.y;
+                a1 += k2 * (double)v.x + k3 * (double)v.y;
+            }
+            a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+            a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+            if (valid && g == 0) {
+                const int i = e.node[pc.row0 + l];
+                const T r0 = fixed[2 * i] ? (T)0 : sr[l].x - (T)a0, r1 = fixed[2 * i + 1] ? (T)0 : sr[l].y - (T)a1;
+                T m0, m1, m2, m3;
+                load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+                Vec2<T> dv = sd[l], xv = xa[l];
+                dv.x = c1 * dv.x + c2 * (m0 * r0 + m1 * r1);
+                dv.y = c1 * dv.y + c2 * (m2 * r0 + m3 * r1);
+                xv.x += dv.x;
+                xv.y += dv.y;
+                sd[l] = dv;
+                xb[l] = xv;
+            }
+        }
+        __syncthreads();
+    }
+    const Vec2<T>* xl = ((kChebSteps - 1) & 1) ? sx2 : sx;
+    for (int l = threadIdx.x; l < pc.end[0]; l += kPieceThreads) {
+        const int i = e.node[pc.row0 + l];
+        Vec2<T> v = xl[l];
+        if (POST) {
+            const Vec2<T> o = ld2(xin, i);
+            v.x += o.x;
+            v.y += o.y;
+        }
+        st2(xout, i, v.x, v.y);
+    }
+}
+
+// Level-0 residual at the regular nodes of a tile of coarse nodes, restricted
+// to them: b_1 = mask(P^T (b - K x)).  Tiles of 8 x 8 coarse nodes need the
+// residual of 17 x 17 fine ones (13% computed twice), which saves writing it
+// and a launch.  The tile marked first in its RVE also ends the CG iteration:
+// it sets the RVE's done flag when the update's r.r has reached the tolerance.
+constexpr int kDownTile = 8;
+constexpr int kDownFine = 2 * kDownTile + 1;
+
+template <typename T>
+__device__ __forceinline__ void restrict_tile(const Vec2<T>* s, int I0, int J0, const Pair& p,
+                                              const uint8_t* __restrict__ fixed_c, T* __restrict__ bc) {
+    // s: the residual on fine nodes (2 I0 - 1 .., 2 J0 - 1 ..), kDownFine per side, 0 outside the grid
+    const int t = threadIdx.x;
+    if (t >= kDownTile * kDownTile) return;
+    const int I = I0 + t % kDownTile, J = J0 + t / kDownTile;
+    if (I > p.cnx || J > p.cny) return;
+    const int px = grid_pos(I, p.fnx) - (2 * I0 - 1), py = grid_pos(J, p.fny) - (2 * J0 - 1);
+    T s0 = 0, s1 = 0;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy) {
+        const int ly = py + dy;
+        if (ly < 0 || ly >= kDownFine) continue;
+        const T wy = (T)grid_w(2 * J0 - 1 + ly, p.fny, J);
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            const int lx = px + dx;
+            if (lx < 0 || lx >= kDownFine) continue;
+            const T w = wy * (T)grid_w(2 * I0 - 1 + lx, p.fnx, I);
+            if (w == (T)0) continue;
+            const Vec2<T> v = s[ly * kDownFine + lx];
+            s0 += w * v.x;
+            s1 += w * v.y;
+        }
+    }
+    const int a = p.coff + I + J * (p.cnx + 1);
+    st2(bc, a, fixed_c[2 * a] ? (T)0 : s0, fixed_c[2 * a + 1] ? (T)0 : s1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSpanThreads) k_mg_down0(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+                                                           const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                                           const T* __restrict__ K, const uint8_t* __restrict__ fixed,
+                                                           const double* __restrict__ b, const T* __restrict__ x,
+                                                           const uint8_t* __restrict__ fixed_c, T* __restrict__ bc,
+                                                           Spans sp, const double* __restrict__ part_rr, const double* sc,
+                                                           int* fl, int check) {
+    __shared__ Vec2<T> s[kDownFine * kDownFine];
+    const int4 tl = tile[blockIdx.x];
+    const Pair p = pair[tl.x];
+    if (fl && fl[kFlags * tl.x]) return;
+    if (check && tl.w) {
+        const double rr = range_sum(part_rr, sp.range[tl.x]);
+        if (threadIdx.x == 0 && rr <= sc[kScal * tl.x + 4]) fl[kFlags * tl.x] = 1;
+    }
+    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1, g = threadIdx.x % kRowLanes;
+    for (int base = 0; base < kDownFine * kDownFine; base += kSpanThreads / kRowLanes) {
+        const int l = base + threadIdx.x / kRowLanes;
+        const int gx = gx0 + l % kDownFine, gy = gy0 + l / kDownFine;
+        const bool in = l < kDownFine * kDownFine;
+        const bool valid = in && gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny;
+        const int i = valid ? p.foff + gx + gy * (p.fnx + 1) : 0;
+        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        double y0, y1;
+        row_lanes(r0, r1, g, col, K, [&](int j) {
+            const Vec2<T> a = ld2(x, j);
+            Vec2<double> v;
+            v.x = (double)a.x;
+            v.y = (double)a.y;
+            return v;
+        }, y0, y1);
+        if (in && g == 0) {
+            Vec2<T> rv;
+            rv.x = rv.y = 0;
+            if (valid) {
+                const Vec2<double> bv = ld2(b, i);
+                rv.x = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0;
+                rv.y = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
+            }
+            s[l] = rv;
+        }
+    }
+    __syncthreads();
+    restrict_tile(s, tl.y, tl.z, p, fixed_c, bc);
+}
+
+// The last smoothing sweep (regular nodes) and z: z_r = x_r + omega D^-1 (b - K x), z_e = x_e (already
+// smoothed, in xe); partials of b.z, which CG takes as r.z
+template <typename T>
+__global__ void __launch_bounds__(kSpanThreads) k_mg_post(Spans sp, const int* __restrict__ row_ptr,
+                                                          const int* __restrict__ col, const T* __restrict__ K,
+                                                          const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
+                                                          const double* __restrict__ b, const T* __restrict__ x,
+                                                          const T* __restrict__ xe, double* __restrict__ z, const int* fl,
+                                                          double* part_rz) {
+    const int4 S = sp.span[blockIdx.x];
+    if (fl && fl[kFlags * S.x]) return;
+    const int reg = sp.reg_end[S.x];
+    const int g = threadIdx.x % kRowLanes;
+    double acc = 0.0;
+    const int end = min(S.z, reg);
+    for (int base = S.y; base < end; base += kSpanThreads / kRowLanes) {
+        const int i = base + threadIdx.x / kRowLanes;
+        const bool valid = i < end;
+        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        double y0, y1;
+        row_lanes(r0, r1, g, col, K, [&](int j) {
+            const Vec2<T> a = ld2(j < reg ? x : xe, j);
+            Vec2<double> v;
+            v.x = (double)a.x;
+            v.y = (double)a.y;
+            return v;
+        }, y0, y1);
+        if (valid && g == 0) {
+            const Vec2<double> bv = ld2(b, i);
+            const Vec2<T> xv = ld2(x, i);
+            const T t0 = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0, t1 = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
+            T m0, m1, m2, m3;
+            load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+            const double z0 = (double)(xv.x + (T)kOmegaReg * (m0 * t0 + m1 * t1));
+            const double z1 = (double)(xv.y + (T)kOmegaReg * (m2 * t0 + m3 * t1));
+            st2(z, i, z0, z1);
+            acc += bv.x * z0 + bv.y * z1;
+        }
+    }
+    for (int i = max(S.y, reg) + threadIdx.x; i < S.z; i += kSpanThreads) {
+        const Vec2<double> bv = ld2(b, i);
+        const Vec2<T> xv = ld2(xe, i);
+        st2(z, i, (double)xv.x, (double)xv.y);
+        acc += bv.x * (double)xv.x + bv.y * (double)xv.y;
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part_rz[blockIdx.x] = acc;
+}
+
+// ---------------------------------------------------------------------------
+// Coarse levels: 9-point block stencils, two sweeps of damped block Jacobi
+// each way.  One launch per level and direction: a launch on these levels
+// costs 3-5 us whatever its size, and a level took seven.  A CTA recomputes
+// the nodes around its tile that the next phase reads (27% more sweeps)
+// instead of waiting for its neighbours.
+// ---------------------------------------------------------------------------
+constexpr int kTileThreads = 384;
+
+// (A x)(node i) from x staged in shared memory, at s[l] of a region W wide
+template <typename T, int W>
+__device__ __forceinline__ void stencil(const T* __restrict__ A, int i, const Vec2<T>* s, int l, T& y0, T& y1) {
+    T k[9][4];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) load4(A + 36 * (size_t)i + 4 * q, k[q][0], k[q][1], k[q][2], k[q][3]);
+    y0 = y1 = 0;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        const Vec2<T> v = s[l + (q / 3 - 1) * W + q % 3 - 1];
+        y0 += k[q][0] * v.x + k[q][1] * v.y;
+        y1 += k[q][2] * v.x + k[q][3] * v.y;
+    }
+}
+
+// x + omega D^-1 mask(b - y) at node i
+template <typename T>
+__device__ __forceinline__ Vec2<T> sweep_node(int i, const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
+                                              const T* __restrict__ b, Vec2<T> x, T y0, T y1) {
+    const Vec2<T> bv = ld2(b, i);
+    const T r0 = fixed[2 * i] ? (T)0 : bv.x - y0, r1 = fixed[2 * i + 1] ? (T)0 : bv.y - y1;
+    T m0, m1, m2, m3;
+    load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+    x.x += (T)kOmega * (m0 * r0 + m1 * r1);
+    x.y += (T)kOmega * (m2 * r0 + m3 * r1);
+    return x;
+}
+
+// pre-smoothing from zero, residual, restriction: x of the finer grid's nodes and b of the coarser one's
+template <typename T>
+__global__ void __launch_bounds__(kTileThreads, 2) k_mg_down(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+                                                          const T* __restrict__ A, const T* __restrict__ Dinv,
+                                                          const uint8_t* __restrict__ fixed, const T* __restrict__ b,
+                                                          T* __restrict__ x, const uint8_t* __restrict__ fixed_c,
+                                                          T* __restrict__ bc, const int* fl) {
+    constexpr int W0 = kDownFine, W1 = W0 + 2, W2 = W1 + 2;
+    __shared__ Vec2<T> s1[W2 * W2];  // after one sweep
+    __shared__ Vec2<T> s2[W1 * W1];  // after two
+    __shared__ Vec2<T> s0[W0 * W0];  // residual
+    const int4 tl = tile[blockIdx.x];
+    const Pair p = pair[tl.x];
+    if (fl && fl[kFlags * tl.x]) return;
+    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1;  // of the residual's region
+    for (int l = threadIdx.x; l < W2 * W2; l += kTileThreads) {
+        const int gx = gx0 - 2 + l % W2, gy = gy0 - 2 + l / W2;
+        Vec2<T> v;
+        v.x = v.y = 0;
+        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny)
+            v = sweep_node<T>(p.foff + gx + gy * (p.fnx + 1), Dinv, fixed, b, v, (T)0, (T)0);
+        s1[l] = v;
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < W1 * W1; l += kTileThreads) {
+        const int lx = l % W1, ly = l / W1, gx = gx0 - 1 + lx, gy = gy0 - 1 + ly;
+        Vec2<T> v;
+        v.x = v.y = 0;
+        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny) {
+            const int i = p.foff + gx + gy * (p.fnx + 1), c = (ly + 1) * W2 + lx + 1;
+            T y0, y1;
+            stencil<T, W2>(A, i, s1, c, y0, y1);
+            v = sweep_node<T>(i, Dinv, fixed, b, s1[c], y0, y1);
+            // a fine node belongs to the tile of its index / (2 kDownTile)
+            if (gx >= 2 * tl.y && gx < 2 * (tl.y + kDownTile) && gy >= 2 * tl.z && gy < 2 * (tl.z + kDownTile))
+                st2(x, i, v.x, v.y);
+        }
+        s2[l] = v;
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < W0 * W0; l += kTileThreads) {
+        const int lx = l % W0, ly = l / W0, gx = gx0 + lx, gy = gy0 + ly;
+        Vec2<T> v;
+        v.x = v.y = 0;
+        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny) {
+            const int i = p.foff + gx + gy * (p.fnx + 1);
+            T y0, y1;
+            stencil<T, W1>(A, i, s2, (ly + 1) * W1 + lx + 1, y0, y1);
+            const Vec2<T> bv = ld2(b, i);
+            if (!fixed[2 * i]) v.x = bv.x - y0;
+            if (!fixed[2 * i + 1]) v.y = bv.y - y1;
+        }
+        s0[l] = v;
+    }
+    __syncthreads();
+    restrict_tile(s0, tl.y, tl.z, p, fixed_c, bc);
+}
+
+// the coarse correction at fine node (gx, gy)
+template <typename T>
+__device__ __forceinline__ Vec2<T> interpolate(int gx, int gy, const Pair& p, const T* __restrict__ xc) {
+    int I0, I1, J0, J1;
+    T w;
+    parents<T>(gx, p.fnx, I0, I1, w);
+    parents<T>(gy, p.fny, J0, J1, w);
+    const int W = p.cnx + 1;
+    const Vec2<T> a = ld2(xc, p.coff + I0 + J0 * W), b = ld2(xc, p.coff + I1 + J0 * W);
+    const Vec2<T> c = ld2(xc, p.coff + I0 + J1 * W), d = ld2(xc, p.coff + I1 + J1 * W);
+    Vec2<T> v;
+    v.x = (T)0.25 * ((a.x + b.x) + (c.x + d.x));
+    v.y = (T)0.25 * ((a.y + b.y) + (c.y + d.y));
+    return v;
+}
+
+// Coarse correction and post-smoothing of one level (the coarse side of
+// `pair`, the fine side of `pairc`).  FINE: its result is interpolated
+// straight into level 0's x; otherwise it goes to xo.
+constexpr int kUpTile = 16;
+template <typename T, bool FINE>
+__global__ void __launch_bounds__(kTileThreads, 2) k_mg_up(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+                                                        const Pair* __restrict__ pairc, const T* __restrict__ A,
+                                                        const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
+                                                        const T* __restrict__ b, const T* __restrict__ x,
+                                                        const T* __restrict__ xc, T* __restrict__ xo,
+                                                        const uint8_t* __restrict__ fixed0, T* __restrict__ x0,
+                                                        const int* fl) {
+    constexpr int W0 = kUpTile + (FINE ? 1 : 0), W1 = W0 + 2, W2 = W1 + 2;
+    __shared__ Vec2<T> s2[W2 * W2];  // corrected
+    __shared__ Vec2<T> s1[W1 * W1];  // after one sweep
+    __shared__ Vec2<T> s0[W0 * W0];  // after two
+    const int4 tl = tile[blockIdx.x];
+    if (fl && fl[kFlags * tl.x]) return;
+    const Pair pf = pair[tl.x], p = pairc[tl.x];
+    const int off = p.foff, nx = p.fnx, ny = p.fny, gx0 = tl.y, gy0 = tl.z;
+    for (int l = threadIdx.x; l < W2 * W2; l += kTileThreads) {
+        const int gx = gx0 - 2 + l % W2, gy = gy0 - 2 + l / W2;
+        Vec2<T> v;
+        v.x = v.y = 0;
+        if (gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) {
+            const int i = off + gx + gy * (nx + 1);
+            v = ld2(x, i);
+            const Vec2<T> e = interpolate(gx, gy, p, xc);
+            if (!fixed[2 * i]) v.x += e.x;
+            if (!fixed[2 * i + 1]) v.y += e.y;
+        }
+        s2[l] = v;
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < W1 * W1; l += kTileThreads) {
+        const int lx = l % W1, ly = l / W1, gx = gx0 - 1 + lx, gy = gy0 - 1 + ly;
+        Vec2<T> v;
+        v.x = v.y = 0;
+        if (gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) {
+            const int i = off + gx + gy * (nx + 1), c = (ly + 1) * W2 + lx + 1;
+            T y0, y1;
+            stencil<T, W2>(A, i, s2, c, y0, y1);
+            v = sweep_node<T>(i, Dinv, fixed, b, s2[c], y0, y1);
+        }
+        s1[l] = v;
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < W0 * W0; l += kTileThreads) {
+        const int lx = l % W0, ly = l / W0, gx = gx0 + lx, gy = gy0 + ly;
+        if (gx > nx || gy > ny) continue;
+        const int i = off + gx + gy * (nx + 1), c = (ly + 1) * W1 + lx + 1;
+        T y0, y1;
+        stencil<T, W1>(A, i, s1, c, y0, y1);
+        const Vec2<T> v = sweep_node<T>(i, Dinv, fixed, b, s1[c], y0, y1);
+        if (FINE) s0[l] = v;
+        else st2(xo, i, v.x, v.y);
+    }
+    if (!FINE) return;
+    __syncthreads();
+    constexpr int F = 2 * kUpTile;
+    for (int l = threadIdx.x; l < F * F; l += kTileThreads) {
+        const int gx = 2 * gx0 + l % F, gy = 2 * gy0 + l / F;
+        if (gx > pf.fnx || gy > pf.fny) continue;
+        int I0, I1, J0, J1;
+        T w;
+        parents<T>(gx, pf.fnx, I0, I1, w);
+        parents<T>(gy, pf.fny, J0, J1, w);
+        I0 -= gx0;
+        I1 -= gx0;
+        J0 -= gy0;
+        J1 -= gy0;
+        const Vec2<T> a = s0[J0 * W0 + I0], bq = s0[J0 * W0 + I1], c = s0[J1 * W0 + I0], d = s0[J1 * W0 + I1];
+        const int i = pf.foff + gx + gy * (pf.fnx + 1);
+        Vec2<T> v = ld2((const T*)x0, i);
+        if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + bq.x) + (c.x + d.x));
+        if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + bq.y) + (c.y + d.y));
+        st2(x0, i, v.x, v.y);
+    }
+}
+
+// The levels of at most kBottomNodes nodes of one RVE, down to the coarsest
+// and back, in one CTA: operators and vectors staged in shared memory, value
+// by value (each of a block's four numbers of all nodes together, so that
+// the threads of a warp, one node each, read neighbouring words), a block
+// barrier between the phases.  Bound by the latency of its ~16 phases.
+constexpr int kBottomNodes = 300;
+constexpr int kBottomThreads = 512;
+constexpr int kBottomLevels = 8;
+
+struct Bottom {
+    int nlev, first;                       // levels, and the first one's number in the hierarchy
+    int nx[kBottomLevels], ny[kBottomLevels], off[kBottomLevels];
+    int foff, fnx, fny;                    // the grid its result is interpolated to when `first` is level 1
+    int pad;
+};
+
+template <typename T>
+struct BottomArrays {                      // of the hierarchy's levels, by number
+    const T* A[17];
+    const T* Dinv[17];
+    const uint8_t* fixed[17];
+    const T* b[17];
+    T* xo[17];
+};
+
+__host__ __device__ inline size_t bottom_level_bytes(int n, size_t t, bool coarsest) {
+    return ((coarsest ? 0 : (size_t)40 * n) + (size_t)8 * n) * t + (((size_t)2 * n + 15) & ~(size_t)15);
+}
+
+template <typename T>
+__device__ __forceinline__ void bottom_stencil(const T* sA, int n, int nx, int i, const Vec2<T>* x, T& y0, T& y1) {
+    y0 = y1 = 0;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        // out-of-grid blocks are zero; the neighbour's index is kept within the level
+        const int j = min(max(i + (q / 3 - 1) * (nx + 1) + q % 3 - 1, 0), n - 1);
+        const Vec2<T> v = x[j];
+        y0 += sA[(4 * q) * n + i] * v.x + sA[(4 * q + 1) * n + i] * v.y;
+        y1 += sA[(4 * q + 2) * n + i] * v.x + sA[(4 * q + 3) * n + i] * v.y;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const Bottom* __restrict__ bottoms, BottomArrays<T> ar,
+                                                              const double* __restrict__ XT,
+                                                              const uint8_t* __restrict__ fixed0, T* __restrict__ x0,
+                                                              const int* fl) {
+    extern __shared__ __align__(16) unsigned char bottom_smem[];
+    __shared__ Bottom B;
+    __shared__ double s_inv[kCoarseStride];
+    __shared__ double s_rhs[kCoarseMaxDof];
+    __shared__ double s_part[8][64];
+    const int r = blockIdx.x, tid = threadIdx.x;
+    if (tid < (int)(sizeof(Bottom) / sizeof(int)))
+        reinterpret_cast<int*>(&B)[tid] = reinterpret_cast<const int*>(&bottoms[r])[tid];
+    __syncthreads();
+    if (fl && fl[kFlags * r]) return;
+    T* sA[kBottomLevels];
+    Vec2<T>* sv[kBottomLevels];  // b, x, x', residual
+    uint8_t* sf[kBottomLevels];
+    unsigned char* at = bottom_smem;
+    for (int k = 0; k < B.nlev; ++k) {
+        const int n = (B.nx[k] + 1) * (B.ny[k] + 1), l = B.first + k;
+        const bool coarsest = k == B.nlev - 1;
+        sv[k] = reinterpret_cast<Vec2<T>*>(at);
+        sA[k] = reinterpret_cast<T*>(sv[k] + 4 * n);
+        sf[k] = reinterpret_cast<uint8_t*>(sA[k] + (coarsest ? 0 : 40 * n));
+        at += bottom_level_bytes(n, sizeof(T), coarsest);
+        if (!coarsest) {
+            const T* A = ar.A[l] + 36 * (size_t)B.off[k];
+            const T* D = ar.Dinv[l] + 4 * (size_t)B.off[k];
+            for (int q = tid; q < 36 * n; q += kBottomThreads) sA[k][(q % 36) * n + q / 36] = A[q];
+            for (int q = tid; q < 4 * n; q += kBottomThreads) sA[k][(36 + q % 4) * n + q / 4] = D[q];
+        }
+        const uint8_t* f = ar.fixed[l] + 2 * (size_t)B.off[k];
+        for (int q = tid; q < 2 * n; q += kBottomThreads) sf[k][q] = f[q];
+    }
+    const int kc = B.nlev - 1, nc = 2 * (B.nx[kc] + 1) * (B.ny[kc] + 1);
+    for (int q = tid; q < nc * nc; q += kBottomThreads) s_inv[q] = XT[(size_t)r * kCoarseStride + q];
+    {
+        const int n = (B.nx[0] + 1) * (B.ny[0] + 1);
+        for (int i = tid; i < n; i += kBottomThreads) sv[0][i] = ld2(ar.b[B.first], B.off[0] + i);
+    }
+    __syncthreads();
+    for (int k = 0; k < kc; ++k) {
+        const int nx = B.nx[k], ny = B.ny[k], n = (nx + 1) * (ny + 1);
+        const T* D = sA[k] + 36 * n;
+        Vec2<T>*b = sv[k], *x = b + n, *x2 = x + n, *rs = x2 + n;
+        auto sweep = [&](int i, Vec2<T> v, T y0, T y1) {
+            const T r0 = sf[k][2 * i] ? (T)0 : b[i].x - y0, r1 = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
+            v.x += (T)kOmega * (D[i] * r0 + D[n + i] * r1);
+            v.y += (T)kOmega * (D[2 * n + i] * r0 + D[3 * n + i] * r1);
+            return v;
+        };
+        for (int i = tid; i < n; i += kBottomThreads) {
+            Vec2<T> v;
+            v.x = v.y = 0;
+            x2[i] = sweep(i, v, (T)0, (T)0);
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kBottomThreads) {
+            T y0, y1;
+            bottom_stencil(sA[k], n, nx, i, x2, y0, y1);
+            x[i] = sweep(i, x2[i], y0, y1);
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kBottomThreads) {
+            T y0, y1;
+            bottom_stencil(sA[k], n, nx, i, x, y0, y1);
+            Vec2<T> v;
+            v.x = sf[k][2 * i] ? (T)0 : b[i].x - y0;
+            v.y = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
+            rs[i] = v;
+        }
+        __syncthreads();
+        const int cx = B.nx[k + 1], cn = (cx + 1) * (B.ny[k + 1] + 1);
+        for (int a = tid; a < cn; a += kBottomThreads) {
+            const int I = a % (cx + 1), J = a / (cx + 1);
+            const int px = grid_pos(I, nx), py = grid_pos(J, ny);
+            T s0 = 0, s1 = 0;
+#pragma unroll
+            for (int dy = -1; dy <= 1; ++dy) {
+                const int gy = py + dy;
+                if (gy < 0 || gy > ny) continue;
+                const T wy = (T)grid_w(gy, ny, J);
+#pragma unroll
+                for (int dx = -1; dx <= 1; ++dx) {
+                    const int gx = px + dx;
+                    if (gx < 0 || gx > nx) continue;
+                    const T w = wy * (T)grid_w(gx, nx, I);
+                    const Vec2<T> v = rs[gx + gy * (nx + 1)];
+                    s0 += w * v.x;
+                    s1 += w * v.y;
+                }
+            }
+            Vec2<T> v;
+            v.x = sf[k + 1][2 * a] ? (T)0 : s0;
+            v.y = sf[k + 1][2 * a + 1] ? (T)0 : s1;
+            sv[k + 1][a] = v;
+        }
+        __syncthreads();
+    }
+    // the coarsest grid: x = X b with the explicit masked inverse, eight threads per DOF
+    {
+        const int n = nc / 2;
+        const T* b = reinterpret_cast<const T*>(sv[kc]);
+        T* x = reinterpret_cast<T*>(sv[kc] + n);
+        for (int q = tid; q < nc; q += kBottomThreads) s_rhs[q] = sf[kc][q] ? 0.0 : (double)b[q];
+        __syncthreads();
+        const int q = tid % 64, part = tid / 64;
+        double acc = 0.0;
+        if (q < nc)
+            for (int j = part; j < nc; j += kBottomThreads / 64) acc += s_inv[j * nc + q] * s_rhs[j];
+        s_part[part][q] = acc;
+        __syncthreads();
+        if (tid < nc) {
+            double v = 0.0;
+#pragma unroll
+            for (int k = 0; k < kBottomThreads / 64; ++k) v += s_part[k][tid];
+            x[tid] = sf[kc][tid] ? (T)0 : (T)v;
+        }
+        __syncthreads();
+    }
+    for (int k = kc - 1; k >= 0; --k) {
+        const int nx = B.nx[k], ny = B.ny[k], n = (nx + 1) * (ny + 1);
+        const T* D = sA[k] + 36 * n;
+        Vec2<T>*b = sv[k], *x = b + n, *x2 = x + n;
+        const int cx = B.nx[k + 1], cn = (cx + 1) * (B.ny[k + 1] + 1);
+        const Vec2<T>* xc = sv[k + 1] + cn;
+        auto sweep = [&](int i, Vec2<T> v, T y0, T y1) {
+            const T r0 = sf[k][2 * i] ? (T)0 : b[i].x - y0, r1 = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
+            v.x += (T)kOmega * (D[i] * r0 + D[n + i] * r1);
+            v.y += (T)kOmega * (D[2 * n + i] * r0 + D[3 * n + i] * r1);
+            return v;
+        };
+        for (int i = tid; i < n; i += kBottomThreads) {
+            int I0, I1, J0, J1;
+            T w;
+            parents<T>(i % (nx + 1), nx, I0, I1, w);
+            parents<T>(i / (nx + 1), ny, J0, J1, w);
+            const Vec2<T> a = xc[I0 + J0 * (cx + 1)], bb = xc[I1 + J0 * (cx + 1)];
+            const Vec2<T> c = xc[I0 + J1 * (cx + 1)], d = xc[I1 + J1 * (cx + 1)];
+            if (!sf[k][2 * i]) x[i].x += (T)0.25 * ((a.x + bb.x) + (c.x + d.x));
+            if (!sf[k][2 * i + 1]) x[i].y += (T)0.25 * ((a.y + bb.y) + (c.y + d.y));
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kBottomThreads) {
+            T y0, y1;
+            bottom_stencil(sA[k], n, nx, i, x, y0, y1);
+            x2[i] = sweep(i, x[i], y0, y1);
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kBottomThreads) {
+            T y0, y1;
+            bottom_stencil(sA[k], n, nx, i, x2, y0, y1);
+            x[i] = sweep(i, x2[i], y0, y1);
+        }
+        __syncthreads();
+    }
+    const int nx = B.nx[0], n0 = (nx + 1) * (B.ny[0] + 1);
+    const Vec2<T>* x = sv[0] + n0;
+    if (B.first > 1) {
+        for (int i = tid; i < n0; i += kBottomThreads) st2(ar.xo[B.first], B.off[0] + i, x[i].x, x[i].y);
+        return;
+    }
+    const int nf = (B.fnx + 1) * (B.fny + 1);
+    for (int l = tid; l < nf; l += kBottomThreads) {
+        int I0, I1, J0, J1;
+        T w;
+        parents<T>(l % (B.fnx + 1), B.fnx, I0, I1, w);
+        parents<T>(l / (B.fnx + 1), B.fny, J0, J1, w);
+        const Vec2<T> a = x[I0 + J0 * (nx + 1)], b = x[I1 + J0 * (nx + 1)];
+        const Vec2<T> c = x[I0 + J1 * (nx + 1)], d = x[I1 + J1 * (nx + 1)];
+        const int i = B.foff + l;
+        Vec2<T> v = ld2((const T*)x0, i);
+        if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + b.x) + (c.x + d.x));
+        if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + b.y) + (c.y + d.y));
+        st2(x0, i, v.x, v.y);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Numeric set-up
+// ---------------------------------------------------------------------------
+
+// Coarse mask by injection: the coarse node takes the mask of the finer node at its position.
+__global__ inline void k_mg_inject_mask(int n, const int* __restrict__ node_rve, const Pair* __restrict__ pair,
+                                        const uint8_t* fixed_f, uint8_t* fixed_c) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= n) return;
+    const Pair p = pair[node_rve ? node_rve[a] : 0];
+    const int la = a - p.coff, I = la % (p.cnx + 1), J = la / (p.cnx + 1);
+    const int i = p.foff + grid_pos(I, p.fnx) + grid_pos(J, p.fny) * (p.fnx + 1);
+    fixed_c[2 * a] = fixed_f[2 * i];
+    fixed_c[2 * a + 1] = fixed_f[2 * i + 1];
+}
+
+// inverse of a node's masked diagonal block
+__device__ __forceinline__ void masked_inverse(const double b[4], bool f0, bool f1, double m[4]) {
+    m[0] = m[1] = m[2] = m[3] = 0.0;
+    if (!f0 && !f1) {
+        const double det = b[0] * b[3] - b[1] * b[2];
+        if (det != 0.0) {
+            m[0] = b[3] / det;
+            m[1] = -b[1] / det;
+            m[2] = -b[2] / det;
+            m[3] = b[0] / det;
+        }
+    } else {
+        m[0] = (f0 || b[0] == 0.0) ? 0.0 : 1.0 / b[0];
+        m[3] = (f1 || b[3] == 0.0) ? 0.0 : 1.0 / b[3];
+    }
+}
+
+// Galerkin product A_c = M_c P^T M A M P M_c of one level and its diagonal
+// inverses, in FP64, with FP32 copies on request.  One thread per child of a
+// coarse node (nine of them, those of zero weight idle): it spreads its
+// row's blocks over the coarse node's nine in its own column of shared
+// memory; then the nine columns are added in order.  (A thread per output
+// block that scans all the children's rows took 180 us at 512^2 and 31 us on
+// every level below, whatever its size.)
+constexpr int kGalNodes = 16;
+constexpr int kGalThreads = 9 * kGalNodes;
+
+template <bool FINE_BSR>
+__global__ void __launch_bounds__(kGalThreads) k_mg_galerkin(int n, const int* __restrict__ node_rve,
+                                                             const Pair* __restrict__ pair, const int* __restrict__ row_ptr,
+                                                             const int* __restrict__ col, const double* __restrict__ K,
+                                                             const double* __restrict__ A,
+                                                             const uint8_t* __restrict__ fixed_f,
+                                                             const uint8_t* __restrict__ fixed_c, double* __restrict__ Ac,
+                                                             float* __restrict__ Acf, double* __restrict__ Dinv,
+                                                             float* __restrict__ Dinvf) {
+    __shared__ double acc[36 * kGalThreads];
+    const int t = threadIdx.x, a0 = blockIdx.x * kGalNodes;
+#pragma unroll
+    for (int k = 0; k < 36; ++k) acc[k * kGalThreads + t] = 0.0;
+    const int a = a0 + t / 9;
+    if (a < n) {
+        const Pair p = pair[node_rve ? node_rve[a] : 0];
+        const int la = a - p.coff, Ia = la % (p.cnx + 1), Ja = la / (p.cnx + 1);
+        const int cx = grid_pos(Ia, p.fnx) + t % 9 % 3 - 1, cy = grid_pos(Ja, p.fny) + t % 9 / 3 - 1;
+        double wi = 0.0;
+        if (cx >= 0 && cx <= p.fnx && cy >= 0 && cy <= p.fny) wi = grid_w(cx, p.fnx, Ia) * grid_w(cy, p.fny, Ja);
+        if (wi != 0.0) {
+            const int W = p.fnx + 1, i = p.foff + cx + cy * W, nreg = W * (p.fny + 1);
+            const double w0 = fixed_f[2 * i] ? 0.0 : wi, w1 = fixed_f[2 * i + 1] ? 0.0 : wi;
+            auto spread = [&](int gx, int gy, int j, const double* blk) {
+                double b0, b1, b2, b3;
+                load_block(blk, b0, b1, b2, b3);
+                const bool f0 = fixed_f[2 * j], f1 = fixed_f[2 * j + 1];
+                b0 = f0 ? 0.0 : w0 * b0;
+                b1 = f1 ? 0.0 : w0 * b1;
+                b2 = f0 ? 0.0 : w1 * b2;
+                b3 = f1 ? 0.0 : w1 * b3;
+#pragma unroll
+                for (int oy = -1; oy <= 1; ++oy) {
+                    const double wy = grid_w(gy, p.fny, Ja + oy);
+                    if (wy == 0.0) continue;
+#pragma unroll
+                    for (int ox = -1; ox <= 1; ++ox) {
+                        const double w = wy * grid_w(gx, p.fnx, Ia + ox);
+                        if (w == 0.0) continue;
+                        double* o = acc + 4 * ((oy + 1) * 3 + ox + 1) * kGalThreads + t;
+                        o[0] += w * b0;
+                        o[kGalThreads] += w * b1;
+                        o[2 * kGalThreads] += w * b2;
+                        o[3 * kGalThreads] += w * b3;
+                    }
+                }
+            };
+            if (FINE_BSR) {
+                const int r1 = row_ptr[i + 1];
+                for (int q = row_ptr[i]; q < r1; ++q) {
+                    const int lj = col[q] - p.foff;
+                    if (lj < 0 || lj >= nreg) continue;  // enrichment columns: no coarse part
+                    const int gy = lj / W;
+                    spread(lj - gy * W, gy, p.foff + lj, K + 4 * (size_t)q);
+                }
+            } else {
+                for (int s = 0; s < 9; ++s) {
+                    const int gx = cx + s % 3 - 1, gy = cy + s / 3 - 1;
+                    if (gx < 0 || gx > p.fnx || gy < 0 || gy > p.fny) continue;
+                    spread(gx, gy, p.foff + gx + gy * W, A + 36 * (size_t)i + 4 * s);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int q = t; q < 36 * kGalNodes; q += kGalThreads) {
+        const int node = q / 36, k = q % 36, c = a0 + node;
+        if (c >= n) break;
+        double v = 0.0;
+#pragma unroll
+        for (int ch = 0; ch < 9; ++ch) v += acc[k * kGalThreads + node * 9 + ch];
+        const Pair p = pair[node_rve ? node_rve[c] : 0];
+        const int la = c - p.coff, Ib = la % (p.cnx + 1) + k / 4 % 3 - 1, Jb = la / (p.cnx + 1) + k / 12 - 1;
+        if (Ib < 0 || Ib > p.cnx || Jb < 0 || Jb > p.cny || fixed_c[2 * c + k % 4 / 2] ||
+            fixed_c[2 * (p.coff + Ib + Jb * (p.cnx + 1)) + k % 2])
+            v = 0.0;
+        Ac[36 * (size_t)c + k] = v;
+        if (Acf) Acf[36 * (size_t)c + k] = (float)v;
+    }
+    if (t < kGalNodes && a0 + t < n) {
+        const int c = a0 + t;
+        const bool f0 = fixed_c[2 * c], f1 = fixed_c[2 * c + 1];
+        double b[4], m[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            b[k] = 0.0;
+#pragma unroll
+            for (int ch = 0; ch < 9; ++ch) b[k] += acc[(16 + k) * kGalThreads + t * 9 + ch];
+        }
+        masked_inverse(b, f0, f1, m);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            Dinv[4 * (size_t)c + k] = m[k];
+            if (Dinvf) Dinvf[4 * (size_t)c + k] = (float)m[k];
+        }
+    }
+}
+
+__global__ inline void k_mg_to_f32(size_t n, const double* a, float* b) {
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < n) b[i] = (float)a[i];
+}
+
+// The coarsest operator of each RVE (one CTA each) inverted explicitly, by
+// Gauss-Jordan elimination with partial pivoting on [M | I]: fixed DOFs get
+// identity rows and columns, and zero rows and columns in the result.  Two
+// barriers per pivot; every warp finds the pivot for itself.  Stored
+// transposed (XT[j n + r] = X[r][j]).  Flag 3 = 1 on a zero pivot.
+struct Coarse {
+    const double* A;
+    const uint8_t* fixed;
+    int off, nx, ny, pad;
+};
+constexpr int kFactorThreads = 512;
+
+__global__ void __launch_bounds__(kFactorThreads) k_mg_coarse_inverse(const Coarse* __restrict__ cd, double* XT, int* fl) {
+    constexpr int kW = 2 * kCoarseMaxDof;
+    extern __shared__ __align__(16) unsigned char factor_smem[];
+    double(*M)[kW] = reinterpret_cast<double(*)[kW]>(factor_smem);
+    const Coarse C = cd[blockIdx.x];
+    const int nn = (C.nx + 1) * (C.ny + 1), n = 2 * nn, t = threadIdx.x, lane = t & 31;
+    const uint8_t* fixed = C.fixed + 2 * (size_t)C.off;
+    const double* A = C.A + 36 * (size_t)C.off;
+    for (int e = t; e < n * 2 * n; e += kFactorThreads) {
+        const int r = e / (2 * n), c = e % (2 * n);
+        M[r][c] = (c - n == r || (c == r && fixed[r])) ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    for (int e = t; e < 9 * nn; e += kFactorThreads) {
+        const int a = e / 9, o = e % 9, I = a % (C.nx + 1) + o % 3 - 1, J = a / (C.nx + 1) + o / 3 - 1;
+        if (I < 0 || I > C.nx || J < 0 || J > C.ny) continue;
+        const int b = I + J * (C.nx + 1);
+        for (int d = 0; d < 2; ++d)
+            for (int f = 0; f < 2; ++f)
+                if (!fixed[2 * a + d] && !fixed[2 * b + f]) M[2 * a + d][2 * b + f] = A[36 * (size_t)a + 4 * o + 2 * d + f];
+    }
+    __syncthreads();
+    // a thread keeps to one column: rows t / 128, t / 128 + 4, ...
+    constexpr int kCols = 128, kRowStep = kFactorThreads / kCols, kPer = (kCoarseMaxDof + kRowStep - 1) / kRowStep;
+    const int c = t % kCols, rg = t / kCols;
+    for (int k = 0; k < n; ++k) {
+        // the largest entry of column k at or below the diagonal (the first such row)
+        double best = -1.0;
+        int pr = k;
+        for (int r = k + lane; r < n; r += 32)
+            if (fabs(M[r][k]) > best) {
+                best = fabs(M[r][k]);
+                pr = r;
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int op = __shfl_xor_sync(0xffffffffu, pr, o);
+            if (ob > best || (ob == best && op < pr)) {
+                best = ob;
+                pr = op;
+            }
+        }
+        const double piv = M[pr][k];
+        if (piv == 0.0 && t == 0) fl[kFlags * blockIdx.x + 3] = 1;
+        double v[kPer];
+        if (c < 2 * n) {
+            const double pc = piv != 0.0 ? M[pr][c] / piv : 0.0;
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int r = rg + u * kRowStep;
+                const int src = r == pr ? k : r;  // rows k and pr change places
+                if (r < n) v[u] = r == k ? pc : M[src][c] - M[src][k] * pc;
+            }
+        }
+        __syncthreads();
+        if (c < 2 * n) {
+#pragma unroll
+            for (int u = 0; u < kPer; ++u)
+                if (rg + u * kRowStep < n) M[rg + u * kRowStep][c] = v[u];
+        }
+        __syncthreads();
+    }
+    double* X = XT + (size_t)blockIdx.x * kCoarseStride;
+    for (int e = t; e < n * n; e += kFactorThreads) {
+        const int j = e / n, r = e % n;
+        X[e] = (fixed[r] || fixed[j]) ? 0.0 : M[r][n + j];
+    }
+}
+
+// D^-1/2 of a symmetric positive definite block (false if it is not)
+__device__ __forceinline__ bool inv_sqrt(const double b[4], double s[4]) {
+    const double o = 0.5 * (b[1] + b[2]), det = b[0] * b[3] - o * o, tr = b[0] + b[3];
+    if (!(det > 0.0 && tr > 0.0 && isfinite(det))) return false;
+    // sqrt(B) = (B + q I) / t, q = sqrt(det), t = sqrt(tr + 2 q); its determinant is q
+    const double q = sqrt(det), w = 1.0 / (q * sqrt(tr + 2.0 * q));
+    s[0] = (b[3] + q) * w;
+    s[1] = s[2] = -o * w;
+    s[3] = (b[0] + q) * w;
+    return true;
+}
+
+// Per RVE the largest block row sum of the scaled enrichment block, max_i
+// sum_j ||D_i^-1/2 K_ij D_j^-1/2||_2 >= lambda_max(D^-1 K_ee) (2.2-2.4 on these
+// meshes, whose lambda_max is 1.9); infinite when a diagonal block is not
+// positive definite.  Kept as the bits of a non-negative double, so the
+// maximum does not depend on the order.
+__global__ inline void k_enr_bound(int n, const int* __restrict__ node, const int* __restrict__ rve,
+                                   const int* __restrict__ reg_end, const int* __restrict__ node_end,
+                                   const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                   const int* __restrict__ diag, const double* __restrict__ K, unsigned long long* bound) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int i = node[t], r = rve[t], lo = reg_end[r], hi = node_end[r];
+    double si[4], sum = 0.0;
+    bool ok = inv_sqrt(K + 4 * (size_t)diag[i], si);
+    for (int q = row_ptr[i]; ok && q < row_ptr[i + 1]; ++q) {
+        const int j = col[q];
+        if (j < lo || j >= hi) continue;
+        double sj[4];
+        ok = inv_sqrt(K + 4 * (size_t)diag[j], sj);
+        const double* b = K + 4 * (size_t)q;
+        const double u0 = si[0] * b[0] + si[1] * b[2], u1 = si[0] * b[1] + si[1] * b[3];
+        const double u2 = si[2] * b[0] + si[3] * b[2], u3 = si[2] * b[1] + si[3] * b[3];
+        const double x0 = u0 * sj[0] + u1 * sj[2], x1 = u0 * sj[1] + u1 * sj[3];
+        const double x2 = u2 * sj[0] + u3 * sj[2], x3 = u2 * sj[1] + u3 * sj[3];
+        const double f = x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3, d = x0 * x3 - x1 * x2;
+        sum += sqrt(0.5 * (f + sqrt(fmax(f * f - 4.0 * d * d, 0.0))));
+    }
+    if (!ok || !isfinite(sum)) sum = INFINITY;
+    atomicMax(&bound[r], (unsigned long long)__double_as_longlong(sum));
+}
+
+// The Chebyshev recurrence's factors (Saad, Iterative Methods for Sparse
+// Linear Systems, Alg. 12.1) for the spectrum (b / kChebRatio, b), b the bound
+// with a margin; one damped Jacobi sweep (1/2) where there is no bound.
+__global__ inline void k_enr_coef(int nr, const unsigned long long* bound, double* coef) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nr) return;
+    const double b = 1.01 * __longlong_as_double((long long)bound[r]);
+    double* c = coef + kChebCoef * r;
+    if (!(b > 0.0) || !isfinite(b)) {
+        c[0] = 0.5;
+        for (int k = 1; k < kChebCoef; ++k) c[k] = 0.0;
+        return;
+    }
+    const double theta = 0.5 * (b + b / kChebRatio), delta = 0.5 * (b - b / kChebRatio), sigma = theta / delta;
+    double rho = 1.0 / sigma;
+    c[0] = 1.0 / theta;
+    for (int k = 1; k < kChebSteps; ++k) {
+        const double rho1 = 1.0 / (2.0 * sigma - rho);
+        c[2 * k - 1] = rho1 * rho;
+        c[2 * k] = 2.0 * rho1 / delta;
+        rho = rho1;
+    }
+}
+
+}  // namespace mg
+}  // namespace pgb

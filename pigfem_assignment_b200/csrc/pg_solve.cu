@@ -120,7 +120,7 @@ int gmres_solve(Ctx& c, const pg_solver_cfg& cfg, double rtol, int max_iter, pg_
             double* w = c.V + (size_t)(j + 1) * nd;
             // w = K M^-1 v_j
             if (cfg.precond == PG_PREC_MG)
-                mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, s, vj, c.z);
+                mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, vj, c.z);
             else
                 k_apply_prec_vec<<<nblk(n), kThreads, 0, s>>>(n, c.minv, vj, c.z);
             k_spmv_plain<double, double><<<nblk(n), kThreads, 0, s>>>(n, c.row_ptr, c.col, c.K, c.z, c.fixed, w);
@@ -169,7 +169,7 @@ int gmres_solve(Ctx& c, const pg_solver_cfg& cfg, double rtol, int max_iter, pg_
         k_fill<double><<<nblk(nd), kThreads, 0, s>>>(nd, c.q, 0.0);
         k_multi_axpy_add<<<nblk(nd), kThreads, 0, s>>>(nd, j, c.V, c.hbuf, c.q);
         if (cfg.precond == PG_PREC_MG)
-            mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, s, c.q, c.z);
+            mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, c.q, c.z);
         else
             k_apply_prec_vec<<<nblk(n), kThreads, 0, s>>>(n, c.minv, c.q, c.z);
         k_axpy_free<double><<<nblk(nd), kThreads, 0, s>>>(nd, c.fixed, c.dx, c.z, 1.0);
@@ -296,6 +296,10 @@ int krylov_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStrea
     }
     if (cfg.precond == PG_PREC_MG) {
         // one multigrid V-cycle per iteration (FP32 cycle under PG_PRECISION_MIXED)
+        if (c.hm.spec.nx < 1 || c.hm.spec.ny < 1) {  // (a batch is solved through pg_batch_solve)
+            set_error("multigrid: mesh without a structured background grid");
+            return PG_ERR_ARG;
+        }
         if (cfg.krylov == PG_KRYLOV_GMRES) {
             const int rc = mg_prepare(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s);
             if (rc == PG_ERR_BREAKDOWN) { st.status = rc; return PG_OK; }
