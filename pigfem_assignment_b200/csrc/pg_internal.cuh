@@ -344,6 +344,8 @@ int krylov_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStrea
 // out = mask(b - K x) (b nullable: 0); returns ||out||^2
 double residual_into(Ctx& c, cudaStream_t s, const double* x, const double* b, double* out);
 // geometric multigrid (pg_mg.cu)
+int mg_build(Ctx& c);                                    // the hierarchies' structure, once per context
+void mg_depths(const Ctx& c, std::vector<int>& depth);   // coarse levels per RVE
 int mg_pcg_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStream_t s);
 int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s);
 void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z);

@@ -85,6 +85,7 @@ struct Level {
 struct MgHierarchy {
     int R = 0;                           // RVEs
     int nlev = 0;                        // coarse levels 1..nlev
+    std::vector<int> depth;              // and those of each RVE
     Level L[kMaxLevels + 1];
     Spans spans{};
     int n_cta = 0;
@@ -439,6 +440,7 @@ int build_hierarchy(Ctx& c) {
     MgHierarchy& m = *mp;
     m.R = R;
     m.nlev = nlev;
+    for (const auto& d : dims) m.depth.push_back((int)d.size() - 1);
     Arena ar;
     // the bottom of each RVE's cycle: its levels of at most kBottomNodes nodes
     std::vector<Bottom> bottom(R);
@@ -624,13 +626,6 @@ int build_hierarchy(Ctx& c) {
     PG_CUDA(cudaGetLastError());
     PG_CUDA(cudaStreamSynchronize(s));
     return R == 1 ? modes_build(c, m) : PG_OK;
-}
-
-int mg_build(Ctx& c) {
-    if (c.mg) return PG_OK;
-    const int rc = build_hierarchy(c);
-    if (rc != PG_OK) mg_free(c);
-    return rc;
 }
 
 // the FP32 cycle's arrays, on its first use
@@ -848,6 +843,15 @@ int cg_run(Ctx& c, MgHierarchy& m, bool modes, const pg_solver_cfg& cfg, cudaStr
 }
 
 }  // namespace
+
+int mg_build(Ctx& c) {
+    if (c.mg) return PG_OK;
+    const int rc = build_hierarchy(c);
+    if (rc != PG_OK) mg_free(c);
+    return rc;
+}
+
+void mg_depths(const Ctx& c, std::vector<int>& depth) { depth = c.mg->depth; }
 
 int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s) {
     int rc = mg_build(c);

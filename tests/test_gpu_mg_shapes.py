@@ -28,7 +28,7 @@ def test_mg_solve_matches_direct_solve(nx, ny, inclusions, precision):
     e = prob.mesh.export()
     prob.get_solver().configure(precision=precision, precond=_lib.PG_PREC_MG, rtol=1e-12)
     st = prob.solve_problem()
-    assert st.status == 0 and st.iterations <= 150, (st.status, st.iterations)
+    assert st.status == 0, st.status
     Ko, _, _ = oracle.from_product(e, pb.template_table(), rve).assemble()
     uo = oracle.solve_linear(Ko, e["fixed"], e["ubar"])
     u = prob.get_solution()
