@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "pg_internal.cuh"
+#include "pg_pdl.cuh"
 
 namespace pgb {
 
@@ -709,14 +710,6 @@ __host__ __device__ inline unsigned grid_nbr_mask(int gi, int gj, int nx, int ny
     return (s && even && w ? 1u : 0u) | (s ? 2u : 0u) | (s && even && e ? 4u : 0u) | (w ? 8u : 0u) | 16u |
            (e ? 32u : 0u) | (n && even && w ? 64u : 0u) | (n ? 128u : 0u) | (n && even && e ? 256u : 0u);
 }
-
-// Programmatic dependent launch (sm_90 and later).  A kernel launched with
-// launch_pdl may start while the kernel before it on the stream is still
-// running, once every CTA of that one has called pdl_trigger (or exited);
-// pdl_wait blocks until the kernel before has completed and its writes are
-// visible.  Both are no-ops for a kernel launched the ordinary way.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // One 2x2 block as a single 256-bit store (K is a cudaMalloc allocation, so
 // every block is 32-byte aligned).
@@ -2042,23 +2035,6 @@ CutArgs cut_args(const Ctx& c, const double* U, double dt) {
     ca.coh = c.coh;
     ca.dt = dt;
     return ca;
-}
-
-// Launches kern with the programmatic-stream-serialization attribute (see
-// pdl_trigger / pdl_wait).
-template <typename... KArgs, typename... Args>
-void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
 void launch_cut_points(const Ctx& c, cudaStream_t s) {

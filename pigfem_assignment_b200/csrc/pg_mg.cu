@@ -98,7 +98,6 @@ struct MgHierarchy {
     double* coef = nullptr;
     // the bottom of every RVE's cycle
     Bottom* bottom = nullptr;
-    size_t bottom_smem[2] = {0, 0};      // FP64, FP32
     Coarse* coarse = nullptr;
     double* XT = nullptr;
     // level-0 vectors of the cycle: x, and the enrichment nodes' after post-smoothing
@@ -359,9 +358,29 @@ struct RvePieces {
 
 void build_pieces(const HostMesh& hm, int rve, int lo, int hi, RvePieces& out) {
     const int n = hi - lo;
-    std::vector<int> order, stack, local(n, -1);
+    std::vector<int> order, stack, local(n, -1), rep(n);
     std::vector<char> seen(n, 0);
     order.reserve(n);
+    // a node and its mirror across a cohesive interface (the same place) follow each other in the order, so that
+    // a core spans the interface instead of one side of it (108 against 60 local rows)
+    for (int v = 0; v < n; ++v) {
+        rep[v] = v;
+        for (int q = hm.row_ptr[lo + v]; q < hm.row_ptr[lo + v + 1]; ++q) {
+            const int j = hm.col[q];
+            if (j >= lo && j < lo + v && hm.x[j] == hm.x[lo + v] && hm.y[j] == hm.y[lo + v]) {
+                rep[v] = rep[j - lo];
+                break;
+            }
+        }
+    }
+    auto visit = [&](int v) {
+        seen[v] = 1;
+        order.push_back(v);
+        for (int q = hm.row_ptr[lo + v + 1] - 1; q >= hm.row_ptr[lo + v]; --q) {
+            const int j = hm.col[q] - lo;
+            if (j >= 0 && j < n && !seen[j] && rep[j] != rep[v]) stack.push_back(j);
+        }
+    };
     for (int s = 0; s < n; ++s) {
         if (seen[s]) continue;
         stack.push_back(s);
@@ -369,11 +388,10 @@ void build_pieces(const HostMesh& hm, int rve, int lo, int hi, RvePieces& out) {
             const int v = stack.back();
             stack.pop_back();
             if (seen[v]) continue;
-            seen[v] = 1;
-            order.push_back(v);
-            for (int q = hm.row_ptr[lo + v + 1] - 1; q >= hm.row_ptr[lo + v]; --q) {
-                const int j = hm.col[q];
-                if (j >= lo && j < hi && !seen[j - lo]) stack.push_back(j - lo);
+            visit(v);
+            for (int q = hm.row_ptr[lo + v]; q < hm.row_ptr[lo + v + 1]; ++q) {
+                const int j = hm.col[q] - lo;
+                if (j >= 0 && j < n && !seen[j] && rep[j] == rep[v]) visit(j);
             }
         }
     }
@@ -442,23 +460,20 @@ int build_hierarchy(Ctx& c) {
     m.nlev = nlev;
     for (const auto& d : dims) m.depth.push_back((int)d.size() - 1);
     Arena ar;
-    // the bottom of each RVE's cycle: its levels of at most kBottomNodes nodes
+    // the bottom of each RVE's cycle: its levels of at most kBottomNodes nodes, as many as its threads own
     std::vector<Bottom> bottom(R);
     std::vector<int> kb(R);
-    size_t smem[2] = {0, 0};
     for (int r = 0; r < R; ++r) {
         const int depth = (int)dims[r].size() - 1;
-        int k = depth;
-        while (k > 1 && depth - k + 1 < kBottomLevels && nodes(r, k - 1) <= kBottomNodes) --k;
-        kb[r] = k;
-        for (int t = 0; t < 2; ++t) {
-            size_t bytes = 0;
-            for (int l = k; l <= depth; ++l) bytes += bottom_level_bytes(nodes(r, l), t ? sizeof(float) : sizeof(double), l == depth);
-            smem[t] = std::max(smem[t], bytes);
+        int k = depth, threads = 0, vec = nodes(r, depth);
+        while (k > 1 && depth - k + 1 < kBottomLevels && nodes(r, k - 1) <= kBottomNodes) {
+            threads += (nodes(r, k - 1) + 31) / 32 * 32;
+            vec += nodes(r, k - 1);
+            if (threads > kBottomThreads || vec > kBottomVec) break;
+            --k;
         }
+        kb[r] = k;
     }
-    m.bottom_smem[0] = smem[0];
-    m.bottom_smem[1] = smem[1];
     // levels: offsets, transfers, tiles
     std::vector<std::vector<int>> off(nlev + 1, std::vector<int>(R, 0));
     std::vector<std::vector<Pair>> pairs(nlev + 1);
@@ -503,6 +518,9 @@ int build_hierarchy(Ctx& c) {
             B.nx[k] = dims[r][kb[r] + k].first;
             B.ny[k] = dims[r][kb[r] + k].second;
             B.off[k] = off[kb[r] + k][r];
+            const int n = nodes(r, kb[r] + k);
+            if (k + 1 < B.nlev) B.thread[k + 1] = B.thread[k] + (n + 31) / 32 * 32;
+            if (k + 1 < B.nlev) B.vec[k + 1] = B.vec[k] + n;
         }
         B.foff = off[kb[r] - 1][r];
         B.fnx = dims[r][kb[r] - 1].first;
@@ -604,13 +622,14 @@ int build_hierarchy(Ctx& c) {
     for (cudaEvent_t& e : m.ev) PG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // kernels whose shared memory exceeds the default (the attribute belongs to the device, so the largest any
     // hierarchy on it may ask for)
-    constexpr int kSmemMax = 190 * 1024;
-    if (smem[0] > kSmemMax || (size_t)m.max_piece * 8 * sizeof(double) > 100 * 1024) {
-        set_error("multigrid: level too large for shared memory");
+    if ((size_t)m.max_piece * 8 * sizeof(double) > 100 * 1024) {
+        set_error("multigrid: enrichment piece too large for shared memory");
         return PG_ERR_LIMIT;
     }
-    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
-    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 4 * kBottomStride * (int)sizeof(Vec2<double>)));
+    PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 4 * kBottomStride * (int)sizeof(Vec2<float>)));
     for (auto k : {k_mg_enr<double, false>, k_mg_enr<double, true>})
         PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     for (auto k : {k_mg_enr<float, false>, k_mg_enr<float, true>})
@@ -698,7 +717,6 @@ struct Cycle<double> {
     static double* x(const MgHierarchy& m) { return m.x0; }
     static double* xe(const MgHierarchy& m) { return m.x0e; }
     static LevelArrays<double>& lev(Level& L) { return L.d; }
-    static size_t bottom_smem(const MgHierarchy& m) { return m.bottom_smem[0]; }
 };
 template <>
 struct Cycle<float> {
@@ -707,7 +725,6 @@ struct Cycle<float> {
     static float* x(const MgHierarchy& m) { return m.x0f; }
     static float* xe(const MgHierarchy& m) { return m.x0ef; }
     static LevelArrays<float>& lev(Level& L) { return L.f; }
-    static size_t bottom_smem(const MgHierarchy& m) { return m.bottom_smem[1]; }
 };
 
 // The V-cycle after its first sweep (which CG's update has formed): z = V(r)
@@ -720,15 +737,15 @@ void mg_cycle(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s, const double* 
     T *x0 = C::x(m), *xe = C::xe(m);
     const size_t esm = (size_t)m.max_piece * 4 * sizeof(Vec2<T>);
     if (m.n_pieces > 0)
-        k_mg_enr<T, false><<<m.n_pieces, kPieceThreads, esm, s>>>(m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
+        launch_pdl(k_mg_enr<T, false>, m.n_pieces, kPieceThreads, esm, s, m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
                                                                   x0, x0, fl);
-    k_mg_down0<T><<<m.L[1].down.n, kSpanThreads, 0, s>>>(m.L[1].down.tile, m.L[1].pair, c.row_ptr, c.col, K, c.fixed, r, x0,
+    launch_pdl(k_mg_down0<T>, m.L[1].down.n, kDown0Threads, 0, s, m.L[1].down.tile, m.L[1].pair, c.row_ptr, c.col, K, c.fixed, r, x0,
                                                          m.L[1].fixed, C::lev(m.L[1]).b, m.spans, m.part_rr, m.sc, fl,
                                                          check ? 1 : 0);
     for (int l = 2; l <= m.nlev && m.L[l].down.n > 0; ++l) {
         Level &F = m.L[l - 1], &L = m.L[l];
         LevelArrays<T>& f = C::lev(F);
-        k_mg_down<T><<<L.down.n, kTileThreads, 0, s>>>(L.down.tile, L.pair, f.A, f.Dinv, F.fixed, f.b, f.x, L.fixed,
+        launch_pdl(k_mg_down<T>, L.down.n, kTileThreads, 0, s, L.down.tile, L.pair, f.A, f.Dinv, f.b, f.x, L.fixed,
                                                        C::lev(L).b, fl);
     }
     BottomArrays<T> ba{};
@@ -740,29 +757,29 @@ void mg_cycle(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s, const double* 
         ba.b[l] = v.b;
         ba.xo[l] = v.xo;
     }
-    k_mg_bottom<T><<<m.R, kBottomThreads, C::bottom_smem(m), s>>>(m.bottom, ba, m.XT, c.fixed, x0, fl);
+    launch_pdl(k_mg_bottom<T>, m.R, kBottomThreads, 4 * kBottomStride * sizeof(Vec2<T>), s, m.bottom, ba, m.XT, c.fixed, x0, fl);
     for (int l = m.nlev - 1; l >= 1; --l) {
         Level& L = m.L[l];
         if (L.up.n == 0) continue;
         LevelArrays<T>& v = C::lev(L);
         const T* xc = C::lev(m.L[l + 1]).xo;
         if (l == 1)
-            k_mg_up<T, true><<<L.up.n, kTileThreads, 0, s>>>(L.up.tile, L.pair, m.L[2].pair, v.A, v.Dinv, L.fixed, v.b, v.x, xc,
+            launch_pdl(k_mg_up<T, true>, L.up.n, kTileThreads, 0, s, L.up.tile, L.pair, m.L[2].pair, v.A, v.Dinv, L.fixed, v.b, v.x, xc,
                                                              nullptr, c.fixed, x0, fl);
         else
-            k_mg_up<T, false><<<L.up.n, kTileThreads, 0, s>>>(L.up.tile, L.pair, m.L[l + 1].pair, v.A, v.Dinv, L.fixed, v.b,
+            launch_pdl(k_mg_up<T, false>, L.up.n, kTileThreads, 0, s, L.up.tile, L.pair, m.L[l + 1].pair, v.A, v.Dinv, L.fixed, v.b,
                                                               v.x, xc, v.xo, nullptr, nullptr, fl);
     }
     if (m.n_pieces > 0)
-        k_mg_enr<T, true><<<m.n_pieces, kPieceThreads, esm, s>>>(m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
+        launch_pdl(k_mg_enr<T, true>, m.n_pieces, kPieceThreads, esm, s, m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
                                                                  x0, xe, fl);
-    k_mg_post<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.row_ptr, c.col, K, D0, c.fixed, r, x0, xe, z, fl, m.part_rz);
+    launch_pdl(k_mg_post<T>, m.n_cta, kSpanThreads, 0, s, m.spans, c.row_ptr, c.col, K, D0, c.fixed, r, x0, xe, z, fl, m.part_rz);
     if (m.n_inc > 0 && modes) {
         const int n = c.n_nodes;
         k_modes_zero<<<nb(3 * m.n_inc), kThreads, 0, s>>>(3 * m.n_inc, m.w, fl);
         k_modes_dot<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, r, m.w, fl);
         k_modes_add<<<nb(n), kThreads, 0, s>>>(n, m.z_inc, m.zval, c.fixed, m.Einv, m.w, z, fl);
-        k_cg_dot<<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, r, z, fl, m.part_rz);
+        launch_pdl(k_cg_dot, m.n_cta, kSpanThreads, 0, s, m.spans, r, z, fl, m.part_rz);
     }
 }
 
@@ -772,9 +789,9 @@ void cg_iterations(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s) {
     double* pb[2] = {c.p, c.xi};
     for (int it = 0; it < kChunk; ++it) {
         const int P = it & 1;
-        k_cg_spmv<<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.row_ptr, c.col, c.K, c.fixed, c.z, pb[1 - P], pb[P], c.q,
+        launch_pdl(k_cg_spmv, m.n_cta, kSpanThreads, 0, s, m.spans, c.row_ptr, c.col, c.K, c.fixed, c.z, pb[1 - P], pb[P], c.q,
                                                    m.part_rz, m.sc, m.fl, m.part_pq, P);
-        k_cg_update<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.dx, c.r, pb[P], c.q, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
+        launch_pdl(k_cg_update<T>, m.n_cta, kSpanThreads, 0, s, m.spans, c.dx, c.r, pb[P], c.q, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
                                                         m.part_pq, m.sc, m.fl, m.part_rr, P);
         mg_cycle<T>(c, m, modes, s, c.r, c.z, m.fl, true);
     }
@@ -788,9 +805,9 @@ int cg_run(Ctx& c, MgHierarchy& m, bool modes, const pg_solver_cfg& cfg, cudaStr
     const size_t fl_bytes = (size_t)kFlags * m.R * sizeof(int);
     int rc = mg_numeric(c, f32, modes, s);
     if (rc) return rc;
-    k_cg_start<T><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, c.b, c.r, c.dx, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
+    launch_pdl(k_cg_start<T>, m.n_cta, kSpanThreads, 0, s, m.spans, c.fixed, c.b, c.r, c.dx, Cycle<T>::Dinv(c, m), Cycle<T>::x(m),
                                                    m.part_rr);
-    k_cg_tol<<<m.R, kSpanThreads, 0, s>>>(m.spans, m.part_rr, cfg.rtol * cfg.rtol, m.sc, m.fl);
+    launch_pdl(k_cg_tol, m.R, kSpanThreads, 0, s, m.spans, m.part_rr, cfg.rtol * cfg.rtol, m.sc, m.fl);
     cudaMemsetAsync(c.xi, 0, (size_t)c.n_dof * sizeof(double), s);  // p before the first iteration
     mg_cycle<T>(c, m, modes, s, c.r, c.z, nullptr, false);
     cudaMemcpyAsync(m.h_sc, m.sc, (size_t)kScal * m.R * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -870,10 +887,10 @@ int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s) {
 void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z) {
     MgHierarchy& m = *c.mg;
     if (f32) {
-        k_mg_pre<float><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, r, m.Dinv0f, m.x0f);
+        launch_pdl(k_mg_pre<float>, m.n_cta, kSpanThreads, 0, s, m.spans, c.fixed, r, m.Dinv0f, m.x0f);
         mg_cycle<float>(c, m, modes, s, r, z, nullptr, false);
     } else {
-        k_mg_pre<double><<<m.n_cta, kSpanThreads, 0, s>>>(m.spans, c.fixed, r, c.minv, m.x0);
+        launch_pdl(k_mg_pre<double>, m.n_cta, kSpanThreads, 0, s, m.spans, c.fixed, r, c.minv, m.x0);
         mg_cycle<double>(c, m, modes, s, r, z, nullptr, false);
     }
 }

@@ -3,8 +3,15 @@
 // Every kernel covers all the RVEs of a context (one, or a batch): the work
 // is cut into tiles or row spans that lie in one RVE each, listed in a table,
 // and a CTA whose RVE is done returns at once.
+//
+// The kernels are chained by programmatic dependent launch: each starts while
+// the one before it runs, reads what no kernel of the chain writes (tables,
+// operators, masks, diagonal inverses) and then waits.  Vectors, partial sums,
+// scalars and flags are read after the wait only, through loads (lv2, __ldcg)
+// that the compiler cannot take for invariant and move ahead of it.
 #pragma once
 
+#include "pg_pdl.cuh"
 #include "pg_solve_kernels.cuh"
 
 namespace pgb {
@@ -48,20 +55,21 @@ __host__ __device__ __forceinline__ double grid_w(int g, int nf, int I) {
     return (I == ((g - 1) >> 1) || I == ((g + 1) >> 1)) ? 0.5 : 0.0;
 }
 
-// the coarse indices a fine index interpolates from (I0 = I1 where it is only one) and the weight of each
+// The fine indices that restrict to a coarse node at fine index g: g with
+// weight 1 and, where g is even, its neighbours with weight 1/2 (an odd g is
+// the short last cell's end; its neighbour g - 1 is a coarse node of its own,
+// and so is the short cell's other end).
 template <typename T>
-__device__ __forceinline__ void parents(int g, int nf, int& I0, int& I1, T& w) {
-    if ((g & 1) == 0) {
-        I0 = I1 = g >> 1;
-        w = (T)0.5;
-    } else if (g == nf) {
-        I0 = I1 = (nf + 1) >> 1;
-        w = (T)0.5;
-    } else {
-        I0 = (g - 1) >> 1;
-        I1 = (g + 1) >> 1;
-        w = (T)0.5;
-    }
+__device__ __forceinline__ void side_weights(int g, int nf, T& lo, T& hi) {
+    lo = (g & 1) == 0 && g > 0 ? (T)0.5 : (T)0;
+    hi = (g & 1) == 0 && g + 1 < nf ? (T)0.5 : (T)0;
+}
+
+// the two coarse indices a fine index interpolates from, each with weight 1/2 (I0 = I1 where it is only one)
+__device__ __forceinline__ void parents(int g, int nf, int& I0, int& I1) {
+    I0 = g >> 1;
+    I1 = (g + 1) >> 1;
+    if (g == nf) I0 = I1;
 }
 
 template <typename T>
@@ -69,9 +77,16 @@ struct alignas(2 * sizeof(T)) Vec2 {
     T x, y;
 };
 
-template <typename T>
-__device__ __forceinline__ Vec2<T> ld2(const T* p, size_t i) {
-    return reinterpret_cast<const Vec2<T>*>(p)[i];
+// a vector's pair (see the head of the file)
+__device__ __forceinline__ Vec2<double> lv2(const double* p, size_t i) {
+    Vec2<double> v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p + 2 * i));
+    return v;
+}
+__device__ __forceinline__ Vec2<float> lv2(const float* p, size_t i) {
+    Vec2<float> v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p + 2 * i));
+    return v;
 }
 template <typename T>
 __device__ __forceinline__ void st2(T* p, size_t i, T x, T y) {
@@ -106,15 +121,71 @@ __device__ __forceinline__ double block_sum_all(double v) {
 // boundary orders the two, so no CTA waits on a fence and a ticket (which held
 // every CTA of the earlier fused sums: 33 us against 21 us for the same matrix
 // product without a sum at 512^2), and the result is the same bits on every run.
-__device__ __forceinline__ double range_sum(const double* __restrict__ part, int2 rg) {
+__device__ __forceinline__ double range_sum(const double* part, int2 rg) {
     double v = 0.0;
-    for (int k = rg.x + threadIdx.x; k < rg.y; k += blockDim.x) v += part[k];
+    for (int k = rg.x + threadIdx.x; k < rg.y; k += blockDim.x) v += __ldcg(&part[k]);
     return block_sum_all(v);
 }
 
-// Block row i of K times a vector, kRowLanes lanes per row (bsr_row_group);
-// get(j) gives the vector's pair at column node j (a Vec2<double>), and
-// columns with skip(j) are left out.
+// Block rows of K times a vector, kRowLanes lanes per row: lane g takes the
+// row's blocks g, g + kRowLanes, ... (a group's loads of K are contiguous).
+// RowFrag holds the columns and blocks of a lane's first kRowUnroll of them
+// (rows of up to 12 blocks), issued together; the first rows' are loaded
+// before the kernel's wait.
+template <typename MT>
+struct RowFrag {
+    int r1, next;              // end of the row, and the lane's first block beyond the fragment
+    int j[kRowUnroll];
+    MT b[kRowUnroll][4];
+
+    __device__ __forceinline__ void blocks(int base, const int* __restrict__ col, const MT* __restrict__ K) {
+#pragma unroll
+        for (int u = 0; u < kRowUnroll; ++u) {
+            const int k = base + u * kRowLanes;
+            j[u] = -1;
+            if (k < r1) {
+                j[u] = __ldg(&col[k]);
+                load4(K + 4 * (size_t)k, b[u][0], b[u][1], b[u][2], b[u][3]);
+            }
+        }
+        next = base + kRowUnroll * kRowLanes;
+    }
+    __device__ __forceinline__ void load(int i, bool valid, int g, const int* __restrict__ row_ptr,
+                                         const int* __restrict__ col, const MT* __restrict__ K) {
+        const int r0 = valid ? __ldg(&row_ptr[i]) : 0;
+        r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        blocks(r0 + g, col, K);
+    }
+    // the row's product, in every lane of its group; get(j) is the vector's pair at column node j
+    template <typename Get>
+    __device__ __forceinline__ void dot(const int* __restrict__ col, const MT* __restrict__ K, Get get, double& y0,
+                                        double& y1) {
+        double a0 = 0.0, a1 = 0.0;
+        while (true) {
+            Vec2<double> v[kRowUnroll];
+#pragma unroll
+            for (int u = 0; u < kRowUnroll; ++u)
+                if (j[u] >= 0) v[u] = get(j[u]);
+#pragma unroll
+            for (int u = 0; u < kRowUnroll; ++u)
+                if (j[u] >= 0) {
+                    a0 += (double)b[u][0] * v[u].x + (double)b[u][1] * v[u].y;
+                    a1 += (double)b[u][2] * v[u].x + (double)b[u][3] * v[u].y;
+                }
+            if (next >= r1) break;
+            blocks(next, col, K);
+        }
+        a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+        a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+        y0 = a0;
+        y1 = a1;
+    }
+};
+// The same without the early loads, for kernels that live on many warps (the
+// level-0 products: with a fragment loaded ahead, 64 registers and spills,
+// the 512^2 product took 36 us instead of 26).
 template <typename MT, typename Get>
 __device__ __forceinline__ void row_lanes(int r0, int r1, int g, const int* __restrict__ col, const MT* __restrict__ K,
                                           Get get, double& y0, double& y1) {
@@ -148,6 +219,13 @@ __device__ __forceinline__ void row_lanes(int r0, int r1, int g, const int* __re
     y0 = a0;
     y1 = a1;
 }
+template <typename T>
+__device__ __forceinline__ Vec2<double> widen(Vec2<T> a) {
+    Vec2<double> v;
+    v.x = (double)a.x;
+    v.y = (double)a.y;
+    return v;
+}
 
 // ---------------------------------------------------------------------------
 // CG.  Iteration parity P; part_* hold one partial per CTA of the spans.
@@ -155,15 +233,15 @@ __device__ __forceinline__ void row_lanes(int r0, int r1, int g, const int* __re
 
 // x = 0, r = mask(b); partials of r.r; the first regular smoothing sweep x1 = omega D^-1 r
 template <typename T>
-__global__ void __launch_bounds__(kSpanThreads) k_cg_start(Spans sp, const uint8_t* __restrict__ fixed,
-                                                           const double* __restrict__ b, double* __restrict__ r,
-                                                           double* __restrict__ x, const T* __restrict__ Dinv,
-                                                           T* __restrict__ x1, double* part_rr) {
+__global__ void __launch_bounds__(kSpanThreads) k_cg_start(Spans sp, const uint8_t* __restrict__ fixed, const double* b,
+                                                           double* r, double* x, const T* Dinv, T* x1, double* part_rr) {
+    pdl_wait();
+    pdl_trigger();
     const int4 S = sp.span[blockIdx.x];
     const int reg = sp.reg_end[S.x];
     double acc = 0.0;
     for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
-        const Vec2<double> v = ld2(b, i);
+        const Vec2<double> v = lv2(b, i);
         const double r0 = fixed[2 * i] ? 0.0 : v.x, r1 = fixed[2 * i + 1] ? 0.0 : v.y;
         st2(r, i, r0, r1);
         st2(x, i, 0.0, 0.0);
@@ -180,13 +258,14 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_start(Spans sp, const uint8
 
 // the first regular smoothing sweep alone (a V-cycle applied outside CG)
 template <typename T>
-__global__ void __launch_bounds__(kSpanThreads) k_mg_pre(Spans sp, const uint8_t* __restrict__ fixed,
-                                                         const double* __restrict__ r, const T* __restrict__ Dinv,
-                                                         T* __restrict__ x1) {
+__global__ void __launch_bounds__(kSpanThreads) k_mg_pre(Spans sp, const uint8_t* __restrict__ fixed, const double* r,
+                                                         const T* Dinv, T* x1) {
+    pdl_wait();
+    pdl_trigger();
     const int4 S = sp.span[blockIdx.x];
     const int end = min(S.z, sp.reg_end[S.x]);
     for (int i = S.y + threadIdx.x; i < end; i += kSpanThreads) {
-        const Vec2<double> v = ld2(r, i);
+        const Vec2<double> v = lv2(r, i);
         const T r0 = fixed[2 * i] ? (T)0 : (T)v.x, r1 = fixed[2 * i + 1] ? (T)0 : (T)v.y;
         T m0, m1, m2, m3;
         load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
@@ -196,6 +275,8 @@ __global__ void __launch_bounds__(kSpanThreads) k_mg_pre(Spans sp, const uint8_t
 
 // per RVE: tol^2 = rtol^2 b.b, and the r.z that the first iteration divides by
 __global__ inline void k_cg_tol(Spans sp, const double* part_rr, double rtol2, double* sc, int* fl) {
+    pdl_wait();
+    pdl_trigger();
     const int r = blockIdx.x;
     const double bb = range_sum(part_rr, sp.range[r]);
     if (threadIdx.x == 0) {
@@ -213,19 +294,20 @@ __global__ inline void k_cg_tol(Spans sp, const double* part_rr, double rtol2, d
 // kernel that writes p.  Bound by the reads of K (32 bytes a block).
 __global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* __restrict__ row_ptr,
                                                           const int* __restrict__ col, const double* __restrict__ K,
-                                                          const uint8_t* __restrict__ fixed,
-                                                          const double* __restrict__ z, const double* __restrict__ p_old,
-                                                          double* __restrict__ p, double* __restrict__ q,
-                                                          const double* __restrict__ part_rz, double* sc, const int* fl,
-                                                          double* part_pq, int P) {
+                                                          const uint8_t* __restrict__ fixed, const double* z,
+                                                          const double* p_old, double* p, double* q, const double* part_rz,
+                                                          double* sc, const int* fl, double* part_pq, int P) {
     const int4 S = sp.span[blockIdx.x];
-    if (fl[kFlags * S.x]) return;
     const int2 rg = sp.range[S.x];
-    const double rz = range_sum(part_rz, rg);
-    double* s = sc + kScal * S.x;
-    const double beta = rz / s[1 - P];
-    if ((int)blockIdx.x == rg.x && threadIdx.x == 0) s[P] = rz;
     const int g = threadIdx.x % kRowLanes;
+    pdl_wait();
+    pdl_trigger();
+    if (__ldcg(&fl[kFlags * S.x])) return;
+    double* s = sc + kScal * S.x;
+    const double rz_old = __ldcg(&s[1 - P]);
+    const double rz = range_sum(part_rz, rg);
+    const double beta = rz / rz_old;
+    if ((int)blockIdx.x == rg.x && threadIdx.x == 0) s[P] = rz;
     double acc = 0.0;
     for (int base = S.y; base < S.z; base += kSpanThreads / kRowLanes) {
         const int i = base + threadIdx.x / kRowLanes;
@@ -233,14 +315,14 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* _
         const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
         double y0, y1;
         row_lanes(r0, r1, g, col, K, [&](int j) {
-            Vec2<double> a = ld2(z, j);
-            const Vec2<double> b = ld2(p_old, j);
+            Vec2<double> a = lv2(z, j);
+            const Vec2<double> b = lv2(p_old, j);
             a.x += beta * b.x;
             a.y += beta * b.y;
             return a;
         }, y0, y1);
         if (valid && g == 0) {
-            const Vec2<double> a = ld2(z, i), b = ld2(p_old, i);
+            const Vec2<double> a = lv2(z, i), b = lv2(p_old, i);
             const double p0 = a.x + beta * b.x, p1 = a.y + beta * b.y;
             if (fixed[2 * i]) y0 = 0.0;
             if (fixed[2 * i + 1]) y1 = 0.0;
@@ -255,15 +337,17 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* _
 
 // x += alpha p, r -= alpha q, partials of r.r, and the first regular smoothing sweep of the coming V-cycle
 template <typename T>
-__global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* __restrict__ x, double* __restrict__ r,
-                                                            const double* __restrict__ p, const double* __restrict__ q,
-                                                            const T* __restrict__ Dinv, T* __restrict__ x1,
-                                                            const double* __restrict__ part_pq, const double* sc, int* fl,
-                                                            double* part_rr, int P) {
+__global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* x, double* r, const double* p, const double* q,
+                                                            const T* __restrict__ Dinv, T* x1, const double* part_pq,
+                                                            const double* sc, int* fl, double* part_rr, int P) {
     const int4 S = sp.span[blockIdx.x];
-    int* f = fl + kFlags * S.x;
-    if (f[0]) return;
     const int2 rg = sp.range[S.x];
+    const int reg = sp.reg_end[S.x];
+    pdl_wait();
+    pdl_trigger();
+    int* f = fl + kFlags * S.x;
+    if (__ldcg(&f[0])) return;
+    const double rz = __ldcg(&sc[kScal * S.x + P]);
     const double pq = range_sum(part_pq, rg);
     const bool first = (int)blockIdx.x == rg.x && threadIdx.x == 0;
     if (!(pq > 0.0)) {
@@ -274,11 +358,10 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* __
         return;
     }
     if (first) f[2] += 1;
-    const double alpha = sc[kScal * S.x + P] / pq;
-    const int reg = sp.reg_end[S.x];
+    const double alpha = rz / pq;
     double acc = 0.0;
     for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
-        const Vec2<double> xv = ld2((const double*)x, i), rv = ld2((const double*)r, i), pv = ld2(p, i), qv = ld2(q, i);
+        const Vec2<double> xv = lv2(x, i), rv = lv2(r, i), pv = lv2(p, i), qv = lv2(q, i);
         const double r0 = rv.x - alpha * qv.x, r1 = rv.y - alpha * qv.y;
         st2(x, i, xv.x + alpha * pv.x, xv.y + alpha * pv.y);
         st2(r, i, r0, r1);
@@ -294,13 +377,15 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* __
 }
 
 // partials of a.b
-__global__ inline void __launch_bounds__(kSpanThreads) k_cg_dot(Spans sp, const double* __restrict__ a,
-                                                                const double* __restrict__ b, const int* fl, double* part) {
+__global__ inline void __launch_bounds__(kSpanThreads) k_cg_dot(Spans sp, const double* a, const double* b, const int* fl,
+                                                                double* part) {
+    pdl_wait();
+    pdl_trigger();
     const int4 S = sp.span[blockIdx.x];
-    if (fl && fl[kFlags * S.x]) return;
+    if (fl && __ldcg(&fl[kFlags * S.x])) return;
     double acc = 0.0;
     for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
-        const Vec2<double> u = ld2(a, i), v = ld2(b, i);
+        const Vec2<double> u = lv2(a, i), v = lv2(b, i);
         acc += u.x * v.x + u.y * v.y;
     }
     acc = block_sum(acc);
@@ -340,14 +425,12 @@ struct Enr {
 };
 
 template <typename T, bool POST>
-__global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __restrict__ row_ptr, const int* __restrict__ col,
+__global__ void __launch_bounds__(kPieceThreads, 3) k_mg_enr(Enr e, const int* __restrict__ row_ptr, const int* __restrict__ col,
                                                           const T* __restrict__ K, const T* __restrict__ Dinv,
                                                           const uint8_t* __restrict__ fixed, const int* __restrict__ reg_end,
-                                                          const double* __restrict__ b, const T* __restrict__ xin,
-                                                          T* __restrict__ xout, const int* fl) {
+                                                          const double* b, const T* xin, T* xout, const int* fl) {
     extern __shared__ __align__(16) unsigned char enr_smem[];
     const Piece pc = e.piece[blockIdx.x];
-    if (fl && fl[kFlags * pc.rve]) return;
     const int n = pc.end[kChebSteps - 1];
     Vec2<T>* sx = reinterpret_cast<Vec2<T>*>(enr_smem);  // two copies of x, then d and r
     Vec2<T>* sx2 = sx + n;
@@ -355,34 +438,56 @@ __global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __re
     Vec2<T>* sr = sd + n;
     const double* cf = e.coef + kChebCoef * pc.rve;
     const int reg = reg_end[pc.rve];
-    const int g = threadIdx.x % kRowLanes;
+    const int g = threadIdx.x % kRowLanes, l0 = threadIdx.x / kRowLanes;
     constexpr int kRows = kPieceThreads / kRowLanes;
-    const T ith = (T)cf[0];
+    constexpr int kEnt = 2;  // entries of K_ee that a lane keeps of its row among the first kRows (8 a row)
+    int i = l0 < n ? e.node[pc.row0 + l0] : 0;
+    RowFrag<T> f;
+    f.load(i, l0 < n, g, row_ptr, col, K);
+    const int e0 = l0 < n ? e.eptr[pc.row0 + l0] : 0, e1 = l0 < n ? e.eptr[pc.row0 + l0 + 1] : 0;
+    int ec[kEnt];
+    T eb[kEnt][4];
+#pragma unroll
+    for (int u = 0; u < kEnt; ++u) {
+        const int q = e0 + g + u * kRowLanes;
+        ec[u] = -1;
+        if (q < e1) {
+            const int2 en = __ldg(&e.ent[q]);
+            ec[u] = en.y;
+            load4(K + 4 * (size_t)en.x, eb[u][0], eb[u][1], eb[u][2], eb[u][3]);
+        }
+    }
+    T m0, m1, m2, m3;  // of the row among the first kRows
+    load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+    const bool f0 = fixed[2 * i], f1 = fixed[2 * i + 1];
+    T c[2 * kChebSteps - 1];
+#pragma unroll
+    for (int k = 0; k < 2 * kChebSteps - 1; ++k) c[k] = (T)cf[k];
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * pc.rve])) return;
     for (int base = 0; base < n; base += kRows) {
-        const int l = base + threadIdx.x / kRowLanes;
-        const bool valid = l < n;
-        const int i = valid ? e.node[pc.row0 + l] : 0;
-        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+        const int l = base + l0;
+        if (base > 0) {
+            i = l < n ? e.node[pc.row0 + l] : 0;
+            f.load(i, l < n, g, row_ptr, col, K);
+        }
+        const Vec2<double> bv = lv2(b, i);
         double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) {
+        f.dot(col, K, [&](int j) {
             Vec2<double> v;
             v.x = v.y = 0.0;
-            if (POST || j < reg) {  // before the coarse correction x_e is zero
-                const Vec2<T> a = ld2(xin, j);
-                v.x = (double)a.x;
-                v.y = (double)a.y;
-            }
+            if (POST || j < reg) v = widen(lv2(xin, j));  // before the coarse correction x_e is zero
             return v;
         }, y0, y1);
-        if (valid && g == 0) {
-            const Vec2<double> bv = ld2(b, i);
+        if (l < n && g == 0) {
             Vec2<T> rv, dv;
+            T a0 = m0, a1 = m1, a2 = m2, a3 = m3;
+            if (base > 0) load4(Dinv + 4 * (size_t)i, a0, a1, a2, a3);
             rv.x = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0;
             rv.y = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
-            T m0, m1, m2, m3;
-            load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
-            dv.x = ith * (m0 * rv.x + m1 * rv.y);
-            dv.y = ith * (m2 * rv.x + m3 * rv.y);
+            dv.x = c[0] * (a0 * rv.x + a1 * rv.y);
+            dv.y = c[0] * (a2 * rv.x + a3 * rv.y);
             sr[l] = rv;
             sd[l] = dv;
             sx[l] = dv;
@@ -391,16 +496,28 @@ __global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __re
     __syncthreads();
 #pragma unroll
     for (int k = 1; k < kChebSteps; ++k) {
-        const T c1 = (T)cf[2 * k - 1], c2 = (T)cf[2 * k];
+        const T c1 = c[2 * k - 1], c2 = c[2 * k];
         const int rows = pc.end[kChebSteps - 1 - k];
         const Vec2<T>* xa = (k & 1) ? sx : sx2;
         Vec2<T>* xb = (k & 1) ? sx2 : sx;
         for (int base = 0; base < rows; base += kRows) {
-            const int l = base + threadIdx.x / kRowLanes;
-            const bool valid = l < rows;
-            const int e0 = valid ? e.eptr[pc.row0 + l] : 0, e1 = valid ? e.eptr[pc.row0 + l + 1] : 0;
+            const int l = base + l0;
             double a0 = 0.0, a1 = 0.0;
-            for (int q = e0 + g; q < e1; q += kRowLanes) {
+            int q = e0 + g, q1 = e1;
+            if (base == 0) {
+#pragma unroll
+                for (int u = 0; u < kEnt; ++u)
+                    if (ec[u] >= 0) {
+                        const Vec2<T> v = xa[ec[u]];
+                        a0 += (double)eb[u][0] * (double)v.x + (double)eb[u][1] * (double)v.y;
+                        a1 += (double)eb[u][2] * (double)v.x + (double)eb[u][3] * (double)v.y;
+                    }
+                q += kEnt * kRowLanes;
+            } else {
+                q = l < rows ? e.eptr[pc.row0 + l] + g : 0;
+                q1 = l < rows ? e.eptr[pc.row0 + l + 1] : 0;
+            }
+            for (; q < q1; q += kRowLanes) {
                 const int2 en = __ldg(&e.ent[q]);
                 double k0, k1, k2, k3;
                 load_block(K + 4 * (size_t)en.x, k0, k1, k2, k3);
@@ -412,14 +529,19 @@ __global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __re
             a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
             a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
             a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-            if (valid && g == 0) {
-                const int i = e.node[pc.row0 + l];
-                const T r0 = fixed[2 * i] ? (T)0 : sr[l].x - (T)a0, r1 = fixed[2 * i + 1] ? (T)0 : sr[l].y - (T)a1;
-                T m0, m1, m2, m3;
-                load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+            if (l < rows && g == 0) {
+                T n0 = m0, n1 = m1, n2 = m2, n3 = m3;
+                bool g0 = f0, g1 = f1;
+                if (base > 0) {
+                    const int il = e.node[pc.row0 + l];
+                    load4(Dinv + 4 * (size_t)il, n0, n1, n2, n3);
+                    g0 = fixed[2 * il];
+                    g1 = fixed[2 * il + 1];
+                }
+                const T r0 = g0 ? (T)0 : sr[l].x - (T)a0, r1 = g1 ? (T)0 : sr[l].y - (T)a1;
                 Vec2<T> dv = sd[l], xv = xa[l];
-                dv.x = c1 * dv.x + c2 * (m0 * r0 + m1 * r1);
-                dv.y = c1 * dv.y + c2 * (m2 * r0 + m3 * r1);
+                dv.x = c1 * dv.x + c2 * (n0 * r0 + n1 * r1);
+                dv.y = c1 * dv.y + c2 * (n2 * r0 + n3 * r1);
                 xv.x += dv.x;
                 xv.y += dv.y;
                 sd[l] = dv;
@@ -430,14 +552,14 @@ __global__ void __launch_bounds__(kPieceThreads) k_mg_enr(Enr e, const int* __re
     }
     const Vec2<T>* xl = ((kChebSteps - 1) & 1) ? sx2 : sx;
     for (int l = threadIdx.x; l < pc.end[0]; l += kPieceThreads) {
-        const int i = e.node[pc.row0 + l];
+        const int il = e.node[pc.row0 + l];
         Vec2<T> v = xl[l];
         if (POST) {
-            const Vec2<T> o = ld2(xin, i);
+            const Vec2<T> o = lv2(xin, il);
             v.x += o.x;
             v.y += o.y;
         }
-        st2(xout, i, v.x, v.y);
+        st2(xout, il, v.x, v.y);
     }
 }
 
@@ -451,71 +573,67 @@ constexpr int kDownFine = 2 * kDownTile + 1;
 
 template <typename T>
 __device__ __forceinline__ void restrict_tile(const Vec2<T>* s, int I0, int J0, const Pair& p,
-                                              const uint8_t* __restrict__ fixed_c, T* __restrict__ bc) {
+                                              const uint8_t* __restrict__ fixed_c, T* bc) {
     // s: the residual on fine nodes (2 I0 - 1 .., 2 J0 - 1 ..), kDownFine per side, 0 outside the grid
     const int t = threadIdx.x;
     if (t >= kDownTile * kDownTile) return;
     const int I = I0 + t % kDownTile, J = J0 + t / kDownTile;
     if (I > p.cnx || J > p.cny) return;
-    const int px = grid_pos(I, p.fnx) - (2 * I0 - 1), py = grid_pos(J, p.fny) - (2 * J0 - 1);
+    const int gx = grid_pos(I, p.fnx), gy = grid_pos(J, p.fny);
+    T wx[3], wy[3];
+    side_weights(gx, p.fnx, wx[0], wx[2]);
+    side_weights(gy, p.fny, wy[0], wy[2]);
+    wx[1] = wy[1] = (T)1;
+    const Vec2<T>* c = s + (gy - (2 * J0 - 1)) * kDownFine + gx - (2 * I0 - 1);
     T s0 = 0, s1 = 0;
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
-        const int ly = py + dy;
-        if (ly < 0 || ly >= kDownFine) continue;
-        const T wy = (T)grid_w(2 * J0 - 1 + ly, p.fny, J);
+    for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
         for (int dx = -1; dx <= 1; ++dx) {
-            const int lx = px + dx;
-            if (lx < 0 || lx >= kDownFine) continue;
-            const T w = wy * (T)grid_w(2 * I0 - 1 + lx, p.fnx, I);
+            const T w = wy[dy + 1] * wx[dx + 1];
             if (w == (T)0) continue;
-            const Vec2<T> v = s[ly * kDownFine + lx];
+            const Vec2<T> v = c[dy * kDownFine + dx];
             s0 += w * v.x;
             s1 += w * v.y;
         }
-    }
     const int a = p.coff + I + J * (p.cnx + 1);
     st2(bc, a, fixed_c[2 * a] ? (T)0 : s0, fixed_c[2 * a + 1] ? (T)0 : s1);
 }
 
+// 304 threads take the tile's 289 rows in four rounds.
+constexpr int kDown0Threads = 304;
 template <typename T>
-__global__ void __launch_bounds__(kSpanThreads) k_mg_down0(const int4* __restrict__ tile, const Pair* __restrict__ pair,
-                                                           const int* __restrict__ row_ptr, const int* __restrict__ col,
-                                                           const T* __restrict__ K, const uint8_t* __restrict__ fixed,
-                                                           const double* __restrict__ b, const T* __restrict__ x,
-                                                           const uint8_t* __restrict__ fixed_c, T* __restrict__ bc,
-                                                           Spans sp, const double* __restrict__ part_rr, const double* sc,
-                                                           int* fl, int check) {
+__global__ void __launch_bounds__(kDown0Threads) k_mg_down0(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+                                                            const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                                            const T* __restrict__ K, const uint8_t* __restrict__ fixed,
+                                                            const double* b, const T* x, const uint8_t* __restrict__ fixed_c,
+                                                            T* bc, Spans sp, const double* part_rr, const double* sc,
+                                                            int* fl, int check) {
     __shared__ Vec2<T> s[kDownFine * kDownFine];
     const int4 tl = tile[blockIdx.x];
     const Pair p = pair[tl.x];
-    if (fl && fl[kFlags * tl.x]) return;
+    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1, g = threadIdx.x % kRowLanes;
+    constexpr int kRows = kDown0Threads / kRowLanes, kN = kDownFine * kDownFine;
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
     if (check && tl.w) {
         const double rr = range_sum(part_rr, sp.range[tl.x]);
-        if (threadIdx.x == 0 && rr <= sc[kScal * tl.x + 4]) fl[kFlags * tl.x] = 1;
+        if (threadIdx.x == 0 && rr <= __ldcg(&sc[kScal * tl.x + 4])) fl[kFlags * tl.x] = 1;
     }
-    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1, g = threadIdx.x % kRowLanes;
-    for (int base = 0; base < kDownFine * kDownFine; base += kSpanThreads / kRowLanes) {
+    for (int base = 0; base < kN; base += kRows) {
         const int l = base + threadIdx.x / kRowLanes;
         const int gx = gx0 + l % kDownFine, gy = gy0 + l / kDownFine;
-        const bool in = l < kDownFine * kDownFine;
-        const bool valid = in && gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny;
+        const bool valid = l < kN && gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny;
         const int i = valid ? p.foff + gx + gy * (p.fnx + 1) : 0;
         const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
         double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) {
-            const Vec2<T> a = ld2(x, j);
-            Vec2<double> v;
-            v.x = (double)a.x;
-            v.y = (double)a.y;
-            return v;
-        }, y0, y1);
-        if (in && g == 0) {
+        row_lanes(r0, r1, g, col, K, [&](int j) { return widen(lv2(x, j)); }, y0, y1);
+        if (l < kN && g == 0) {
             Vec2<T> rv;
             rv.x = rv.y = 0;
             if (valid) {
-                const Vec2<double> bv = ld2(b, i);
+                const Vec2<double> bv = lv2(b, i);
                 rv.x = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0;
                 rv.y = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
             }
@@ -532,30 +650,25 @@ template <typename T>
 __global__ void __launch_bounds__(kSpanThreads) k_mg_post(Spans sp, const int* __restrict__ row_ptr,
                                                           const int* __restrict__ col, const T* __restrict__ K,
                                                           const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                                          const double* __restrict__ b, const T* __restrict__ x,
-                                                          const T* __restrict__ xe, double* __restrict__ z, const int* fl,
+                                                          const double* b, const T* x, const T* xe, double* z, const int* fl,
                                                           double* part_rz) {
     const int4 S = sp.span[blockIdx.x];
-    if (fl && fl[kFlags * S.x]) return;
     const int reg = sp.reg_end[S.x];
     const int g = threadIdx.x % kRowLanes;
-    double acc = 0.0;
     const int end = min(S.z, reg);
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * S.x])) return;
+    double acc = 0.0;
     for (int base = S.y; base < end; base += kSpanThreads / kRowLanes) {
         const int i = base + threadIdx.x / kRowLanes;
         const bool valid = i < end;
         const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
         double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) {
-            const Vec2<T> a = ld2(j < reg ? x : xe, j);
-            Vec2<double> v;
-            v.x = (double)a.x;
-            v.y = (double)a.y;
-            return v;
-        }, y0, y1);
+        row_lanes(r0, r1, g, col, K, [&](int j) { return widen(lv2(j < reg ? x : xe, j)); }, y0, y1);
         if (valid && g == 0) {
-            const Vec2<double> bv = ld2(b, i);
-            const Vec2<T> xv = ld2(x, i);
+            const Vec2<double> bv = lv2(b, i);
+            const Vec2<T> xv = lv2(x, i);
             const T t0 = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0, t1 = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
             T m0, m1, m2, m3;
             load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
@@ -565,11 +678,10 @@ __global__ void __launch_bounds__(kSpanThreads) k_mg_post(Spans sp, const int* _
             acc += bv.x * z0 + bv.y * z1;
         }
     }
-    for (int i = max(S.y, reg) + threadIdx.x; i < S.z; i += kSpanThreads) {
-        const Vec2<double> bv = ld2(b, i);
-        const Vec2<T> xv = ld2(xe, i);
-        st2(z, i, (double)xv.x, (double)xv.y);
-        acc += bv.x * (double)xv.x + bv.y * (double)xv.y;
+    for (int k = max(S.y, reg) + threadIdx.x; k < S.z; k += kSpanThreads) {
+        const Vec2<double> bv = lv2(b, k), xv = widen(lv2(xe, k));
+        st2(z, k, xv.x, xv.y);
+        acc += bv.x * xv.x + bv.y * xv.y;
     }
     acc = block_sum(acc);
     if (threadIdx.x == 0) part_rz[blockIdx.x] = acc;
@@ -582,89 +694,98 @@ __global__ void __launch_bounds__(kSpanThreads) k_mg_post(Spans sp, const int* _
 // the nodes around its tile that the next phase reads (27% more sweeps)
 // instead of waiting for its neighbours.
 // ---------------------------------------------------------------------------
+//
+// A thread keeps one node of the tile's first swept region through all the
+// phases, so its operator row is loaded once, before the wait.
 constexpr int kTileThreads = 384;
 
-// (A x)(node i) from x staged in shared memory, at s[l] of a region W wide
-template <typename T, int W>
-__device__ __forceinline__ void stencil(const T* __restrict__ A, int i, const Vec2<T>* s, int l, T& y0, T& y1) {
-    T k[9][4];
-#pragma unroll
-    for (int q = 0; q < 9; ++q) load4(A + 36 * (size_t)i + 4 * q, k[q][0], k[q][1], k[q][2], k[q][3]);
-    y0 = y1 = 0;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const Vec2<T> v = s[l + (q / 3 - 1) * W + q % 3 - 1];
-        y0 += k[q][0] * v.x + k[q][1] * v.y;
-        y1 += k[q][2] * v.x + k[q][3] * v.y;
-    }
-}
-
-// x + omega D^-1 mask(b - y) at node i
 template <typename T>
-__device__ __forceinline__ Vec2<T> sweep_node(int i, const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                              const T* __restrict__ b, Vec2<T> x, T y0, T y1) {
-    const Vec2<T> bv = ld2(b, i);
-    const T r0 = fixed[2 * i] ? (T)0 : bv.x - y0, r1 = fixed[2 * i + 1] ? (T)0 : bv.y - y1;
-    T m0, m1, m2, m3;
-    load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
-    x.x += (T)kOmega * (m0 * r0 + m1 * r1);
-    x.y += (T)kOmega * (m2 * r0 + m3 * r1);
-    return x;
-}
+struct NodeRow {
+    T k[9][4], m[4];
+    __device__ __forceinline__ void load(int i, const T* __restrict__ A, const T* __restrict__ Dinv) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) load4(A + 36 * (size_t)i + 4 * q, k[q][0], k[q][1], k[q][2], k[q][3]);
+        load4(Dinv + 4 * (size_t)i, m[0], m[1], m[2], m[3]);
+    }
+    // b - A x from x staged in shared memory, at s[l] of a region W wide (0 at a fixed DOF: its row and b are)
+    __device__ __forceinline__ Vec2<T> residual(Vec2<T> b, const Vec2<T>* s, int l, int W) const {
+        T y0 = 0, y1 = 0;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const Vec2<T> v = s[l + (q / 3 - 1) * W + q % 3 - 1];
+            y0 += k[q][0] * v.x + k[q][1] * v.y;
+            y1 += k[q][2] * v.x + k[q][3] * v.y;
+        }
+        b.x -= y0;
+        b.y -= y1;
+        return b;
+    }
+    // x + omega D^-1 r
+    __device__ __forceinline__ Vec2<T> relax(Vec2<T> x, Vec2<T> r) const {
+        x.x += (T)kOmega * (m[0] * r.x + m[1] * r.y);
+        x.y += (T)kOmega * (m[2] * r.x + m[3] * r.y);
+        return x;
+    }
+};
 
 // pre-smoothing from zero, residual, restriction: x of the finer grid's nodes and b of the coarser one's
 template <typename T>
-__global__ void __launch_bounds__(kTileThreads, 2) k_mg_down(const int4* __restrict__ tile, const Pair* __restrict__ pair,
-                                                          const T* __restrict__ A, const T* __restrict__ Dinv,
-                                                          const uint8_t* __restrict__ fixed, const T* __restrict__ b,
-                                                          T* __restrict__ x, const uint8_t* __restrict__ fixed_c,
-                                                          T* __restrict__ bc, const int* fl) {
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_down(const int4* __restrict__ tile,
+                                                                                  const Pair* __restrict__ pair,
+                                                                                  const T* __restrict__ A,
+                                                                                  const T* __restrict__ Dinv, const T* b, T* x,
+                                                                                  const uint8_t* __restrict__ fixed_c, T* bc,
+                                                                                  const int* fl) {
     constexpr int W0 = kDownFine, W1 = W0 + 2, W2 = W1 + 2;
+    static_assert(W1 * W1 <= kTileThreads, "one thread per node of the swept region");
     __shared__ Vec2<T> s1[W2 * W2];  // after one sweep
     __shared__ Vec2<T> s2[W1 * W1];  // after two
     __shared__ Vec2<T> s0[W0 * W0];  // residual
     const int4 tl = tile[blockIdx.x];
     const Pair p = pair[tl.x];
-    if (fl && fl[kFlags * tl.x]) return;
-    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1;  // of the residual's region
-    for (int l = threadIdx.x; l < W2 * W2; l += kTileThreads) {
-        const int gx = gx0 - 2 + l % W2, gy = gy0 - 2 + l / W2;
+    const int gx0 = 2 * tl.y - 2, gy0 = 2 * tl.z - 2;  // of the swept region
+    const int t = threadIdx.x, lx = t % W1, ly = t / W1, gx = gx0 + lx, gy = gy0 + ly;
+    const bool in = t < W1 * W1 && gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny;
+    const int i = in ? p.foff + gx + gy * (p.fnx + 1) : p.foff;
+    NodeRow<T> row;
+    row.load(i, A, Dinv);
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
+    Vec2<T> bv = lv2(b, i);
+    for (int l = t; l < W2 * W2; l += kTileThreads) {
+        const int hx = gx0 - 1 + l % W2, hy = gy0 - 1 + l / W2;
         Vec2<T> v;
         v.x = v.y = 0;
-        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny)
-            v = sweep_node<T>(p.foff + gx + gy * (p.fnx + 1), Dinv, fixed, b, v, (T)0, (T)0);
+        if (hx >= 0 && hx <= p.fnx && hy >= 0 && hy <= p.fny) {
+            const int h = p.foff + hx + hy * (p.fnx + 1);
+            const Vec2<T> r = lv2(b, h);  // (masked by the restriction)
+            T m0, m1, m2, m3;
+            load4(Dinv + 4 * (size_t)h, m0, m1, m2, m3);
+            v.x = (T)kOmega * (m0 * r.x + m1 * r.y);
+            v.y = (T)kOmega * (m2 * r.x + m3 * r.y);
+        }
         s1[l] = v;
     }
     __syncthreads();
-    for (int l = threadIdx.x; l < W1 * W1; l += kTileThreads) {
-        const int lx = l % W1, ly = l / W1, gx = gx0 - 1 + lx, gy = gy0 - 1 + ly;
+    const int c = (ly + 1) * W2 + lx + 1;
+    if (t < W1 * W1) {
         Vec2<T> v;
         v.x = v.y = 0;
-        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny) {
-            const int i = p.foff + gx + gy * (p.fnx + 1), c = (ly + 1) * W2 + lx + 1;
-            T y0, y1;
-            stencil<T, W2>(A, i, s1, c, y0, y1);
-            v = sweep_node<T>(i, Dinv, fixed, b, s1[c], y0, y1);
+        if (in) {
+            v = row.relax(s1[c], row.residual(bv, s1, c, W2));
             // a fine node belongs to the tile of its index / (2 kDownTile)
             if (gx >= 2 * tl.y && gx < 2 * (tl.y + kDownTile) && gy >= 2 * tl.z && gy < 2 * (tl.z + kDownTile))
                 st2(x, i, v.x, v.y);
         }
-        s2[l] = v;
+        s2[t] = v;
     }
     __syncthreads();
-    for (int l = threadIdx.x; l < W0 * W0; l += kTileThreads) {
-        const int lx = l % W0, ly = l / W0, gx = gx0 + lx, gy = gy0 + ly;
+    if (lx >= 1 && lx <= W0 && ly >= 1 && ly <= W0) {
         Vec2<T> v;
         v.x = v.y = 0;
-        if (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny) {
-            const int i = p.foff + gx + gy * (p.fnx + 1);
-            T y0, y1;
-            stencil<T, W1>(A, i, s2, (ly + 1) * W1 + lx + 1, y0, y1);
-            const Vec2<T> bv = ld2(b, i);
-            if (!fixed[2 * i]) v.x = bv.x - y0;
-            if (!fixed[2 * i + 1]) v.y = bv.y - y1;
-        }
-        s0[l] = v;
+        if (in) v = row.residual(bv, s2, t, W1);
+        s0[(ly - 1) * W0 + lx - 1] = v;
     }
     __syncthreads();
     restrict_tile(s0, tl.y, tl.z, p, fixed_c, bc);
@@ -672,14 +793,13 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_mg_down(const int4* __restr
 
 // the coarse correction at fine node (gx, gy)
 template <typename T>
-__device__ __forceinline__ Vec2<T> interpolate(int gx, int gy, const Pair& p, const T* __restrict__ xc) {
+__device__ __forceinline__ Vec2<T> interpolate(int gx, int gy, const Pair& p, const T* xc) {
     int I0, I1, J0, J1;
-    T w;
-    parents<T>(gx, p.fnx, I0, I1, w);
-    parents<T>(gy, p.fny, J0, J1, w);
+    parents(gx, p.fnx, I0, I1);
+    parents(gy, p.fny, J0, J1);
     const int W = p.cnx + 1;
-    const Vec2<T> a = ld2(xc, p.coff + I0 + J0 * W), b = ld2(xc, p.coff + I1 + J0 * W);
-    const Vec2<T> c = ld2(xc, p.coff + I0 + J1 * W), d = ld2(xc, p.coff + I1 + J1 * W);
+    const Vec2<T> a = lv2(xc, p.coff + I0 + J0 * W), b = lv2(xc, p.coff + I1 + J0 * W);
+    const Vec2<T> c = lv2(xc, p.coff + I0 + J1 * W), d = lv2(xc, p.coff + I1 + J1 * W);
     Vec2<T> v;
     v.x = (T)0.25 * ((a.x + b.x) + (c.x + d.x));
     v.y = (T)0.25 * ((a.y + b.y) + (c.y + d.y));
@@ -691,56 +811,53 @@ __device__ __forceinline__ Vec2<T> interpolate(int gx, int gy, const Pair& p, co
 // straight into level 0's x; otherwise it goes to xo.
 constexpr int kUpTile = 16;
 template <typename T, bool FINE>
-__global__ void __launch_bounds__(kTileThreads, 2) k_mg_up(const int4* __restrict__ tile, const Pair* __restrict__ pair,
-                                                        const Pair* __restrict__ pairc, const T* __restrict__ A,
-                                                        const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
-                                                        const T* __restrict__ b, const T* __restrict__ x,
-                                                        const T* __restrict__ xc, T* __restrict__ xo,
-                                                        const uint8_t* __restrict__ fixed0, T* __restrict__ x0,
-                                                        const int* fl) {
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_up(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+                                                           const Pair* __restrict__ pairc, const T* __restrict__ A,
+                                                           const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
+                                                           const T* b, const T* x, const T* xc, T* xo,
+                                                           const uint8_t* __restrict__ fixed0, T* x0, const int* fl) {
     constexpr int W0 = kUpTile + (FINE ? 1 : 0), W1 = W0 + 2, W2 = W1 + 2;
+    static_assert(W1 * W1 <= kTileThreads, "one thread per node of the swept region");
     __shared__ Vec2<T> s2[W2 * W2];  // corrected
     __shared__ Vec2<T> s1[W1 * W1];  // after one sweep
     __shared__ Vec2<T> s0[W0 * W0];  // after two
     const int4 tl = tile[blockIdx.x];
-    if (fl && fl[kFlags * tl.x]) return;
     const Pair pf = pair[tl.x], p = pairc[tl.x];
     const int off = p.foff, nx = p.fnx, ny = p.fny, gx0 = tl.y, gy0 = tl.z;
-    for (int l = threadIdx.x; l < W2 * W2; l += kTileThreads) {
-        const int gx = gx0 - 2 + l % W2, gy = gy0 - 2 + l / W2;
+    const int t = threadIdx.x, lx = t % W1, ly = t / W1, gx = gx0 - 1 + lx, gy = gy0 - 1 + ly;
+    const bool in = t < W1 * W1 && gx >= 0 && gx <= nx && gy >= 0 && gy <= ny;
+    const int i = in ? off + gx + gy * (nx + 1) : off;
+    NodeRow<T> row;
+    row.load(i, A, Dinv);
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
+    const Vec2<T> bv = lv2(b, i);
+    for (int l = t; l < W2 * W2; l += kTileThreads) {
+        const int hx = gx0 - 2 + l % W2, hy = gy0 - 2 + l / W2;
         Vec2<T> v;
         v.x = v.y = 0;
-        if (gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) {
-            const int i = off + gx + gy * (nx + 1);
-            v = ld2(x, i);
-            const Vec2<T> e = interpolate(gx, gy, p, xc);
-            if (!fixed[2 * i]) v.x += e.x;
-            if (!fixed[2 * i + 1]) v.y += e.y;
+        if (hx >= 0 && hx <= nx && hy >= 0 && hy <= ny) {
+            const int h = off + hx + hy * (nx + 1);
+            v = lv2(x, h);
+            const Vec2<T> e = interpolate(hx, hy, p, xc);
+            if (!fixed[2 * h]) v.x += e.x;
+            if (!fixed[2 * h + 1]) v.y += e.y;
         }
         s2[l] = v;
     }
     __syncthreads();
-    for (int l = threadIdx.x; l < W1 * W1; l += kTileThreads) {
-        const int lx = l % W1, ly = l / W1, gx = gx0 - 1 + lx, gy = gy0 - 1 + ly;
+    const int c = (ly + 1) * W2 + lx + 1;
+    if (t < W1 * W1) {
         Vec2<T> v;
         v.x = v.y = 0;
-        if (gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) {
-            const int i = off + gx + gy * (nx + 1), c = (ly + 1) * W2 + lx + 1;
-            T y0, y1;
-            stencil<T, W2>(A, i, s2, c, y0, y1);
-            v = sweep_node<T>(i, Dinv, fixed, b, s2[c], y0, y1);
-        }
-        s1[l] = v;
+        if (in) v = row.relax(s2[c], row.residual(bv, s2, c, W2));
+        s1[t] = v;
     }
     __syncthreads();
-    for (int l = threadIdx.x; l < W0 * W0; l += kTileThreads) {
-        const int lx = l % W0, ly = l / W0, gx = gx0 + lx, gy = gy0 + ly;
-        if (gx > nx || gy > ny) continue;
-        const int i = off + gx + gy * (nx + 1), c = (ly + 1) * W1 + lx + 1;
-        T y0, y1;
-        stencil<T, W1>(A, i, s1, c, y0, y1);
-        const Vec2<T> v = sweep_node<T>(i, Dinv, fixed, b, s1[c], y0, y1);
-        if (FINE) s0[l] = v;
+    if (in && lx >= 1 && lx <= W0 && ly >= 1 && ly <= W0) {
+        const Vec2<T> v = row.relax(s1[t], row.residual(bv, s1, t, W1));
+        if (FINE) s0[(ly - 1) * W0 + lx - 1] = v;
         else st2(xo, i, v.x, v.y);
     }
     if (!FINE) return;
@@ -750,16 +867,15 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_mg_up(const int4* __restric
         const int gx = 2 * gx0 + l % F, gy = 2 * gy0 + l / F;
         if (gx > pf.fnx || gy > pf.fny) continue;
         int I0, I1, J0, J1;
-        T w;
-        parents<T>(gx, pf.fnx, I0, I1, w);
-        parents<T>(gy, pf.fny, J0, J1, w);
+        parents(gx, pf.fnx, I0, I1);
+        parents(gy, pf.fny, J0, J1);
         I0 -= gx0;
         I1 -= gx0;
         J0 -= gy0;
         J1 -= gy0;
         const Vec2<T> a = s0[J0 * W0 + I0], bq = s0[J0 * W0 + I1], c = s0[J1 * W0 + I0], d = s0[J1 * W0 + I1];
         const int i = pf.foff + gx + gy * (pf.fnx + 1);
-        Vec2<T> v = ld2((const T*)x0, i);
+        Vec2<T> v = lv2(x0, i);
         if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + bq.x) + (c.x + d.x));
         if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + bq.y) + (c.y + d.y));
         st2(x0, i, v.x, v.y);
@@ -767,10 +883,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_mg_up(const int4* __restric
 }
 
 // The levels of at most kBottomNodes nodes of one RVE, down to the coarsest
-// and back, in one CTA: operators and vectors staged in shared memory, value
-// by value (each of a block's four numbers of all nodes together, so that
-// the threads of a warp, one node each, read neighbouring words), a block
-// barrier between the phases.  Bound by the latency of its ~16 phases.
+// and back, in one CTA.  Every thread owns one node of one level (a level
+// starts at a warp boundary): its operator row, its place in the transfers
+// and its masks are in registers before the wait, and shared memory holds the
+// vectors alone.  Bound by the latency of its 16 or so phases, each a block
+// barrier and one node's arithmetic.  (With the operators staged in shared
+// memory and a loop over each level's nodes the phases took 11 us of 16.)
 constexpr int kBottomNodes = 300;
 constexpr int kBottomThreads = 512;
 constexpr int kBottomLevels = 8;
@@ -778,9 +896,16 @@ constexpr int kBottomLevels = 8;
 struct Bottom {
     int nlev, first;                       // levels, and the first one's number in the hierarchy
     int nx[kBottomLevels], ny[kBottomLevels], off[kBottomLevels];
+    int thread[kBottomLevels];             // first thread of each level but the coarsest
+    int vec[kBottomLevels];                // and its place in the shared vectors
     int foff, fnx, fny;                    // the grid its result is interpolated to when `first` is level 1
-    int pad;
 };
+// Its vectors (right-hand sides, two iterates, the residual of every level):
+// at most so many nodes each, with a margin on both sides, as a boundary
+// node's row of (zero) blocks reads up to a line of nodes past its level.
+constexpr int kBottomVec = 544, kBottomPad = 160, kBottomStride = kBottomVec + 2 * kBottomPad;
+static_assert(kBottomVec >= kBottomThreads + (kCoarseCells + 1) * (kCoarseCells + 1), "room for every thread's node");
+static_assert(kBottomPad > kBottomNodes / 2 + 1, "a line of the narrowest level");
 
 template <typename T>
 struct BottomArrays {                      // of the hierarchy's levels, by number
@@ -791,198 +916,175 @@ struct BottomArrays {                      // of the hierarchy's levels, by numb
     T* xo[17];
 };
 
-__host__ __device__ inline size_t bottom_level_bytes(int n, size_t t, bool coarsest) {
-    return ((coarsest ? 0 : (size_t)40 * n) + (size_t)8 * n) * t + (((size_t)2 * n + 15) & ~(size_t)15);
-}
-
-template <typename T>
-__device__ __forceinline__ void bottom_stencil(const T* sA, int n, int nx, int i, const Vec2<T>* x, T& y0, T& y1) {
-    y0 = y1 = 0;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        // out-of-grid blocks are zero; the neighbour's index is kept within the level
-        const int j = min(max(i + (q / 3 - 1) * (nx + 1) + q % 3 - 1, 0), n - 1);
-        const Vec2<T> v = x[j];
-        y0 += sA[(4 * q) * n + i] * v.x + sA[(4 * q + 1) * n + i] * v.y;
-        y1 += sA[(4 * q + 2) * n + i] * v.x + sA[(4 * q + 3) * n + i] * v.y;
-    }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const Bottom* __restrict__ bottoms, BottomArrays<T> ar,
                                                               const double* __restrict__ XT,
-                                                              const uint8_t* __restrict__ fixed0, T* __restrict__ x0,
-                                                              const int* fl) {
+                                                              const uint8_t* __restrict__ fixed0, T* x0, const int* fl) {
+    constexpr int kPad = kBottomPad;
     extern __shared__ __align__(16) unsigned char bottom_smem[];
+    Vec2<T>* s_vec = reinterpret_cast<Vec2<T>*>(bottom_smem);
     __shared__ Bottom B;
     __shared__ double s_inv[kCoarseStride];
     __shared__ double s_rhs[kCoarseMaxDof];
     __shared__ double s_part[8][64];
-    const int r = blockIdx.x, tid = threadIdx.x;
-    if (tid < (int)(sizeof(Bottom) / sizeof(int)))
-        reinterpret_cast<int*>(&B)[tid] = reinterpret_cast<const int*>(&bottoms[r])[tid];
-    __syncthreads();
-    if (fl && fl[kFlags * r]) return;
-    T* sA[kBottomLevels];
-    Vec2<T>* sv[kBottomLevels];  // b, x, x', residual
-    uint8_t* sf[kBottomLevels];
-    unsigned char* at = bottom_smem;
-    for (int k = 0; k < B.nlev; ++k) {
-        const int n = (B.nx[k] + 1) * (B.ny[k] + 1), l = B.first + k;
-        const bool coarsest = k == B.nlev - 1;
-        sv[k] = reinterpret_cast<Vec2<T>*>(at);
-        sA[k] = reinterpret_cast<T*>(sv[k] + 4 * n);
-        sf[k] = reinterpret_cast<uint8_t*>(sA[k] + (coarsest ? 0 : 40 * n));
-        at += bottom_level_bytes(n, sizeof(T), coarsest);
-        if (!coarsest) {
-            const T* A = ar.A[l] + 36 * (size_t)B.off[k];
-            const T* D = ar.Dinv[l] + 4 * (size_t)B.off[k];
-            for (int q = tid; q < 36 * n; q += kBottomThreads) sA[k][(q % 36) * n + q / 36] = A[q];
-            for (int q = tid; q < 4 * n; q += kBottomThreads) sA[k][(36 + q % 4) * n + q / 4] = D[q];
-        }
-        const uint8_t* f = ar.fixed[l] + 2 * (size_t)B.off[k];
-        for (int q = tid; q < 2 * n; q += kBottomThreads) sf[k][q] = f[q];
+    const int r = blockIdx.x, t = threadIdx.x;
+    if (t < (int)(sizeof(Bottom) / sizeof(int)))
+        reinterpret_cast<int*>(&B)[t] = reinterpret_cast<const int*>(&bottoms[r])[t];
+    for (int q = t; q < 4 * kBottomStride; q += kBottomThreads) {
+        Vec2<T> z;
+        z.x = z.y = 0;
+        s_vec[q] = z;
     }
+    __syncthreads();
     const int kc = B.nlev - 1, nc = 2 * (B.nx[kc] + 1) * (B.ny[kc] + 1);
-    for (int q = tid; q < nc * nc; q += kBottomThreads) s_inv[q] = XT[(size_t)r * kCoarseStride + q];
+    // the thread's node
+    int lev = -1;
+    for (int k = 0; k < kc; ++k)
+        if (t >= B.thread[k]) lev = k;
+    int node = 0, W = 1, nx = 0, ny = 0;
+    if (lev >= 0) {
+        nx = B.nx[lev];
+        ny = B.ny[lev];
+        W = nx + 1;
+        node = t - B.thread[lev];
+        if (node >= W * (ny + 1)) lev = -1;
+    }
+    NodeRow<T> row;
+    int at = kPad, cat = kPad;             // of the node, and of its level's coarser one, in the vectors
+    int pa = 0, pb = 0, pc = 0, pd = 0;    // its parents there
+    bool f0 = true, f1 = true;             // its masks
+    int cn = -1, fat = 0;                  // the coarse node it restricts to: number, and its place on this level
+    T wx[3], wy[3];
+    bool cf0 = true, cf1 = true;
+    if (lev >= 0) {
+        const int l = B.first + lev, gx = node % W, gy = node / W;
+        row.load(B.off[lev] + node, ar.A[l], ar.Dinv[l]);
+        f0 = ar.fixed[l][2 * (size_t)(B.off[lev] + node)];
+        f1 = ar.fixed[l][2 * (size_t)(B.off[lev] + node) + 1];
+        at = kPad + B.vec[lev] + node;
+        cat = kPad + B.vec[lev + 1];
+        const int cW = B.nx[lev + 1] + 1, cN = cW * (B.ny[lev + 1] + 1);
+        int I0, I1, J0, J1;
+        parents(gx, nx, I0, I1);
+        parents(gy, ny, J0, J1);
+        pa = cat + I0 + J0 * cW;
+        pb = cat + I1 + J0 * cW;
+        pc = cat + I0 + J1 * cW;
+        pd = cat + I1 + J1 * cW;
+        if (node < cN) {                   // a level has at least as many nodes as the one below it
+            cn = node;
+            const int px = grid_pos(cn % cW, nx), py = grid_pos(cn / cW, ny);
+            side_weights(px, nx, wx[0], wx[2]);
+            side_weights(py, ny, wy[0], wy[2]);
+            wx[1] = wy[1] = (T)1;
+            fat = kPad + B.vec[lev] + px + py * W;
+            cf0 = ar.fixed[l + 1][2 * (size_t)(B.off[lev + 1] + cn)];
+            cf1 = ar.fixed[l + 1][2 * (size_t)(B.off[lev + 1] + cn) + 1];
+        }
+    }
+    for (int q = t; q < nc * nc; q += kBottomThreads) s_inv[q] = XT[(size_t)r * kCoarseStride + q];
+    Vec2<T>*vb = s_vec, *v1 = vb + kBottomStride, *v2 = v1 + kBottomStride, *vr = v2 + kBottomStride;
+    pdl_wait();
+    pdl_trigger();
+    if (fl && __ldcg(&fl[kFlags * r])) return;
     {
         const int n = (B.nx[0] + 1) * (B.ny[0] + 1);
-        for (int i = tid; i < n; i += kBottomThreads) sv[0][i] = ld2(ar.b[B.first], B.off[0] + i);
+        if (t < n) vb[kPad + B.vec[0] + t] = lv2(ar.b[B.first], B.off[0] + t);
     }
     __syncthreads();
+    Vec2<T> b, x;
+    b.x = b.y = x.x = x.y = 0;
     for (int k = 0; k < kc; ++k) {
-        const int nx = B.nx[k], ny = B.ny[k], n = (nx + 1) * (ny + 1);
-        const T* D = sA[k] + 36 * n;
-        Vec2<T>*b = sv[k], *x = b + n, *x2 = x + n, *rs = x2 + n;
-        auto sweep = [&](int i, Vec2<T> v, T y0, T y1) {
-            const T r0 = sf[k][2 * i] ? (T)0 : b[i].x - y0, r1 = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
-            v.x += (T)kOmega * (D[i] * r0 + D[n + i] * r1);
-            v.y += (T)kOmega * (D[2 * n + i] * r0 + D[3 * n + i] * r1);
-            return v;
-        };
-        for (int i = tid; i < n; i += kBottomThreads) {
-            Vec2<T> v;
-            v.x = v.y = 0;
-            x2[i] = sweep(i, v, (T)0, (T)0);
+        const bool mine = lev == k;
+        if (mine) {
+            Vec2<T> z;
+            z.x = z.y = 0;
+            b = vb[at];
+            x = row.relax(z, b);
+            v1[at] = x;
         }
         __syncthreads();
-        for (int i = tid; i < n; i += kBottomThreads) {
-            T y0, y1;
-            bottom_stencil(sA[k], n, nx, i, x2, y0, y1);
-            x[i] = sweep(i, x2[i], y0, y1);
+        if (mine) {
+            x = row.relax(x, row.residual(b, v1, at, W));
+            v2[at] = x;
         }
         __syncthreads();
-        for (int i = tid; i < n; i += kBottomThreads) {
-            T y0, y1;
-            bottom_stencil(sA[k], n, nx, i, x, y0, y1);
-            Vec2<T> v;
-            v.x = sf[k][2 * i] ? (T)0 : b[i].x - y0;
-            v.y = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
-            rs[i] = v;
-        }
+        if (mine) vr[at] = row.residual(b, v2, at, W);
         __syncthreads();
-        const int cx = B.nx[k + 1], cn = (cx + 1) * (B.ny[k + 1] + 1);
-        for (int a = tid; a < cn; a += kBottomThreads) {
-            const int I = a % (cx + 1), J = a / (cx + 1);
-            const int px = grid_pos(I, nx), py = grid_pos(J, ny);
+        if (mine && cn >= 0) {
             T s0 = 0, s1 = 0;
 #pragma unroll
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int gy = py + dy;
-                if (gy < 0 || gy > ny) continue;
-                const T wy = (T)grid_w(gy, ny, J);
+            for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
                 for (int dx = -1; dx <= 1; ++dx) {
-                    const int gx = px + dx;
-                    if (gx < 0 || gx > nx) continue;
-                    const T w = wy * (T)grid_w(gx, nx, I);
-                    const Vec2<T> v = rs[gx + gy * (nx + 1)];
+                    const T w = wy[dy + 1] * wx[dx + 1];
+                    const Vec2<T> v = vr[fat + dx + dy * W];
                     s0 += w * v.x;
                     s1 += w * v.y;
                 }
-            }
             Vec2<T> v;
-            v.x = sf[k + 1][2 * a] ? (T)0 : s0;
-            v.y = sf[k + 1][2 * a + 1] ? (T)0 : s1;
-            sv[k + 1][a] = v;
+            v.x = cf0 ? (T)0 : s0;
+            v.y = cf1 ? (T)0 : s1;
+            vb[cat + cn] = v;
         }
         __syncthreads();
     }
     // the coarsest grid: x = X b with the explicit masked inverse, eight threads per DOF
     {
-        const int n = nc / 2;
-        const T* b = reinterpret_cast<const T*>(sv[kc]);
-        T* x = reinterpret_cast<T*>(sv[kc] + n);
-        for (int q = tid; q < nc; q += kBottomThreads) s_rhs[q] = sf[kc][q] ? 0.0 : (double)b[q];
+        const T* bc = reinterpret_cast<const T*>(vb + kPad + B.vec[kc]);
+        T* xc = reinterpret_cast<T*>(v2 + kPad + B.vec[kc]);
+        if (t < nc) s_rhs[t] = (double)bc[t];
         __syncthreads();
-        const int q = tid % 64, part = tid / 64;
+        const int q = t % 64, part = t / 64;
         double acc = 0.0;
         if (q < nc)
             for (int j = part; j < nc; j += kBottomThreads / 64) acc += s_inv[j * nc + q] * s_rhs[j];
         s_part[part][q] = acc;
         __syncthreads();
-        if (tid < nc) {
+        if (t < nc) {
             double v = 0.0;
 #pragma unroll
-            for (int k = 0; k < kBottomThreads / 64; ++k) v += s_part[k][tid];
-            x[tid] = sf[kc][tid] ? (T)0 : (T)v;
+            for (int k = 0; k < kBottomThreads / 64; ++k) v += s_part[k][t];
+            xc[t] = (T)v;
         }
         __syncthreads();
     }
     for (int k = kc - 1; k >= 0; --k) {
-        const int nx = B.nx[k], ny = B.ny[k], n = (nx + 1) * (ny + 1);
-        const T* D = sA[k] + 36 * n;
-        Vec2<T>*b = sv[k], *x = b + n, *x2 = x + n;
-        const int cx = B.nx[k + 1], cn = (cx + 1) * (B.ny[k + 1] + 1);
-        const Vec2<T>* xc = sv[k + 1] + cn;
-        auto sweep = [&](int i, Vec2<T> v, T y0, T y1) {
-            const T r0 = sf[k][2 * i] ? (T)0 : b[i].x - y0, r1 = sf[k][2 * i + 1] ? (T)0 : b[i].y - y1;
-            v.x += (T)kOmega * (D[i] * r0 + D[n + i] * r1);
-            v.y += (T)kOmega * (D[2 * n + i] * r0 + D[3 * n + i] * r1);
-            return v;
-        };
-        for (int i = tid; i < n; i += kBottomThreads) {
-            int I0, I1, J0, J1;
-            T w;
-            parents<T>(i % (nx + 1), nx, I0, I1, w);
-            parents<T>(i / (nx + 1), ny, J0, J1, w);
-            const Vec2<T> a = xc[I0 + J0 * (cx + 1)], bb = xc[I1 + J0 * (cx + 1)];
-            const Vec2<T> c = xc[I0 + J1 * (cx + 1)], d = xc[I1 + J1 * (cx + 1)];
-            if (!sf[k][2 * i]) x[i].x += (T)0.25 * ((a.x + bb.x) + (c.x + d.x));
-            if (!sf[k][2 * i + 1]) x[i].y += (T)0.25 * ((a.y + bb.y) + (c.y + d.y));
+        const bool mine = lev == k;
+        if (mine) {
+            const Vec2<T> a = v2[pa], bq = v2[pb], c = v2[pc], d = v2[pd];
+            if (!f0) x.x += (T)0.25 * ((a.x + bq.x) + (c.x + d.x));
+            if (!f1) x.y += (T)0.25 * ((a.y + bq.y) + (c.y + d.y));
+            vr[at] = x;
         }
         __syncthreads();
-        for (int i = tid; i < n; i += kBottomThreads) {
-            T y0, y1;
-            bottom_stencil(sA[k], n, nx, i, x, y0, y1);
-            x2[i] = sweep(i, x[i], y0, y1);
+        if (mine) {
+            x = row.relax(x, row.residual(b, vr, at, W));
+            v1[at] = x;
         }
         __syncthreads();
-        for (int i = tid; i < n; i += kBottomThreads) {
-            T y0, y1;
-            bottom_stencil(sA[k], n, nx, i, x2, y0, y1);
-            x[i] = sweep(i, x2[i], y0, y1);
+        if (mine) {
+            x = row.relax(x, row.residual(b, v1, at, W));
+            v2[at] = x;
         }
         __syncthreads();
     }
-    const int nx = B.nx[0], n0 = (nx + 1) * (B.ny[0] + 1);
-    const Vec2<T>* x = sv[0] + n0;
+    const int n0 = (B.nx[0] + 1) * (B.ny[0] + 1);
+    const Vec2<T>* xr = v2 + kPad + B.vec[0];
     if (B.first > 1) {
-        for (int i = tid; i < n0; i += kBottomThreads) st2(ar.xo[B.first], B.off[0] + i, x[i].x, x[i].y);
+        if (t < n0) st2(ar.xo[B.first], B.off[0] + t, xr[t].x, xr[t].y);
         return;
     }
-    const int nf = (B.fnx + 1) * (B.fny + 1);
-    for (int l = tid; l < nf; l += kBottomThreads) {
+    const int W0 = B.nx[0] + 1, nf = (B.fnx + 1) * (B.fny + 1);
+    for (int l = t; l < nf; l += kBottomThreads) {
         int I0, I1, J0, J1;
-        T w;
-        parents<T>(l % (B.fnx + 1), B.fnx, I0, I1, w);
-        parents<T>(l / (B.fnx + 1), B.fny, J0, J1, w);
-        const Vec2<T> a = x[I0 + J0 * (nx + 1)], b = x[I1 + J0 * (nx + 1)];
-        const Vec2<T> c = x[I0 + J1 * (nx + 1)], d = x[I1 + J1 * (nx + 1)];
+        parents(l % (B.fnx + 1), B.fnx, I0, I1);
+        parents(l / (B.fnx + 1), B.fny, J0, J1);
+        const Vec2<T> a = xr[I0 + J0 * W0], bq = xr[I1 + J0 * W0], c = xr[I0 + J1 * W0], d = xr[I1 + J1 * W0];
         const int i = B.foff + l;
-        Vec2<T> v = ld2((const T*)x0, i);
-        if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + b.x) + (c.x + d.x));
-        if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + b.y) + (c.y + d.y));
+        Vec2<T> v = lv2(x0, i);
+        if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + bq.x) + (c.x + d.x));
+        if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + bq.y) + (c.y + d.y));
         st2(x0, i, v.x, v.y);
     }
 }
