@@ -21,7 +21,7 @@ SOURCES = ["igfem_host.cpp", "pg_assemble.cu", "pg_solve.cu", "pg_newton.cu", "p
 # operation on its own, as the host builder does (no FMA contraction)
 EXTRA_FLAGS = {"pg_mesh_gpu.cu": ["-fmad=false"]}
 HEADERS = ["igfem_host.h", "pg_internal.cuh", "pg_solve_kernels.cuh", "pg_mg_kernels.cuh",
-           "pg_pdl.cuh"]
+           "pg_pdl.cuh", "pg_pcg_cluster.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -190,6 +190,8 @@ struct Ctx {
     int n_fold_f = 0;
     int* coh_rec = nullptr;            // per cohesive point: class-ordered element << 8 | sub-element << 1 | point
     double* coh_rows = nullptr;        // per cohesive point: kCohRowDoubles FP64 (k_coh_points)
+    // the one-launch CG's cut of the rows (its largest part; cluster_halo < 0: not looked at yet)
+    int cluster_rows = 0, cluster_blocks = 0, cluster_halo = -1;
     MgHierarchy* mg = nullptr;         // multigrid hierarchy, built at the first multigrid solve
     // system
     double* K = nullptr;               // 4 * n_blocks
