@@ -15,6 +15,15 @@
 // bounded; on timeout the kernel records an error, frees its tensor memory
 // and returns.
 //
+// A tile is a chain of GEMMs that wait for one another, so what counts is how
+// many tiles an SM has in flight.  Inference (k_mlp_forward) therefore has a
+// kernel of its own with one 16 KB operand buffer and 64 columns of tensor
+// memory per CTA, seven CTAs per SM: 1.13M rows in 56 us (bound by the
+// shared-memory and tensor-memory path), where the training
+// kernel's shape (182 KB, 512 columns, one CTA per SM) took 170.  The BF16
+// operand images of the weights are kept beside the FP32 masters (k_pack and
+// the optimizer step write them), so a CTA copies them instead of converting.
+//
 // Weight gradients: dW2 and dW1 come out of one M=128 GEMM whose A stacks
 // dZ2^T over dZ1^T and whose B stacks H1^T over X^T (the off-diagonal blocks
 // are not read); dW3 uses A = [dY^T; 0].  They accumulate in tensor memory
@@ -23,6 +32,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -31,6 +41,7 @@
 #include <vector>
 
 #include "pg_internal.cuh"
+#include "pg_pdl.cuh"
 
 namespace pgb {
 namespace mlp {
@@ -38,28 +49,40 @@ namespace mlp {
 constexpr int IN = 16, HID = 64, OUT = 16, USED = 2, TILE = 128, NT = 128;
 constexpr uint32_t TMEM_COLS = 512;
 // tensor-memory columns
-constexpr uint32_t C_Z1 = 0, C_Z2 = 64, C_Y = 128, C_DW12 = 256, C_DW3 = 384;
+constexpr uint32_t C_Z1 = 0, C_Z2 = 64, C_DW12 = 256, C_DW3 = 384, C_Y = 128;
 
-// shared-memory map (bytes from the 1024-aligned dynamic base)
-constexpr uint32_t O_X = 0;                       // A 128 x 16        4 KB
-constexpr uint32_t O_W1 = O_X + 4096;             // B  64 x 16        2 KB
-constexpr uint32_t O_H1 = O_W1 + 2048;            // A 128 x 64       16 KB
-constexpr uint32_t O_W2 = O_H1 + 16384;           // B  64 x 64        8 KB
-constexpr uint32_t O_H2 = O_W2 + 8192;            // A 128 x 64       16 KB
-constexpr uint32_t O_W3 = O_H2 + 16384;           // B  16 x 64        2 KB
-constexpr uint32_t O_DY = O_W3 + 2048;            // A 128 x 16        4 KB
-constexpr uint32_t O_W3T = O_DY + 4096;           // B  64 x 16        2 KB
-constexpr uint32_t O_DZ2 = O_W3T + 2048;          // A 128 x 64       16 KB
-constexpr uint32_t O_W2T = O_DZ2 + 16384;         // B  64 x 64        8 KB
-constexpr uint32_t O_AT = O_W2T + 8192;           // A 128 x 128 (dZ2^T ; dZ1^T)   32 KB
+// BF16 operand images of the weights (bytes from the image's start): W1, W2,
+// W3, then the transposes the backward pass multiplies by
+constexpr uint32_t P_W1 = 0;                      // B  64 x 16        2 KB
+constexpr uint32_t P_W2 = P_W1 + 2048;            // B  64 x 64        8 KB
+constexpr uint32_t P_W3 = P_W2 + 8192;            // B  16 x 64        2 KB
+constexpr uint32_t P_FORWARD = P_W3 + 2048;       // what inference needs
+constexpr uint32_t P_W3T = P_FORWARD;             // B  64 x 16        2 KB
+constexpr uint32_t P_W2T = P_W3T + 2048;          // B  64 x 64        8 KB
+constexpr uint32_t P_BYTES = P_W2T + 8192;
+
+// shared-memory map of the training kernel (bytes from the 1024-aligned dynamic base)
+constexpr uint32_t O_W = 0;                       // the image
+constexpr uint32_t O_W1 = O_W + P_W1, O_W2 = O_W + P_W2, O_W3 = O_W + P_W3, O_W3T = O_W + P_W3T, O_W2T = O_W + P_W2T;
+constexpr uint32_t O_X = O_W + 22528;             // A 128 x 16        4 KB
+constexpr uint32_t O_H1 = O_X + 4096;             // A 128 x 64       16 KB
+constexpr uint32_t O_H2 = O_H1 + 16384;           // A 128 x 64       16 KB
+constexpr uint32_t O_DY = O_H2 + 16384;           // A 128 x 16        4 KB
+constexpr uint32_t O_DZ2 = O_DY + 4096;           // A 128 x 64       16 KB
+constexpr uint32_t O_AT = O_DZ2 + 16384;          // A 128 x 128 (dZ2^T ; dZ1^T)   32 KB
 constexpr uint32_t O_BT = O_AT + 32768;           // B  80 x 128 (H1^T ; X^T)      20 KB
 constexpr uint32_t O_A3 = O_BT + 20480;           // A 128 x 128 (dY^T ; 0)        32 KB
 constexpr uint32_t O_B3 = O_A3 + 32768;           // B  64 x 128 (H2^T)            16 KB
-constexpr uint32_t SMEM_BYTES = O_B3 + 16384;     // 182 KB
+static_assert(P_BYTES <= O_X - O_W, "the image's place");
 // The allocation also covers O_B3 + 32 KB: every operand's core-matrix grid
 // (rows/8 x K/8 groups of 128 B) read with either stride interpretation stays
 // inside the allocation.
 constexpr uint32_t SMEM_ALLOC = O_B3 + 32768 + 1024;
+// and of the inference kernel: the image, one A operand (X, H1 and H2 in turn), the biases
+constexpr uint32_t F_W = 0, F_A = F_W + P_FORWARD, F_B = F_A + 16384;
+constexpr uint32_t F_ALLOC = F_B + 4 * (HID + HID + OUT) + 1024;
+constexpr uint32_t F_COLS = 64;
+constexpr int kForwardCtasPerSm = 7;
 
 struct Params {
     float* W1; float* b1; float* W2; float* b2; float* W3; float* b3;
@@ -67,6 +90,7 @@ struct Params {
 
 constexpr int kW1 = HID * IN, kB1 = HID, kW2 = HID * HID, kB2 = HID, kW3 = OUT * HID, kB3 = OUT;
 constexpr int kNParams = kW1 + kB1 + kW2 + kB2 + kW3 + kB3;
+constexpr int kParamBlocks = (kNParams + 255) / 256;  // of 256 threads, one per parameter
 
 __host__ __device__ inline Params carve(float* base) {
     Params q;
@@ -168,6 +192,29 @@ __device__ __forceinline__ void st_row(uint8_t* base, int row, const float* v, i
     }
 }
 
+// parameter i as BF16 into its places in the operand images
+__device__ __forceinline__ void pack_param(uint8_t* img, int i, float v) {
+    if (i < kW1) {
+        st_bf16(img, P_W1 + kmaj(i / IN, i % IN, IN), v);
+        return;
+    }
+    i -= kW1 + kB1;
+    if (i >= 0 && i < kW2) {
+        st_bf16(img, P_W2 + kmaj(i / HID, i % HID, HID), v);
+        st_bf16(img, P_W2T + kmaj(i % HID, i / HID, HID), v);
+    }
+    i -= kW2 + kB2;
+    if (i >= 0 && i < kW3) {
+        st_bf16(img, P_W3 + kmaj(i / HID, i % HID, HID), v);
+        st_bf16(img, P_W3T + kmaj(i % HID, i / HID, OUT), v);
+    }
+}
+
+__global__ void k_pack(const float* p, uint8_t* img) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kNParams) pack_param(img, i, p[i]);
+}
+
 // How the completion waits of one launch behave: polls before a wait gives
 // up, and (self-test only) a GEMM whose MMAs are not issued, so that nothing
 // ever arrives on its mbarrier and its wait must run out.
@@ -207,16 +254,201 @@ __device__ __forceinline__ bool gemm(uint32_t sbase, uint32_t a_off, uint32_t b_
     return ok;
 }
 
-// Training (kTrain) or inference pass over n rows.  Training writes this
-// CTA's gradient (kNParams floats, summed over its tiles) to gpart + CTA *
-// kNParams and its share of the loss to lpart[CTA]; k_grad_sum adds the CTAs'
-// parts in CTA order.  Every sum inside a CTA has a fixed order too (warp
-// butterflies, then the four warps in order, then the tiles in order), so a
-// gradient is the same bits on every run.
-template <bool kTrain>
-__global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, const float* __restrict__ T, int n,
-                                               Params p, float* gpart, float* Y_out, double* lpart, int* err,
-                                               WaitCfg wc) {
+__device__ __forceinline__ void mbar_init(uint32_t mbar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(1));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+template <uint32_t COLS>
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(slot)),
+                 "r"(COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+template <uint32_t COLS>
+__device__ __forceinline__ void tmem_free(uint32_t tmem) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
+}
+
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float* v) {
+    uint32_t r0, r1;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    v[0] = __uint_as_float(r0);
+    v[1] = __uint_as_float(r1);
+}
+
+// 32 consecutive columns of the thread's row
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+#define PG_R(i) "=r"(r[i])
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : PG_R(0), PG_R(1), PG_R(2), PG_R(3), PG_R(4), PG_R(5), PG_R(6), PG_R(7), PG_R(8), PG_R(9), PG_R(10), PG_R(11),
+          PG_R(12), PG_R(13), PG_R(14), PG_R(15), PG_R(16), PG_R(17), PG_R(18), PG_R(19), PG_R(20), PG_R(21), PG_R(22),
+          PG_R(23), PG_R(24), PG_R(25), PG_R(26), PG_R(27), PG_R(28), PG_R(29), PG_R(30), PG_R(31)
+        : "r"(taddr));
+#undef PG_R
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The thread's share of a tile of X, 16 floats.  VEC (X is 16-byte aligned):
+// four 16-byte loads, each of a warp's 32 covering 512 consecutive bytes, so
+// its share is a quarter of the rows 32 warp + 8 k + lane / 4; otherwise its
+// own row.
+template <bool VEC>
+__device__ __forceinline__ void load_x(const float* __restrict__ X, int tile, int n, float* x) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (VEC) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = tile * TILE + 32 * warp + 8 * k + lane / 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < n) v = __ldg(reinterpret_cast<const float4*>(X + (size_t)row * IN) + lane % 4);
+            x[4 * k] = v.x;
+            x[4 * k + 1] = v.y;
+            x[4 * k + 2] = v.z;
+            x[4 * k + 3] = v.w;
+        }
+    } else {
+        const int row = tile * TILE + tid;
+#pragma unroll
+        for (int i = 0; i < IN; ++i) x[i] = row < n ? X[(size_t)row * IN + i] : 0.f;
+    }
+}
+// and into the A operand
+template <bool VEC>
+__device__ __forceinline__ void store_x(uint8_t* base, const float* x) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (VEC) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            __align__(8) __nv_bfloat162 h[2];
+            h[0] = __floats2bfloat162_rn(x[4 * k], x[4 * k + 1]);
+            h[1] = __floats2bfloat162_rn(x[4 * k + 2], x[4 * k + 3]);
+            *reinterpret_cast<uint2*>(base + kmaj(32 * warp + 8 * k + lane / 4, 4 * (lane % 4), IN)) =
+                *reinterpret_cast<const uint2*>(h);
+        }
+    } else {
+        st_row(base, tid, x, IN);
+    }
+}
+
+// Inference over n rows.  The next tile's row is loaded while this one's
+// GEMMs run; a layer is read back 32 columns at a time and stored at once as
+// the next layer's operand, over the one the finished GEMM has read.
+template <bool VEC>
+__global__ void __launch_bounds__(NT, kForwardCtasPerSm) k_mlp_forward(const float* __restrict__ X, int n, Params p,
+                                                                       const uint4* __restrict__ img, float* Y_out, int* err,
+                                                                       WaitCfg wc) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
+    __shared__ __align__(8) uint64_t mbar_storage;
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(&mbar_storage);
+    float* sb = reinterpret_cast<float*>(sm + F_B);  // b1, b2, b3
+    const int ntiles = (n + TILE - 1) / TILE;
+    float x[IN];
+    load_x<VEC>(X, blockIdx.x, n, x);
+    for (uint32_t i = tid; i < P_FORWARD / 16; i += NT) reinterpret_cast<uint4*>(sm + F_W)[i] = img[i];
+    if (tid < HID) {
+        sb[tid] = p.b1[tid];
+        sb[HID + tid] = p.b2[tid];
+    }
+    if (tid < OUT) sb[2 * HID + tid] = p.b3[tid];
+    if (tid == 0) mbar_init(mbar);
+    if (warp == 0) tmem_alloc<F_COLS>(&tmem_slot);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_slot;
+    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    uint32_t phase = 0;
+    bool ok = true;
+    int gi = 0;             // GEMMs issued so far (WaitCfg::skip_gemm)
+    bool inflight = false;  // a timed-out wait left MMAs of this CTA pending
+    // relu(accumulator + bias) of the thread's row as the next operand
+    auto hidden = [&](const float* bias) {
+#pragma unroll
+        for (int c = 0; c < HID; c += 32) {
+            float z[32];
+            tmem_ld32(tmem + lane_base + c, z);
+#pragma unroll
+            for (int q = 0; q < 32; q += 8) {
+                __align__(16) __nv_bfloat162 h[4];
+                const float4 b0 = *reinterpret_cast<const float4*>(bias + c + q);
+                const float4 b1 = *reinterpret_cast<const float4*>(bias + c + q + 4);
+                h[0] = __floats2bfloat162_rn(fmaxf(z[q] + b0.x, 0.f), fmaxf(z[q + 1] + b0.y, 0.f));
+                h[1] = __floats2bfloat162_rn(fmaxf(z[q + 2] + b0.z, 0.f), fmaxf(z[q + 3] + b0.w, 0.f));
+                h[2] = __floats2bfloat162_rn(fmaxf(z[q + 4] + b1.x, 0.f), fmaxf(z[q + 5] + b1.y, 0.f));
+                h[3] = __floats2bfloat162_rn(fmaxf(z[q + 6] + b1.z, 0.f), fmaxf(z[q + 7] + b1.w, 0.f));
+                *reinterpret_cast<uint4*>(sm + F_A + kmaj(tid, c + q, HID)) = *reinterpret_cast<const uint4*>(h);
+            }
+        }
+    };
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int row = tile * TILE + tid;
+        store_x<VEC>(sm + F_A, x);
+        load_x<VEC>(X, min(tile + (int)gridDim.x, ntiles), n, x);  // (past the last tile: nothing)
+        ok = gemm(sbase, F_A, F_W + P_W1, IN, HID, tmem, false, mbar, phase, wc, gi, inflight);
+        if (!ok) break;
+        hidden(sb);
+        ok = gemm(sbase, F_A, F_W + P_W2, HID, HID, tmem, false, mbar, phase, wc, gi, inflight);
+        if (!ok) break;
+        hidden(sb + HID);
+        ok = gemm(sbase, F_A, F_W + P_W3, HID, OUT, tmem, false, mbar, phase, wc, gi, inflight);
+        if (!ok) break;
+        float y[2];
+        tmem_ld2(tmem + lane_base, y);
+        if (row < n) {
+            const float y0 = y[0] + sb[2 * HID], y1 = y[1] + sb[2 * HID + 1];
+            if (VEC) {
+                *reinterpret_cast<float2*>(Y_out + 2 * (size_t)row) = make_float2(y0, y1);
+            } else {
+                Y_out[2 * (size_t)row] = y0;
+                Y_out[2 * (size_t)row + 1] = y1;
+            }
+        }
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    // MMAs still pending after a timed-out wait write tensor memory: wait for
+    // them (bounded again) before that memory is freed below
+    if (!ok && inflight) mbar_wait(mbar, phase, kPollLimit);
+    fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_free<F_COLS>(tmem);
+}
+
+// Sums of 32 values over a warp's lanes, all at once: lane l ends with the
+// sum of v[l], by the pairing of a butterfly (the lanes 16 apart first).  31
+// exchanges, where a butterfly per value takes 160.
+__device__ __forceinline__ float warp_sum32(float* v, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool hi = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = hi ? v[i] : v[i + o], keep = hi ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+// Training pass over n rows: this CTA's gradient (kNParams floats, summed
+// over its tiles) to gpart + CTA * kNParams and its share of the loss to
+// lpart[CTA]; the CTAs' parts are added in CTA order by the next kernel.
+// Every sum inside a CTA has a fixed order too (warp butterflies, then the
+// four warps in order, then the tiles in order), so a gradient is the same
+// bits on every run.
+__global__ void __launch_bounds__(NT, 1) k_mlp_train(const float* __restrict__ X, const float* __restrict__ T, int n,
+                                                     Params p, const uint4* img, float* gpart, double* lpart,
+                                                     int* err, WaitCfg wc) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
@@ -224,42 +456,27 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
     __shared__ uint32_t tmem_slot;
     constexpr int NB = HID + HID + OUT;  // bias gradients: b1, b2, b3
     __shared__ float sgb[NB];
+    __shared__ float sbias[NB];
     __shared__ float sloss;
     __shared__ float swarp[NT / 32][NB + 1];  // per warp: this tile's bias-gradient and loss sums
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(&mbar_storage);
 
-    // stage the weights as BF16 B operands (and transposes for the backward)
-    for (int i = tid; i < HID * IN; i += NT) {
-        const int o = i / IN, k = i % IN;
-        st_bf16(sm, O_W1 + kmaj(o, k, IN), p.W1[i]);
+    for (int i = tid; i < 32768 / 16; i += NT) reinterpret_cast<uint4*>(sm + O_A3)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < NB; i += NT) sgb[i] = 0.f;
+    for (int i = tid; i < (NT / 32) * (NB + 1); i += NT) (&swarp[0][0])[i] = 0.f;
+    if (tid == 0) sloss = 0.f;
+    if (tid == 0) mbar_init(mbar);
+    if (warp == 0) tmem_alloc<TMEM_COLS>(&tmem_slot);
+    // the minibatch before has stepped the network (and read the parts that this one writes)
+    pdl_wait();
+    pdl_trigger();
+    for (uint32_t i = tid; i < P_BYTES / 16; i += NT) reinterpret_cast<uint4*>(sm + O_W)[i] = __ldcg(&img[i]);
+    if (tid < HID) {
+        sbias[tid] = __ldcg(&p.b1[tid]);
+        sbias[HID + tid] = __ldcg(&p.b2[tid]);
     }
-    for (int i = tid; i < HID * HID; i += NT) {
-        const int o = i / HID, k = i % HID;
-        st_bf16(sm, O_W2 + kmaj(o, k, HID), p.W2[i]);
-        if (kTrain) st_bf16(sm, O_W2T + kmaj(k, o, HID), p.W2[i]);
-    }
-    for (int i = tid; i < OUT * HID; i += NT) {
-        const int o = i / HID, k = i % HID;
-        st_bf16(sm, O_W3 + kmaj(o, k, HID), p.W3[i]);
-        if (kTrain) st_bf16(sm, O_W3T + kmaj(k, o, OUT), p.W3[i]);
-    }
-    if (kTrain) {
-        for (int i = tid; i < 32768 / 16; i += NT) reinterpret_cast<uint4*>(sm + O_A3)[i] = make_uint4(0, 0, 0, 0);
-        for (int i = tid; i < NB; i += NT) sgb[i] = 0.f;
-        for (int i = tid; i < (NT / 32) * (NB + 1); i += NT) (&swarp[0][0])[i] = 0.f;
-        if (tid == 0) sloss = 0.f;
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(1));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(&tmem_slot)),
-                     "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    if (tid < OUT) sbias[2 * HID + tid] = __ldcg(&p.b3[tid]);
     fence_before();
     __syncthreads();
     fence_after();
@@ -275,52 +492,46 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
         const int row = tile * TILE + tid;
         const bool valid = row < n;
         float x[IN];
-#pragma unroll
-        for (int i = 0; i < IN; ++i) x[i] = valid ? X[(size_t)row * IN + i] : 0.f;
+        load_x<false>(X, tile, n, x);
         st_row(sm + O_X, tid, x, IN);
-        if (kTrain)
-            for (int i = 0; i < IN; ++i) st_bf16(sm, O_BT + kmaj(HID + i, tid, TILE), x[i]);
+#pragma unroll
+        for (int i = 0; i < IN; ++i) st_bf16(sm, O_BT + kmaj(HID + i, tid, TILE), x[i]);
         // ---- layer 1
         ok = gemm(sbase, O_X, O_W1, IN, HID, tmem + C_Z1, false, mbar, phase, wc, gi, inflight);
         if (!ok) break;
         float h1[HID];
         uint64_t m1 = 0;
-        for (int c = 0; c < HID; c += 16) tmem_ld16(tmem + lane_base + C_Z1 + c, h1 + c);
+        for (int c = 0; c < HID; c += 32) tmem_ld32(tmem + lane_base + C_Z1 + c, h1 + c);
+#pragma unroll
         for (int j = 0; j < HID; ++j) {
-            const float z = h1[j] + p.b1[j];
+            const float z = h1[j] + sbias[j];
             h1[j] = z > 0.f ? z : 0.f;
             if (z > 0.f) m1 |= (1ull << j);
         }
         st_row(sm + O_H1, tid, h1, HID);
-        if (kTrain)
-            for (int j = 0; j < HID; ++j) st_bf16(sm, O_BT + kmaj(j, tid, TILE), h1[j]);
+#pragma unroll
+        for (int j = 0; j < HID; ++j) st_bf16(sm, O_BT + kmaj(j, tid, TILE), h1[j]);
         // ---- layer 2
         ok = gemm(sbase, O_H1, O_W2, HID, HID, tmem + C_Z2, false, mbar, phase, wc, gi, inflight);
         if (!ok) break;
         float h2[HID];
         uint64_t m2 = 0;
-        for (int c = 0; c < HID; c += 16) tmem_ld16(tmem + lane_base + C_Z2 + c, h2 + c);
+        for (int c = 0; c < HID; c += 32) tmem_ld32(tmem + lane_base + C_Z2 + c, h2 + c);
+#pragma unroll
         for (int j = 0; j < HID; ++j) {
-            const float z = h2[j] + p.b2[j];
+            const float z = h2[j] + sbias[HID + j];
             h2[j] = z > 0.f ? z : 0.f;
             if (z > 0.f) m2 |= (1ull << j);
         }
         st_row(sm + O_H2, tid, h2, HID);
-        if (kTrain)
-            for (int j = 0; j < HID; ++j) st_bf16(sm, O_B3 + kmaj(j, tid, TILE), h2[j]);
+#pragma unroll
+        for (int j = 0; j < HID; ++j) st_bf16(sm, O_B3 + kmaj(j, tid, TILE), h2[j]);
         // ---- layer 3
         ok = gemm(sbase, O_H2, O_W3, HID, OUT, tmem + C_Y, false, mbar, phase, wc, gi, inflight);
         if (!ok) break;
         float y[OUT];
         tmem_ld16(tmem + lane_base + C_Y, y);
-        for (int o = 0; o < OUT; ++o) y[o] += p.b3[o];
-        if (!kTrain) {
-            if (valid) {
-                Y_out[2 * (size_t)row] = y[0];
-                Y_out[2 * (size_t)row + 1] = y[1];
-            }
-            continue;
-        }
+        for (int o = 0; o < OUT; ++o) y[o] += sbias[2 * HID + o];
         // ---- backward
         float dy[OUT];
         float lrow = 0.f;
@@ -331,7 +542,6 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
                 dy[o] = 2.f * e / (float)n;
                 lrow += e * e;
             }
-        const int lane = tid & 31;
         {
             const float ls = warp_sum(lrow);
             if (lane == 0) swarp[warp][NB] = ls;
@@ -345,25 +555,31 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
         ok = gemm(sbase, O_DY, O_W3T, OUT, HID, tmem + C_Z1, false, mbar, phase, wc, gi, inflight);  // dH2
         if (!ok) break;
         float d2[HID];
-        for (int c = 0; c < HID; c += 16) tmem_ld16(tmem + lane_base + C_Z1 + c, d2 + c);
+        for (int c = 0; c < HID; c += 32) tmem_ld32(tmem + lane_base + C_Z1 + c, d2 + c);
 #pragma unroll
         for (int j = 0; j < HID; ++j) {
             d2[j] = ((m2 >> j) & 1ull) ? d2[j] : 0.f;
-            const float v = warp_sum(d2[j]);
-            if (lane == 0) swarp[warp][HID + j] = v;
+            st_bf16(sm, O_AT + kmaj(j, tid, TILE), d2[j]);
         }
         st_row(sm + O_DZ2, tid, d2, HID);
-        for (int j = 0; j < HID; ++j) st_bf16(sm, O_AT + kmaj(j, tid, TILE), d2[j]);
+#pragma unroll
+        for (int c = 0; c < HID; c += 32) {
+            const float v = warp_sum32(d2 + c, lane);
+            swarp[warp][HID + c + lane] = v;
+        }
         ok = gemm(sbase, O_DZ2, O_W2T, HID, HID, tmem + C_Z2, false, mbar, phase, wc, gi, inflight);  // dH1
         if (!ok) break;
         float d1[HID];
-        for (int c = 0; c < HID; c += 16) tmem_ld16(tmem + lane_base + C_Z2 + c, d1 + c);
+        for (int c = 0; c < HID; c += 32) tmem_ld32(tmem + lane_base + C_Z2 + c, d1 + c);
 #pragma unroll
         for (int j = 0; j < HID; ++j) {
             d1[j] = ((m1 >> j) & 1ull) ? d1[j] : 0.f;
-            const float v = warp_sum(d1[j]);
-            if (lane == 0) swarp[warp][j] = v;
             st_bf16(sm, O_AT + kmaj(HID + j, tid, TILE), d1[j]);
+        }
+#pragma unroll
+        for (int c = 0; c < HID; c += 32) {
+            const float v = warp_sum32(d1 + c, lane);
+            swarp[warp][c + lane] = v;
         }
         // this tile's sums, the warps added in order (the tile's other smem
         // writes are fenced by the barrier inside the next GEMM)
@@ -384,7 +600,7 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
     // MMAs still pending after a timed-out wait write tensor memory: wait for
     // them (bounded again) before that memory is freed below
     if (!ok && inflight) mbar_wait(mbar, phase, kPollLimit);
-    if (kTrain) {
+    {
         // this CTA's part: D12 rows 0..63: dW2 (cols 0..63); rows 64..127:
         // dW1 (cols 64..79); D3 rows 0..15: dW3 (the rows of unused outputs
         // zero); every entry written, zero when the CTA stopped early
@@ -416,37 +632,79 @@ __global__ void __launch_bounds__(NT, 1) k_mlp(const float* __restrict__ X, cons
     }
     fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    if (warp == 0) tmem_free<TMEM_COLS>(tmem);
 }
 
-// g[i] = the CTAs' parts of parameter i added in CTA order; *loss likewise
+// the CTAs' parts of parameter i (or of the loss) added in CTA order
+__device__ __forceinline__ float part_sum(const float* part, int nparts, int i) {
+    float acc = 0.f;
+    int b = 0;
+    for (; b + 32 <= nparts; b += 32) {  // (the loads together, the sum in order)
+        float v[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = __ldcg(&part[(size_t)(b + k) * kNParams + i]);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) acc += v[k];
+    }
+    for (; b < nparts; ++b) acc += __ldcg(&part[(size_t)b * kNParams + i]);
+    return acc;
+}
+__device__ __forceinline__ double loss_sum(const double* lpart, int nparts) {
+    double l = 0.0;
+    int b = 0;
+    for (; b + 16 <= nparts; b += 16) {
+        double v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = __ldcg(&lpart[b + k]);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) l += v[k];
+    }
+    for (; b < nparts; ++b) l += __ldcg(&lpart[b]);
+    return l;
+}
+
+// g[i] = the CTAs' parts of parameter i; *loss likewise
 __global__ void k_grad_sum(const float* __restrict__ part, int nparts, float* g, const double* __restrict__ lpart,
                            double* loss) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kNParams) {
-        float acc = 0.f;
-        for (int b = 0; b < nparts; ++b) acc += part[(size_t)b * kNParams + i];
-        g[i] = acc;
-    }
-    if (i == 0) {
-        double l = 0.0;
-        for (int b = 0; b < nparts; ++b) l += lpart[b];
-        *loss = l;
-    }
+    if (i < kNParams) g[i] = part_sum(part, nparts, i);
+    if (i == 0) *loss = loss_sum(lpart, nparts);
 }
 
-__global__ void k_adam(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+struct AdamArgs {
+    float lr, b1, b2, eps, c1, c2;
+};
+
+__device__ __forceinline__ void adam_param(int i, float gi, float* p, float* m, float* v, uint8_t* img, const AdamArgs& a) {
+    const float mi = a.b1 * m[i] + (1.f - a.b1) * gi;
+    const float vi = a.b2 * v[i] + (1.f - a.b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float pi = p[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+    p[i] = pi;
+    pack_param(img, i, pi);
 }
 
+__global__ void k_adam(float* p, const float* g, float* m, float* v, uint8_t* img, AdamArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kNParams) adam_param(i, g[i], p, m, v, img, a);
+}
+
+// k_grad_sum and k_adam of one minibatch; *loss_acc gains the minibatch's
+// loss.  After a timed-out wait (*err) the network is left as it is.
+__global__ void k_grad_adam(const float* part, int nparts, float* g, const double* lpart, double* loss_acc, float* p,
+                            float* m, float* v, uint8_t* img, AdamArgs a, const int* err) {
+    pdl_wait();
+    pdl_trigger();
+    if (__ldcg(err)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kNParams) {
+        const float gi = part_sum(part, nparts, i);
+        g[i] = gi;
+        adam_param(i, gi, p, m, v, img, a);
+    }
+    if (i == 0) *loss_acc += loss_sum(lpart, nparts);
+}
 
 }  // namespace mlp
 }  // namespace pgb
@@ -454,10 +712,12 @@ __global__ void k_adam(float* p, const float* g, float* m, float* v, int n, floa
 struct pg_mlp {
     int device = 0;
     cudaStream_t stream = nullptr;
+    void* memory = nullptr;    // holds all of the below
     float* params = nullptr;   // kNParams
     float* grads = nullptr;
     float* m = nullptr;
     float* v = nullptr;
+    uint8_t* img = nullptr;    // BF16 operand images of the weights (P_BYTES), always those of params
     double* loss = nullptr;
     float* gpart = nullptr;    // per CTA of a gradient launch: its part of the gradient (kNParams)
     double* lpart = nullptr;   // and of the loss
@@ -480,21 +740,34 @@ int pg_mlp_create(int32_t device, uint64_t seed, pg_mlp** out) {
     m->device = device;
     PG_CUDA(cudaSetDevice(device));
     PG_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
-    PG_CUDA(cudaMalloc((void**)&m->params, 4 * kNParams * sizeof(float)));
+    cudaDeviceGetAttribute(&m->n_sms, cudaDevAttrMultiProcessorCount, device);
+    // one allocation, each part on a 256-byte boundary
+    struct Part {
+        void** p;
+        size_t bytes;
+    };
+    const Part parts[] = {{(void**)&m->params, 4 * (size_t)kNParams * sizeof(float)},
+                          {(void**)&m->img, P_BYTES},
+                          {(void**)&m->loss, sizeof(double)},
+                          {(void**)&m->err, sizeof(int)},
+                          {(void**)&m->probe, TILE * (IN + 2) * sizeof(float)},
+                          {(void**)&m->lpart, (size_t)m->n_sms * sizeof(double)},
+                          {(void**)&m->gpart, (size_t)m->n_sms * kNParams * sizeof(float)}};
+    size_t bytes = 0;
+    for (const Part& q : parts) bytes += (q.bytes + 255) & ~size_t(255);
+    PG_CUDA(cudaMalloc(&m->memory, bytes));
+    PG_CUDA(fill_sync(m->memory, 0, bytes));
+    char* at = (char*)m->memory;
+    for (const Part& q : parts) {
+        *q.p = at;
+        at += (q.bytes + 255) & ~size_t(255);
+    }
     m->grads = m->params + kNParams;
     m->m = m->grads + kNParams;
     m->v = m->m + kNParams;
-    PG_CUDA(fill_sync(m->params, 0, 4 * kNParams * sizeof(float)));
-    PG_CUDA(cudaMalloc((void**)&m->loss, sizeof(double)));
-    PG_CUDA(cudaMalloc((void**)&m->err, sizeof(int)));
-    PG_CUDA(fill_sync(m->err, 0, sizeof(int)));
-    PG_CUDA(cudaMalloc((void**)&m->probe, TILE * (IN + 2) * sizeof(float)));
-    PG_CUDA(fill_sync(m->probe, 0, TILE * (IN + 2) * sizeof(float)));
-    cudaDeviceGetAttribute(&m->n_sms, cudaDevAttrMultiProcessorCount, device);
-    PG_CUDA(cudaMalloc((void**)&m->gpart, (size_t)m->n_sms * kNParams * sizeof(float)));
-    PG_CUDA(cudaMalloc((void**)&m->lpart, (size_t)m->n_sms * sizeof(double)));
-    PG_CUDA(cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));
-    PG_CUDA(cudaFuncSetAttribute(k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));
+    PG_CUDA(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));
+    for (auto k : {k_mlp_forward<true>, k_mlp_forward<false>})  // room for kForwardCtasPerSm of them on an SM
+        PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     // He initialisation (host, seeded), last layer scaled to start near zero output
     std::mt19937_64 rng(seed);
     std::normal_distribution<float> nd(0.f, 1.f);
@@ -505,6 +778,8 @@ int pg_mlp_create(int32_t device, uint64_t seed, pg_mlp** out) {
     for (int o = 0; o < USED; ++o)
         for (int j = 0; j < HID; ++j) hp.W3[o * HID + j] = 0.1f * nd(rng) * std::sqrt(1.f / HID);
     PG_CUDA(h2d_sync(m->params, h.data(), kNParams * sizeof(float)));
+    k_pack<<<kParamBlocks, 256, 0, m->stream>>>(m->params, m->img);
+    PG_CUDA(cudaStreamSynchronize(m->stream));
     *out = m;
     return PG_OK;
 }
@@ -512,12 +787,7 @@ int pg_mlp_create(int32_t device, uint64_t seed, pg_mlp** out) {
 void pg_mlp_destroy(pg_mlp* m) {
     if (!m) return;
     cudaSetDevice(m->device);
-    if (m->params) cudaFree(m->params);
-    if (m->loss) cudaFree(m->loss);
-    if (m->gpart) cudaFree(m->gpart);
-    if (m->lpart) cudaFree(m->lpart);
-    if (m->err) cudaFree(m->err);
-    if (m->probe) cudaFree(m->probe);
+    if (m->memory) cudaFree(m->memory);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
@@ -531,6 +801,8 @@ int pg_mlp_params(pg_mlp* m, float* host, int32_t set) {
     if (set) {
         PG_CUDA(h2d_sync(m->params, host, kNParams * sizeof(float)));
         PG_CUDA(fill_sync(m->m, 0, 2 * kNParams * sizeof(float)));
+        k_pack<<<kParamBlocks, 256, 0, m->stream>>>(m->params, m->img);
+        PG_CUDA(cudaStreamSynchronize(m->stream));  // a forward pass may follow on another stream
         m->step = 0;
     } else {
         PG_CUDA(cudaMemcpy(host, m->params, kNParams * sizeof(float), cudaMemcpyDeviceToHost));
@@ -558,17 +830,23 @@ static int mlp_check_err(pg_mlp* m) {
     return PG_OK;
 }
 
+static void launch_forward(pg_mlp* m, const float* X, int n, float* Y, cudaStream_t s, WaitCfg wc) {
+    const int tiles = (n + TILE - 1) / TILE, grid = std::min(tiles, m->n_sms * kForwardCtasPerSm);
+    const Params p = carve(m->params);
+    const uint4* img = reinterpret_cast<const uint4*>(m->img);
+    // 16-byte loads of X and 8-byte stores of Y where the caller's buffers are so aligned
+    const bool vec = (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;
+    if (vec) k_mlp_forward<true><<<grid, NT, F_ALLOC, s>>>(X, n, p, img, Y, m->err, wc);
+    else k_mlp_forward<false><<<grid, NT, F_ALLOC, s>>>(X, n, p, img, Y, m->err, wc);
+}
+
 // Y_dev[2n] = MLP(X_dev[16n]) (device pointers)
 int pg_mlp_forward(pg_mlp* m, const float* X_dev, int32_t n, float* Y_dev, void* stream) {
     if (!m || (n > 0 && (!X_dev || !Y_dev))) { set_error("pg_mlp_forward: null argument"); return PG_ERR_ARG; }
     if (n <= 0) return PG_OK;
     cudaSetDevice(m->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : m->stream;
-    const int tiles = (n + TILE - 1) / TILE;
-    const int grid = tiles < m->n_sms ? tiles : m->n_sms;
-    Params p = carve(m->params);
-    k_mlp<false><<<grid, NT, SMEM_ALLOC, s>>>(X_dev, nullptr, n, p, nullptr, Y_dev, nullptr, m->err,
-                                              WaitCfg{kPollLimit, -1});
+    launch_forward(m, X_dev, n, Y_dev, s, WaitCfg{kPollLimit, -1});
     PG_CUDA(cudaGetLastError());
     if (s == m->stream) return mlp_check_err(m);
     return PG_OK;
@@ -582,25 +860,39 @@ int pg_mlp_forward(pg_mlp* m, const float* X_dev, int32_t n, float* Y_dev, void*
 int pg_mlp_wait_selftest(pg_mlp* m, int32_t polls) {
     if (!m || polls < 1) { set_error("pg_mlp_wait_selftest: bad argument"); return PG_ERR_ARG; }
     cudaSetDevice(m->device);
-    Params p = carve(m->params);
-    k_mlp<false><<<1, NT, SMEM_ALLOC, m->stream>>>(m->probe, nullptr, TILE, p, nullptr, m->probe + TILE * IN, nullptr, m->err,
-                                                   WaitCfg{polls, 0});
+    launch_forward(m, m->probe, TILE, m->probe + TILE * IN, m->stream, WaitCfg{polls, 0});
     PG_CUDA(cudaGetLastError());
     return mlp_check_err(m);
+}
+
+// the CTAs' gradient parts over n rows; returns their number
+static int launch_train(pg_mlp* m, const float* X, const float* T, int n) {
+    const int tiles = (n + TILE - 1) / TILE, grid = std::min(tiles, m->n_sms);
+    launch_pdl(k_mlp_train, grid, NT, SMEM_ALLOC, m->stream, X, T, n, carve(m->params),
+               reinterpret_cast<const uint4*>(m->img), m->gpart, m->lpart, m->err, WaitCfg{kPollLimit, -1});
+    return grid;
+}
+
+// Adam's constants of the next step
+static AdamArgs next_step(pg_mlp* m, float lr) {
+    m->step += 1;
+    AdamArgs a;
+    a.lr = lr;
+    a.b1 = 0.9f;
+    a.b2 = 0.999f;
+    a.eps = 1e-8f;
+    a.c1 = 1.f - std::pow(a.b1, (float)m->step);
+    a.c2 = 1.f - std::pow(a.b2, (float)m->step);
+    return a;
 }
 
 // gradients of the mean-squared loss over all n rows into the internal buffer; loss to *loss_host
 int pg_mlp_gradient(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n, double* loss_host) {
     if (!m || !X_dev || !T_dev || n <= 0) { set_error("pg_mlp_gradient: bad argument"); return PG_ERR_ARG; }
     cudaSetDevice(m->device);
-    cudaStream_t s = m->stream;
-    const int tiles = (n + TILE - 1) / TILE;
-    const int grid = tiles < m->n_sms ? tiles : m->n_sms;
-    Params p = carve(m->params);
-    k_mlp<true><<<grid, NT, SMEM_ALLOC, s>>>(X_dev, T_dev, n, p, m->gpart, nullptr, m->lpart, m->err,
-                                             WaitCfg{kPollLimit, -1});
+    const int parts = launch_train(m, X_dev, T_dev, n);
     PG_CUDA(cudaGetLastError());
-    k_grad_sum<<<(kNParams + 255) / 256, 256, 0, s>>>(m->gpart, grid, m->grads, m->lpart, m->loss);
+    k_grad_sum<<<kParamBlocks, 256, 0, m->stream>>>(m->gpart, parts, m->grads, m->lpart, m->loss);
     PG_CUDA(cudaGetLastError());
     int rc = mlp_check_err(m);
     if (rc) return rc;
@@ -611,11 +903,7 @@ int pg_mlp_gradient(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n
 int pg_mlp_adam(pg_mlp* m, float lr) {
     if (!m) { set_error("pg_mlp_adam: null"); return PG_ERR_ARG; }
     cudaSetDevice(m->device);
-    m->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    k_adam<<<(kNParams + 255) / 256, 256, 0, m->stream>>>(m->params, m->grads, m->m, m->v, kNParams, lr, b1, b2, 1e-8f,
-                                                        c1, c2);
+    k_adam<<<kParamBlocks, 256, 0, m->stream>>>(m->params, m->grads, m->m, m->v, m->img, next_step(m, lr));
     PG_CUDA(cudaGetLastError());
     return PG_OK;
 }
@@ -625,19 +913,23 @@ int pg_mlp_adam(pg_mlp* m, float lr) {
 int pg_mlp_train(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n, int32_t epochs, int32_t batch, float lr,
                  double* loss_hist) {
     if (!m || !X_dev || !T_dev || n <= 0 || batch <= 0) { set_error("pg_mlp_train: bad argument"); return PG_ERR_ARG; }
+    cudaSetDevice(m->device);
+    // an epoch is queued whole: the host looks at its loss and at the error word once, at its end
     for (int ep = 0; ep < epochs; ++ep) {
-        double acc = 0.0;
+        PG_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream));
         int nb = 0;
         for (int s0 = 0; s0 < n; s0 += batch) {
             const int nn = (n - s0) < batch ? (n - s0) : batch;
-            double l = 0.0;
-            int rc = pg_mlp_gradient(m, X_dev + (size_t)s0 * IN, T_dev + (size_t)s0 * 2, nn, &l);
-            if (rc) return rc;
-            rc = pg_mlp_adam(m, lr);
-            if (rc) return rc;
-            acc += l;
+            const int parts = launch_train(m, X_dev + (size_t)s0 * IN, T_dev + (size_t)s0 * 2, nn);
+            launch_pdl(k_grad_adam, kParamBlocks, 256, 0, m->stream, m->gpart, parts, m->grads, m->lpart, m->loss,
+                       m->params, m->m, m->v, m->img, next_step(m, lr), m->err);
+            PG_CUDA(cudaGetLastError());
             ++nb;
         }
+        double acc = 0.0;
+        PG_CUDA(cudaMemcpyAsync(&acc, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
+        const int rc = mlp_check_err(m);
+        if (rc) return rc;
         if (loss_hist) loss_hist[ep] = acc / (nb ? nb : 1);
     }
     return PG_OK;
