@@ -594,13 +594,36 @@ __device__ __forceinline__ void cut_point_row(const CutPoint& P, const double* _
     cut_row(row, 1, nl, g_quad[type], q, nc, ln, cx, cy, dm, pbx, pby);
 }
 
+// The same row from the element's node coordinates XY (local numbers; the
+// parent's nodes are the first three) and the record's third part.
+__device__ __forceinline__ void cut_point_row_local(const int4 r2, const double2* XY, const double* __restrict__ dmat,
+                                                    double* row) {
+    const int mat = r2.y, lnp = r2.z, meta = r2.w;
+    const int q = meta & 255, type = (meta >> 8) & 3, nc = (meta >> 10) & 7, nl = (meta >> 13) & 15;
+    const double dm[3] = {__ldg(&dmat[3 * mat]), __ldg(&dmat[3 * mat + 1]), __ldg(&dmat[3 * mat + 2])};
+    int ln[kMaxChildNodes];
+    double cx[kMaxChildNodes], cy[kMaxChildNodes];
+#pragma unroll
+    for (int k = 0; k < kMaxChildNodes; ++k) {
+        ln[k] = (lnp >> (4 * k)) & 15;
+        const double2 v = XY[k < nc ? ln[k] : 0];
+        cx[k] = v.x;
+        cy[k] = v.y;
+    }
+    const double2 P0 = XY[0], P1 = XY[1], P2 = XY[2];
+    const double PX[3] = {P0.x, P1.x, P2.x}, PY[3] = {P0.y, P1.y, P2.y};
+    double pbx[3], pby[3];
+    parent_gradients(PX, PY, pbx, pby);
+    cut_row(row, 1, nl, g_quad[type], q, nc, ln, cx, cy, dm, pbx, pby);
+}
+
 // Point records of the cut-element kernel, per point kCutPointInts ints:
 // global nodes of its child (6, unused ones repeat the first), of the parent
 // (3), the child's material, the child nodes' local numbers (4 bits each),
 // then point q (8 bits), child type (2), child node count (3) and the
 // element's local-function count (4), then the offset in doubles of the
-// point's row (2 ints, low first: the element's first row + l (4 + 2 NL)),
-// the element's point count and the point's number l within it.  Points are
+// point's row (2 ints, low first: the element's first row + l (4 + 2 NL) for
+// its point l), the element and an unused int.  Points are
 // in class order, each element's in the order of its rows; one sentinel
 // record follows the last point, holding only the rows' total length.
 void build_cut_points(const std::vector<int>& nodes, const std::vector<int>& tmpl, const std::vector<int>& chm,
@@ -620,7 +643,6 @@ void build_cut_points(const std::vector<int>& nodes, const std::vector<int>& tmp
         const int k = cls[oi];
         const CutTemplate& T = cut_template(tmpl[oi]);
         const int* en = &nodes[(size_t)kCutNodeStride * oi];
-        const int nq_e = device_point_count(tmpl[oi]);
         int* r = &out[(size_t)rec0[oi] * kCutPointInts];
         int l = 0;
         for (int ch = 0; ch < T.n_child; ++ch) {
@@ -639,8 +661,7 @@ void build_cut_points(const std::vector<int>& nodes, const std::vector<int>& tmp
                 const long long off = roff[oi] + (long long)l * (4 + 2 * kCutClassNl[k]);
                 r[12] = (int)(unsigned)(off & 0xffffffffLL);
                 r[13] = (int)(off >> 32);
-                r[14] = nq_e;
-                r[15] = l;
+                r[14] = (int)oi;
             }
         }
     });
@@ -837,23 +858,58 @@ __device__ __forceinline__ void grid_store(double* K, int q0, unsigned mask, con
 // Tile of the structured-grid kernel: kGridTileC node columns (I0 even) x
 // TR node rows (2 or 4, picked by the autotuner), one thread per node; warp
 // 2 r + q takes the nodes of parity q in tile row r (every other column).
-// Staged window: the tile's nodes with a one-node halo, the cells around them.
+// Staged window: the tile's nodes with a one-node halo, the cells around
+// them.  A window row keeps its even columns first, then its odd ones: the
+// lanes of a warp, two columns apart, read consecutive places (a 16-byte read
+// takes 4 passes of the shared memory instead of the 8 of a stride of 32
+// bytes).  The odd half starts 16 banks off the even one, so that the copies
+// into the window don't conflict either.
 constexpr int kGridTileC = kGridTileCols;
 constexpr int kGridWinX = kGridTileC + 2;   // staged node columns
 constexpr int kGridCellX = kGridTileC + 1;  // staged cell columns
+constexpr int kGridWinHalf = 36, kGridWinRow = kGridWinHalf + kGridWinX / 2;
+constexpr int kGridCellHalf = 40, kGridCellRow = kGridCellHalf + kGridCellX / 2;
+__device__ __forceinline__ int grid_win(int c) { return (c & 1) * kGridWinHalf + (c >> 1); }
+__device__ __forceinline__ int grid_cell_at(int c) { return (c & 1) * kGridCellHalf + (c >> 1); }
 
+// A node's places in a window row: its own column, the one to the left (the
+// one to the right follows that), and the cells to its left and right.
+struct GridAt {
+    int c, l, ml, mr;
+};
+
+// cell (OX, OY) of the node in window row ly: its corner (cx, cy) is in
+// window row ly - 1 + OY + cy, column offset OX + cx - 1
 template <int OX, int OY, bool WF>
 __device__ __forceinline__ void grid_load_cell(GridCell& C, double2 (&U)[4], const double2* sXY, const double2* sU,
-                                               const int2* sM, int lx, int ly) {
-    // cell (OX, OY) of the node at window position (lx, ly): its corner (cx, cy)
-    // is window node (lx - 1 + OX + cx, ly - 1 + OY + cy)
+                                               const int2* sM, const GridAt& at, int ly) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int w = (ly - 1 + OY + (k >> 1)) * kGridWinX + lx - 1 + OX + (k & 1);
+        const int dx = OX + (k & 1);
+        const int w = (ly - 1 + OY + (k >> 1)) * kGridWinRow + (dx == 1 ? at.c : at.l + (dx >> 1));
         C.p[k] = sXY[w];
         if (WF) U[k] = sU[w];
     }
-    const int2 m = sM[(ly - 1 + OY) * kGridCellX + lx - 1 + OX];
+    const int2 m = sM[(ly - 1 + OY) * kGridCellRow + (OX ? at.mr : at.ml)];
+    C.m0 = m.x;
+    C.m1 = m.y;
+}
+
+// cell (1, OY) after cell (0, OY): its left corners are that one's right ones
+template <int OY, bool WF>
+__device__ __forceinline__ void grid_next_cell(GridCell& C, double2 (&U)[4], const double2* sXY, const double2* sU,
+                                               const int2* sM, const GridAt& at, int ly) {
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+        const int w = (ly - 1 + OY + (k >> 1)) * kGridWinRow + at.l + 1;
+        C.p[k] = C.p[k + 1];
+        C.p[k + 1] = sXY[w];
+        if (WF) {
+            U[k] = U[k + 1];
+            U[k + 1] = sU[w];
+        }
+    }
+    const int2 m = sM[(ly - 1 + OY) * kGridCellRow + at.mr];
     C.m0 = m.x;
     C.m1 = m.y;
 }
@@ -870,24 +926,25 @@ __device__ __forceinline__ void grid_node(const GridArgs& a, const int4 B, int g
     double fx = 0.0, fy = 0.0;
     GridCell C;
     double2 U[4];
+    const GridAt at = {grid_win(lx), grid_win(lx - 1), grid_cell_at(lx - 1), grid_cell_at(lx)};
     // cells in the order that completes blocks early: below (d = 0, 1, 2
     // done), above left (d = 3, 6), above right (d = 4, 5, 7, 8)
-    grid_load_cell<0, 0, WF>(C, U, sXY, sU, sM, lx, ly);
+    grid_load_cell<0, 0, WF>(C, U, sXY, sU, sM, at, ly);
     grid_cell<Q, 0, 0, WK, WF>(C, U, a.dmat, acc, fx, fy);
-    grid_load_cell<1, 0, WF>(C, U, sXY, sU, sM, lx, ly);
+    grid_next_cell<0, WF>(C, U, sXY, sU, sM, at, ly);
     grid_cell<Q, 1, 0, WK, WF>(C, U, a.dmat, acc, fx, fy);
     if (WK) {
         if (Q == 0) grid_store<0>(a.K, q0, mask, acc);
         grid_store<1>(a.K, q0, mask, acc);
         if (Q == 0) grid_store<2>(a.K, q0, mask, acc);
     }
-    grid_load_cell<0, 1, WF>(C, U, sXY, sU, sM, lx, ly);
+    grid_load_cell<0, 1, WF>(C, U, sXY, sU, sM, at, ly);
     grid_cell<Q, 0, 1, WK, WF>(C, U, a.dmat, acc, fx, fy);
     if (WK) {
         grid_store<3>(a.K, q0, mask, acc);
         if (Q == 0) grid_store<6>(a.K, q0, mask, acc);
     }
-    grid_load_cell<1, 1, WF>(C, U, sXY, sU, sM, lx, ly);
+    grid_next_cell<1, WF>(C, U, sXY, sU, sM, at, ly);
     grid_cell<Q, 1, 1, WK, WF>(C, U, a.dmat, acc, fx, fy);
     if (WK) {
         grid_store<4>(a.K, q0, mask, acc);
@@ -903,32 +960,42 @@ __device__ __forceinline__ void grid_node(const GridArgs& a, const int4 B, int g
 
 // One CTA per tile: the window's coordinates (and displacements) and cell
 // materials are staged with coalesced loads, all in flight together; then
-// every thread forms its node's row from shared memory.
+// every thread forms its node's row from shared memory.  Bound by the L1:
+// a warp's block store goes to 32 lines, and the window reads.  Two resident
+// groups of 256 threads with both outputs (three spilled 328 bytes per
+// thread: 122 us at 1024^2, now 84 in the persistent kernel).  128 threads
+// per CTA are never slower than 256 (a halo row more per node row, but
+// smaller steps at the end of the grid): stiffness of 256^2 16.5 us against
+// 20.5, 512^2 34.9 against 37.5, with the cut elements.
 template <bool WK, bool WF, int TR>
-__global__ void __launch_bounds__(kGridTileC * TR, 12 / TR) k_grid_rows(GridArgs a) {
+__global__ void __launch_bounds__(kGridTileC * TR, (WK && WF ? 8 : 12) / TR) k_grid_rows(GridArgs a) {
     pdl_trigger();  // the cut elements' row kernels may fill the SMs this grid frees
     constexpr int kGridThreads = kGridTileC * TR, kGridWinY = TR + 2, kGridCellY = TR + 1;
-    __shared__ double2 sXY[kGridWinX * kGridWinY];
-    __shared__ double2 sU[WF ? kGridWinX * kGridWinY : 1];
-    __shared__ int2 sM[kGridCellX * kGridCellY];
+    __shared__ double2 sXY[kGridWinRow * kGridWinY];
+    __shared__ double2 sU[WF ? kGridWinRow * kGridWinY : 1];
+    __shared__ int2 sM[kGridCellRow * kGridCellY];
     const int4 T = __ldg(&a.tiles[blockIdx.x]);
     const int4 B = __ldg(&a.rves[T.x]);  // this tile's grid block: nx, ny, first node, first element
     const int nx = B.x, ny = B.y, NX1 = nx + 1;
     const int I0 = T.y, J0 = T.z;
     for (int i = threadIdx.x; i < kGridWinX * kGridWinY; i += kGridThreads) {
-        const int gi = I0 - 1 + i % kGridWinX, gj = J0 - 1 + i / kGridWinX;
+        const int wc = i % kGridWinX, wr = i / kGridWinX;
+        const int gi = I0 - 1 + wc, gj = J0 - 1 + wr;
         double2 v = make_double2(0.0, 0.0), uv = make_double2(0.0, 0.0);
         if (gi >= 0 && gi <= nx && gj >= 0 && gj <= ny) {
             const size_t n = (size_t)B.z + gi + (size_t)gj * NX1;
             v = make_double2(__ldg(&a.x[n]), __ldg(&a.y[n]));
             if (WF) uv = make_double2(__ldg(&a.u[2 * n]), __ldg(&a.u[2 * n + 1]));
         }
-        sXY[i] = v;
-        if (WF) sU[i] = uv;
+        const int w = wr * kGridWinRow + grid_win(wc);
+        sXY[w] = v;
+        if (WF) sU[w] = uv;
     }
     for (int i = threadIdx.x; i < kGridCellX * kGridCellY; i += kGridThreads) {
-        const int ci = I0 - 1 + i % kGridCellX, cj = J0 - 1 + i / kGridCellX;
-        sM[i] = (ci >= 0 && ci < nx && cj >= 0 && cj < ny)
+        const int wc = i % kGridCellX, wr = i / kGridCellX;
+        const int ci = I0 - 1 + wc, cj = J0 - 1 + wr;
+        sM[wr * kGridCellRow + grid_cell_at(wc)] =
+                    (ci >= 0 && ci < nx && cj >= 0 && cj < ny)
                     ? __ldg(reinterpret_cast<const int2*>(a.emat) + ((size_t)B.w / 2 + ci + (size_t)cj * nx))
                     : make_int2(-1, -1);
     }
@@ -958,9 +1025,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // pairs, displacements, cell materials.
 template <int TR, bool WF>
 struct GridWin {
-    double2 xy[kGridWinX * (TR + 2)];
-    double2 u[WF ? kGridWinX * (TR + 2) : 1];
-    int2 m[kGridCellX * (TR + 1)];
+    double2 xy[kGridWinRow * (TR + 2)];
+    double2 u[WF ? kGridWinRow * (TR + 2) : 1];
+    int2 m[kGridCellRow * (TR + 1)];
 };
 
 // Issues the copies of tile t's window into W (every thread its share).
@@ -971,21 +1038,23 @@ __device__ __forceinline__ void grid_stage_async(const GridArgs& a, int t, GridW
     const int4 B = __ldg(&a.rves[T.x]);
     const int nx = B.x, ny = B.y, NX1 = nx + 1;
     for (int i = threadIdx.x; i < kGridWinX * kWinY; i += kThreads) {
-        const int gi = T.y - 1 + i % kGridWinX, gj = T.z - 1 + i / kGridWinX;
+        const int wc = i % kGridWinX, wr = i / kGridWinX;
+        const int gi = T.y - 1 + wc, gj = T.z - 1 + wr, w = wr * kGridWinRow + grid_win(wc);
         const bool in = gi >= 0 && gi <= nx && gj >= 0 && gj <= ny;
         const size_t n = in ? (size_t)B.z + gi + (size_t)gj * NX1 : 0;
-        cp_async8(&W.xy[i].x, a.x + n, in);
-        cp_async8(&W.xy[i].y, a.y + n, in);
+        cp_async8(&W.xy[w].x, a.x + n, in);
+        cp_async8(&W.xy[w].y, a.y + n, in);
         if (WF) {
-            cp_async8(&W.u[i].x, a.u + 2 * n, in);
-            cp_async8(&W.u[i].y, a.u + 2 * n + 1, in);
+            cp_async8(&W.u[w].x, a.u + 2 * n, in);
+            cp_async8(&W.u[w].y, a.u + 2 * n + 1, in);
         }
     }
     for (int i = threadIdx.x; i < kGridCellX * kCellY; i += kThreads) {
-        const int ci = T.y - 1 + i % kGridCellX, cj = T.z - 1 + i / kGridCellX;
+        const int wc = i % kGridCellX, wr = i / kGridCellX;
+        const int ci = T.y - 1 + wc, cj = T.z - 1 + wr;
         const bool in = ci >= 0 && ci < nx && cj >= 0 && cj < ny;
         const size_t k = in ? (size_t)B.w / 2 + ci + (size_t)cj * nx : 0;
-        cp_async8(&W.m[i], reinterpret_cast<const int2*>(a.emat) + k, in);
+        cp_async8(&W.m[wr * kGridCellRow + grid_cell_at(wc)], reinterpret_cast<const int2*>(a.emat) + k, in);
     }
 }
 
@@ -999,8 +1068,12 @@ __device__ __forceinline__ void grid_stage_async(const GridArgs& a, int t, GridW
 // barrier.  Out-of-grid window entries are zero-filled (materials:
 // out-of-grid cells read as material 0 from the fill, so they are set to -1
 // after the copy lands).
+// Its 64-thread groups per SM: stiffness and residual together keep 126
+// registers, one of them 96, without spills.
+__host__ __device__ constexpr int grid_ctas(bool wk, bool wf) { return wk && wf ? 8 : 10; }
+
 template <bool WK, bool WF, int TR>
-__global__ void __launch_bounds__(kGridTileC * TR, 12 / TR) k_grid_rows_pipe(GridArgs a, int n_tiles) {
+__global__ void __launch_bounds__(kGridTileC * TR, grid_ctas(WK, WF) / TR) k_grid_rows_pipe(GridArgs a, int n_tiles) {
     pdl_trigger();
     __shared__ GridWin<TR, WF> W[3];
     int t = blockIdx.x;
@@ -1018,8 +1091,10 @@ __global__ void __launch_bounds__(kGridTileC * TR, 12 / TR) k_grid_rows_pipe(Gri
         const int nx = B.x, ny = B.y;
         // cells outside the grid are no triangles
         for (int i = threadIdx.x; i < kGridCellX * (TR + 1); i += kGridTileC * TR) {
-            const int ci = T.y - 1 + i % kGridCellX, cj = T.z - 1 + i / kGridCellX;
-            if (!(ci >= 0 && ci < nx && cj >= 0 && cj < ny)) cur.m[i] = make_int2(-1, -1);
+            const int wc = i % kGridCellX, wr = i / kGridCellX;
+            const int ci = T.y - 1 + wc, cj = T.z - 1 + wr;
+            if (!(ci >= 0 && ci < nx && cj >= 0 && cj < ny))
+                cur.m[wr * kGridCellRow + grid_cell_at(wc)] = make_int2(-1, -1);
         }
         __syncthreads();
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1091,15 +1166,18 @@ void launch_grid(const Ctx& c, const double* U, bool want_f, bool want_K, cudaSt
     ga.tiles = c.grid_tiles[tr == 2 ? 0 : 1];
     const int blocks = c.n_grid_tiles[tr == 2 ? 0 : 1];
     if (blocks == 0) return;
-    if (c.tuning.tri_persistent) {
-        // persistent, pipelined: as many CTAs as fit on the SMs at once
-        int dev = 0, n_sm = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    // Persistent, pipelined: as many CTAs as fit on the SMs at once -- unless
+    // the tiles fit all at once anyway: then nothing is pipelined, and the
+    // plain kernel's smaller CTAs leave room for the cut elements' first ones
+    // (256^2: 16.6 us against 18.4 with the cut kernels; 512^2, 2313 tiles on
+    // 740 places: 39.0 against 34.9).
+    const bool one_wave = blocks <= c.n_sm * (grid_ctas(want_K, want_f) / tr) && c.tuning.cut_overlap == 0;
+    if (c.tuning.tri_persistent && !one_wave) {
         auto go = [&](auto kern) {
+            int per_sm = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridTileC * tr, 0);
             if (c.tuning.cut_overlap > 0 && c.n_cut > 0) per_sm -= c.tuning.cut_overlap;  // room for the cut kernels
-            const int grid = std::min(blocks, std::max(1, per_sm) * n_sm);
+            const int grid = std::min(blocks, std::max(1, per_sm) * c.n_sm);
             kern<<<grid, kGridTileC * tr, 0, s>>>(ga, blocks);
         };
         if (tr == 2) {
@@ -1130,15 +1208,17 @@ void launch_grid(const Ctx& c, const double* U, bool want_f, bool want_K, cudaSt
 // Every cut element's (3 + n_enr)^2 node-pair blocks have a fixed place in
 // the element's slot table (cut_slot: pair (a, b) at cut_slot_ptr + a nl +
 // b, holding the block's K slot).  k_cut_elems forms the element's
-// quadrature rows in shared memory and integrates one row of blocks (a, *)
-// per thread.  A block whose K slot takes no other contribution (half of
+// quadrature rows and its cohesive Gauss points (traction-separation law,
+// trial delta_max, row) in shared memory and integrates one row of blocks
+// (a, *) per thread.  A block whose K slot takes no other contribution (half of
 // them) goes into K there: stored where only cut elements reach the slot
 // (enrichment rows and columns), else added to the triangle kernel's value
 // by a reduction that waits for nothing -- with a single addend its result
 // is the same in any order.  The others are stored at their position in
 // fold order (kpos, built once per mesh: all contributions to one K slot
-// next to each other, by element and pair), and for residual passes K_ab
-// u_b at its position in the node-sorted order (fpos).  k_fold_K then gives
+// next to each other, by element and pair), and for residual passes the
+// row's force term sum_b K_ab u_b at its position in the node-sorted order
+// (fpos).  k_fold_K then gives
 // every K slot of two or more contributions its final value in one thread:
 // the triangle kernel's value (or zero, for blocks in enrichment rows or
 // columns, which only cut elements reach) plus its contiguous run of
@@ -1146,12 +1226,10 @@ void launch_grid(const Ctx& c, const double* U, bool want_f, bool want_K, cudaSt
 // the same on every run.
 //
 // After the triangle kernel on the same stream, chained by programmatic
-// dependent launch: k_coh_points forms every cohesive Gauss point (one
-// thread each: traction-separation law, trial delta_max, row), k_cut_elems
-// (one launch per size class) the quadrature rows and the blocks, then the
-// folds.  k_cut_points forms the same quadrature rows in global memory for
+// dependent launch: k_cut_elems (one launch per size class), then the folds.
+// k_cut_points forms the same quadrature rows in global memory for
 // the stress recovery.
-constexpr int kCohRow = kCohRowDoubles;  // {w dA, N0, N1, (R^T D R) 4, (R^T t) 2, pad}
+constexpr int kCohRow = 9;  // {w dA, N0, N1, (R^T D R) 4, (R^T t) 2}
 
 // One thread per quadrature point: its row, point-major (the element's point
 // l at row_off[element] + l (4 + 2 NL), NL its size class's largest local
@@ -1189,57 +1267,28 @@ __global__ void __launch_bounds__(kPointThreads) k_cut_points(int n_pts, const i
     pdl_wait();  // completes only after the kernel before it: the chain stays ordered
 }
 
-// One thread per cohesive Gauss point (CohEdge2, 2 points, w = 1): the law
-// at its opening (writing the trial delta_max) and its row.  Point qp of
-// sub-element ce of element ci (class order) is qp = cut_coh_qp0[ci] + 2 ce
-// + q; coh_rec[qp] packs ci << 8 | ce << 1 | q.
-struct CohArgs {
-    int n_qp;
-    const int* __restrict__ coh_rec;
-    const int* __restrict__ cut_nodes;
-    const int* __restrict__ cut_tmpl;
-    const double* __restrict__ x;
-    const double* __restrict__ y;
-    const double* __restrict__ u;
-    const double* __restrict__ isv_c;
-    double* isv_t;
-    double* coh_rows;
-    DevCohLaw coh;
-    double dt;
-};
-
-__global__ void __launch_bounds__(128) k_coh_points(CohArgs a) {
-    pdl_trigger();
-    const int qp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qp >= a.n_qp) {
-        pdl_wait();
-        return;
-    }
-    const int rec = __ldg(&a.coh_rec[qp]);
-    const int ci = rec >> 8, ce = (rec >> 1) & 127, q = rec & 1;
-    const DevTemplate& T = g_tmpl[__ldg(&a.cut_tmpl[ci])];
-    const int* en = a.cut_nodes + (size_t)kCutNodeStride * ci;
-    int n[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) n[m] = __ldg(&en[T.coh_nodes[ce][m]]);
-    const double jx = 0.5 * (__ldg(&a.x[n[1]]) - __ldg(&a.x[n[0]]));
-    const double jy = 0.5 * (__ldg(&a.y[n[1]]) - __ldg(&a.y[n[0]]));
+// Cohesive Gauss point q of a cut element's sub-element with local nodes cn
+// (CohEdge2, 2 points, w = 1): the law at its opening, from the element's
+// local coordinates and displacements, writing the trial delta_max of point
+// qp (mesh numbering), and its row {dA, N0, N1, R^T D R, R^T t}.
+__device__ __forceinline__ void coh_point_row(const int* cn, int q, const double2* XY, const double2* U,
+                                              double isv_c, double* isv_t, const DevCohLaw& coh, double dt,
+                                              double* row) {
+    const int n0 = cn[0], n1 = cn[1], n2 = cn[2], n3 = cn[3];
+    const double jx = 0.5 * (XY[n1].x - XY[n0].x);
+    const double jy = 0.5 * (XY[n1].y - XY[n0].y);
     const double mag = sqrt(jx * jx + jy * jy);
     const double nx = -jy, ny = jx;
     const double dA = sqrt(nx * nx + ny * ny);
     const double R[2][2] = {{jx / mag, jy / mag}, {nx / dA, ny / dA}};
     const double xi = q == 0 ? -0.57735026918962576450914878050196 : 0.57735026918962576450914878050196;
     const double N0 = 0.5 * (1.0 - xi), N1 = 0.5 * (1 + xi);
-    double dg[2];
-#pragma unroll
-    for (int d = 0; d < 2; ++d)
-        dg[d] = N0 * (__ldg(&a.u[2 * n[2] + d]) - __ldg(&a.u[2 * n[0] + d])) +
-                N1 * (__ldg(&a.u[2 * n[3] + d]) - __ldg(&a.u[2 * n[1] + d]));
+    const double dg[2] = {N0 * (U[n2].x - U[n0].x) + N1 * (U[n3].x - U[n1].x),
+                          N0 * (U[n2].y - U[n0].y) + N1 * (U[n3].y - U[n1].y)};
     double dl[2] = {R[0][0] * dg[0] + R[0][1] * dg[1], R[1][0] * dg[0] + R[1][1] * dg[1]};
     double tr[2], Dc[2][2], dmax_t;
-    cohesive_law(a.coh, a.dt, __ldg(&a.isv_c[qp]), dl, tr, Dc, dmax_t);
-    a.isv_t[qp] = dmax_t;
-    double* row = a.coh_rows + (size_t)kCohRow * qp;
+    cohesive_law(coh, dt, isv_c, dl, tr, Dc, dmax_t);
+    *isv_t = dmax_t;
     row[0] = dA * 1.0;
     row[1] = N0;
     row[2] = N1;
@@ -1256,8 +1305,6 @@ __global__ void __launch_bounds__(128) k_coh_points(CohArgs a) {
         }
     row[7] = R[0][0] * tr[0] + R[1][0] * tr[1];
     row[8] = R[0][1] * tr[0] + R[1][1] * tr[1];
-    row[9] = 0.0;
-    pdl_wait();
 }
 
 struct ElemArgs {
@@ -1270,17 +1317,22 @@ struct ElemArgs {
     const int* __restrict__ kpos;   // slot-table entry -> position in fold order (-1: no K slot)
     const long long* __restrict__ kdir;  // slot-table entry -> slot << 1 | cut_only of a one-entry run,
                                          // else -2 - (fold position), -1 without a K slot (direct passes)
-    const int* __restrict__ fpos;   // slot-table entry -> position in node order
+    const int* __restrict__ fpos;   // kCutNodeStride element + local node -> position in node order
     const int4* __restrict__ pts;   // point records (build_cut_points)
     const int* __restrict__ pt_off; // per element its first point record
     const long long* __restrict__ row_off;
     const double* __restrict__ x;
     const double* __restrict__ y;
     const double* __restrict__ dmat;
-    const double* __restrict__ coh_rows;
     const double* __restrict__ u;
+    const double* __restrict__ isv_c;
+    double* isv_t;
+    DevCohLaw coh;
+    double dt;
+    int coh_max;                    // most cohesive sub-elements of one element of this class
+    int node_off;                   // doubles of shared memory before the nodes' coordinates and displacements
     double* ke;                     // 4 FP64 per fold position
-    double* fe;                     // 2 FP64 per node-order position
+    double* fe;                     // 2 FP64 per node-order position (one per element and local node)
     double* K;
     int want_K, want_f;
     int direct;                     // 1: one-entry runs go straight into K (the triangle kernel has finished)
@@ -1295,8 +1347,8 @@ __device__ __forceinline__ double2 lds2(const double* p) { return *reinterpret_c
 // local function a of an element integrates the element's row a of blocks:
 // K_ab = sum_q w_q B_a^T D B_b over the rows for every b, plus the cohesive
 // sub-elements' N_a N_b (+-) R^T D R terms where both nodes are cohesive
-// nodes.  Residual passes store K_ab u_b (bulk) for every b and, on the
-// diagonal block, add the node's cohesive traction term.  In direct passes
+// nodes.  Residual passes store one force term per local function: the bulk
+// sum_b K_ab u_b plus the node's cohesive tractions.  In direct passes
 // a block whose K slot no other contribution reaches goes straight into K
 // (stored, or added to the triangle kernel's value by a single-addend
 // reduction); every other block goes to its place in fold order.
@@ -1309,20 +1361,49 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
     const int e0 = blockIdx.x * epc, e1 = min(a.n_elem, e0 + epc);
     const int c0 = a.first + e0;
     const long long base = __ldg(&a.row_off[c0]);
-    // this thread's element and local function; its static tables are
-    // loaded while the rows are formed
+    // this thread's element and local function; its static tables and the
+    // first point record are loaded while the nodes are staged
     const int le = threadIdx.x / NL, pa = threadIdx.x - le * NL;
     const bool act = le < epc && e0 + le < a.n_elem;
     const int ci = c0 + (act ? le : 0);
     const int tm = __ldg(&a.cut_tmpl[ci]);
     const long long r0 = __ldg(&a.row_off[ci]), r1 = __ldg(&a.row_off[ci + 1]);
     const int sp_e = __ldg(&a.cut_slot_ptr[ci]);
-    {
-        const int p0 = __ldg(&a.pt_off[c0]), p1 = __ldg(&a.pt_off[a.first + e1]);
-        for (int p = p0 + (int)threadIdx.x; p < p1; p += blockDim.x) {
-            const CutPoint cp = cut_point_load(a.pts + 4 * (size_t)p);
-            const long long off = (long long)(unsigned)cp.r3.x | ((long long)cp.r3.y << 32);
-            cut_point_row(cp, a.x, a.y, a.dmat, sRow + (off - base));
+    double2* sXY = reinterpret_cast<double2*>(sRow + a.node_off);
+    double2* sU = sXY + epc * NL;
+    double* sCoh = reinterpret_cast<double*>(WF || COH ? sU + epc * NL : sU);
+    int p = __ldg(&a.pt_off[c0]) + (int)threadIdx.x;
+    const int p1 = __ldg(&a.pt_off[a.first + e1]);
+    int4 r2 = make_int4(0, 0, 0, 0), r3 = r2;
+    if (p < p1) {
+        r2 = __ldg(a.pts + 4 * (size_t)p + 2);
+        r3 = __ldg(a.pts + 4 * (size_t)p + 3);
+    }
+    const int nd = act ? __ldg(&a.cut_nodes[(size_t)kCutNodeStride * ci + pa]) : -1;  // -1: fewer local nodes
+    if (nd >= 0) {
+        sXY[le * NL + pa] = make_double2(__ldg(&a.x[nd]), __ldg(&a.y[nd]));
+        if (WF || COH) sU[le * NL + pa] = make_double2(__ldg(&a.u[2 * (size_t)nd]), __ldg(&a.u[2 * (size_t)nd + 1]));
+    }
+    __syncthreads();
+    while (p < p1) {
+        const long long off = (long long)(unsigned)r3.x | ((long long)r3.y << 32);
+        cut_point_row_local(r2, sXY + (r3.z - c0) * NL, a.dmat, sRow + (off - base));
+        p += blockDim.x;
+        if (p < p1) {
+            r2 = __ldg(a.pts + 4 * (size_t)p + 2);
+            r3 = __ldg(a.pts + 4 * (size_t)p + 3);
+        }
+    }
+    if (COH) {
+        // from the last thread down: the first ones have the bulk points
+        const int m = 2 * a.coh_max;
+        for (int i = blockDim.x - 1 - threadIdx.x; i < (e1 - e0) * m; i += blockDim.x) {
+            const int l = i / m, j = i - l * m;
+            const DevTemplate& Tc = g_tmpl[__ldg(&a.cut_tmpl[c0 + l])];
+            const int qp = __ldg(&a.cut_coh_qp0[c0 + l]) + j;
+            if (j < 2 * Tc.n_coh)
+                coh_point_row(Tc.coh_nodes[j >> 1], j & 1, sXY + l * NL, sU + l * NL, __ldg(&a.isv_c[qp]),
+                              a.isv_t + qp, a.coh, a.dt, sCoh + (size_t)kCohRow * i);
         }
     }
     __syncthreads();
@@ -1332,7 +1413,6 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
     if (pa >= nl) return;
     const int nq = (int)((r1 - r0) / W);
     const long long sp0 = sp_e + (long long)pa * nl;
-    const int* en = a.cut_nodes + (size_t)kCutNodeStride * ci;
     // where the row's blocks go (static tables), in flight during the
     // integration: kdir in direct mode, else the fold position
     long long kd[NL];
@@ -1363,28 +1443,19 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
         }
     }
     // bulk internal force terms K_ab u_b (the cohesive part of f_int is the
-    // traction integral below, not the cohesive tangent times u); every
-    // block but the diagonal one is final here
+    // traction integral below, not the cohesive tangent times u)
     double fx = 0.0, fy = 0.0;
     if (WF) {
 #pragma unroll
         for (int b = 0; b < NL; ++b) {
             if (b < nl) {
-                const int nb = __ldg(&en[b]);
-                const double ux = __ldg(&a.u[2 * nb]), uy = __ldg(&a.u[2 * nb + 1]);
-                const double gx = k[b][0] * ux + k[b][1] * uy, gy = k[b][2] * ux + k[b][3] * uy;
-                if (b == pa) {
-                    fx = gx;
-                    fy = gy;
-                } else {
-                    const int fp = __ldg(&a.fpos[sp0 + b]);
-                    if (fp >= 0) reinterpret_cast<double2*>(a.fe)[fp] = make_double2(gx, gy);
-                }
+                const double2 ub = sU[le * NL + b];
+                fx += k[b][0] * ub.x + k[b][1] * ub.y;
+                fy += k[b][2] * ub.x + k[b][3] * ub.y;
             }
         }
     }
     if (COH && T.n_coh > 0) {
-        const int qp0 = __ldg(&a.cut_coh_qp0[ci]);
         for (int ce = 0; ce < T.n_coh; ++ce) {
             int i = -1;
 #pragma unroll
@@ -1394,16 +1465,16 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
             const double sa = i < 2 ? -1.0 : 1.0;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-                const double* row = a.coh_rows + (size_t)kCohRow * (qp0 + 2 * ce + q);
-                const double wgt = __ldg(&row[0]);
+                const double* row = sCoh + kCohRow * (2 * (le * a.coh_max + ce) + q);
+                const double wgt = row[0];
                 if (wgt == 0.0) continue;
-                const double Na = __ldg(&row[1 + (i & 1)]);
-                const double D0 = __ldg(&row[3]), D1 = __ldg(&row[4]), D2 = __ldg(&row[5]), D3 = __ldg(&row[6]);
+                const double Na = row[1 + (i & 1)];
+                const double D0 = row[3], D1 = row[4], D2 = row[5], D3 = row[6];
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const int b = T.coh_nodes[ce][m];
                     const double sgn = ((i < 2) == (m < 2)) ? 1.0 : -1.0;
-                    const double v = wgt * sgn * Na * __ldg(&row[1 + (m & 1)]);
+                    const double v = wgt * sgn * Na * row[1 + (m & 1)];
 #pragma unroll
                     for (int bb = 0; bb < NL; ++bb)
                         if (bb == b) {
@@ -1413,14 +1484,13 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
                             k[bb][3] += v * D3;
                         }
                 }
-                fx += wgt * sa * Na * __ldg(&row[7]);
-                fy += wgt * sa * Na * __ldg(&row[8]);
+                fx += wgt * sa * Na * row[7];
+                fy += wgt * sa * Na * row[8];
             }
         }
     }
     if (WF) {
-        const int fp = __ldg(&a.fpos[sp0 + pa]);
-        if (fp >= 0) reinterpret_cast<double2*>(a.fe)[fp] = make_double2(fx, fy);
+        reinterpret_cast<double2*>(a.fe)[__ldg(&a.fpos[(size_t)kCutNodeStride * ci + pa])] = make_double2(fx, fy);
     }
     // kd >= 0: the slot's only contribution (slot << 1 | cut_only): stored
     // (a block only cut elements reach) or added to the triangle kernel's
@@ -1493,7 +1563,7 @@ __global__ void __launch_bounds__(256) k_fold_K(int n, const long long* __restri
 
 // f_int of the nodes cut elements touch, one thread each: f = (the triangle
 // kernel's value, or 0 for enrichment nodes) + the node's contiguous run of
-// pair terms.  fold_node[j] = node << 1 | cut_only.
+// element terms.  fold_node[j] = node << 1 | cut_only.
 __global__ void __launch_bounds__(256) k_fold_f(int n, const int* __restrict__ fold_node,
                                                 const int* __restrict__ fold_ptr, const double* __restrict__ fe,
                                                 double* f) {
@@ -1941,11 +2011,9 @@ void launch_tri_tn(const Ctx& c, const RowArgs& ra, cudaStream_t s) {
     if (n_tiles <= 0) return;
     int grid = n_tiles;
     if (c.tuning.tri_persistent) {
-        int per_sm = 0, dev = 0, n_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+        int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_assemble_tri<WANT_F, TN>, 2 * TN, 0);
-        grid = std::min(n_tiles, std::max(1, per_sm) * n_sm);
+        grid = std::min(n_tiles, std::max(1, per_sm) * c.n_sm);
     }
     k_assemble_tri<WANT_F, TN><<<grid, 2 * TN, 0, s>>>(ra, n_tiles);
 }
@@ -2043,24 +2111,6 @@ void launch_cut_points(const Ctx& c, cudaStream_t s) {
                    reinterpret_cast<const int4*>(c.cut_pts), c.x, c.y, c.dmat, c.cut_rows);
 }
 
-void launch_coh_points(const Ctx& c, const double* U, double dt, cudaStream_t s) {
-    if (c.n_coh_qp <= 0) return;
-    CohArgs ca;
-    ca.n_qp = c.n_coh_qp;
-    ca.coh_rec = c.coh_rec;
-    ca.cut_nodes = c.cut_nodes;
-    ca.cut_tmpl = c.cut_tmpl;
-    ca.x = c.x;
-    ca.y = c.y;
-    ca.u = U;
-    ca.isv_c = c.isv_c;
-    ca.isv_t = c.isv_t;
-    ca.coh_rows = c.coh_rows;
-    ca.coh = c.coh;
-    ca.dt = dt;
-    launch_pdl(k_coh_points, (c.n_coh_qp + 127) / 128, 128, 0, s, ca);
-}
-
 template <int NL, bool WF, bool COH>
 int launch_elems_inst(const ElemArgs& ea, int blocks, int bs, size_t smem, cudaStream_t s) {
     if (smem > 48 * 1024) {
@@ -2087,7 +2137,7 @@ int launch_elems_nl(const ElemArgs& ea, bool coh, int blocks, int bs, size_t sme
 // one launch per size class; cut_warps x 32 threads per CTA.  direct: the
 // blocks of one-contribution slots go into K (the triangle kernel runs
 // before on the same stream); otherwise every block goes to fold order.
-int launch_cut_elems(const Ctx& c, const double* U, bool want_f, bool want_K, bool direct, cudaStream_t s) {
+int launch_cut_elems(const Ctx& c, const double* U, double dt, bool want_f, bool want_K, bool direct, cudaStream_t s) {
     ElemArgs ea;
     ea.cut_nodes = c.cut_nodes;
     ea.cut_tmpl = c.cut_tmpl;
@@ -2102,8 +2152,11 @@ int launch_cut_elems(const Ctx& c, const double* U, bool want_f, bool want_K, bo
     ea.x = c.x;
     ea.y = c.y;
     ea.dmat = c.dmat;
-    ea.coh_rows = c.coh_rows;
     ea.u = U;
+    ea.isv_c = c.isv_c;
+    ea.isv_t = c.isv_t;
+    ea.coh = c.coh;
+    ea.dt = dt;
     ea.ke = c.cut_ke;
     ea.fe = c.cut_fe;
     ea.K = c.K;
@@ -2119,13 +2172,16 @@ int launch_cut_elems(const Ctx& c, const double* U, bool want_f, bool want_K, bo
         ea.first = c.cut_class_off[k];
         const int epc = cut_elems_per_cta(bs, kCutClassNl[k]);
         const int blocks = (n + epc - 1) / epc;
-        const size_t smem = sizeof(double) * (size_t)std::max(2, c.cut_span[k][w]);
+        ea.coh_max = c.cut_class_coh[k];
+        ea.node_off = std::max(2, c.cut_span[k][w]);
+        const bool coh = c.n_coh_qp > 0 && ea.coh_max > 0;
+        const size_t smem = sizeof(double) * ((size_t)ea.node_off + (want_f || coh ? 4 : 2) * epc * kCutClassNl[k] +
+                                              2 * (size_t)kCohRow * ea.coh_max * epc);
         if (smem > 227 * 1024) {
             set_error("cut elements: a CTA's quadrature rows exceed the shared memory (use fewer warps per CTA)");
             return PG_ERR_LIMIT;
         }
         int rc;
-        const bool coh = c.n_coh_qp > 0;
         if (k == 0) rc = launch_elems_nl<5>(ea, coh, blocks, bs, smem, s);
         else if (k == 1) rc = launch_elems_nl<7>(ea, coh, blocks, bs, smem, s);
         else if (k == 2) rc = launch_elems_nl<11>(ea, coh, blocks, bs, smem, s);
@@ -2148,8 +2204,7 @@ void launch_cut_fold(const Ctx& c, bool want_f, bool want_K, bool direct, cudaSt
 
 // the cut elements' whole pass after the triangle kernel on stream s
 int launch_cut_all(const Ctx& c, const double* U, double dt, bool want_f, bool want_K, cudaStream_t s) {
-    launch_coh_points(c, U, dt, s);
-    const int rc = launch_cut_elems(c, U, want_f, want_K, true, s);
+    const int rc = launch_cut_elems(c, U, dt, want_f, want_K, true, s);
     if (rc != PG_OK) return rc;
     launch_cut_fold(c, want_f, want_K, true, s);
     return PG_OK;
@@ -2179,8 +2234,7 @@ int launch_assemble(Ctx& c, const double* U, double dt, bool want_f, bool want_K
         // persistent grid kernel (which leaves them CTA slots); the fold joins
         PG_CUDA(cudaEventRecord(c.fork_ev, s));
         PG_CUDA(cudaStreamWaitEvent(c.aux, c.fork_ev, 0));
-        launch_coh_points(c, U, dt, c.aux);
-        const int rc = launch_cut_elems(c, U, want_f, want_K, false, c.aux);
+        const int rc = launch_cut_elems(c, U, dt, want_f, want_K, false, c.aux);
         if (rc != PG_OK) return rc;
         PG_CUDA(cudaEventRecord(c.join_ev, c.aux));
         launch_tri(c, ra, want_f, s);

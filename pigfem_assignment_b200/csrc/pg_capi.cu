@@ -64,7 +64,7 @@ void free_ctx(Ctx& c) {
                     c.grid_rves, c.grid_tiles[0], c.grid_tiles[1], c.qp_off, c.qp_elem_cut, c.qp_cut_elem,
                     c.qp_class_off, c.qp_out,
                     c.cut_ke, c.cut_fe, c.cut_kpos, c.cut_fpos, c.fold_K_slot, c.fold_K_ptr, c.fold_f_node,
-                    c.fold_f_ptr, c.coh_rec, c.coh_rows, c.K, c.Kf, c.fixed, c.ubar,
+                    c.fold_f_ptr, c.K, c.Kf, c.fixed, c.ubar,
                     c.U, c.F, c.isv_c, c.isv_t, c.r, c.z, c.p, c.q, c.dx, c.minv, c.rf, c.zf, c.pf, c.qf, c.xf,
                     c.minvf, c.scal, c.iflags};
     for (void* p : ptrs)
@@ -110,6 +110,7 @@ int ctx_create(HostMesh mesh, int device, Ctx& c) {
     PG_CUDA(cudaEventCreate(&c.ea0));
     PG_CUDA(cudaEventCreate(&c.ea1));
     PG_CUDA(cudaEventCreate(&c.ea2));
+    PG_CUDA(cudaDeviceGetAttribute(&c.n_sm, cudaDevAttrMultiProcessorCount, c.device));
     c.hm = std::move(mesh);
     const HostMesh& hm = c.hm;
     c.n_nodes = hm.n_nodes();
@@ -163,6 +164,7 @@ int ctx_create(HostMesh mesh, int device, Ctx& c) {
             c.n_grid_tiles[h] = (int)tiles.size();
             if ((rc = dev_upload(&c.grid_tiles[h], tiles))) return rc;
         }
+        c.tuning.tri_persistent = 1;
     } else {
         c.tuning.tri_grid = 0;
     }
@@ -242,29 +244,25 @@ int ctx_create(HostMesh mesh, int device, Ctx& c) {
             (rc = dev_upload(&c.cut_pt_off, pt_off)))
             return rc;
         c.cut_rows_len = roff[nc];  // allocated by the stress recovery, the only user of rows in global memory
-        // cohesive Gauss points: the owning element, sub-element and point
+        // every cohesive Gauss point belongs to one cut element, whose thread forms it
         if (hm.n_coh_qp > 0) {
-            std::vector<int> rec(hm.n_coh_qp, -1);
-            for (int oi = 0; oi < nc; ++oi) {
-                const CutTemplate& T = cut_template(tmpl[oi]);
-                for (int ce = 0; ce < T.n_coh; ++ce)
-                    for (int q = 0; q < 2; ++q) rec[qp0[oi] + 2 * ce + q] = (oi << 8) | (ce << 1) | q;
-            }
-            for (int v : rec)
-                if (v < 0) {
+            std::vector<uint8_t> owned(hm.n_coh_qp, 0);
+            for (int k = 0; k < kCutClasses; ++k)
+                for (int oi = c.cut_class_off[k]; oi < c.cut_class_off[k + 1]; ++oi) {
+                    const int n = cut_template(tmpl[oi]).n_coh;
+                    c.cut_class_coh[k] = std::max(c.cut_class_coh[k], n);
+                    for (int q = 0; q < 2 * n; ++q) owned[qp0[oi] + q] = 1;
+                }
+            for (uint8_t v : owned)
+                if (!v) {
                     set_error("cohesive Gauss point not owned by any cut element");
                     return PG_ERR_MESH;
                 }
-            if ((rc = dev_upload(&c.coh_rec, rec)) ||
-                (rc = dev_alloc(&c.coh_rows, (size_t)kCohRowDoubles * hm.n_coh_qp)))
-                return rc;
         }
         c.setup_s[2] = secs(t_phase, now());
         t_phase = now();
         // deterministic assembly: the pair buffers and the fold order (built on the GPU)
-        if ((rc = dev_alloc(&c.cut_ke, 4 * std::max<size_t>(1, sl.size()))) ||
-            (rc = dev_alloc(&c.cut_fe, 2 * std::max<size_t>(1, sl.size()))))
-            return rc;
+        if ((rc = dev_alloc(&c.cut_ke, 4 * std::max<size_t>(1, sl.size())))) return rc;
         if ((rc = build_fold_device(c, node_enr, (int)sl.size()))) return rc;
         c.setup_s[3] = secs(t_phase, now());
     }

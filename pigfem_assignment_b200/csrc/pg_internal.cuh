@@ -69,7 +69,6 @@ struct DevCohLaw {
 constexpr int kCutClasses = 4;
 constexpr int kCutClassNl[kCutClasses] = {5, 7, 11, 15};
 constexpr int kCutNodeStride = 16;
-constexpr int kCohRowDoubles = 10;  // row of a cohesive Gauss point (k_coh_points)
 
 struct DevTemplate {
     int n_enr, n_child, n_coh, pad;
@@ -111,7 +110,7 @@ constexpr int kGridTileCols = 64;          // node columns per structured-grid t
 // one CTA per tile, and the warps per CTA of the cut-element kernel.
 struct AsmTuning {
     int tri_grid = 1;      // 1: the structured-grid kernel (when the mesh has one grid)
-    int grid_block = 256;  // its threads per CTA: 128 or 256
+    int grid_block = 128;  // its threads per CTA: 128 or 256
     int tri_variant = 1;   // otherwise: index into kTriTileSizes
     int tri_persistent = 0;
     int cut_warps = 4;     // 2, 4 or 8
@@ -122,7 +121,7 @@ struct AsmTuning {
 };
 
 struct Ctx {
-    int device = 0;
+    int device = 0, n_sm = 148;
     cudaStream_t stream = nullptr;
     HostMesh hm;                       // host copy (sizes, maps, export)
     int n_nodes = 0, n_reg = 0, n_elem = 0, n_cut = 0, n_blocks = 0, n_dof = 0, n_coh_qp = 0;
@@ -167,6 +166,7 @@ struct Ctx {
     int* cut_slot_ptr = nullptr;
     int* cut_slot = nullptr;           // (3 + n_enr)^2 block slots per element
     int cut_class_off[5] = {0, 0, 0, 0, 0};
+    int cut_class_coh[4] = {0, 0, 0, 0};  // most cohesive sub-elements of one element of the class
     // deterministic assembly of the cut elements: pair blocks (4 FP64) in
     // fold order and residual terms (2 FP64) in node order, each slot-table
     // entry's positions there, and the runs the folds sum
@@ -188,8 +188,6 @@ struct Ctx {
     int* fold_f_node = nullptr;        // node << 1 | cut_only
     int* fold_f_ptr = nullptr;
     int n_fold_f = 0;
-    int* coh_rec = nullptr;            // per cohesive point: class-ordered element << 8 | sub-element << 1 | point
-    double* coh_rows = nullptr;        // per cohesive point: kCohRowDoubles FP64 (k_coh_points)
     // the one-launch CG's cut of the rows (its largest part; cluster_halo < 0: not looked at yet)
     int cluster_rows = 0, cluster_blocks = 0, cluster_halo = -1;
     MgHierarchy* mg = nullptr;         // multigrid hierarchy, built at the first multigrid solve

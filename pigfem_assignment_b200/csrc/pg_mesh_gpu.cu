@@ -715,7 +715,8 @@ cudaError_t download(std::vector<T>& h, const T* d, size_t n, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Fold order of the cut elements' pair blocks (pg_assemble.cu), built on the
 // GPU by a counting sort: every slot-table entry (class-ordered element oi,
-// pair p = a nl + b) counts itself into its K slot and into its row node a;
+// pair p = a nl + b) counts itself into its K slot, every local node into its
+// node;
 // exclusive scans give every slot's and node's run; the entries scatter into
 // their runs; each run is then put in entry order, so the result is the
 // order (key, entry) a sort would give, the same on every run.
@@ -736,8 +737,8 @@ __global__ void k_fold_count(int nc, const int* __restrict__ sp, const int* __re
             atomicAdd(&cntK[slot], 1);
             if (node_enr[na] || node_enr[nb]) cutK[slot] = 1;
         }
-        atomicAdd(&cntF[na], 1);
     }
+    for (int a = 0; a < nl; ++a) atomicAdd(&cntF[nodes[(size_t)kCutNodeStride * oi + a]], 1);
 }
 
 // runs: a key i is touched when start[i + 1] > start[i]; touched_idx holds
@@ -766,11 +767,12 @@ __global__ void k_fold_scatter(int nc, const int* __restrict__ sp, const int* __
     int nl = 0;
     while (nl * nl < np) ++nl;
     for (int p = 0; p < np; ++p) {
-        const int a = p / nl;
-        const int na = nodes[(size_t)kCutNodeStride * oi + a];
         const int slot = sl[s0 + p];
         if (slot >= 0) tmpK[startK[slot] + atomicAdd(&fillK[slot], 1)] = s0 + p;
-        tmpF[startF[na] + atomicAdd(&fillF[na], 1)] = s0 + p;
+    }
+    for (int a = 0; a < nl; ++a) {
+        const int e = kCutNodeStride * oi + a, na = nodes[e];
+        tmpF[startF[na] + atomicAdd(&fillF[na], 1)] = e;
     }
 }
 
@@ -1072,7 +1074,8 @@ int build_fold_device(Ctx& c, const std::vector<uint8_t>& node_enr, int n_entrie
     MESH_CUDA(S.alloc(&fillK, nbk));
     MESH_CUDA(S.alloc(&fillF, nn));
     MESH_CUDA(S.alloc(&tmpK, n_entries));
-    MESH_CUDA(S.alloc(&tmpF, n_entries));
+    const int n_fpos = kCutNodeStride * nc;  // one force term per (cut element, local node)
+    MESH_CUDA(S.alloc(&tmpF, n_fpos));
     MESH_CUDA(S.alloc(&runK, nbk));
     MESH_CUDA(S.alloc(&runF, nn));
     MESH_CUDA(cudaMemcpyAsync(enr, node_enr.data(), nn, cudaMemcpyHostToDevice, s));
@@ -1098,9 +1101,10 @@ int build_fold_device(Ctx& c, const std::vector<uint8_t>& node_enr, int n_entrie
     MESH_CUDA(cudaMalloc((void**)&c.fold_f_node, std::max(1, nrunF) * sizeof(int)));
     MESH_CUDA(cudaMalloc((void**)&c.fold_f_ptr, (nrunF + 1) * sizeof(int)));
     MESH_CUDA(cudaMalloc((void**)&c.cut_kpos, std::max(1, n_entries) * sizeof(int)));
-    MESH_CUDA(cudaMalloc((void**)&c.cut_fpos, std::max(1, n_entries) * sizeof(int)));
+    MESH_CUDA(cudaMalloc((void**)&c.cut_fpos, std::max(1, n_fpos) * sizeof(int)));
+    MESH_CUDA(cudaMalloc((void**)&c.cut_fe, std::max(1, totF) * sizeof(double2)));
     MESH_CUDA(cudaMemsetAsync(c.cut_kpos, 0xff, std::max(1, n_entries) * sizeof(int), s));
-    MESH_CUDA(cudaMemsetAsync(c.cut_fpos, 0xff, std::max(1, n_entries) * sizeof(int), s));
+    MESH_CUDA(cudaMemsetAsync(c.cut_fpos, 0xff, std::max(1, n_fpos) * sizeof(int), s));
     k_fold_runs<long long><<<nb_mesh(nbk), kThreadsMesh, 0, s>>>(nbk, cntK, runK, cutK, c.fold_K_slot, c.fold_K_ptr);
     k_fold_runs<int><<<nb_mesh(nn), kThreadsMesh, 0, s>>>(nn, cntF, runF, cutF, c.fold_f_node, c.fold_f_ptr);
     MESH_CUDA(cudaMemcpyAsync(c.fold_K_ptr + nrunK, &totK, sizeof(int), cudaMemcpyHostToDevice, s));
