@@ -23,7 +23,7 @@
 // error in the energy norm (kOmegaReg and the polynomial's bound), so the
 // cycle is positive definite.  Coarse levels take two sweeps of damped block
 // Jacobi each way, the coarsest grid (at most 4 cells per side) its inverse.
-// Against two sweeps over all of level 0 each way: 74 -> 51 CG iterations at
+// Against two sweeps over all of level 0 each way: 74 -> 57 CG iterations at
 // 512^2 (rtol 1e-12), each with three products by K instead of five.
 //
 // A CG iteration is 7 launches and two per coarse level that has more than
@@ -55,7 +55,6 @@ using namespace mg;
 namespace {
 
 constexpr int kMaxLevels = 16;
-constexpr int kSpanCtasPerSm = 5;        // CTAs of the level-0 kernels that an SM holds
 constexpr int kChunk = 2;                // CG iterations per graph (the parity of p and r.z is baked in)
 
 // Level vectors in the V-cycle's precision
@@ -527,10 +526,10 @@ int build_hierarchy(Ctx& c) {
         B.fny = dims[r][kb[r] - 1].second;
     }
     // row spans of the level-0 kernels: as many CTAs as the GPU holds, each with about as many blocks of K, in
-    // steps of the rows a CTA takes at once
+    // steps of kStep rows
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    constexpr int kStep = kSpanThreads / kRowLanes;
+    constexpr int kStep = 16;
     const long long total = hm.n_blocks() + 2LL * c.n_nodes;
     const double per_cta = std::max((double)total / (sms * kSpanCtasPerSm), 1.0);
     std::vector<int4> span;

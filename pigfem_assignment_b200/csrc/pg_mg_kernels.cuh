@@ -26,6 +26,7 @@ constexpr int kChebCoef = 8;          // doubles per RVE: 1 / theta, then per la
 constexpr int kScal = 8;              // doubles per RVE: r.z of even and odd iterations, -, -, tol^2, b.b, true r.r
 constexpr int kFlags = 4;             // ints per RVE: done, breakdown, iterations, coarsest operator singular
 constexpr int kSpanThreads = 256;
+constexpr int kSpanCtasPerSm = 3;     // CTAs of the level-0 kernels that an SM holds: 80 registers, no spills
 constexpr int kCoarseCells = 4;       // an RVE is coarsened until both sides have at most this many cells
 constexpr int kCoarseMaxDof = 2 * (kCoarseCells + 1) * (kCoarseCells + 1);
 constexpr int kCoarseStride = kCoarseMaxDof * kCoarseMaxDof;
@@ -183,41 +184,69 @@ struct RowFrag {
         y1 = a1;
     }
 };
-// The same without the early loads, for kernels that live on many warps (the
-// level-0 products: with a fragment loaded ahead, 64 registers and spills,
-// the 512^2 product took 36 us instead of 26).
-template <typename MT, typename Get>
-__device__ __forceinline__ void row_lanes(int r0, int r1, int g, const int* __restrict__ col, const MT* __restrict__ K,
-                                          Get get, double& y0, double& y1) {
-    double a0 = 0.0, a1 = 0.0;
-    for (int base = r0 + g; base < r1; base += kRowLanes * kRowUnroll) {
-        int j[kRowUnroll];
-        double b[kRowUnroll][4];
+// Block rows i0 .. i0 + n (n <= 32) of K times a vector, one warp: lane l
+// returns row i0 + l.  The lanes take the rows' blocks in storage order, U at
+// a time (a warp's loads of K are whole lines, and no lane waits for a longer
+// row's), leave each block's product in shared memory (sp, kWarpBlocks
+// entries of the warp's own) and then each sums its row there, in order.
+// For the level-0 products, which four lanes per row read with half the lanes
+// of a last round idle: K p of 512^2 26.6 -> 20.5 us, of 1000 x 700 68 -> 60
+// (bound by the latency of its trips to memory -- row, blocks and columns,
+// vector -- at 24 warps per SM; K alone takes 24 at the DRAM's rate).  More
+// warps with fewer blocks in flight, chunks of K copied ahead with cp.async,
+// and K kept in an order without column indices were all slower.
+constexpr int kWarpBlocks = 256;
+template <int U, typename MT, typename Get>
+__device__ __forceinline__ void warp_rows(int i0, int n, const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                          const MT* __restrict__ K, Get get, double2* sp, double& y0, double& y1) {
+    const int lane = threadIdx.x & 31;
+    const int r0 = __ldg(&row_ptr[i0 + min(lane, n)]), r1 = __ldg(&row_ptr[i0 + min(lane + 1, n)]);
+    const int begin = __shfl_sync(0xffffffffu, r0, 0), end = __shfl_sync(0xffffffffu, r1, 31);
+    y0 = y1 = 0.0;
+    for (int c0 = begin; c0 < end; c0 += kWarpBlocks) {
+        const int c1 = min(end, c0 + kWarpBlocks);
+        for (int base = c0 + lane; base < c1; base += 32 * U) {
+            int j[U];
+            MT b[U][4];
 #pragma unroll
-        for (int u = 0; u < kRowUnroll; ++u) {
-            const int k = base + u * kRowLanes;
-            j[u] = -1;
-            b[u][0] = b[u][1] = b[u][2] = b[u][3] = 0.0;
-            if (k < r1) {
-                j[u] = __ldg(&col[k]);
-                load_block(K + 4 * (size_t)k, b[u][0], b[u][1], b[u][2], b[u][3]);
+            for (int u = 0; u < U; ++u) {
+                const int k = base + 32 * u;
+                j[u] = -1;
+                if (k < c1) {
+                    j[u] = __ldg(&col[k]);
+                    load4(K + 4 * (size_t)k, b[u][0], b[u][1], b[u][2], b[u][3]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (j[u] >= 0) {
+                    const Vec2<double> v = get(j[u]);
+                    sp[base + 32 * u - c0] = make_double2((double)b[u][0] * v.x + (double)b[u][1] * v.y,
+                                                          (double)b[u][2] * v.x + (double)b[u][3] * v.y);
+                }
             }
         }
-#pragma unroll
-        for (int u = 0; u < kRowUnroll; ++u) {
-            if (j[u] >= 0) {
-                const Vec2<double> v = get(j[u]);
-                a0 += b[u][0] * v.x + b[u][1] * v.y;
-                a1 += b[u][2] * v.x + b[u][3] * v.y;
-            }
+        __syncwarp();
+        const int k1 = min(r1, c1);
+        for (int k = max(r0, c0); k < k1; ++k) {
+            y0 += sp[k - c0].x;
+            y1 += sp[k - c0].y;
         }
+        __syncwarp();
     }
-    a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
-    a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-    y0 = a0;
-    y1 = a1;
+}
+// the part of a CTA's rows that a warp takes, and how many of them at once
+struct WarpSpan {
+    int i, end, step;
+};
+__device__ __forceinline__ WarpSpan warp_span(int begin, int end) {
+    const int w = threadIdx.x >> 5, n = max(0, end - begin);
+    WarpSpan s;
+    s.i = begin + (int)((long long)n * w / (kSpanThreads / 32));
+    s.end = begin + (int)((long long)n * (w + 1) / (kSpanThreads / 32));
+    const int parts = (s.end - s.i + 31) / 32;
+    s.step = parts > 0 ? (s.end - s.i + parts - 1) / parts : 32;
+    return s;
 }
 template <typename T>
 __device__ __forceinline__ Vec2<double> widen(Vec2<T> a) {
@@ -292,14 +321,14 @@ __global__ inline void k_cg_tol(Spans sp, const double* part_rr, double rtol2, d
 // p = z + beta p_old, q = mask(K p), partials of p.q.  p is formed where it is
 // read: a row gathers z and p_old of its columns instead of waiting for a
 // kernel that writes p.  Bound by the reads of K (32 bytes a block).
-__global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* __restrict__ row_ptr,
+__global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_cg_spmv(Spans sp, const int* __restrict__ row_ptr,
                                                           const int* __restrict__ col, const double* __restrict__ K,
                                                           const uint8_t* __restrict__ fixed, const double* z,
                                                           const double* p_old, double* p, double* q, const double* part_rz,
                                                           double* sc, const int* fl, double* part_pq, int P) {
+    __shared__ double2 s_rows[kSpanThreads / 32 * kWarpBlocks];
     const int4 S = sp.span[blockIdx.x];
     const int2 rg = sp.range[S.x];
-    const int g = threadIdx.x % kRowLanes;
     pdl_wait();
     pdl_trigger();
     if (__ldcg(&fl[kFlags * S.x])) return;
@@ -309,19 +338,17 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_spmv(Spans sp, const int* _
     const double beta = rz / rz_old;
     if ((int)blockIdx.x == rg.x && threadIdx.x == 0) s[P] = rz;
     double acc = 0.0;
-    for (int base = S.y; base < S.z; base += kSpanThreads / kRowLanes) {
-        const int i = base + threadIdx.x / kRowLanes;
-        const bool valid = i < S.z;
-        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+    for (WarpSpan ws = warp_span(S.y, S.z); ws.i < ws.end; ws.i += ws.step) {
+        const int n = min(ws.step, ws.end - ws.i), i = ws.i + (threadIdx.x & 31);
         double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) {
+        warp_rows<4>(ws.i, n, row_ptr, col, K, [&](int j) {
             Vec2<double> a = lv2(z, j);
             const Vec2<double> b = lv2(p_old, j);
             a.x += beta * b.x;
             a.y += beta * b.y;
             return a;
-        }, y0, y1);
-        if (valid && g == 0) {
+        }, s_rows + kWarpBlocks * (threadIdx.x >> 5), y0, y1);
+        if (i < ws.i + n) {
             const Vec2<double> a = lv2(z, i), b = lv2(p_old, i);
             const double p0 = a.x + beta * b.x, p1 = a.y + beta * b.y;
             if (fixed[2 * i]) y0 = 0.0;
@@ -600,20 +627,20 @@ __device__ __forceinline__ void restrict_tile(const Vec2<T>* s, int I0, int J0, 
     st2(bc, a, fixed_c[2 * a] ? (T)0 : s0, fixed_c[2 * a + 1] ? (T)0 : s1);
 }
 
-// 304 threads take the tile's 289 rows in four rounds.
-constexpr int kDown0Threads = 304;
+// 9 warps take the tile's 17 rows of 17 nodes in two rounds.
+constexpr int kDown0Threads = 288;
 template <typename T>
-__global__ void __launch_bounds__(kDown0Threads) k_mg_down0(const int4* __restrict__ tile, const Pair* __restrict__ pair,
+__global__ void __launch_bounds__(kDown0Threads, sizeof(T) == 8 ? 4 : 3) k_mg_down0(const int4* __restrict__ tile, const Pair* __restrict__ pair,
                                                             const int* __restrict__ row_ptr, const int* __restrict__ col,
                                                             const T* __restrict__ K, const uint8_t* __restrict__ fixed,
                                                             const double* b, const T* x, const uint8_t* __restrict__ fixed_c,
                                                             T* bc, Spans sp, const double* part_rr, const double* sc,
                                                             int* fl, int check) {
     __shared__ Vec2<T> s[kDownFine * kDownFine];
+    __shared__ double2 s_rows[kDown0Threads / 32 * kWarpBlocks];
     const int4 tl = tile[blockIdx.x];
     const Pair p = pair[tl.x];
-    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1, g = threadIdx.x % kRowLanes;
-    constexpr int kRows = kDown0Threads / kRowLanes, kN = kDownFine * kDownFine;
+    const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1;
     pdl_wait();
     pdl_trigger();
     if (fl && __ldcg(&fl[kFlags * tl.x])) return;
@@ -621,24 +648,26 @@ __global__ void __launch_bounds__(kDown0Threads) k_mg_down0(const int4* __restri
         const double rr = range_sum(part_rr, sp.range[tl.x]);
         if (threadIdx.x == 0 && rr <= __ldcg(&sc[kScal * tl.x + 4])) fl[kFlags * tl.x] = 1;
     }
-    for (int base = 0; base < kN; base += kRows) {
-        const int l = base + threadIdx.x / kRowLanes;
-        const int gx = gx0 + l % kDownFine, gy = gy0 + l / kDownFine;
-        const bool valid = l < kN && gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny;
-        const int i = valid ? p.foff + gx + gy * (p.fnx + 1) : 0;
-        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
-        double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) { return widen(lv2(x, j)); }, y0, y1);
-        if (l < kN && g == 0) {
-            Vec2<T> rv;
-            rv.x = rv.y = 0;
-            if (valid) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int gxa = max(gx0, 0), n = min(gx0 + kDownFine - 1, p.fnx) + 1 - gxa;  // the tile's columns inside the grid
+    for (int ly = w; ly < kDownFine; ly += kDown0Threads / 32) {
+        const int gy = gy0 + ly, i0 = p.foff + gxa + gy * (p.fnx + 1);
+        Vec2<T> rv;
+        rv.x = rv.y = 0;
+        if (gy >= 0 && gy <= p.fny) {
+            double y0, y1;
+            warp_rows<sizeof(T) == 8 ? 2 : 4>(i0, n, row_ptr, col, K, [&](int j) { return widen(lv2(x, j)); },
+                                              s_rows + kWarpBlocks * w, y0, y1);
+            if (lane < n) {
+                const int i = i0 + lane;
                 const Vec2<double> bv = lv2(b, i);
                 rv.x = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0;
                 rv.y = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
             }
-            s[l] = rv;
         }
+        // lanes beyond the grid's columns clear the tile's others
+        const int lx = lane < n ? lane + gxa - gx0 : lane - n < gxa - gx0 ? lane - n : lane;
+        if (lx < kDownFine) s[ly * kDownFine + lx] = rv;
     }
     __syncthreads();
     restrict_tile(s, tl.y, tl.z, p, fixed_c, bc);
@@ -647,31 +676,35 @@ __global__ void __launch_bounds__(kDown0Threads) k_mg_down0(const int4* __restri
 // The last smoothing sweep (regular nodes) and z: z_r = x_r + omega D^-1 (b - K x), z_e = x_e (already
 // smoothed, in xe); partials of b.z, which CG takes as r.z
 template <typename T>
-__global__ void __launch_bounds__(kSpanThreads) k_mg_post(Spans sp, const int* __restrict__ row_ptr,
+__global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_mg_post(Spans sp, const int* __restrict__ row_ptr,
                                                           const int* __restrict__ col, const T* __restrict__ K,
                                                           const T* __restrict__ Dinv, const uint8_t* __restrict__ fixed,
                                                           const double* b, const T* x, const T* xe, double* z, const int* fl,
                                                           double* part_rz) {
+    __shared__ double2 s_rows[kSpanThreads / 32 * kWarpBlocks];
     const int4 S = sp.span[blockIdx.x];
     const int reg = sp.reg_end[S.x];
-    const int g = threadIdx.x % kRowLanes;
-    const int end = min(S.z, reg);
     pdl_wait();
     pdl_trigger();
     if (fl && __ldcg(&fl[kFlags * S.x])) return;
     double acc = 0.0;
-    for (int base = S.y; base < end; base += kSpanThreads / kRowLanes) {
-        const int i = base + threadIdx.x / kRowLanes;
-        const bool valid = i < end;
-        const int r0 = valid ? __ldg(&row_ptr[i]) : 0, r1 = valid ? __ldg(&row_ptr[i + 1]) : 0;
+    for (WarpSpan ws = warp_span(S.y, min(S.z, reg)); ws.i < ws.end; ws.i += ws.step) {
+        const int n = min(ws.step, ws.end - ws.i), i = ws.i + (threadIdx.x & 31);
         double y0, y1;
-        row_lanes(r0, r1, g, col, K, [&](int j) { return widen(lv2(j < reg ? x : xe, j)); }, y0, y1);
-        if (valid && g == 0) {
-            const Vec2<double> bv = lv2(b, i);
-            const Vec2<T> xv = lv2(x, i);
-            const T t0 = fixed[2 * i] ? (T)0 : (T)bv.x - (T)y0, t1 = fixed[2 * i + 1] ? (T)0 : (T)bv.y - (T)y1;
-            T m0, m1, m2, m3;
+        Vec2<double> bv;
+        Vec2<T> xv;
+        T m0, m1, m2, m3;
+        uchar2 fx;
+        if (i < ws.i + n) {
+            bv = lv2(b, i);
+            xv = lv2(x, i);
+            fx = __ldg(reinterpret_cast<const uchar2*>(fixed) + i);
             load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
+        }
+        warp_rows<4>(ws.i, n, row_ptr, col, K, [&](int j) { return widen(lv2(j < reg ? x : xe, j)); },
+                     s_rows + kWarpBlocks * (threadIdx.x >> 5), y0, y1);
+        if (i < ws.i + n) {
+            const T t0 = fx.x ? (T)0 : (T)bv.x - (T)y0, t1 = fx.y ? (T)0 : (T)bv.y - (T)y1;
             const double z0 = (double)(xv.x + (T)kOmegaReg * (m0 * t0 + m1 * t1));
             const double z1 = (double)(xv.y + (T)kOmegaReg * (m2 * t0 + m3 * t1));
             st2(z, i, z0, z1);
