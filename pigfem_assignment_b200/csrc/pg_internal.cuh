@@ -87,6 +87,7 @@ struct DevChildQuad {
 };
 
 struct MgHierarchy;
+struct SensData;
 
 // Uncut-triangle assembly tiling (k_assemble_tri) and the per-block map that
 // tells each 2x2 block which staged (node, triangle) entries of its CTA
@@ -191,6 +192,7 @@ struct Ctx {
     // the one-launch CG's cut of the rows (its largest part; cluster_halo < 0: not looked at yet)
     int cluster_rows = 0, cluster_blocks = 0, cluster_halo = -1;
     MgHierarchy* mg = nullptr;         // multigrid hierarchy, built at the first multigrid solve
+    SensData* sens = nullptr;          // shape sensitivities, on their first call (pg_sens.cu)
     // system
     double* K = nullptr;               // 4 * n_blocks
     float* Kf = nullptr;               // FP32 copy for mixed precision
@@ -358,6 +360,7 @@ struct MgCgResult {
 };
 int mg_cg(Ctx& c, const pg_solver_cfg& cfg, MgCgResult& res, cudaStream_t s);
 void mg_free(Ctx& c);
+void sens_free(Ctx& c);
 // ||v||^2 of a device vector (synchronises)
 double dev_norm2(Ctx& c, const double* v, int n, cudaStream_t s);
 void set_prescribed(Ctx& c, double t_frac, cudaStream_t s);

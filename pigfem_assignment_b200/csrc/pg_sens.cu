@@ -44,6 +44,21 @@ __global__ void k_sens_weight(int nd, const uint8_t* __restrict__ fixed, const d
     if (i < nd) w[i] = fixed[i] ? L[i] : -lambda[i];
 }
 
+// partials of a.b, one per CTA
+constexpr int kDotCtas = 148;
+__global__ void k_sens_dot(int n, const double* __restrict__ a, const double* __restrict__ b, double* part) {
+    double acc = 0.0;
+    for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) acc += a[i] * b[i];
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) part[blockIdx.x] = acc;
+}
+
+}  // namespace
+
+// What the sensitivities need beside the solver's arrays, in one allocation of
+// the context: the mesh decides all of it but w, sens and part, which every
+// call writes.  (Nine allocations, uploads and frees per call were most of a
+// call at 256^2: 15 of 20 ms.)
 struct SensData {
     int n_inc = 0;
     int* node_inc = nullptr;
@@ -51,19 +66,32 @@ struct SensData {
     double* radius = nullptr;
     double* L = nullptr;
     double* w = nullptr;
-    double* sens = nullptr;
-    int* param_of = nullptr;
-    std::vector<double> hL;
+    double* sens = nullptr;                        // 3 per inclusion
+    double* part = nullptr;
+    int* param_of = nullptr;                       // 3 per inclusion
+    void* base = nullptr;
 };
 
-int sens_setup(Ctx& c, SensData& d, int n_slots) {
+void sens_free(Ctx& c) {
+    if (!c.sens) return;
+    if (c.sens->base) cudaFree(c.sens->base);
+    delete c.sens;
+    c.sens = nullptr;
+}
+
+namespace {
+
+int sens_build(Ctx& c) {
     const HostMesh& m = c.hm;
-    const int nn = m.n_nodes();
+    const size_t nn = m.n_nodes(), nd = 2 * nn;
+    SensData& d = *c.sens;
     d.n_inc = (int)m.spec.inclusions.size();
-    std::vector<int> inc(nn, -1);
+    const size_t ni = std::max(1, d.n_inc);
+    // only enrichment nodes move
+    std::vector<int> inc(std::max(1, m.n_enr), -1);
     std::vector<double> vel[3];
-    for (auto& v : vel) v.assign(2 * (size_t)nn, 0.0);
-    std::vector<double> rad(std::max(1, d.n_inc), 0.0);
+    for (auto& v : vel) v.assign(2 * inc.size(), 0.0);
+    std::vector<double> rad(ni, 0.0);
     for (int i = 0; i < d.n_inc; ++i) rad[i] = m.spec.inclusions[i].r;
     for (int k = 0; k < m.n_enr; ++k) {
         const int node = m.n_reg + k, ic = m.enr_inc[k];
@@ -74,38 +102,54 @@ int sens_setup(Ctx& c, SensData& d, int n_slots) {
         const double px = m.x[node] - I.cx, py = m.y[node] - I.cy;
         const double den = px * dx + py * dy;
         if (den == 0.0) continue;  // tangent edge: the node does not move to first order
-        inc[node] = ic;
+        inc[k] = ic;
         const double s[3] = {px, py, I.r};
         for (int kind = 0; kind < 3; ++kind) {
-            vel[kind][2 * (size_t)node] = dx * s[kind] / den;
-            vel[kind][2 * (size_t)node + 1] = dy * s[kind] / den;
+            vel[kind][2 * (size_t)k] = dx * s[kind] / den;
+            vel[kind][2 * (size_t)k + 1] = dy * s[kind] / den;
         }
     }
     // right edge, x direction: 1 / height (SensitivityRightLoad's L / area)
-    d.hL.assign(2 * (size_t)nn, 0.0);
     const int nx = m.spec.nx, ny = m.spec.ny;
-    const double H = m.spec.y1 - m.spec.y0;
-    for (int j = 0; j <= ny; ++j) d.hL[2 * (size_t)(nx + j * (nx + 1))] = 1.0 / H;
-    PG_CUDA(cudaMalloc((void**)&d.node_inc, nn * sizeof(int)));
-    for (int kind = 0; kind < 3; ++kind) {
-        PG_CUDA(cudaMalloc((void**)&d.vel[kind], vel[kind].size() * sizeof(double)));
-        PG_CUDA(h2d_sync(d.vel[kind], vel[kind].data(), vel[kind].size() * sizeof(double)));
+    const std::vector<double> edge(ny + 1, 1.0 / (m.spec.y1 - m.spec.y0));
+    const size_t doubles = 5 * nd + ni + 3 * ni + kDotCtas, ints = nn + 3 * ni;
+    PG_CUDA(cudaMalloc(&d.base, doubles * sizeof(double) + ints * sizeof(int)));
+    double* q = static_cast<double*>(d.base);
+    auto take = [&](size_t n) {
+        double* r = q;
+        q += n;
+        return r;
+    };
+    for (double*& v : d.vel) v = take(nd);
+    d.L = take(nd);
+    d.w = take(nd);
+    d.radius = take(ni);
+    d.sens = take(3 * ni);
+    d.part = take(kDotCtas);
+    d.node_inc = reinterpret_cast<int*>(q);
+    d.param_of = d.node_inc + nn;
+    cudaStream_t s = c.stream;
+    PG_CUDA(cudaMemsetAsync(d.vel[0], 0, 4 * nd * sizeof(double), s));  // the three velocities and L
+    PG_CUDA(cudaMemsetAsync(d.node_inc, 0xff, nn * sizeof(int), s));
+    if (m.n_enr > 0) {
+        for (int kind = 0; kind < 3; ++kind)
+            PG_CUDA(cudaMemcpyAsync(d.vel[kind] + 2 * (size_t)m.n_reg, vel[kind].data(), 2 * (size_t)m.n_enr * sizeof(double),
+                                    cudaMemcpyHostToDevice, s));
+        PG_CUDA(cudaMemcpyAsync(d.node_inc + m.n_reg, inc.data(), m.n_enr * sizeof(int), cudaMemcpyHostToDevice, s));
     }
-    PG_CUDA(cudaMalloc((void**)&d.radius, rad.size() * sizeof(double)));
-    PG_CUDA(cudaMalloc((void**)&d.L, d.hL.size() * sizeof(double)));
-    PG_CUDA(cudaMalloc((void**)&d.w, d.hL.size() * sizeof(double)));
-    PG_CUDA(cudaMalloc((void**)&d.sens, std::max(1, n_slots) * sizeof(double)));
-    PG_CUDA(cudaMalloc((void**)&d.param_of, 3 * (size_t)std::max(1, d.n_inc) * sizeof(int)));
-    PG_CUDA(h2d_sync(d.node_inc, inc.data(), nn * sizeof(int)));
-    PG_CUDA(h2d_sync(d.radius, rad.data(), rad.size() * sizeof(double)));
-    PG_CUDA(h2d_sync(d.L, d.hL.data(), d.hL.size() * sizeof(double)));
+    PG_CUDA(cudaMemcpy2DAsync(d.L + 2 * (size_t)nx, 2 * (nx + 1) * sizeof(double), edge.data(), sizeof(double), sizeof(double),
+                              ny + 1, cudaMemcpyHostToDevice, s));
+    PG_CUDA(cudaMemcpyAsync(d.radius, rad.data(), rad.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+    PG_CUDA(cudaStreamSynchronize(s));
     return PG_OK;
 }
 
-void sens_free(SensData& d) {
-    for (void* p : {(void*)d.node_inc, (void*)d.vel[0], (void*)d.vel[1], (void*)d.vel[2], (void*)d.radius,
-                    (void*)d.L, (void*)d.w, (void*)d.sens, (void*)d.param_of})
-        if (p) cudaFree(p);
+int sens_setup(Ctx& c) {
+    if (c.sens) return PG_OK;
+    c.sens = new SensData();
+    const int rc = sens_build(c);
+    if (rc != PG_OK) sens_free(c);
+    return rc;
 }
 
 // f and the adjoint weights w = L - lambda at the context's U (committed
@@ -115,11 +159,12 @@ int sens_adjoint(Ctx& c, const pg_solver_cfg& cfg, SensData& d, double& f, pg_so
     cudaMemsetAsync(c.F, 0, (size_t)nd * sizeof(double), s);
     launch_assemble(c, c.U, 1.0, true, true, s);
     c.assembled = true;
-    std::vector<double> F(nd);
-    PG_CUDA(cudaMemcpyAsync(F.data(), c.F, (size_t)nd * sizeof(double), cudaMemcpyDeviceToHost, s));
+    double part[kDotCtas];
+    k_sens_dot<<<kDotCtas, kThreads, 0, s>>>(nd, d.L, c.F, d.part);
+    PG_CUDA(cudaMemcpyAsync(part, d.part, sizeof part, cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaStreamSynchronize(s));
     f = 0.0;
-    for (int i = 0; i < nd; ++i) f += d.hL[i] * F[i];
+    for (double v : part) f += v;
     // adjoint: mask(K) lambda = mask(K L)
     residual_into(c, s, d.L, nullptr, c.b);  // c.b = -mask(K L)
     k_scale_inplace<<<nb(nd), kThreads, 0, s>>>(nd, c.b, -1.0);
@@ -176,16 +221,13 @@ extern "C" int pg_sensitivity_shape(pg_ctx* cx, const pg_solver_cfg* cfg, int32_
         slot[p] = sl;
     }
     cudaStream_t s = c.stream;
-    SensData d;
-    rc = sens_setup(c, d, n_slots);
+    rc = sens_setup(c);
     double f = 0.0;
     pg_solve_stats st{};
-    if (rc == PG_OK) rc = sens_adjoint(c, *cfg, d, f, st, s);
+    if (rc == PG_OK) rc = sens_adjoint(c, *cfg, *c.sens, f, st, s);
     if (adjoint_stats) *adjoint_stats = st;
-    if (rc != PG_OK) {
-        sens_free(d);
-        return rc;
-    }
+    if (rc != PG_OK) return rc;
+    SensData& d = *c.sens;
     if (f_out) *f_out = f;
     std::vector<double> hs(std::max(1, n_slots), 0.0);
     if (n_slots > 0 && c.n_cut > 0) {
@@ -212,7 +254,6 @@ extern "C" int pg_sensitivity_shape(pg_ctx* cx, const pg_solver_cfg* cfg, int32_
         cudaMemcpyAsync(hs.data(), d.sens, n_slots * sizeof(double), cudaMemcpyDeviceToHost, s);
     }
     const cudaError_t e = cudaStreamSynchronize(s);
-    sens_free(d);
     if (e != cudaSuccess) return cuda_fail(e, "pg_sensitivity_shape");
     PG_CUDA(cudaGetLastError());
     if (dfdp)
@@ -249,16 +290,13 @@ extern "C" int pg_sensitivity_c11(pg_ctx* cx, const pg_solver_cfg* cfg, double h
     }
     // central difference of each cut element's internal force (cross-check)
     cudaStream_t s = c.stream;
-    SensData d;
-    rc = sens_setup(c, d, n_inc);
+    rc = sens_setup(c);
     double f = 0.0;
     pg_solve_stats st{};
-    if (rc == PG_OK) rc = sens_adjoint(c, *cfg, d, f, st, s);
+    if (rc == PG_OK) rc = sens_adjoint(c, *cfg, *c.sens, f, st, s);
     if (adjoint_stats) *adjoint_stats = st;
-    if (rc != PG_OK) {
-        sens_free(d);
-        return rc;
-    }
+    if (rc != PG_OK) return rc;
+    SensData& d = *c.sens;
     if (c11) *c11 = f / strain;
     cudaMemsetAsync(d.sens, 0, std::max(1, d.n_inc) * sizeof(double), s);
     CutArgs ca = cut_args(c, c.U, 1.0);
@@ -278,7 +316,6 @@ extern "C" int pg_sensitivity_c11(pg_ctx* cx, const pg_solver_cfg* cfg, double h
     std::vector<double> hs(std::max(1, d.n_inc));
     cudaMemcpyAsync(hs.data(), d.sens, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
-    sens_free(d);
     if (e != cudaSuccess) return cuda_fail(e, "pg_sensitivity_c11");
     if (dc11_dr)
         for (int i = 0; i < d.n_inc; ++i) dc11_dr[i] = hs[i] / strain;
