@@ -721,17 +721,6 @@ __host__ __device__ constexpr int tri_corner(int cp, int t, int m) {
                    : (t == 0 ? (m == 0 ? 0 : m == 1 ? 1 : 2) : (m == 0 ? 1 : m == 1 ? 3 : 2));
 }
 
-// Grid neighbours of node (gi, gj) present in its row, as bits d = 3 (dy + 1)
-// + (dx + 1) (bit 4 the node itself): axis neighbours inside the grid, and
-// the diagonal ones too for even nodes.  A block's place in the row is the
-// number of lower bits set.
-__host__ __device__ inline unsigned grid_nbr_mask(int gi, int gj, int nx, int ny) {
-    const bool even = ((gi + gj) & 1) == 0;
-    const bool w = gi > 0, e = gi < nx, s = gj > 0, n = gj < ny;
-    return (s && even && w ? 1u : 0u) | (s ? 2u : 0u) | (s && even && e ? 4u : 0u) | (w ? 8u : 0u) | 16u |
-           (e ? 32u : 0u) | (n && even && w ? 64u : 0u) | (n ? 128u : 0u) | (n && even && e ? 256u : 0u);
-}
-
 // One 2x2 block as a single 256-bit store (K is a cudaMalloc allocation, so
 // every block is 32-byte aligned).
 __device__ __forceinline__ void store_block(double* K, long long q, double k0, double k1, double k2, double k3) {

@@ -103,6 +103,17 @@ constexpr int kTriTileSizes[kTriTileVariants] = {32, 64};
 constexpr int kTriMapDiag = 1 << 28;
 constexpr int kTriMapSlow = 1 << 29;
 void build_tri_map(const HostMesh& hm, int tile_nodes, std::vector<int>& map);
+// Grid neighbours of node (gi, gj) present in its row, as bits d = 3 (dy + 1)
+// + (dx + 1) (bit 4 the node itself): axis neighbours inside the grid, and
+// the diagonal ones too for even nodes.  A block's place in the row is the
+// number of lower bits set.
+__host__ __device__ inline unsigned grid_nbr_mask(int gi, int gj, int nx, int ny) {
+    const bool even = ((gi + gj) & 1) == 0;
+    const bool w = gi > 0, e = gi < nx, s = gj > 0, n = gj < ny;
+    return (s && even && w ? 1u : 0u) | (s ? 2u : 0u) | (s && even && e ? 4u : 0u) | (w ? 8u : 0u) | 16u |
+           (e ? 32u : 0u) | (n && even && w ? 64u : 0u) | (n ? 128u : 0u) | (n && even && e ? 256u : 0u);
+}
+
 bool grid_pattern_ok(const HostMesh& hm);  // block rows laid out as the structured-grid kernel assumes
 constexpr int kGridTileCols = 64;          // node columns per structured-grid tile
 // Autotuned launch shapes of the assembly kernels (pg_ctx_autotune):

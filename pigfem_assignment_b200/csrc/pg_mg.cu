@@ -434,6 +434,10 @@ int build_hierarchy(Ctx& c) {
         set_error("multigrid: mesh without a structured background grid");
         return PG_ERR_ARG;
     }
+    if (!c.grid_emat) {  // (no builder makes one: their rows begin with the grid neighbours, see grid_pattern_ok)
+        set_error("multigrid: the background grid's rows are not laid out as its Galerkin product reads them");
+        return PG_ERR_ARG;
+    }
     // each RVE's grids, coarsened until both sides have at most kCoarseCells cells
     std::vector<std::vector<std::pair<int, int>>> dims(R);
     int nlev = 0;
@@ -689,10 +693,10 @@ int mg_numeric(Ctx& c, bool f32, bool modes, cudaStream_t s) {
         float* Af = f32 ? L.f.A : nullptr;
         float* Df = f32 ? L.f.Dinv : nullptr;
         if (l == 1)
-            k_mg_galerkin<true><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, c.row_ptr, c.col, c.K,
+            k_mg_galerkin<true><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, c.row_ptr, c.K,
                                                                            nullptr, ff, L.fixed, L.d.A, Af, L.d.Dinv, Df);
         else
-            k_mg_galerkin<false><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, nullptr, nullptr, nullptr,
+            k_mg_galerkin<false><<<nb(L.n, kGalNodes), kGalThreads, 0, s>>>(L.n, L.node_rve, L.pair, nullptr, nullptr,
                                                                             m.L[l - 1].d.A, ff, L.fixed, L.d.A, Af, L.d.Dinv,
                                                                             Df);
     }
@@ -701,7 +705,7 @@ int mg_numeric(Ctx& c, bool f32, bool modes, cudaStream_t s) {
         k_modes_E<<<nb(n0), kThreads, 0, s>>>(n0, m.z_inc, m.zval, c.row_ptr, c.col, c.K, c.fixed, m.E);
         k_modes_inv<<<nb(m.n_inc), kThreads, 0, s>>>(m.n_inc, m.E, m.Einv);
     }
-    k_mg_coarse_inverse<<<m.R, kFactorThreads, 2 * kCoarseStride * sizeof(double), s>>>(m.coarse, m.XT, m.fl);
+    k_mg_coarse_inverse<<<m.R, kFactorThreads, 0, s>>>(m.coarse, m.XT, m.fl);
     PG_CUDA(cudaGetLastError());
     return PG_OK;
 }

@@ -106,6 +106,10 @@ __device__ __forceinline__ void load4(const float* p, float& a, float& b, float&
     asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "l"(p));
 }
 
+__device__ __forceinline__ void load2(const double* p, double& a, double& b) {
+    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p));
+}
+
 // block_sum, valid in every thread
 __device__ __forceinline__ double block_sum_all(double v) {
     __shared__ double s_all;
@@ -1156,104 +1160,127 @@ __device__ __forceinline__ void masked_inverse(const double b[4], bool f0, bool 
 }
 
 // Galerkin product A_c = M_c P^T M A M P M_c of one level and its diagonal
-// inverses, in FP64, with FP32 copies on request.  One thread per child of a
-// coarse node (nine of them, those of zero weight idle): it spreads its
-// row's blocks over the coarse node's nine in its own column of shared
-// memory; then the nine columns are added in order.  (A thread per output
-// block that scans all the children's rows took 180 us at 512^2 and 31 us on
-// every level below, whatever its size.)
-constexpr int kGalNodes = 16;
-constexpr int kGalThreads = 9 * kGalNodes;
+// inverses, in FP64, with FP32 copies on request.  A CTA takes 32 coarse
+// nodes, a warp one component of one of their nine children each: its lanes'
+// rows have the same pattern and the same weights, but at the grid's edge, so
+// a block goes only to the one to four coarse blocks it has a weight for.  Sums in registers,
+// added through shared memory in the order of the children.  (With the nine
+// children of a node in neighbouring lanes every block took the instructions
+// of all nine targets: 230 us on level 1 of 512^2 and 152 on the six below;
+// now 125 and 82, bound by the instructions of 18 warps per SM.)
+constexpr int kGalNodes = 32;
+constexpr int kGalThreads = 2 * 9 * kGalNodes;
+constexpr int kGalRow = kGalNodes + 1;  // odd: different entries of a node in different banks
 
 template <bool FINE_BSR>
 __global__ void __launch_bounds__(kGalThreads) k_mg_galerkin(int n, const int* __restrict__ node_rve,
                                                              const Pair* __restrict__ pair, const int* __restrict__ row_ptr,
-                                                             const int* __restrict__ col, const double* __restrict__ K,
+                                                             const double* __restrict__ K,
                                                              const double* __restrict__ A,
                                                              const uint8_t* __restrict__ fixed_f,
                                                              const uint8_t* __restrict__ fixed_c, double* __restrict__ Ac,
                                                              float* __restrict__ Acf, double* __restrict__ Dinv,
                                                              float* __restrict__ Dinvf) {
-    __shared__ double acc[36 * kGalThreads];
-    const int t = threadIdx.x, a0 = blockIdx.x * kGalNodes;
+    __shared__ double acc[3][36 * kGalRow];
+    const int t = threadIdx.x, a0 = blockIdx.x * kGalNodes, ch = (t >> 5) % 9, d = t / (9 * kGalNodes), node = t & 31;
+    double v[9][2];
 #pragma unroll
-    for (int k = 0; k < 36; ++k) acc[k * kGalThreads + t] = 0.0;
-    const int a = a0 + t / 9;
+    for (int o = 0; o < 9; ++o) v[o][0] = v[o][1] = 0.0;
+    const int a = a0 + node;
     if (a < n) {
         const Pair p = pair[node_rve ? node_rve[a] : 0];
         const int la = a - p.coff, Ia = la % (p.cnx + 1), Ja = la / (p.cnx + 1);
-        const int cx = grid_pos(Ia, p.fnx) + t % 9 % 3 - 1, cy = grid_pos(Ja, p.fny) + t % 9 / 3 - 1;
+        const int cx = grid_pos(Ia, p.fnx) + ch % 3 - 1, cy = grid_pos(Ja, p.fny) + ch / 3 - 1;
         double wi = 0.0;
         if (cx >= 0 && cx <= p.fnx && cy >= 0 && cy <= p.fny) wi = grid_w(cx, p.fnx, Ia) * grid_w(cy, p.fny, Ja);
         if (wi != 0.0) {
-            const int W = p.fnx + 1, i = p.foff + cx + cy * W, nreg = W * (p.fny + 1);
-            const double w0 = fixed_f[2 * i] ? 0.0 : wi, w1 = fixed_f[2 * i + 1] ? 0.0 : wi;
-            auto spread = [&](int gx, int gy, int j, const double* blk) {
-                double b0, b1, b2, b3;
-                load_block(blk, b0, b1, b2, b3);
-                const bool f0 = fixed_f[2 * j], f1 = fixed_f[2 * j + 1];
-                b0 = f0 ? 0.0 : w0 * b0;
-                b1 = f1 ? 0.0 : w0 * b1;
-                b2 = f0 ? 0.0 : w1 * b2;
-                b3 = f1 ? 0.0 : w1 * b3;
-#pragma unroll
-                for (int oy = -1; oy <= 1; ++oy) {
-                    const double wy = grid_w(gy, p.fny, Ja + oy);
-                    if (wy == 0.0) continue;
-#pragma unroll
-                    for (int ox = -1; ox <= 1; ++ox) {
-                        const double w = wy * grid_w(gx, p.fnx, Ia + ox);
-                        if (w == 0.0) continue;
-                        double* o = acc + 4 * ((oy + 1) * 3 + ox + 1) * kGalThreads + t;
-                        o[0] += w * b0;
-                        o[kGalThreads] += w * b1;
-                        o[2 * kGalThreads] += w * b2;
-                        o[3 * kGalThreads] += w * b3;
-                    }
-                }
+            const int W = p.fnx + 1, i = p.foff + cx + cy * W;
+            const double wd = fixed_f[2 * i + d] ? 0.0 : wi;
+            // 2 bits per neighbour column (row) and coarse column (row): weight 0, 1 or 1/2 as 0, 1, 2
+            auto code = [](int g, int nf, int I) {
+                const double w = grid_w(g, nf, I);
+                return w == 0.0 ? 0u : w == 1.0 ? 1u : 2u;
             };
-            if (FINE_BSR) {
-                const int r1 = row_ptr[i + 1];
-                for (int q = row_ptr[i]; q < r1; ++q) {
-                    const int lj = col[q] - p.foff;
-                    if (lj < 0 || lj >= nreg) continue;  // enrichment columns: no coarse part
-                    const int gy = lj / W;
-                    spread(lj - gy * W, gy, p.foff + lj, K + 4 * (size_t)q);
+            unsigned wx = 0, wy = 0, in = 0;  // in: the neighbours inside the grid
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                wx |= code(cx + e / 3 - 1, p.fnx, Ia + e % 3 - 1) << 2 * e;
+                wy |= code(cy + e / 3 - 1, p.fny, Ja + e % 3 - 1) << 2 * e;
+                const int gx = cx + e % 3 - 1, gy = cy + e / 3 - 1;
+                in |= (gx >= 0 && gx <= p.fnx && gy >= 0 && gy <= p.fny ? 1u : 0u) << e;
+            }
+            // level 0: the row's first blocks are its grid neighbours in order (no enrichment node has a coarse part)
+            const unsigned mask = FINE_BSR ? grid_nbr_mask(cx, cy, p.fnx, p.fny) : in;
+            const double* blk = (FINE_BSR ? K + 4 * (size_t)row_ptr[i] : A + 36 * (size_t)i) + 2 * d;
+            const uchar2* fix = reinterpret_cast<const uchar2*>(fixed_f) + i;
+#pragma unroll
+            for (int s = 0; s < 9; s += 3) {
+                double b[3][2];
+                uchar2 f[3];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    b[u][0] = b[u][1] = 0.0;
+                    if (!(mask >> (s + u) & 1)) continue;
+                    const int q = FINE_BSR ? __popc(mask & ((1u << (s + u)) - 1u)) : s + u;
+                    load2(blk + 4 * q, b[u][0], b[u][1]);
+                    f[u] = fix[(s / 3 - 1) * W + u - 1];
                 }
-            } else {
-                for (int s = 0; s < 9; ++s) {
-                    const int gx = cx + s % 3 - 1, gy = cy + s / 3 - 1;
-                    if (gx < 0 || gx > p.fnx || gy < 0 || gy > p.fny) continue;
-                    spread(gx, gy, p.foff + gx + gy * W, A + 36 * (size_t)i + 4 * s);
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    if (!(mask >> (s + u) & 1)) continue;
+                    const double b0 = f[u].x ? 0.0 : wd * b[u][0], b1 = f[u].y ? 0.0 : wd * b[u][1];
+#pragma unroll
+                    for (int oy = 0; oy < 3; ++oy) {
+                        const unsigned ky = wy >> 2 * (s + oy) & 3u;
+                        if (!ky) continue;
+#pragma unroll
+                        for (int ox = 0; ox < 3; ++ox) {
+                            const unsigned kx = wx >> 2 * (3 * u + ox) & 3u;
+                            if (!kx) continue;
+                            // 2^(2 - kx - ky)
+                            const double w = __hiloint2double((int)((1025u - kx - ky) << 20), 0);
+                            v[3 * oy + ox][0] += w * b0;
+                            v[3 * oy + ox][1] += w * b1;
+                        }
+                    }
                 }
             }
         }
     }
-    __syncthreads();
-    for (int q = t; q < 36 * kGalNodes; q += kGalThreads) {
-        const int node = q / 36, k = q % 36, c = a0 + node;
-        if (c >= n) break;
-        double v = 0.0;
+    // a group of three children each, then the groups
 #pragma unroll
-        for (int ch = 0; ch < 9; ++ch) v += acc[k * kGalThreads + node * 9 + ch];
+    for (int turn = 0; turn < 3; ++turn) {
+        if (ch % 3 == turn) {
+            double* o = acc[ch / 3] + 2 * d * kGalRow + node;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    double& x = o[(4 * k + e) * kGalRow];
+                    x = turn ? x + v[k][e] : v[k][e];
+                }
+        }
+        __syncthreads();
+    }
+    auto total = [&](int k, int nd) { return acc[0][k * kGalRow + nd] + acc[1][k * kGalRow + nd] + acc[2][k * kGalRow + nd]; };
+    for (int q = t; q < 36 * kGalNodes; q += kGalThreads) {
+        const int nd = q / 36, k = q % 36, c = a0 + nd;
+        if (c >= n) break;
+        double s = total(k, nd);
         const Pair p = pair[node_rve ? node_rve[c] : 0];
         const int la = c - p.coff, Ib = la % (p.cnx + 1) + k / 4 % 3 - 1, Jb = la / (p.cnx + 1) + k / 12 - 1;
         if (Ib < 0 || Ib > p.cnx || Jb < 0 || Jb > p.cny || fixed_c[2 * c + k % 4 / 2] ||
             fixed_c[2 * (p.coff + Ib + Jb * (p.cnx + 1)) + k % 2])
-            v = 0.0;
-        Ac[36 * (size_t)c + k] = v;
-        if (Acf) Acf[36 * (size_t)c + k] = (float)v;
+            s = 0.0;
+        Ac[36 * (size_t)c + k] = s;
+        if (Acf) Acf[36 * (size_t)c + k] = (float)s;
     }
     if (t < kGalNodes && a0 + t < n) {
         const int c = a0 + t;
         const bool f0 = fixed_c[2 * c], f1 = fixed_c[2 * c + 1];
         double b[4], m[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            b[k] = 0.0;
-#pragma unroll
-            for (int ch = 0; ch < 9; ++ch) b[k] += acc[(16 + k) * kGalThreads + t * 9 + ch];
-        }
+        for (int k = 0; k < 4; ++k) b[k] = total(16 + k, t);
         masked_inverse(b, f0, f1, m);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1269,28 +1296,35 @@ __global__ inline void k_mg_to_f32(size_t n, const double* a, float* b) {
 }
 
 // The coarsest operator of each RVE (one CTA each) inverted explicitly, by
-// Gauss-Jordan elimination with partial pivoting on [M | I]: fixed DOFs get
-// identity rows and columns, and zero rows and columns in the result.  Two
-// barriers per pivot; every warp finds the pivot for itself.  Stored
-// transposed (XT[j n + r] = X[r][j]).  Flag 3 = 1 on a zero pivot.
+// Gauss-Jordan elimination in place with partial pivoting: fixed DOFs get
+// identity rows and columns, and zero rows and columns in the result.  A
+// thread keeps its column's rows t / 64, t / 64 + 4, ... in registers; rows
+// stay where they are, and step k's pivot is the largest entry of column k in
+// a row that no step has taken.  A step's column and pivot row pass through
+// shared memory.  Stored transposed (XT[j n + r] = X[r][j]).  Flag 3 = 1 on a
+// zero pivot.  Bound by the latency of a step, 50 of them at most.  (With
+// [M | I] in shared memory and row exchanges: 102 us, now 64.)
 struct Coarse {
     const double* A;
     const uint8_t* fixed;
     int off, nx, ny, pad;
 };
-constexpr int kFactorThreads = 512;
+constexpr int kFactorThreads = 256;
 
 __global__ void __launch_bounds__(kFactorThreads) k_mg_coarse_inverse(const Coarse* __restrict__ cd, double* XT, int* fl) {
-    constexpr int kW = 2 * kCoarseMaxDof;
-    extern __shared__ __align__(16) unsigned char factor_smem[];
-    double(*M)[kW] = reinterpret_cast<double(*)[kW]>(factor_smem);
+    constexpr int kCols = 64, kRowStep = kFactorThreads / kCols, kPer = (kCoarseMaxDof + kRowStep - 1) / kRowStep;
+    static_assert(kCoarseMaxDof <= kCols, "a thread per column");
+    constexpr int kW = kCoarseMaxDof + 1;  // odd: a column's entries in different banks
+    __shared__ double M[kCoarseMaxDof][kW];
+    __shared__ double s_colk[2][kPer * kRowStep], s_row[kCols], s_best[2][kRowStep];
+    __shared__ int s_arg[2][kRowStep], s_step[kCoarseMaxDof], s_pivot[kCoarseMaxDof];
     const Coarse C = cd[blockIdx.x];
-    const int nn = (C.nx + 1) * (C.ny + 1), n = 2 * nn, t = threadIdx.x, lane = t & 31;
+    const int nn = (C.nx + 1) * (C.ny + 1), n = 2 * nn, t = threadIdx.x;
     const uint8_t* fixed = C.fixed + 2 * (size_t)C.off;
     const double* A = C.A + 36 * (size_t)C.off;
-    for (int e = t; e < n * 2 * n; e += kFactorThreads) {
-        const int r = e / (2 * n), c = e % (2 * n);
-        M[r][c] = (c - n == r || (c == r && fixed[r])) ? 1.0 : 0.0;
+    for (int e = t; e < n * n; e += kFactorThreads) {
+        const int r = e / n, c = e % n;
+        M[r][c] = c == r && fixed[r] ? 1.0 : 0.0;
     }
     __syncthreads();
     for (int e = t; e < 9 * nn; e += kFactorThreads) {
@@ -1302,51 +1336,76 @@ __global__ void __launch_bounds__(kFactorThreads) k_mg_coarse_inverse(const Coar
                 if (!fixed[2 * a + d] && !fixed[2 * b + f]) M[2 * a + d][2 * b + f] = A[36 * (size_t)a + 4 * o + 2 * d + f];
     }
     __syncthreads();
-    // a thread keeps to one column: rows t / 128, t / 128 + 4, ...
-    constexpr int kCols = 128, kRowStep = kFactorThreads / kCols, kPer = (kCoarseMaxDof + kRowStep - 1) / kRowStep;
     const int c = t % kCols, rg = t / kCols;
-    for (int k = 0; k < n; ++k) {
-        // the largest entry of column k at or below the diagonal (the first such row)
-        double best = -1.0;
-        int pr = k;
-        for (int r = k + lane; r < n; r += 32)
-            if (fabs(M[r][k]) > best) {
-                best = fabs(M[r][k]);
-                pr = r;
-            }
+    unsigned taken = 0;  // this thread's rows that were pivots (bit u)
+    double v[kPer];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int op = __shfl_xor_sync(0xffffffffu, pr, o);
+    for (int u = 0; u < kPer; ++u) {
+        const int r = rg + u * kRowStep;
+        v[u] = r < n && c < n ? M[r][c] : 0.0;
+    }
+    // column k for the step, and its largest entry among this thread's free rows (the first such row)
+    auto publish = [&](int k) {
+        if (c != k) return;
+        double best = -1.0;
+        int arg = n;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int r = rg + u * kRowStep;
+            s_colk[k & 1][r] = v[u];
+            if (r < n && !(taken >> u & 1)) {
+                if (arg == n) arg = r;  // (entries that don't compare: the first free row)
+                if (fabs(v[u]) > best) {
+                    best = fabs(v[u]);
+                    arg = r;
+                }
+            }
+        }
+        s_best[k & 1][rg] = best;
+        s_arg[k & 1][rg] = arg;
+    };
+    publish(0);
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+        double best = s_best[k & 1][0];
+        int pr = s_arg[k & 1][0];
+#pragma unroll
+        for (int g = 1; g < kRowStep; ++g) {
+            const double ob = s_best[k & 1][g];
+            const int op = s_arg[k & 1][g];
             if (ob > best || (ob == best && op < pr)) {
                 best = ob;
                 pr = op;
             }
         }
-        const double piv = M[pr][k];
-        if (piv == 0.0 && t == 0) fl[kFlags * blockIdx.x + 3] = 1;
-        double v[kPer];
-        if (c < 2 * n) {
-            const double pc = piv != 0.0 ? M[pr][c] / piv : 0.0;
+        const double piv = s_colk[k & 1][pr];
+        const int pu = rg == pr % kRowStep ? pr / kRowStep : -1;  // this thread's place of the pivot row
 #pragma unroll
-            for (int u = 0; u < kPer; ++u) {
-                const int r = rg + u * kRowStep;
-                const int src = r == pr ? k : r;  // rows k and pr change places
-                if (r < n) v[u] = r == k ? pc : M[src][c] - M[src][k] * pc;
-            }
+        for (int u = 0; u < kPer; ++u)
+            if (u == pu) s_row[c] = v[u];
+        if (pu >= 0) taken |= 1u << pu;
+        if (t == 0) {
+            s_step[pr] = k;
+            s_pivot[k] = pr;
+            if (piv == 0.0) fl[kFlags * blockIdx.x + 3] = 1;
         }
         __syncthreads();
-        if (c < 2 * n) {
+        // column k is replaced by what the unit matrix's column has become
+        const double pc = piv != 0.0 ? (c == k ? 1.0 : s_row[c]) / piv : 0.0;
 #pragma unroll
-            for (int u = 0; u < kPer; ++u)
-                if (rg + u * kRowStep < n) M[rg + u * kRowStep][c] = v[u];
-        }
+        for (int u = 0; u < kPer; ++u)
+            v[u] = u == pu ? pc : (c == k ? 0.0 : v[u]) - s_colk[k & 1][rg + u * kRowStep] * pc;
+        publish(k + 1);
         __syncthreads();
     }
+    // row pr of the result is row s_step[pr] of the inverse, its column k column s_pivot[k]
     double* X = XT + (size_t)blockIdx.x * kCoarseStride;
-    for (int e = t; e < n * n; e += kFactorThreads) {
-        const int j = e / n, r = e % n;
-        X[e] = (fixed[r] || fixed[j]) ? 0.0 : M[r][n + j];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int r = rg + u * kRowStep;
+        if (r >= n || c >= n) continue;
+        const int R = s_step[r], J = s_pivot[c];
+        X[J * n + R] = (fixed[R] || fixed[J]) ? 0.0 : v[u];
     }
 }
 
