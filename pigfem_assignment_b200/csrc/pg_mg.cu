@@ -633,9 +633,10 @@ int build_hierarchy(Ctx& c) {
                                  4 * kBottomStride * (int)sizeof(Vec2<double>)));
     PG_CUDA(cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  4 * kBottomStride * (int)sizeof(Vec2<float>)));
-    for (auto k : {k_mg_enr<double, false>, k_mg_enr<double, true>})
+    for (auto k : {k_mg_enr<double, false, kPieceThreads>, k_mg_enr<double, true, kPieceThreads>})
         PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    for (auto k : {k_mg_enr<float, false>, k_mg_enr<float, true>})
+    for (auto k : {k_mg_enr<float, false, kPieceThreads>, k_mg_enr<float, true, kPieceThreads>,
+                   k_mg_enr<float, false, kPieceThreadsWide>, k_mg_enr<float, true, kPieceThreadsWide>})
         PG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     // coarse masks by injection
     cudaStream_t s = c.stream;
@@ -730,6 +731,27 @@ struct Cycle<float> {
     static LevelArrays<float>& lev(Level& L) { return L.f; }
 };
 
+// The enrichment nodes' smoothing: x_e of the cycle's x into xout.  Pieces of
+// a cohesive mesh hold some 100 rows (both sides of an interface) and get a
+// thread group per row in the FP32 cycle; in FP64 a row's blocks leave no
+// registers for that.
+template <typename T, bool POST>
+void mg_enr(Ctx& c, MgHierarchy& m, cudaStream_t s, const double* r, T* xout, const int* fl) {
+    using C = Cycle<T>;
+    if (m.n_pieces == 0) return;
+    auto go = [&](auto kern, int threads) {
+        launch_pdl(kern, m.n_pieces, threads, (size_t)m.max_piece * 4 * sizeof(Vec2<T>), s, m.enr, c.row_ptr, c.col, C::K(c),
+                   C::Dinv(c, m), c.fixed, m.spans.reg_end, r, C::x(m), xout, fl);
+    };
+    if constexpr (std::is_same<T, float>::value) {
+        if (m.max_piece > kPieceThreads / kRowLanes) {
+            go(k_mg_enr<T, POST, kPieceThreadsWide>, kPieceThreadsWide);
+            return;
+        }
+    }
+    go(k_mg_enr<T, POST, kPieceThreads>, kPieceThreads);
+}
+
 // The V-cycle after its first sweep (which CG's update has formed): z = V(r)
 // and the partials of r.z.  fl null outside CG; check: this cycle follows a
 // CG update, whose r.r it tests.
@@ -738,10 +760,7 @@ void mg_cycle(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s, const double* 
     using C = Cycle<T>;
     const T *K = C::K(c), *D0 = C::Dinv(c, m);
     T *x0 = C::x(m), *xe = C::xe(m);
-    const size_t esm = (size_t)m.max_piece * 4 * sizeof(Vec2<T>);
-    if (m.n_pieces > 0)
-        launch_pdl(k_mg_enr<T, false>, m.n_pieces, kPieceThreads, esm, s, m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
-                                                                  x0, x0, fl);
+    mg_enr<T, false>(c, m, s, r, x0, fl);
     launch_pdl(k_mg_down0<T>, m.L[1].down.n, kDown0Threads, 0, s, m.L[1].down.tile, m.L[1].pair, c.row_ptr, c.col, K, c.fixed, r, x0,
                                                          m.L[1].fixed, C::lev(m.L[1]).b, m.spans, m.part_rr, m.sc, fl,
                                                          check ? 1 : 0);
@@ -773,9 +792,7 @@ void mg_cycle(Ctx& c, MgHierarchy& m, bool modes, cudaStream_t s, const double* 
             launch_pdl(k_mg_up<T, false>, L.up.n, kTileThreads, 0, s, L.up.tile, L.pair, m.L[l + 1].pair, v.A, v.Dinv, L.fixed, v.b,
                                                               v.x, xc, v.xo, nullptr, nullptr, fl);
     }
-    if (m.n_pieces > 0)
-        launch_pdl(k_mg_enr<T, true>, m.n_pieces, kPieceThreads, esm, s, m.enr, c.row_ptr, c.col, K, D0, c.fixed, m.spans.reg_end, r,
-                                                                 x0, xe, fl);
+    mg_enr<T, true>(c, m, s, r, xe, fl);
     launch_pdl(k_mg_post<T>, m.n_cta, kSpanThreads, 0, s, m.spans, c.row_ptr, c.col, K, D0, c.fixed, r, x0, xe, z, fl, m.part_rz);
     if (m.n_inc > 0 && modes) {
         const int n = c.n_nodes;

@@ -445,7 +445,9 @@ struct Piece {
     int rve, pad0, pad1;
 };
 constexpr int kPieceRows = 48;
-constexpr int kPieceThreads = 256;
+// Threads per CTA: all of a piece's rows at once, as a row beyond the first
+// TH / kRowLanes loads its numbers and blocks again in every step.
+constexpr int kPieceThreads = 256, kPieceThreadsWide = 448;
 
 struct Enr {
     const Piece* piece;
@@ -455,8 +457,8 @@ struct Enr {
     const double* coef;        // kChebCoef per RVE
 };
 
-template <typename T, bool POST>
-__global__ void __launch_bounds__(kPieceThreads, 3) k_mg_enr(Enr e, const int* __restrict__ row_ptr, const int* __restrict__ col,
+template <typename T, bool POST, int TH>
+__global__ void __launch_bounds__(TH, TH == kPieceThreads ? 3 : 2) k_mg_enr(Enr e, const int* __restrict__ row_ptr, const int* __restrict__ col,
                                                           const T* __restrict__ K, const T* __restrict__ Dinv,
                                                           const uint8_t* __restrict__ fixed, const int* __restrict__ reg_end,
                                                           const double* b, const T* xin, T* xout, const int* fl) {
@@ -470,7 +472,7 @@ __global__ void __launch_bounds__(kPieceThreads, 3) k_mg_enr(Enr e, const int* _
     const double* cf = e.coef + kChebCoef * pc.rve;
     const int reg = reg_end[pc.rve];
     const int g = threadIdx.x % kRowLanes, l0 = threadIdx.x / kRowLanes;
-    constexpr int kRows = kPieceThreads / kRowLanes;
+    constexpr int kRows = TH / kRowLanes;
     constexpr int kEnt = 2;  // entries of K_ee that a lane keeps of its row among the first kRows (8 a row)
     int i = l0 < n ? e.node[pc.row0 + l0] : 0;
     RowFrag<T> f;
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(kPieceThreads, 3) k_mg_enr(Enr e, const int* _
         __syncthreads();
     }
     const Vec2<T>* xl = ((kChebSteps - 1) & 1) ? sx2 : sx;
-    for (int l = threadIdx.x; l < pc.end[0]; l += kPieceThreads) {
+    for (int l = threadIdx.x; l < pc.end[0]; l += TH) {
         const int il = e.node[pc.row0 + l];
         Vec2<T> v = xl[l];
         if (POST) {
