@@ -735,8 +735,9 @@ __global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_mg_post(Spans 
 // ---------------------------------------------------------------------------
 //
 // A thread keeps one node of the tile's first swept region through all the
-// phases, so its operator row is loaded once, before the wait.
-constexpr int kTileThreads = 384;
+// phases, so its operator row is loaded once, before the wait.  448 threads:
+// the 441 nodes that the first sweep reads are staged in one round of loads.
+constexpr int kTileThreads = 448;
 
 template <typename T>
 struct NodeRow {
@@ -900,11 +901,19 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_up(
         else st2(xo, i, v.x, v.y);
     }
     if (!FINE) return;
+    // level 0's x is on its way while the sweep ends
+    constexpr int F = 2 * kUpTile, kPer = (F * F + kTileThreads - 1) / kTileThreads;
+    Vec2<T> xv[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int l = threadIdx.x + u * kTileThreads, gx = 2 * gx0 + l % F, gy = 2 * gy0 + l / F;
+        if (l < F * F && gx <= pf.fnx && gy <= pf.fny) xv[u] = lv2(x0, pf.foff + gx + gy * (pf.fnx + 1));
+    }
     __syncthreads();
-    constexpr int F = 2 * kUpTile;
-    for (int l = threadIdx.x; l < F * F; l += kTileThreads) {
-        const int gx = 2 * gx0 + l % F, gy = 2 * gy0 + l / F;
-        if (gx > pf.fnx || gy > pf.fny) continue;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int l = threadIdx.x + u * kTileThreads, gx = 2 * gx0 + l % F, gy = 2 * gy0 + l / F;
+        if (l >= F * F || gx > pf.fnx || gy > pf.fny) continue;
         int I0, I1, J0, J1;
         parents(gx, pf.fnx, I0, I1);
         parents(gy, pf.fny, J0, J1);
@@ -914,7 +923,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_up(
         J1 -= gy0;
         const Vec2<T> a = s0[J0 * W0 + I0], bq = s0[J0 * W0 + I1], c = s0[J1 * W0 + I0], d = s0[J1 * W0 + I1];
         const int i = pf.foff + gx + gy * (pf.fnx + 1);
-        Vec2<T> v = lv2(x0, i);
+        Vec2<T> v = xv[u];
         if (!fixed0[2 * i]) v.x += (T)0.25 * ((a.x + bq.x) + (c.x + d.x));
         if (!fixed0[2 * i + 1]) v.y += (T)0.25 * ((a.y + bq.y) + (c.y + d.y));
         st2(x0, i, v.x, v.y);
