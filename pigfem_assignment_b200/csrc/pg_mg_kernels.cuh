@@ -121,6 +121,15 @@ __device__ __forceinline__ double block_sum_all(double v) {
     return v;
 }
 
+// Whether an RVE is done, for every thread of a CTA alike and before its
+// kernel's wait, so that no load after the wait stands behind this one (each
+// kernel of the chain had a trip to memory more).  The flag may be set
+// meanwhile: a kernel that misses that forms vectors nobody reads, as x and
+// the iteration count change in k_cg_update alone, which looks after its wait.
+__device__ __forceinline__ bool cta_done(const int* fl, int r) {
+    return fl && __syncthreads_or(__ldcg(&fl[kFlags * r]));
+}
+
 // The sum of one RVE's partials, in CTA order.  A reduction's kernel leaves
 // one partial per CTA and the next kernel's CTAs each add them up: the kernel
 // boundary orders the two, so no CTA waits on a fence and a ticket (which held
@@ -333,9 +342,10 @@ __global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_cg_spmv(Spans 
     __shared__ double2 s_rows[kSpanThreads / 32 * kWarpBlocks];
     const int4 S = sp.span[blockIdx.x];
     const int2 rg = sp.range[S.x];
+    const bool done = cta_done(fl, S.x);
     pdl_wait();
     pdl_trigger();
-    if (__ldcg(&fl[kFlags * S.x])) return;
+    if (done) return;
     double* s = sc + kScal * S.x;
     const double rz_old = __ldcg(&s[1 - P]);
     const double rz = range_sum(part_rz, rg);
@@ -374,12 +384,26 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* x,
     const int4 S = sp.span[blockIdx.x];
     const int2 rg = sp.range[S.x];
     const int reg = sp.reg_end[S.x];
+    const bool was_done = cta_done(fl, S.x);
     pdl_wait();
     pdl_trigger();
+    if (was_done) return;
     int* f = fl + kFlags * S.x;
-    if (__ldcg(&f[0])) return;
+    const int done = __ldcg(&f[0]);
+    // a thread's first vectors are on their way while alpha is summed (a small system's CTA has one node per thread)
+    int i = S.y + threadIdx.x;
+    Vec2<double> xv, rv, pv, qv;
+    auto load = [&] {
+        if (i >= S.z) return;
+        xv = lv2(x, i);
+        rv = lv2(r, i);
+        pv = lv2(p, i);
+        qv = lv2(q, i);
+    };
+    load();
     const double rz = __ldcg(&sc[kScal * S.x + P]);
     const double pq = range_sum(part_pq, rg);
+    if (done) return;
     const bool first = (int)blockIdx.x == rg.x && threadIdx.x == 0;
     if (!(pq > 0.0)) {
         if (first) {
@@ -391,8 +415,7 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* x,
     if (first) f[2] += 1;
     const double alpha = rz / pq;
     double acc = 0.0;
-    for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
-        const Vec2<double> xv = lv2(x, i), rv = lv2(r, i), pv = lv2(p, i), qv = lv2(q, i);
+    while (i < S.z) {
         const double r0 = rv.x - alpha * qv.x, r1 = rv.y - alpha * qv.y;
         st2(x, i, xv.x + alpha * pv.x, xv.y + alpha * pv.y);
         st2(r, i, r0, r1);
@@ -402,6 +425,8 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* x,
             load4(Dinv + 4 * (size_t)i, m0, m1, m2, m3);
             st2(x1, i, (T)kOmegaReg * (m0 * (T)r0 + m1 * (T)r1), (T)kOmegaReg * (m2 * (T)r0 + m3 * (T)r1));
         }
+        i += kSpanThreads;
+        load();
     }
     acc = block_sum(acc);
     if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
@@ -410,10 +435,11 @@ __global__ void __launch_bounds__(kSpanThreads) k_cg_update(Spans sp, double* x,
 // partials of a.b
 __global__ inline void __launch_bounds__(kSpanThreads) k_cg_dot(Spans sp, const double* a, const double* b, const int* fl,
                                                                 double* part) {
+    const int4 S = sp.span[blockIdx.x];
+    const bool done = cta_done(fl, S.x);
     pdl_wait();
     pdl_trigger();
-    const int4 S = sp.span[blockIdx.x];
-    if (fl && __ldcg(&fl[kFlags * S.x])) return;
+    if (done) return;
     double acc = 0.0;
     for (int i = S.y + threadIdx.x; i < S.z; i += kSpanThreads) {
         const Vec2<double> u = lv2(a, i), v = lv2(b, i);
@@ -496,9 +522,10 @@ __global__ void __launch_bounds__(TH, TH == kPieceThreads ? 3 : 2) k_mg_enr(Enr 
     T c[2 * kChebSteps - 1];
 #pragma unroll
     for (int k = 0; k < 2 * kChebSteps - 1; ++k) c[k] = (T)cf[k];
+    const bool done = cta_done(fl, pc.rve);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * pc.rve])) return;
+    if (done) return;
     for (int base = 0; base < n; base += kRows) {
         const int l = base + l0;
         if (base > 0) {
@@ -647,9 +674,10 @@ __global__ void __launch_bounds__(kDown0Threads, sizeof(T) == 8 ? 4 : 3) k_mg_do
     const int4 tl = tile[blockIdx.x];
     const Pair p = pair[tl.x];
     const int gx0 = 2 * tl.y - 1, gy0 = 2 * tl.z - 1;
+    const bool done = cta_done(fl, tl.x);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
+    if (done) return;
     if (check && tl.w) {
         const double rr = range_sum(part_rr, sp.range[tl.x]);
         if (threadIdx.x == 0 && rr <= __ldcg(&sc[kScal * tl.x + 4])) fl[kFlags * tl.x] = 1;
@@ -690,9 +718,10 @@ __global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_mg_post(Spans 
     __shared__ double2 s_rows[kSpanThreads / 32 * kWarpBlocks];
     const int4 S = sp.span[blockIdx.x];
     const int reg = sp.reg_end[S.x];
+    const bool done = cta_done(fl, S.x);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * S.x])) return;
+    if (done) return;
     double acc = 0.0;
     for (WarpSpan ws = warp_span(S.y, min(S.z, reg)); ws.i < ws.end; ws.i += ws.step) {
         const int n = min(ws.step, ws.end - ws.i), i = ws.i + (threadIdx.x & 31);
@@ -789,9 +818,10 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_dow
     const int i = in ? p.foff + gx + gy * (p.fnx + 1) : p.foff;
     NodeRow<T> row;
     row.load(i, A, Dinv);
+    const bool done = cta_done(fl, tl.x);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
+    if (done) return;
     Vec2<T> bv = lv2(b, i);
     for (int l = t; l < W2 * W2; l += kTileThreads) {
         const int hx = gx0 - 1 + l % W2, hy = gy0 - 1 + l / W2;
@@ -869,9 +899,10 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2) k_mg_up(
     const int i = in ? off + gx + gy * (nx + 1) : off;
     NodeRow<T> row;
     row.load(i, A, Dinv);
+    const bool done = cta_done(fl, tl.x);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * tl.x])) return;
+    if (done) return;
     const Vec2<T> bv = lv2(b, i);
     for (int l = t; l < W2 * W2; l += kTileThreads) {
         const int hx = gx0 - 2 + l % W2, hy = gy0 - 2 + l / W2;
@@ -1032,9 +1063,10 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const Bottom* __re
     }
     for (int q = t; q < nc * nc; q += kBottomThreads) s_inv[q] = XT[(size_t)r * kCoarseStride + q];
     Vec2<T>*vb = s_vec, *v1 = vb + kBottomStride, *v2 = v1 + kBottomStride, *vr = v2 + kBottomStride;
+    const bool done = cta_done(fl, r);
     pdl_wait();
     pdl_trigger();
-    if (fl && __ldcg(&fl[kFlags * r])) return;
+    if (done) return;
     {
         const int n = (B.nx[0] + 1) * (B.ny[0] + 1);
         if (t < n) vb[kPad + B.vec[0] + t] = lv2(ar.b[B.first], B.off[0] + t);
