@@ -123,7 +123,8 @@ __device__ __forceinline__ double block_sum_all(double v) {
 
 // Whether an RVE is done, for every thread of a CTA alike and before its
 // kernel's wait, so that no load after the wait stands behind this one (each
-// kernel of the chain had a trip to memory more).  The flag may be set
+// kernel of the chain had a trip to memory more: 512^2 FP64 8.96 -> 8.06 ms,
+// the cohesive 256^2 path 162 -> 140).  The flag may be set
 // meanwhile: a kernel that misses that forms vectors nobody reads, as x and
 // the iteration count change in k_cg_update alone, which looks after its wait.
 __device__ __forceinline__ bool cta_done(const int* fl, int r) {
@@ -472,7 +473,8 @@ struct Piece {
 };
 constexpr int kPieceRows = 48;
 // Threads per CTA: all of a piece's rows at once, as a row beyond the first
-// TH / kRowLanes loads its numbers and blocks again in every step.
+// TH / kRowLanes loads its numbers and blocks again in every step (pieces of
+// 60 to 108 rows, 256^2 cohesive, FP32: 9.3 us with 256 threads, 8.4 with 448).
 constexpr int kPieceThreads = 256, kPieceThreadsWide = 448;
 
 struct Enr {
@@ -765,7 +767,8 @@ __global__ void __launch_bounds__(kSpanThreads, kSpanCtasPerSm) k_mg_post(Spans 
 //
 // A thread keeps one node of the tile's first swept region through all the
 // phases, so its operator row is loaded once, before the wait.  448 threads:
-// the 441 nodes that the first sweep reads are staged in one round of loads.
+// the 441 nodes that the first sweep reads are staged in one round of loads
+// (384 threads took two: 3% of a 256^2 solve in FP64, 1.5% of 512^2).
 constexpr int kTileThreads = 448;
 
 template <typename T>
