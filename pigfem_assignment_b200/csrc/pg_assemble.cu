@@ -1331,9 +1331,13 @@ __device__ __forceinline__ double2 lds2(const double* p) { return *reinterpret_c
 
 // One CTA per cut_elems_per_cta(blockDim.x, NL) consecutive elements of size
 // class NL.  The CTA first forms its elements' quadrature rows in shared
-// memory (one thread per point, from the point records; the mesh is all it
-// reads, so this part runs beside the kernel before it), then one thread per
-// local function a of an element integrates the element's row a of blocks:
+// memory (one thread per point, from the point records; it reads nothing that
+// the kernel before it writes, so this part runs beside that one).  A
+// stiffness pass takes the coordinates that a record names straight from
+// global memory: through staged nodes, as the other passes, the row has a
+// block barrier more in its chain (cut elements of 512^2 25.4 us cold, now
+// 23.6; of 64^2 16.4, now 15.4).  Then one thread per local function a of an
+// element integrates the element's row a of blocks:
 // K_ab = sum_q w_q B_a^T D B_b over the rows for every b, plus the cohesive
 // sub-elements' N_a N_b (+-) R^T D R terms where both nodes are cohesive
 // nodes.  Residual passes store one force term per local function: the bulk
@@ -1360,27 +1364,39 @@ __global__ void __launch_bounds__(256, NL <= 5 ? 3 : (NL <= 7 ? 2 : 1)) k_cut_el
     const int sp_e = __ldg(&a.cut_slot_ptr[ci]);
     double2* sXY = reinterpret_cast<double2*>(sRow + a.node_off);
     double2* sU = sXY + epc * NL;
-    double* sCoh = reinterpret_cast<double*>(WF || COH ? sU + epc * NL : sU);
+    double* sCoh = reinterpret_cast<double*>(sU + epc * NL);
     int p = __ldg(&a.pt_off[c0]) + (int)threadIdx.x;
     const int p1 = __ldg(&a.pt_off[a.first + e1]);
-    int4 r2 = make_int4(0, 0, 0, 0), r3 = r2;
-    if (p < p1) {
-        r2 = __ldg(a.pts + 4 * (size_t)p + 2);
-        r3 = __ldg(a.pts + 4 * (size_t)p + 3);
-    }
-    const int nd = act ? __ldg(&a.cut_nodes[(size_t)kCutNodeStride * ci + pa]) : -1;  // -1: fewer local nodes
-    if (nd >= 0) {
-        sXY[le * NL + pa] = make_double2(__ldg(&a.x[nd]), __ldg(&a.y[nd]));
-        if (WF || COH) sU[le * NL + pa] = make_double2(__ldg(&a.u[2 * (size_t)nd]), __ldg(&a.u[2 * (size_t)nd + 1]));
-    }
-    __syncthreads();
-    while (p < p1) {
-        const long long off = (long long)(unsigned)r3.x | ((long long)r3.y << 32);
-        cut_point_row_local(r2, sXY + (r3.z - c0) * NL, a.dmat, sRow + (off - base));
-        p += blockDim.x;
+    if (WF || COH) {
+        // the nodes' coordinates and displacements first, as the cohesive
+        // points and the force terms read them too; the first point record is
+        // loaded meanwhile
+        int4 r2 = make_int4(0, 0, 0, 0), r3 = r2;
         if (p < p1) {
             r2 = __ldg(a.pts + 4 * (size_t)p + 2);
             r3 = __ldg(a.pts + 4 * (size_t)p + 3);
+        }
+        const int nd = act ? __ldg(&a.cut_nodes[(size_t)kCutNodeStride * ci + pa]) : -1;  // -1: fewer local nodes
+        if (nd >= 0) {
+            sXY[le * NL + pa] = make_double2(__ldg(&a.x[nd]), __ldg(&a.y[nd]));
+            sU[le * NL + pa] = make_double2(__ldg(&a.u[2 * (size_t)nd]), __ldg(&a.u[2 * (size_t)nd + 1]));
+        }
+        __syncthreads();
+        while (p < p1) {
+            const long long off = (long long)(unsigned)r3.x | ((long long)r3.y << 32);
+            cut_point_row_local(r2, sXY + (r3.z - c0) * NL, a.dmat, sRow + (off - base));
+            p += blockDim.x;
+            if (p < p1) {
+                r2 = __ldg(a.pts + 4 * (size_t)p + 2);
+                r3 = __ldg(a.pts + 4 * (size_t)p + 3);
+            }
+        }
+    } else {
+        // a stiffness pass needs the coordinates for the rows alone
+        for (; p < p1; p += blockDim.x) {
+            const CutPoint cp = cut_point_load(a.pts + 4 * (size_t)p);
+            const long long off = (long long)(unsigned)cp.r3.x | ((long long)cp.r3.y << 32);
+            cut_point_row(cp, a.x, a.y, a.dmat, sRow + (off - base));
         }
     }
     if (COH) {
@@ -2164,8 +2180,8 @@ int launch_cut_elems(const Ctx& c, const double* U, double dt, bool want_f, bool
         ea.coh_max = c.cut_class_coh[k];
         ea.node_off = std::max(2, c.cut_span[k][w]);
         const bool coh = c.n_coh_qp > 0 && ea.coh_max > 0;
-        const size_t smem = sizeof(double) * ((size_t)ea.node_off + (want_f || coh ? 4 : 2) * epc * kCutClassNl[k] +
-                                              2 * (size_t)kCohRow * ea.coh_max * epc);
+        size_t smem = sizeof(double) * (size_t)ea.node_off;
+        if (want_f || coh) smem += sizeof(double) * (4 * epc * kCutClassNl[k] + 2 * (size_t)kCohRow * ea.coh_max * epc);
         if (smem > 227 * 1024) {
             set_error("cut elements: a CTA's quadrature rows exceed the shared memory (use fewer warps per CTA)");
             return PG_ERR_LIMIT;
