@@ -389,7 +389,9 @@ int pg_sensitivity_c11(pg_ctx* c, const pg_solver_cfg* cfg, double h_rel, double
 int pg_ctx_autotune(pg_ctx* c, int32_t reps, float* ms_tri, float* ms_cut);
 /* the launch shapes in use, and setting them by hand (tile 32 or 64 node rows per CTA of the
  * row-tile kernel, or 128 / 256 threads per CTA of the structured-grid kernel; persistent 0/1
- * for either; warps 2/4/8 per CTA of the cut elements' kernel) */
+ * for either; warps 2/4/8 per CTA of the cut elements' kernel).  Until it is set or tuned, the
+ * structured-grid kernel is persistent where its tiles do not fit the GPU all at once; what is read
+ * then is what a stiffness pass does. */
 int pg_ctx_tuning(pg_ctx* c, int32_t* tri_tile_nodes, int32_t* tri_persistent, int32_t* cut_warps);
 int pg_ctx_set_tuning(pg_ctx* c, int32_t tri_tile_nodes, int32_t tri_persistent, int32_t cut_warps);
 /* With the structured-grid kernel: 0 runs the cut elements' kernels after it on the same

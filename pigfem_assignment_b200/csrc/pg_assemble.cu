@@ -1140,6 +1140,17 @@ bool grid_pattern_ok(const HostMesh& hm) {
     return ok.load();
 }
 
+// Left to itself (kGridAuto) the grid kernel is persistent and pipelined,
+// unless the tiles fit the SMs all at once anyway: then nothing is pipelined,
+// and the plain kernel's smaller CTAs leave room for the cut elements' first
+// ones (256^2: 16.6 us against 18.4 with the cut kernels; 512^2, 2313 tiles on
+// 740 places: 39.0 against 34.9).
+bool grid_persistent(const Ctx& c, bool want_f, bool want_K) {
+    if (c.tuning.tri_persistent != kGridAuto) return c.tuning.tri_persistent != 0;
+    const int tr = c.tuning.grid_block == 128 ? 2 : 4;
+    return c.tuning.cut_overlap > 0 || c.n_grid_tiles[tr == 2 ? 0 : 1] > c.n_sm * (grid_ctas(want_K, want_f) / tr);
+}
+
 void launch_grid(const Ctx& c, const double* U, bool want_f, bool want_K, cudaStream_t s) {
     GridArgs ga;
     ga.rves = c.grid_rves;
@@ -1155,13 +1166,8 @@ void launch_grid(const Ctx& c, const double* U, bool want_f, bool want_K, cudaSt
     ga.tiles = c.grid_tiles[tr == 2 ? 0 : 1];
     const int blocks = c.n_grid_tiles[tr == 2 ? 0 : 1];
     if (blocks == 0) return;
-    // Persistent, pipelined: as many CTAs as fit on the SMs at once -- unless
-    // the tiles fit all at once anyway: then nothing is pipelined, and the
-    // plain kernel's smaller CTAs leave room for the cut elements' first ones
-    // (256^2: 16.6 us against 18.4 with the cut kernels; 512^2, 2313 tiles on
-    // 740 places: 39.0 against 34.9).
-    const bool one_wave = blocks <= c.n_sm * (grid_ctas(want_K, want_f) / tr) && c.tuning.cut_overlap == 0;
-    if (c.tuning.tri_persistent && !one_wave) {
+    if (grid_persistent(c, want_f, want_K)) {
+        // as many CTAs as fit on the SMs at once
         auto go = [&](auto kern) {
             int per_sm = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGridTileC * tr, 0);

@@ -165,7 +165,7 @@ int ctx_create(HostMesh mesh, int device, Ctx& c) {
             c.n_grid_tiles[h] = (int)tiles.size();
             if ((rc = dev_upload(&c.grid_tiles[h], tiles))) return rc;
         }
-        c.tuning.tri_persistent = 1;
+        c.tuning.tri_persistent = kGridAuto;
     } else {
         c.tuning.tri_grid = 0;
     }
@@ -528,7 +528,9 @@ int pg_ctx_tuning(pg_ctx* c, int32_t* tri_tile_nodes, int32_t* tri_persistent, i
     PG_GUARD_CTX(c);
     if (tri_tile_nodes)
         *tri_tile_nodes = c->c.tuning.tri_grid ? c->c.tuning.grid_block : kTriTileSizes[c->c.tuning.tri_variant];
-    if (tri_persistent) *tri_persistent = c->c.tuning.tri_persistent;
+    if (tri_persistent)
+        *tri_persistent = c->c.tuning.tri_persistent == kGridAuto ? grid_persistent(c->c, false, true)
+                                                                  : c->c.tuning.tri_persistent;
     if (cut_warps) *cut_warps = c->c.tuning.cut_warps;
     return PG_OK;
 }

@@ -116,6 +116,7 @@ __host__ __device__ inline unsigned grid_nbr_mask(int gi, int gj, int nx, int ny
 
 bool grid_pattern_ok(const HostMesh& hm);  // block rows laid out as the structured-grid kernel assumes
 constexpr int kGridTileCols = 64;          // node columns per structured-grid tile
+constexpr int kGridAuto = 2;               // AsmTuning::tri_persistent left to grid_persistent's rule
 // Autotuned launch shapes of the assembly kernels (pg_ctx_autotune):
 // the structured-grid kernel's CTA size, or (meshes without one grid) the
 // row-tile kernel's tile size and persistent grid (CTAs walk the tiles) or
@@ -124,7 +125,7 @@ struct AsmTuning {
     int tri_grid = 1;      // 1: the structured-grid kernel (when the mesh has one grid)
     int grid_block = 128;  // its threads per CTA: 128 or 256
     int tri_variant = 1;   // otherwise: index into kTriTileSizes
-    int tri_persistent = 0;
+    int tri_persistent = 0;  // or kGridAuto
     int cut_warps = 4;     // 2, 4 or 8
     // with the structured-grid kernel: 0 runs the cut elements' kernels after
     // it on the same stream; 1 or 2 runs them beside it on a second stream (the
@@ -301,6 +302,8 @@ int stress_prepare(Ctx& c);
 int write_vtk(Ctx& c, const std::string& path, double t);
 int write_cohesive_openings(Ctx& c, const std::string& path);
 int autotune_assembly(Ctx& c, int reps, float* ms_tri, float* ms_cut);
+// whether the structured-grid kernel of such a pass is the persistent one
+bool grid_persistent(const Ctx& c, bool want_f, bool want_K);
 // shape sensitivity (pg_sens.cu): per-node inclusion / velocity and the cut-kernel passes
 // Arguments of the cut elements' shape-sensitivity kernel (pg_assemble.cu)
 struct CutArgs {
