@@ -2122,11 +2122,14 @@ void launch_cut_points(const Ctx& c, cudaStream_t s) {
                    reinterpret_cast<const int4*>(c.cut_pts), c.x, c.y, c.dmat, c.cut_rows);
 }
 
+constexpr int kCutSmem = 227 * 1024;  // the most that a CTA of k_cut_elems may ask for
+
 template <int NL, bool WF, bool COH>
 int launch_elems_inst(const ElemArgs& ea, int blocks, int bs, size_t smem, cudaStream_t s) {
     if (smem > 48 * 1024) {
+        // (the attribute belongs to the device: one value for every context, whatever the host thread)
         const cudaError_t e = cudaFuncSetAttribute(k_cut_elems<NL, WF, COH>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kCutSmem);
         if (e != cudaSuccess) return cuda_fail(e, "k_cut_elems shared memory");
     }
     launch_pdl(k_cut_elems<NL, WF, COH>, blocks, bs, smem, s, ea);
@@ -2188,7 +2191,7 @@ int launch_cut_elems(const Ctx& c, const double* U, double dt, bool want_f, bool
         const bool coh = c.n_coh_qp > 0 && ea.coh_max > 0;
         size_t smem = sizeof(double) * (size_t)ea.node_off;
         if (want_f || coh) smem += sizeof(double) * (4 * epc * kCutClassNl[k] + 2 * (size_t)kCohRow * ea.coh_max * epc);
-        if (smem > 227 * 1024) {
+        if (smem > kCutSmem) {
             set_error("cut elements: a CTA's quadrature rows exceed the shared memory (use fewer warps per CTA)");
             return PG_ERR_LIMIT;
         }

@@ -34,6 +34,8 @@ namespace {
 
 inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
 
+constexpr size_t kClusterSmem = 220 * 1024;  // the most that a CTA of the one-launch CG asks for
+
 // Launches CG as one cluster where the system fits its shared memory (up to
 // some 27k nodes); false where it does not, or where the device cannot hold
 // such a cluster.  The blocks of K go into shared memory too where they fit
@@ -42,7 +44,9 @@ inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
 template <typename MT, bool KS>
 bool cluster_cg_launch(const ClusterCgArgs& args, const MT* K, size_t smem, cudaStream_t s) {
     auto kern = k_pcg_cluster<MT, KS>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    // (the attribute belongs to the device: the largest value, so that a thread with a smaller system does not
+    // lower it between this and the launch)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -75,9 +79,8 @@ bool cluster_cg(Ctx& c, cudaStream_t s, const MT* K, double* x, const double* r,
     const HostMesh& hm = c.hm;
     ClusterCgArgs a{};
     a.n = c.n_nodes;
-    constexpr size_t kSmem = 220 * 1024;
     // rows as in the kernel; 16-bit column numbers
-    if (cluster_cg_smem(a.n / kClusterCtas, 0, 0, 0) > kSmem || a.n > 0xffff) return false;
+    if (cluster_cg_smem(a.n / kClusterCtas, 0, 0, 0) > kClusterSmem || a.n > 0xffff) return false;
     if (c.cluster_halo < 0) {            // the cut of this mesh, once
         std::vector<int> seen(a.n, -1);
         c.cluster_rows = c.cluster_blocks = c.cluster_halo = 0;
@@ -101,7 +104,7 @@ bool cluster_cg(Ctx& c, cudaStream_t s, const MT* K, double* x, const double* r,
     a.blocks = (c.cluster_blocks + 7) & ~7;
     const size_t small = cluster_cg_smem(a.rows, a.blocks, a.halo, 0),
                  full = cluster_cg_smem(a.rows, a.blocks, a.halo, sizeof(MT));
-    if (small > kSmem || a.rows + a.halo > 0xffff || (size_t)a.n * 2 > (size_t)a.rows * 80) return false;
+    if (small > kClusterSmem || a.rows + a.halo > 0xffff || (size_t)a.n * 2 > (size_t)a.rows * 80) return false;
     a.row_ptr = c.row_ptr;
     a.col = c.col;
     a.fixed = c.fixed;
@@ -112,7 +115,7 @@ bool cluster_cg(Ctx& c, cudaStream_t s, const MT* K, double* x, const double* r,
     a.max_iter = max_iter;
     a.flags = c.iflags;
     a.scal = c.scal;
-    return full <= kSmem ? cluster_cg_launch<MT, true>(a, K, full, s) : cluster_cg_launch<MT, false>(a, K, small, s);
+    return full <= kClusterSmem ? cluster_cg_launch<MT, true>(a, K, full, s) : cluster_cg_launch<MT, false>(a, K, small, s);
 }
 
 template <typename MT, typename VT, typename PT>

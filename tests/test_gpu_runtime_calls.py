@@ -25,3 +25,30 @@ for t in (128, 256):
     assert one(t, 0) != one(t, 1), t
 ctx.close()
 """)
+
+
+def test_function_attributes_do_not_depend_on_the_context(tmp_path):
+    # they belong to the device: a value of one context's own size could be
+    # lowered by another host thread before the launch that needs it
+    cudart_shim.run(tmp_path, r"""
+crowded = [(i / 12, j / 12, 0.42 / 12, 1) for j in range(13) for i in range(13)]
+for precision in (_lib.PG_PRECISION_FP64, _lib.PG_PRECISION_MIXED):
+    for precond in (_lib.PG_PREC_BLOCK_JACOBI, _lib.PG_PREC_MG):
+        for nx, inclusions in ((12, crowded), (40, [(0.5, 0.5, 0.25, 1)]), (100, [(0.5, 0.5, 0.25, 1)])):
+            prob = pb.ProblemLinearElasticity(RVE(nx=nx, ny=nx, inclusions=inclusions, strain=0.01))
+            prob.init()
+            for warps in (2, 4, 8):
+                _lib.check(_lib.lib.pg_ctx_set_tuning(prob.ctx.handle, 128, 0, warps))
+                pb.Assembler(prob.ctx).assemble_linear()
+            prob.get_solver().configure(precond=precond, precision=precision, rtol=1e-9)
+            prob.solve_problem()
+            prob.ctx.close()
+n = var("shim_n_attr").value
+funcs, attrs, values = (var(name, k * 65536) for name, k in
+                        (("shim_attr_func", C.c_void_p), ("shim_attr", C.c_int), ("shim_attr_value", C.c_int)))
+seen = {}
+for i in range(n):
+    seen.setdefault((funcs[i], attrs[i]), set()).add(values[i])
+assert len(seen) > 8, seen
+assert all(len(v) == 1 for v in seen.values()), seen
+""")
