@@ -364,7 +364,7 @@ int mg_build(Ctx& c);                                    // the hierarchies' str
 void mg_depths(const Ctx& c, std::vector<int>& depth);   // coarse levels per RVE
 int mg_pcg_solve(Ctx& c, const pg_solver_cfg& cfg, pg_solve_stats& st, cudaStream_t s);
 int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s);
-void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z);
+int mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z);
 // CG preconditioned by the V-cycle on every RVE of the context; host copies
 // of the scalars (8 per RVE: ..., 4 tol^2, 5 b.b) and flags (4 per RVE: done,
 // breakdown, iterations, coarsest operator singular), valid until the next call

@@ -830,6 +830,7 @@ int cg_run(Ctx& c, MgHierarchy& m, bool modes, const pg_solver_cfg& cfg, cudaStr
     launch_pdl(k_cg_tol, m.R, kSpanThreads, 0, s, m.spans, m.part_rr, cfg.rtol * cfg.rtol, m.sc, m.fl);
     cudaMemsetAsync(c.xi, 0, (size_t)c.n_dof * sizeof(double), s);  // p before the first iteration
     mg_cycle<T>(c, m, modes, s, c.r, c.z, nullptr, false);
+    PG_CUDA(cudaGetLastError());
     cudaMemcpyAsync(m.h_sc, m.sc, (size_t)kScal * m.R * sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(m.h_fl, m.fl, fl_bytes, cudaMemcpyDeviceToHost, s);
     cudaGraphExec_t& exec = m.graph[(f32 ? 1 : 0) + (modes ? 2 : 0)];
@@ -838,8 +839,10 @@ int cg_run(Ctx& c, MgHierarchy& m, bool modes, const pg_solver_cfg& cfg, cudaStr
         cudaGraph_t graph;
         PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         cg_iterations<T>(c, m, modes, s);
+        // (a graph that lacks a refused launch would be kept for every later solve)
+        const cudaError_t le = cudaGetLastError();
         PG_CUDA(cudaStreamEndCapture(s, &graph));
-        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+        const cudaError_t ie = le != cudaSuccess ? le : cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) {
             exec = nullptr;
@@ -904,7 +907,7 @@ int mg_prepare(Ctx& c, bool f32, bool modes, cudaStream_t s) {
     return PG_OK;
 }
 
-void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z) {
+int mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double* r, double* z) {
     MgHierarchy& m = *c.mg;
     if (f32) {
         launch_pdl(k_mg_pre<float>, m.n_cta, kSpanThreads, 0, s, m.spans, c.fixed, r, m.Dinv0f, m.x0f);
@@ -913,6 +916,8 @@ void mg_precondition(Ctx& c, bool f32, bool modes, cudaStream_t s, const double*
         launch_pdl(k_mg_pre<double>, m.n_cta, kSpanThreads, 0, s, m.spans, c.fixed, r, c.minv, m.x0);
         mg_cycle<double>(c, m, modes, s, r, z, nullptr, false);
     }
+    PG_CUDA(cudaGetLastError());
+    return PG_OK;
 }
 
 void mg_free(Ctx& c) {

@@ -218,10 +218,12 @@ int gmres_solve(Ctx& c, const pg_solver_cfg& cfg, double rtol, int max_iter, pg_
             double* vj = c.V + (size_t)j * nd;
             double* w = c.V + (size_t)(j + 1) * nd;
             // w = K M^-1 v_j
-            if (cfg.precond == PG_PREC_MG)
-                mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, vj, c.z);
-            else
+            if (cfg.precond == PG_PREC_MG) {
+                const int rc = mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, vj, c.z);
+                if (rc != PG_OK) return rc;
+            } else {
                 k_apply_prec_vec<<<nblk(n), kThreads, 0, s>>>(n, c.minv, vj, c.z);
+            }
             k_spmv_plain<double, double><<<nblk(n), kThreads, 0, s>>>(n, c.row_ptr, c.col, c.K, c.z, c.fixed, w);
             // classical Gram-Schmidt, twice
             std::fill(hcol.begin(), hcol.end(), 0.0);
@@ -267,10 +269,12 @@ int gmres_solve(Ctx& c, const pg_solver_cfg& cfg, double rtol, int max_iter, pg_
         cudaMemcpyAsync(c.hbuf, y.data(), j * sizeof(double), cudaMemcpyHostToDevice, s);
         k_fill<double><<<nblk(nd), kThreads, 0, s>>>(nd, c.q, 0.0);
         k_multi_axpy_add<<<nblk(nd), kThreads, 0, s>>>(nd, j, c.V, c.hbuf, c.q);
-        if (cfg.precond == PG_PREC_MG)
-            mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, c.q, c.z);
-        else
+        if (cfg.precond == PG_PREC_MG) {
+            const int rc = mg_precondition(c, cfg.precision == PG_PRECISION_MIXED, cfg.inclusion_modes != 0, s, c.q, c.z);
+            if (rc != PG_OK) return rc;
+        } else {
             k_apply_prec_vec<<<nblk(n), kThreads, 0, s>>>(n, c.minv, c.q, c.z);
+        }
         k_axpy_free<double><<<nblk(nd), kThreads, 0, s>>>(nd, c.fixed, c.dx, c.z, 1.0);
         if (done) {
             rnorm = std::sqrt(residual_into(c, s, c.dx, c.b, c.r));

@@ -26,16 +26,15 @@ const void* shim_attr_func[kLog];  /* cudaFuncSetAttribute calls, in order */
 int shim_attr[kLog], shim_attr_value[kLog];
 int shim_n_attr;
 int shim_refuse = -1;              /* launches to let pass before one is refused (-1: none) */
-int shim_refuse_captured;          /* count only launches on a stream that is capturing */
+int shim_refuse_captured;          /* which ones count: 0 launches with attributes, not captured; 1 captured ones */
 static cudaError_t pending;
 
-static int refuse(cudaStream_t s) {
+static int refuse(cudaStream_t s, int attributes) {
+    enum cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (shim_refuse < 0) return 0;
-    if (shim_refuse_captured) {
-        enum cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        ((cudaError_t(*)(cudaStream_t, enum cudaStreamCaptureStatus*))real("cudaStreamIsCapturing"))(s, &st);
-        if (st != cudaStreamCaptureStatusActive) return 0;
-    }
+    ((cudaError_t(*)(cudaStream_t, enum cudaStreamCaptureStatus*))real("cudaStreamIsCapturing"))(s, &st);
+    if (shim_refuse_captured ? st != cudaStreamCaptureStatusActive : st == cudaStreamCaptureStatusActive || !attributes)
+        return 0;
     if (shim_refuse-- > 0) return 0;
     pending = cudaErrorInvalidConfiguration;
     return 1;
@@ -45,12 +44,12 @@ static void note(const void* f) {
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t m, cudaStream_t s) {
     note(f);
-    if (refuse(s)) return pending;
+    if (refuse(s, 0)) return pending;
     return ((cudaError_t(*)(const void*, dim3, dim3, void**, size_t, cudaStream_t))real("cudaLaunchKernel"))(f, g, b, a, m, s);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
     note(f);
-    if (refuse(c->stream)) return pending;
+    if (refuse(c->stream, 1)) return pending;
     return ((cudaError_t(*)(const cudaLaunchConfig_t*, const void*, void**))real("cudaLaunchKernelExC"))(c, f, a);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute k, int v) {

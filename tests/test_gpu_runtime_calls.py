@@ -52,3 +52,34 @@ for i in range(n):
 assert len(seen) > 8, seen
 assert all(len(v) == 1 for v in seen.values()), seen
 """)
+
+
+def test_a_refused_launch_ends_the_multigrid_solve_and_no_later_one(tmp_path):
+    # refused while a V-cycle is queued, or while the iterations are recorded:
+    # an error there and then, and the next solve is that of a fresh context
+    cudart_shim.run(tmp_path, r"""
+def problem():
+    prob = pb.ProblemLinearElasticity(RVE(nx=48, ny=40, inclusions=[(0.5, 0.5, 0.27, 1)], strain=0.01))
+    prob.init()
+    prob.get_assembler().assemble_linear()
+    return prob
+def solve(prob, precision):
+    s = prob.get_solver()
+    s.configure(precond=_lib.PG_PREC_MG, precision=precision, rtol=1e-10, max_iter=300)
+    prob.ctx.set_vector(0, np.zeros(prob.mesh.info["n_dof"]))
+    return _lib.lib.pg_solve_linear(prob.ctx.handle, C.byref(s.cfg), C.byref(s.stats))
+for precision in (_lib.PG_PRECISION_FP64, _lib.PG_PRECISION_MIXED):
+    clean = problem()
+    assert solve(clean, precision) == 0
+    for captured in (0, 1):
+        for nth in range(0, 8):  # fewer than a cycle's launches
+            prob = problem()
+            var("shim_refuse_captured").value = captured
+            var("shim_refuse").value = nth
+            rc = solve(prob, precision)
+            assert var("shim_refuse").value == -1
+            assert rc == _lib.PG_ERR_CUDA, (captured, nth, rc)
+            assert solve(prob, precision) == 0, (captured, nth)
+            assert np.array_equal(prob.get_solution(), clean.get_solution()), (captured, nth)
+            prob.ctx.close()
+""")
