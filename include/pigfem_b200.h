@@ -296,10 +296,11 @@ int pg_mlp_adam(pg_mlp* m, float lr);
 int pg_mlp_train(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n, int32_t epochs, int32_t batch,
                  float lr, double* loss_hist);
 /* Self-test of the kernels' bounded completion waits (the failure path the
- * reference has no counterpart for): one forward tile whose first GEMM is
- * not issued, so its mbarrier is never signalled and the wait gives up after
- * `polls` polls with nothing in flight.  Returns PG_ERR_STATE ("timed out");
- * the network and the device stay usable. */
+ * reference has no counterpart for): one forward tile, then a training epoch
+ * of two minibatches, whose first GEMM is not issued, so its mbarrier is never
+ * signalled and the wait gives up after `polls` polls with nothing in flight.
+ * Returns PG_ERR_STATE ("timed out"); the network is what it was, and it and
+ * the device stay usable. */
 int pg_mlp_wait_selftest(pg_mlp* m, int32_t polls);
 
 /* Learned-predictor plumbing (device pointers).  The history of a step: the

@@ -478,12 +478,12 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_train(const float* __restrict__ X
     }
     if (tid < OUT) sbias[2 * HID + tid] = __ldcg(&p.b3[tid]);
     fence_before();
-    __syncthreads();
+    // after a wait that ran out in an earlier minibatch this one's gradient is not used: it stays zero
+    bool ok = __syncthreads_or(__ldcg(err)) == 0;
     fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     uint32_t phase = 0;
-    bool ok = true;
     bool first = true;
     int gi = 0;             // GEMMs issued so far (WaitCfg::skip_gemm)
     bool inflight = false;  // a timed-out wait left MMAs of this CTA pending
@@ -671,6 +671,12 @@ __global__ void k_grad_sum(const float* __restrict__ part, int nparts, float* g,
     if (i == 0) *loss = loss_sum(lpart, nparts);
 }
 
+// What an epoch adds up on the device
+struct EpochSum {
+    double loss;               // of its minibatches (the gradient call: the loss alone)
+    long long steps;           // minibatches applied
+};
+
 struct AdamArgs {
     float lr, b1, b2, eps, c1, c2;
 };
@@ -690,9 +696,9 @@ __global__ void k_adam(float* p, const float* g, float* m, float* v, uint8_t* im
     if (i < kNParams) adam_param(i, g[i], p, m, v, img, a);
 }
 
-// k_grad_sum and k_adam of one minibatch; *loss_acc gains the minibatch's
-// loss.  After a timed-out wait (*err) the network is left as it is.
-__global__ void k_grad_adam(const float* part, int nparts, float* g, const double* lpart, double* loss_acc, float* p,
+// k_grad_sum and k_adam of one minibatch; the epoch's sums gain it.  After a
+// timed-out wait (*err) the network is left as it is.
+__global__ void k_grad_adam(const float* part, int nparts, float* g, const double* lpart, EpochSum* sum, float* p,
                             float* m, float* v, uint8_t* img, AdamArgs a, const int* err) {
     pdl_wait();
     pdl_trigger();
@@ -703,7 +709,10 @@ __global__ void k_grad_adam(const float* part, int nparts, float* g, const doubl
         g[i] = gi;
         adam_param(i, gi, p, m, v, img, a);
     }
-    if (i == 0) *loss_acc += loss_sum(lpart, nparts);
+    if (i == 0) {
+        sum->loss += loss_sum(lpart, nparts);
+        sum->steps += 1;
+    }
 }
 
 }  // namespace mlp
@@ -718,7 +727,7 @@ struct pg_mlp {
     float* m = nullptr;
     float* v = nullptr;
     uint8_t* img = nullptr;    // BF16 operand images of the weights (P_BYTES), always those of params
-    double* loss = nullptr;
+    pgb::mlp::EpochSum* sum = nullptr;  // what a training epoch adds up
     float* gpart = nullptr;    // per CTA of a gradient launch: its part of the gradient (kNParams)
     double* lpart = nullptr;   // and of the loss
     int* err = nullptr;
@@ -748,7 +757,7 @@ int pg_mlp_create(int32_t device, uint64_t seed, pg_mlp** out) {
     };
     const Part parts[] = {{(void**)&m->params, 4 * (size_t)kNParams * sizeof(float)},
                           {(void**)&m->img, P_BYTES},
-                          {(void**)&m->loss, sizeof(double)},
+                          {(void**)&m->sum, sizeof(EpochSum)},
                           {(void**)&m->err, sizeof(int)},
                           {(void**)&m->probe, TILE * (IN + 2) * sizeof(float)},
                           {(void**)&m->lpart, (size_t)m->n_sms * sizeof(double)},
@@ -852,24 +861,11 @@ int pg_mlp_forward(pg_mlp* m, const float* X_dev, int32_t n, float* Y_dev, void*
     return PG_OK;
 }
 
-// Self-test of the bounded completion wait: one forward tile whose first GEMM
-// is not issued, so nothing arrives on its mbarrier and the wait must give up
-// after `polls` polls.  Nothing is in flight when it does, so the kernel
-// records its error word, frees its tensor memory and returns; the call
-// returns the timeout status and the network stays usable.
-int pg_mlp_wait_selftest(pg_mlp* m, int32_t polls) {
-    if (!m || polls < 1) { set_error("pg_mlp_wait_selftest: bad argument"); return PG_ERR_ARG; }
-    cudaSetDevice(m->device);
-    launch_forward(m, m->probe, TILE, m->probe + TILE * IN, m->stream, WaitCfg{polls, 0});
-    PG_CUDA(cudaGetLastError());
-    return mlp_check_err(m);
-}
-
 // the CTAs' gradient parts over n rows; returns their number
-static int launch_train(pg_mlp* m, const float* X, const float* T, int n) {
+static int launch_train(pg_mlp* m, const float* X, const float* T, int n, WaitCfg wc) {
     const int tiles = (n + TILE - 1) / TILE, grid = std::min(tiles, m->n_sms);
     launch_pdl(k_mlp_train, grid, NT, SMEM_ALLOC, m->stream, X, T, n, carve(m->params),
-               reinterpret_cast<const uint4*>(m->img), m->gpart, m->lpart, m->err, WaitCfg{kPollLimit, -1});
+               reinterpret_cast<const uint4*>(m->img), m->gpart, m->lpart, m->err, wc);
     return grid;
 }
 
@@ -890,13 +886,13 @@ static AdamArgs next_step(pg_mlp* m, float lr) {
 int pg_mlp_gradient(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n, double* loss_host) {
     if (!m || !X_dev || !T_dev || n <= 0) { set_error("pg_mlp_gradient: bad argument"); return PG_ERR_ARG; }
     cudaSetDevice(m->device);
-    const int parts = launch_train(m, X_dev, T_dev, n);
+    const int parts = launch_train(m, X_dev, T_dev, n, WaitCfg{kPollLimit, -1});
     PG_CUDA(cudaGetLastError());
-    k_grad_sum<<<kParamBlocks, 256, 0, m->stream>>>(m->gpart, parts, m->grads, m->lpart, m->loss);
+    k_grad_sum<<<kParamBlocks, 256, 0, m->stream>>>(m->gpart, parts, m->grads, m->lpart, &m->sum->loss);
     PG_CUDA(cudaGetLastError());
     int rc = mlp_check_err(m);
     if (rc) return rc;
-    if (loss_host) PG_CUDA(cudaMemcpy(loss_host, m->loss, sizeof(double), cudaMemcpyDeviceToHost));
+    if (loss_host) PG_CUDA(cudaMemcpy(loss_host, &m->sum->loss, sizeof(double), cudaMemcpyDeviceToHost));
     return PG_OK;
 }
 
@@ -908,31 +904,60 @@ int pg_mlp_adam(pg_mlp* m, float lr) {
     return PG_OK;
 }
 
+// One pass over n rows in batches of `batch` rows, queued whole: the host
+// looks at its loss and at the error word once, at its end.  A minibatch whose
+// wait ran out and those after it are not applied, and not counted as steps.
+// `first` is the first minibatch's WaitCfg.
+static int train_epoch(pg_mlp* m, const float* X, const float* T, int n, int batch, float lr, WaitCfg first, double* loss) {
+    PG_CUDA(cudaMemsetAsync(m->sum, 0, sizeof(EpochSum), m->stream));
+    const int step0 = m->step;
+    int nb = 0;
+    for (int s0 = 0; s0 < n; s0 += batch) {
+        const int nn = (n - s0) < batch ? (n - s0) : batch;
+        const int parts = launch_train(m, X + (size_t)s0 * IN, T + (size_t)s0 * 2, nn, nb ? WaitCfg{kPollLimit, -1} : first);
+        launch_pdl(k_grad_adam, kParamBlocks, 256, 0, m->stream, m->gpart, parts, m->grads, m->lpart, m->sum,
+                   m->params, m->m, m->v, m->img, next_step(m, lr), m->err);
+        PG_CUDA(cudaGetLastError());
+        ++nb;
+    }
+    EpochSum sum{};
+    PG_CUDA(cudaMemcpyAsync(&sum, m->sum, sizeof sum, cudaMemcpyDeviceToHost, m->stream));
+    const int rc = mlp_check_err(m);
+    if (rc) {
+        m->step = step0 + (int)sum.steps;
+        return rc;
+    }
+    if (loss) *loss = sum.loss / (nb ? nb : 1);
+    return PG_OK;
+}
+
 // Minibatch training: `epochs` passes over n rows in batches of `batch` rows
 // (the caller shuffles).  Writes the mean loss of every epoch to loss_hist.
 int pg_mlp_train(pg_mlp* m, const float* X_dev, const float* T_dev, int32_t n, int32_t epochs, int32_t batch, float lr,
                  double* loss_hist) {
     if (!m || !X_dev || !T_dev || n <= 0 || batch <= 0) { set_error("pg_mlp_train: bad argument"); return PG_ERR_ARG; }
     cudaSetDevice(m->device);
-    // an epoch is queued whole: the host looks at its loss and at the error word once, at its end
     for (int ep = 0; ep < epochs; ++ep) {
-        PG_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream));
-        int nb = 0;
-        for (int s0 = 0; s0 < n; s0 += batch) {
-            const int nn = (n - s0) < batch ? (n - s0) : batch;
-            const int parts = launch_train(m, X_dev + (size_t)s0 * IN, T_dev + (size_t)s0 * 2, nn);
-            launch_pdl(k_grad_adam, kParamBlocks, 256, 0, m->stream, m->gpart, parts, m->grads, m->lpart, m->loss,
-                       m->params, m->m, m->v, m->img, next_step(m, lr), m->err);
-            PG_CUDA(cudaGetLastError());
-            ++nb;
-        }
-        double acc = 0.0;
-        PG_CUDA(cudaMemcpyAsync(&acc, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
-        const int rc = mlp_check_err(m);
+        const int rc = train_epoch(m, X_dev, T_dev, n, batch, lr, WaitCfg{kPollLimit, -1}, loss_hist ? loss_hist + ep : nullptr);
         if (rc) return rc;
-        if (loss_hist) loss_hist[ep] = acc / (nb ? nb : 1);
     }
     return PG_OK;
+}
+
+// Self-test of the bounded completion wait: one forward tile, and an epoch of
+// two minibatches, whose first GEMM is not issued, so nothing arrives on its
+// mbarrier and the wait must give up after `polls` polls.  Nothing is in
+// flight when it does, so the kernel records its error word, frees its tensor
+// memory and returns; the call returns the timeout status, and the network is
+// what it was.
+int pg_mlp_wait_selftest(pg_mlp* m, int32_t polls) {
+    if (!m || polls < 1) { set_error("pg_mlp_wait_selftest: bad argument"); return PG_ERR_ARG; }
+    cudaSetDevice(m->device);
+    launch_forward(m, m->probe, TILE, m->probe + TILE * IN, m->stream, WaitCfg{polls, 0});
+    PG_CUDA(cudaGetLastError());
+    const int rc = mlp_check_err(m);
+    if (rc != PG_ERR_STATE) return rc;
+    return train_epoch(m, m->probe, m->probe + TILE * IN, TILE, TILE / 2, 1e-3f, WaitCfg{polls, 0}, nullptr);
 }
 
 }  // extern "C"
