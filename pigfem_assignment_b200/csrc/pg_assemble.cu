@@ -623,7 +623,7 @@ __device__ __forceinline__ void cut_point_row_local(const int4 r2, const double2
 // then point q (8 bits), child type (2), child node count (3) and the
 // element's local-function count (4), then the offset in doubles of the
 // point's row (2 ints, low first: the element's first row + l (4 + 2 NL) for
-// its point l), the element and an unused int.  Points are
+// its point l), the element and four bytes of padding.  Points are
 // in class order, each element's in the order of its rows; one sentinel
 // record follows the last point, holding only the rows' total length.
 void build_cut_points(const std::vector<int>& nodes, const std::vector<int>& tmpl, const std::vector<int>& chm,

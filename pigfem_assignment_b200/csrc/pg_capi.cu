@@ -66,8 +66,7 @@ void free_ctx(Ctx& c) {
                     c.qp_class_off, c.qp_out,
                     c.cut_ke, c.cut_fe, c.cut_kpos, c.cut_fpos, c.fold_K_slot, c.fold_K_ptr, c.fold_f_node,
                     c.fold_f_ptr, c.K, c.Kf, c.fixed, c.ubar,
-                    c.U, c.F, c.isv_c, c.isv_t, c.r, c.z, c.p, c.q, c.dx, c.minv, c.rf, c.zf, c.pf, c.qf, c.xf,
-                    c.minvf, c.scal, c.iflags};
+                    c.U, c.F, c.isv_c, c.isv_t, c.r, c.z, c.p, c.q, c.dx, c.minv, c.scal, c.iflags};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c.h_scal) cudaFreeHost(c.h_scal);
@@ -281,9 +280,6 @@ int ctx_create(HostMesh mesh, int device, Ctx& c) {
         if ((rc = dev_alloc(v, nd))) return rc;
     if ((rc = dev_alloc(&c.minv, 4 * nn))) return rc;
     if ((rc = dev_alloc(&c.mw, 2 * nd))) return rc;
-    for (float** v : {&c.rf, &c.zf, &c.pf, &c.qf, &c.xf})
-        if ((rc = dev_alloc(v, nd))) return rc;
-    if ((rc = dev_alloc(&c.minvf, 4 * nn))) return rc;
     if ((rc = dev_alloc(&c.hbuf, 128))) return rc;
     if ((rc = dev_alloc(&c.scal, 64))) return rc;
     {

@@ -221,13 +221,6 @@ struct Ctx {
     double* q = nullptr;
     double* dx = nullptr;
     double* minv = nullptr;            // 4 per node: inverse of the (masked) diagonal 2x2 block or Jacobi
-    // solver work (FP32)
-    float* rf = nullptr;
-    float* zf = nullptr;
-    float* pf = nullptr;
-    float* qf = nullptr;
-    float* xf = nullptr;
-    float* minvf = nullptr;
     double* b = nullptr;               // right-hand side of the current Krylov solve
     double* res = nullptr;             // Newton residual
     double* Ut = nullptr;              // Newton trial displacement

@@ -110,51 +110,10 @@ __device__ __forceinline__ void load_block(const float* p, double& a, double& b,
     d = v.w;
 }
 
-// Block row i of K times x with kRowLanes lanes per row: lane g of the row's
-// group takes blocks r0 + g, r0 + g + kRowLanes, ..., so a group's loads of K
-// are contiguous; two shuffles give every lane of the group the row's sum.
-// A lane issues the column and block loads of kRowUnroll of its blocks at
-// once, then their x gathers (a row of up to 12 blocks: one round of each).
-// Every lane of the warp must call it (valid = false for padding rows).
+// Lanes that share a block row where a row takes more than one, and the blocks
+// of it that a lane loads at once (a row of up to 12 blocks: one round).
 constexpr int kRowLanes = 4;
 constexpr int kRowUnroll = 3;
-template <typename MT, typename VT>
-__device__ __forceinline__ void bsr_row_group(int i, bool valid, int g, const int* __restrict__ row_ptr,
-                                              const int* __restrict__ col, const MT* __restrict__ K,
-                                              const VT* __restrict__ x, double& y0, double& y1) {
-    double a0 = 0.0, a1 = 0.0;
-    if (valid) {
-        const int r1 = __ldg(&row_ptr[i + 1]);
-        for (int base = __ldg(&row_ptr[i]) + g; base < r1; base += kRowLanes * kRowUnroll) {
-            int j[kRowUnroll];
-            double b[kRowUnroll][4];
-#pragma unroll
-            for (int u = 0; u < kRowUnroll; ++u) {
-                const int k = base + u * kRowLanes;
-                j[u] = -1;
-                b[u][0] = b[u][1] = b[u][2] = b[u][3] = 0.0;
-                if (k < r1) {
-                    j[u] = __ldg(&col[k]);
-                    load_block(K + 4 * (size_t)k, b[u][0], b[u][1], b[u][2], b[u][3]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kRowUnroll; ++u) {
-                if (j[u] >= 0) {
-                    const double x0 = (double)x[2 * j[u]], x1 = (double)x[2 * j[u] + 1];
-                    a0 += b[u][0] * x0 + b[u][1] * x1;
-                    a1 += b[u][2] * x0 + b[u][3] * x1;
-                }
-            }
-        }
-    }
-    a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
-    a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-    y0 = a0;
-    y1 = a1;
-}
 
 template <typename MT, typename VT>
 __global__ void __launch_bounds__(kThreads) k_spmv_plain(int n, const int* __restrict__ row_ptr, const int* __restrict__ col,
@@ -191,12 +150,6 @@ __global__ void __launch_bounds__(kThreads) k_spmv_cg(int n, int P, const int* _
     }
     const double s = block_sum(part);
     grid_add(ws, 0, s, &scal[S_PQ0 + P]);
-}
-
-template <typename VT>
-__global__ void k_neg(int nd, VT* r) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < nd) r[i] = -r[i];
 }
 
 template <typename VT, typename PT>
@@ -322,17 +275,6 @@ template <typename VT>
 __global__ void k_axpy_free(int nd, const uint8_t* __restrict__ fixed, double* U, const VT* __restrict__ e, double s) {
     const int i = blockIdx.x * kThreads + threadIdx.x;
     if (i < nd && !fixed[i]) U[i] += s * (double)e[i];
-}
-
-__global__ inline void k_axpy_free_f(int nd, const uint8_t* __restrict__ fixed, double* U, const float* __restrict__ e,
-                                     double s) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < nd && !fixed[i]) U[i] += s * (double)e[i];
-}
-
-__global__ inline void k_to_float_scaled(int nd, const double* __restrict__ a, float* b, double s) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < nd) b[i] = (float)(a[i] * s);
 }
 
 __global__ inline void k_dot_self(int nd, const double* __restrict__ a, double* out, double* ws) {
