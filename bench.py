@@ -230,6 +230,14 @@ def run_reference_arm(args):
     from pigfem_assignment_b200.rve import config1
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import refio
+    if not refio.driver_available():
+        # the C port that cpu_baseline falls back to is this repository's own restatement, not the reference
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "oracle/_ref/pigfem_ref_driver is not built: it needs the reference's sources"}),
+              flush=True)
+        return
     rve = config1()
     procs = max(1, min(os.cpu_count() or 1, 16))
     res = cpu_reference_sample(rve, args.warmup + args.steps, procs)
