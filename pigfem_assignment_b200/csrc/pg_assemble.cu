@@ -949,11 +949,12 @@ __device__ __forceinline__ void grid_node(const GridArgs& a, const int4 B, int g
 
 // One CTA per tile: the window's coordinates (and displacements) and cell
 // materials are staged with coalesced loads, all in flight together; then
-// every thread forms its node's row from shared memory.  Bound by the L1:
-// a warp's block store goes to 32 lines, and the window reads.  Two resident
-// groups of 256 threads with both outputs (three spilled 328 bytes per
-// thread: 122 us at 1024^2, now 84 in the persistent kernel).  128 threads
-// per CTA are never slower than 256 (a halo row more per node row, but
+// every thread forms its node's row from shared memory.  The L1 is its busiest
+// unit (two thirds of its rate in the persistent kernel at 1024^2: a warp's
+// block store goes to 32 lines, and the window reads), the rest latency.  Two
+// resident groups of 256 threads with both outputs (three spilled 328 bytes
+// per thread: 122 us at 1024^2, now 84 in the persistent kernel, 78 alone
+// under the profiler).  128 threads per CTA are never slower than 256 (a halo row more per node row, but
 // smaller steps at the end of the grid): stiffness of 256^2 16.5 us against
 // 20.5, 512^2 34.9 against 37.5, with the cut elements.
 template <bool WK, bool WF, int TR>

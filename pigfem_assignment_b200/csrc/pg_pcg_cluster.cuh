@@ -15,11 +15,11 @@ namespace pgb {
 // writes its partial into all 16, and each adds them in rank order, so all
 // take the same decisions and the result is the same bits on every run.
 //
-// Three launches per iteration with fused sums took 17.7 us at 64^2 (4.5k
+// Three launches per iteration with fused sums take 17.2 us at 64^2 (4.5k
 // nodes), nearly all of it launch, fence and ticket latency; with z and p
 // gathered remotely for every entry (131 KB a CTA) this kernel took 6.0; as it
-// is, 4.3 (3.6 are the two barriers and sums), and 11.3 at 128^2 (18k nodes, K
-// from L2) against 19.3.
+// is, 4.2 (3.6 were the two barriers and sums), and 9.1 at 128^2 (17k nodes, K
+// from L2) against 17.8.
 constexpr int kClusterCtas = 16;
 constexpr int kClusterThreads = 384;     // one row each at 64^2 (281 a CTA); 1,024 threads: 5.8 us an iteration, 384: 4.3
 constexpr int kClusterUnroll = 4;        // blocks a row loads at once

@@ -37,10 +37,11 @@ inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
 constexpr size_t kClusterSmem = 220 * 1024;  // the most that a CTA of the one-launch CG asks for
 
 // Launches CG as one cluster where the system fits its shared memory (up to
-// some 27k nodes); false where it does not, or where the device cannot hold
+// some 25k nodes); false where it does not, or where the device cannot hold
 // such a cluster.  The blocks of K go into shared memory too where they fit
-// (up to some 9k nodes).  Wherever it fits it is the faster form: 4.3 against
-// 18.6 us an iteration at 64^2, 11.3 against 19.3 at 128^2.
+// (up to some 9k nodes, 13k stored in FP32).  Wherever it fits it is the
+// faster form: 4.2 against 17.2 us an iteration at 64^2, 9.1 against 17.8 at
+// 128^2, 12.4 against 17.7 at 150^2.
 template <typename MT, bool KS>
 bool cluster_cg_launch(const ClusterCgArgs& args, const MT* K, size_t smem, cudaStream_t s) {
     auto kern = k_pcg_cluster<MT, KS>;
