@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -295,6 +296,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Row r of a tile (unsigned: inference asks for the rows of one tile past the
+// last, up to 255 beyond the largest number of rows)
+__host__ __device__ constexpr unsigned tile_row(int tile, int r) { return (unsigned)tile * TILE + r; }
+static_assert(tile_row(INT_MAX / TILE + 1, TILE - 1) > INT_MAX, "no row past the end wraps to one before it");
+
 // The thread's share of a tile of X, 16 floats.  VEC (X is 16-byte aligned):
 // four 16-byte loads, each of a warp's 32 covering 512 consecutive bytes, so
 // its share is a quarter of the rows 32 warp + 8 k + lane / 4; otherwise its
@@ -305,18 +311,18 @@ __device__ __forceinline__ void load_x(const float* __restrict__ X, int tile, in
     if (VEC) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int row = tile * TILE + 32 * warp + 8 * k + lane / 4;
+            const unsigned row = tile_row(tile, 32 * warp + 8 * k + lane / 4);
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < n) v = __ldg(reinterpret_cast<const float4*>(X + (size_t)row * IN) + lane % 4);
+            if (row < (unsigned)n) v = __ldg(reinterpret_cast<const float4*>(X + (size_t)row * IN) + lane % 4);
             x[4 * k] = v.x;
             x[4 * k + 1] = v.y;
             x[4 * k + 2] = v.z;
             x[4 * k + 3] = v.w;
         }
     } else {
-        const int row = tile * TILE + tid;
+        const unsigned row = tile_row(tile, tid);
 #pragma unroll
-        for (int i = 0; i < IN; ++i) x[i] = row < n ? X[(size_t)row * IN + i] : 0.f;
+        for (int i = 0; i < IN; ++i) x[i] = row < (unsigned)n ? X[(size_t)row * IN + i] : 0.f;
     }
 }
 // and into the A operand
