@@ -477,6 +477,7 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_train(const float* __restrict__ X
     // the minibatch before has stepped the network (and read the parts that this one writes)
     pdl_wait();
     pdl_trigger();
+    const int failed = __ldcg(err);
     for (uint32_t i = tid; i < P_BYTES / 16; i += NT) reinterpret_cast<uint4*>(sm + O_W)[i] = __ldcg(&img[i]);
     if (tid < HID) {
         sbias[tid] = __ldcg(&p.b1[tid]);
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_train(const float* __restrict__ X
     if (tid < OUT) sbias[2 * HID + tid] = __ldcg(&p.b3[tid]);
     fence_before();
     // after a wait that ran out in an earlier minibatch this one's gradient is not used: it stays zero
-    bool ok = __syncthreads_or(__ldcg(err)) == 0;
+    bool ok = __syncthreads_or(failed) == 0;
     fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
